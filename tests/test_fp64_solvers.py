@@ -1,0 +1,86 @@
+"""The FP64 solvers' kernels at the edges of their tiles and lists: the
+per-particle walk (bit for bit the oracle's) and the sampled direct sums."""
+
+import numpy as np
+import pytest
+
+from native import lopsided_sphere
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 2, 31, 33, 63, 65, 129, 1000])
+@pytest.mark.parametrize("scale", [1.0, 1e-24, 1e24])
+def test_tree_walk_sizes_and_scales_bitwise(ctx, oracle, n, scale):
+    """Ragged last warps, lists shorter and longer than a lane's 32 entries,
+    and lengths whose squares leave the FP32 range (every test in FP64)."""
+    pos, mass = lopsided_sphere(max(n, 8), 4)
+    pos, mass = np.ascontiguousarray(pos[:n] * scale), mass[:n].copy()
+    kw = dict(G=1.0, theta=0.6, eps=0.02 * scale, quadrupole=True)
+    acc, pot = ctx.tree_force(pos, mass, **kw)
+    st = ctx.stats()
+    want, wpot, (nc, npart) = oracle.tree_force(pos, mass, **kw)
+    assert np.array_equal(acc, want, equal_nan=True) and np.array_equal(pot, wpot, equal_nan=True)
+    assert (st["cell_interactions"], st["body_interactions"]) == (nc, npart)
+
+
+@pytest.mark.parametrize("big", [31, 32, 33, 100])
+def test_tree_walk_leaf_longer_than_a_list_bitwise(ctx, oracle, big):
+    """A leaf of `big` coincident bodies: the lists stop inside it and go on."""
+    pos, mass = lopsided_sphere(400, 9)
+    pos[:big] = pos[0]
+    kw = dict(G=1.7, theta=0.7, eps=0.05, quadrupole=True)
+    acc, pot = ctx.tree_force(pos, mass, **kw)
+    want, wpot, _ = oracle.tree_force(pos, mass, **kw)
+    assert np.array_equal(acc, want) and np.array_equal(pot, wpot)
+
+
+@pytest.mark.parametrize("n,m", [(1, 1), (127, 5), (128, 128), (129, 129), (3001, 257)])
+@pytest.mark.parametrize("scale", [1.0, 1e-160, 1e140])
+def test_fp64_sample_sizes_and_scales(ctx, oracle, n, m, scale):
+    """Ragged tiles of sources and targets; squared distances far from 1 and
+    (the smallest scale) below the normal range. 1e-12 relative, the bound of
+    the other sample tests, where the oracle's own squares are normal."""
+    import torch
+    pos, mass = lopsided_sphere(max(n, 8), 6)
+    pos, mass = np.ascontiguousarray(pos[:n] * scale), mass[:n].copy()
+    idx = (np.arange(m) * 7 % n).astype(np.uint64)
+    kw = dict(G=2.5, eps=0.05 * scale)
+    racc, rpot = oracle.direct_fp64(pos, mass, idx=idx, **kw)
+    d = lambda a: torch.from_numpy(a).cuda()
+    dp, dm, di = d(pos), d(mass), d(idx.astype(np.int64))
+    acc = torch.zeros((m, 3), dtype=torch.float64, device="cuda")
+    pot = torch.zeros(m, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.direct_fp64_device(dp.data_ptr(), dm.data_ptr(), n, di.data_ptr(), m, acc.data_ptr(),
+                           pot.data_ptr(), **kw)
+    acc, pot = acc.cpu().numpy(), pot.cpu().numpy()
+    if scale == 1e-160:  # r^2 is subnormal in both: a few bits only
+        assert np.array_equal(np.isfinite(acc), np.isfinite(racc))
+        return
+    ok = np.linalg.norm(racc, axis=1) > 0
+    err = np.linalg.norm(acc[ok] - racc[ok], axis=1) / np.linalg.norm(racc[ok], axis=1)
+    assert err.size == 0 or err.max() < 1e-12
+    assert np.all(acc[~ok] == 0)
+    assert np.allclose(pot, rpot, rtol=1e-12, atol=0)
+
+
+def test_fp64_sample_coincident_unsoftened(ctx, oracle):
+    """Two bodies at one place without softening: 1/0 gives what it gave."""
+    import torch
+    pos, mass = lopsided_sphere(300, 2)
+    pos[5] = pos[200]
+    idx = np.array([5, 7, 200], np.uint64)
+    with np.errstate(all="ignore"):
+        racc, rpot = oracle.direct_fp64(pos, mass, G=1.0, eps=0.0, idx=idx)
+    d = lambda a: torch.from_numpy(a).cuda()
+    dp, dm, di = d(pos), d(mass), d(idx.astype(np.int64))
+    acc = torch.zeros((3, 3), dtype=torch.float64, device="cuda")
+    pot = torch.zeros(3, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.direct_fp64_device(dp.data_ptr(), dm.data_ptr(), 300, di.data_ptr(), 3, acc.data_ptr(),
+                           pot.data_ptr(), G=1.0, eps=0.0)
+    acc, pot = acc.cpu().numpy(), pot.cpu().numpy()
+    assert np.array_equal(np.isnan(acc), np.isnan(racc))
+    assert np.array_equal(np.isinf(pot), np.isinf(rpot)) and np.array_equal(pot > 0, rpot > 0)
+    assert np.allclose(acc[1], racc[1], rtol=1e-12, atol=0)
