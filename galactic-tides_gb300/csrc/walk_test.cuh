@@ -1,0 +1,92 @@
+// The walks' opening test (group_lists.cpp:145-154): FP64 exactly as the
+// reference computes it, and an FP32 form with a rigorous error band that
+// decides almost every test and leaves the rest to FP64. Users are compiled
+// with -fmad=false.
+#pragma once
+
+#include "pipeline.cuh"
+
+namespace gtc {
+
+// The opening test of group_lists.cpp:145-154 for one node, in FP64 exactly
+// as the reference computes it.
+__device__ __forceinline__ bool accept64(const WalkRec64 &r, const double *gc, const double *gh) {
+  bool overlap = true;
+  double d2 = 0.0;
+  if (fabs(r.cx - gc[0]) > r.slack + gh[0]) overlap = false;
+  double d = fabs(r.mx - gc[0]) - gh[0];
+  if (d > 0) d2 += d * d;
+  if (fabs(r.cy - gc[1]) > r.slack + gh[1]) overlap = false;
+  d = fabs(r.my - gc[1]) - gh[1];
+  if (d > 0) d2 += d * d;
+  if (fabs(r.cz - gc[2]) > r.slack + gh[2]) overlap = false;
+  d = fabs(r.mz - gc[2]) - gh[2];
+  if (d > 0) d2 += d * d;
+  return !overlap && d2 > r.crit2;
+}
+
+// The same test in FP32 with a rigorous error band. Every FP32 input is the
+// FP64 quantity (relative to the root centre) rounded once; the node record
+// carries B_n >= all its |values| + slack and the group B_g >= max|centre| +
+// max half-extent, so every quantity compared below is at most ~2 (B_n + B_g)
+// in size and each FP32 result is within 5 * 2^-24 (B_n + B_g) of the value
+// from the exact inputs (more than the FP64 roundings too). The band
+// E = 2^-20 (B_n + B_g) is over three times that: a comparison whose sides
+// differ by more than E has the FP64 outcome; otherwise the caller runs the
+// FP64 test. Returns 1 accept, 0 open, 2 undecided (NaNs end up undecided).
+constexpr float kBand = 1.0f / (1 << 20);
+
+__device__ __forceinline__ int accept32(const WalkRec32 &r, const float *gf, const float *hf,
+                                        float gbound) {
+  const float e = kBand * (r.bound + gbound);
+  bool separated = false, within = true;
+  float lo2 = 0.f, hi2 = 0.f;
+  const float c[3] = {r.cx, r.cy, r.cz}, mm[3] = {r.mx, r.my, r.mz};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    // overlap: on every axis |c - g| <= slack + gh (group_lists.cpp:147)
+    const float x = fabsf(c[a] - gf[a]), y = r.slack + hf[a];
+    separated |= x > y + e;
+    within &= x < y - e;
+    // distance from the box to the centre of mass (group_lists.cpp:150-151)
+    const float d = fabsf(mm[a] - gf[a]) - hf[a];
+    const float dl = fmaxf(d - e, 0.f), dh = fmaxf(d + e, 0.f);
+    lo2 = fmaf(dl, dl, lo2);
+    hi2 = fmaf(dh, dh, hi2);
+  }
+  const float c2 = r.crit2;
+  // scales where a rounding above may be a subnormal's: left to FP64
+  if (e < 1e-36f || (hi2 < 1e-35f && c2 < 1e-35f)) return 2;
+  if (within) return 0;                                      // overlaps: opened
+  if (hi2 * (1.f + 4.f * kBand) < c2 * (1.f - 4.f * kBand)) return 0;  // too close
+  if (separated && lo2 * (1.f - 4.f * kBand) > c2 * (1.f + 4.f * kBand)) return 1;
+  return 2;
+}
+
+__device__ __forceinline__ WalkRec32 load32(const WalkRec32 *w, u32 i) {
+  const float4 *p = reinterpret_cast<const float4 *>(w + i);
+  const float4 a = __ldg(p), b = __ldg(p + 1);
+  const uint4 c = __ldg(reinterpret_cast<const uint4 *>(p + 2));
+  WalkRec32 r;
+  r.cx = a.x;
+  r.cy = a.y;
+  r.cz = a.z;
+  r.slack = a.w;
+  r.mx = b.x;
+  r.my = b.y;
+  r.mz = b.z;
+  r.crit2 = b.w;
+  r.skip = c.x;
+  r.nbody_leaf = c.y;
+  r.begin = c.z;
+  r.bound = __uint_as_float(c.w);
+  return r;
+}
+
+__device__ __forceinline__ WalkRec64 load64(const WalkRec64 *w, u32 i) {
+  const double2 *p = reinterpret_cast<const double2 *>(w + i);
+  const double2 a0 = __ldg(p), a1 = __ldg(p + 1), b0 = __ldg(p + 2), b1 = __ldg(p + 3);
+  return WalkRec64{a0.x, a0.y, a1.x, a1.y, b0.x, b0.y, b1.x, b1.y};
+}
+
+}  // namespace gtc
