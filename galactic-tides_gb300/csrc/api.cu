@@ -402,7 +402,7 @@ struct GraphStep {
                           ctx->have_model ? ctx->prev_amag.as<float>() : nullptr};
     gtc::evaluate_lists_graph(ws.bodies.as<float4>(), ws.cells.as<float4>(),
                               ws.cell_list.as<u32>(), ws.body_list.as<u32>(),
-                              ws.groups.as<uint4>(), n, sc, static_cast<float>(sp.G),
+                              ws.groups.as<uint4>(), n, caps.groups, sc, static_cast<float>(sp.G),
                               static_cast<float>(sp.eps * sp.eps), sp.quadrupole != 0, eo,
                               ctx->counter.as<u32>(), s, ws.eval_shape);
     mark(5, s);
@@ -729,7 +729,7 @@ struct ForestGraph {
     gtc::join_side(ws, s);  // the cells
     gtc::evaluate_lists_graph(ws.bodies.as<float4>(), ws.cells.as<float4>(),
                               ws.cell_list.as<u32>(), ws.body_list.as<u32>(),
-                              ws.groups.as<uint4>(), f->n, sc, static_cast<float>(f->sp.G),
+                              ws.groups.as<uint4>(), f->n, caps.groups, sc, static_cast<float>(f->sp.G),
                               static_cast<float>(f->sp.eps * f->sp.eps), f->sp.quadrupole != 0,
                               gtc::EvalOut{ws.out.as<float4>()}, f->counter.as<u32>(), s,
                               ws.eval_shape);

@@ -8,16 +8,43 @@
 // instruction itself, rsqrt_normal, as every softened r^2 is a normal
 // float) instead of 1/sqrt.
 //
-// Lane l of a warp owns target begin + l of its group. The warp walks the
-// list 32 entries at a time: each lane loads one entry (coalesced index
-// load, then one 48-byte cell or 16-byte body), scales its mass and
-// quadrupole by G once, and stages it in shared memory; then every lane
-// reads the 32 staged entries back as broadcast loads (one shared-memory
-// transaction serves the whole warp) and accumulates. A group of 16 or
-// fewer targets splits its lists into 2-4 slices worked by separate lane
-// sets (lanes that would otherwise idle), summed by shuffles at the end.
-// Groups are handed out to warps by an atomic counter, so a warp that drew
-// a long list does not hold back the others' next groups.
+// Packed FP32x2: a lane holds two targets of its group, one in each half of
+// its float2 registers, and every FFMA2 / FMUL2 / FADD2 works one list entry
+// against both. Entries (48-byte cells, 16-byte bodies) are copied from
+// global to shared memory by cp.async, two per lane and round, a round ahead
+// of the arithmetic; a slot past the list is filled with zeros, whose zero
+// mass and quadrupole add exactly zero to a softened sum. The staged entries
+// come back as broadcast loads, and the factor G multiplies the sums once.
+//
+// What bounds the kernel is the FP32 FMA pipe: 33 packed instructions per
+// cell and target pair, 13 per body. A packed instruction holds the pipe two
+// cycles when its operands allow; with three different register pairs it
+// takes three (measured in a loop of them: 3.1 cycles, 2.3 with two pairs),
+// so the inner loop alone runs at 80 cycles for 66 of arithmetic. Scalar
+// FFMAs measured no faster (88 cycles: issue). Pairing two targets instead of
+// two entries halves the shared-memory bytes per interaction (the pipe to
+// shared memory was 83% busy, now 43%), and the copies a round ahead take
+// the list's latency off the warps, so 5 blocks of 4 warps (96 registers)
+// serve better than 32 warps per SM did. Copies through L1 (.ca) gain 1% over
+// copies past it: neighbouring groups share cells.
+//
+// Lane fill: a group of T targets has P = ceil(T / 2) target pairs. Its lists
+// are cut into S slices, and the (slice, pair) slots v = s P + q go to the
+// lanes 32 at a time, a pass each, so that ceil(S P / 32) passes keep nearly
+// every lane busy whatever T is (94% of the lanes' work is real at 200k). S is
+// chosen per group from T and the list lengths alone (choose_slices). Each
+// target's partial sums are added in slice order, so the result does not
+// depend on which warp ran which pass.
+//
+// With many groups one warp works a group's passes one after another (groups
+// handed out by an atomic counter). Below kTeamGroups the four warps of a
+// block share a group's passes, so that long lists do not run alone at the
+// end. Kernel times against a kernel pairing two entries for one target, a
+// warp per group, the next round's entries loaded only when needed (seed 1
+// galaxies, quadrupoles): 5k bodies 139 -> 32 us (86 with a warp per group), 50k
+// 140 -> 101 us (133), 200k (8.9k groups) 359 -> 332 us (359 in teams), 2M 3.26 ->
+// 3.21 ms; monopoles only (a scalar kernel before) 200k 276 -> 219 us, 2M 2.39 ->
+// 1.97 ms.
 
 #include <algorithm>
 
@@ -26,46 +53,15 @@
 namespace gtc {
 namespace {
 
-constexpr int kWarpsPerBlock = 8;
+constexpr int kWarpsPerBlock = 4;
 constexpr int kT = 32 * kWarpsPerBlock;
-
-struct Staged {
-  float4 cm;   // com (rel. origin), G * mass
-  float4 q0;   // G * (xx, yy, zz, xy)
-  float4 q1;   // G * (xz, yz, -, -)
-};
-
-template <bool kQuad>
-__device__ __forceinline__ void add_cell(float px, float py, float pz, const Staged &c, float eps2,
-                                         float &ax, float &ay, float &az, float &pot) {
-  const float dx = px - c.cm.x, dy = py - c.cm.y, dz = pz - c.cm.z;
-  const float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-  const float inv = rsqrtf(r2);
-  const float inv2 = inv * inv;
-  const float inv3 = inv * inv2;
-  if (kQuad) {
-    // a = -G m d / r^3 + G Q d / r^5 - 5/2 G (d.Q.d) d / r^7, with G folded
-    // into m and Q: the monopole and quadrupole terms along d share one FMA
-    // per axis.
-    const float qx = fmaf(c.q0.x, dx, fmaf(c.q0.w, dy, c.q1.x * dz));
-    const float qy = fmaf(c.q0.w, dx, fmaf(c.q0.y, dy, c.q1.y * dz));
-    const float qz = fmaf(c.q1.x, dx, fmaf(c.q1.y, dy, c.q0.z * dz));
-    const float rqr = fmaf(dx, qx, fmaf(dy, qy, dz * qz));
-    const float inv5 = inv3 * inv2;
-    const float inv7 = inv5 * inv2;
-    const float along = fmaf(-2.5f * rqr, inv7, -c.cm.w * inv3);
-    ax = fmaf(along, dx, fmaf(qx, inv5, ax));
-    ay = fmaf(along, dy, fmaf(qy, inv5, ay));
-    az = fmaf(along, dz, fmaf(qz, inv5, az));
-    pot = fmaf(-c.cm.w, inv, fmaf(-0.5f * rqr, inv5, pot));
-  } else {
-    const float gm3 = c.cm.w * inv3;
-    ax = fmaf(-gm3, dx, ax);
-    ay = fmaf(-gm3, dy, ay);
-    az = fmaf(-gm3, dz, az);
-    pot = fmaf(-c.cm.w, inv, pot);
-  }
-}
+constexpr int kBlocksPerSm = 5;   // 96 registers: 2M 3.21 ms; 4: 3.24, 6: 3.26, 7: 3.4 ms
+constexpr float kSoftEps2 = 1e-14f;  // eps^-5 stays below 1e35
+constexpr u32 kNone = 0xffffffffu;
+constexpr u32 kMaxSlices = 32;    // slices per group at most
+constexpr u32 kStage = 64;        // entries a warp stages per round, two per lane
+constexpr int kPer = kStage / 32;    // entries a lane stages per round
+constexpr u32 kChunk = 256;       // entries a slice holds at most (up to kMaxSlices slices)
 
 // Target i's results (tree order) into eo: the FP32 record, and the caller's
 // FP64 arrays (FP32 -> FP64 exactly) and |a| when eo asks for them.
@@ -80,422 +76,389 @@ __device__ __forceinline__ void write_target(const EvalOut &eo, u32 i, float4 a)
   if (eo.amag) eo.amag[j] = sqrtf(__fmaf_rn(a.x, a.x, __fmaf_rn(a.y, a.y, __fmul_rn(a.z, a.z))));
 }
 
-// kSoft: eps2 > 0. Every target appears exactly once in its own group's body
-// list (each body is covered once and no accepted cell holds a target), and
-// with softening its self term adds exactly zero acceleration (d = 0) and a
-// known -G m_i / eps to the potential, so the loop needs no self test and
-// the self potential is taken back out at the end. Without softening the
-// self term is singular and each entry is tested as in the reference.
-template <bool kQuad, bool kSoft>
-__global__ void __launch_bounds__(kT)
+// Slices for a group of T targets with ec cells and eb bodies (warp-uniform):
+// of the S in 1..32 whose slices hold at most kChunk entries, the one that
+// minimises passes x (entries per slice + pass_cost); 32 when the lists are
+// longer than that. pass_cost is a pass's fixed cost in entries worked
+// against one target: half as many against the lane's two.
+__device__ __forceinline__ u32 choose_slices(u32 T, u32 ec, u32 eb, int lane, u32 pass_cost) {
+  const u32 P = (T + 1) / 2;
+  const u32 S = static_cast<u32>(lane) + 1u;
+  const u32 passes = (S * P + 31u) / 32u;
+  const u32 each = (ec + S - 1) / S + (eb + S - 1) / S;
+  const u32 cost = each <= kChunk ? passes * (each + pass_cost / 2u) : (1u << 26);
+  // ties: the most slices
+  return kMaxSlices - (__reduce_min_sync(kFullMask, cost << 5 | (kMaxSlices - S)) & 31u);
+}
+
+// 16 (8) bytes from global to shared memory without a register in between;
+// zeros where `real` is false.
+__device__ __forceinline__ void copy_async16(void *dst, const void *src, bool real) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(
+                   static_cast<u32>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(real ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void copy_async8(void *dst, const void *src, bool real) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(
+                   static_cast<u32>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(real ? 8 : 0)
+               : "memory");
+}
+template <bool kQuad>
+__device__ __forceinline__ void copy_cell(float4 *dst, const float4 *cells, u32 c) {
+  const bool real = c != kNone;
+  const float4 *src = cells + 3ull * (real ? c : 0u);
+  copy_async16(dst, src, real);
+  if (kQuad) {
+    copy_async16(dst + 1, src + 1, real);
+    copy_async8(dst + 2, src + 2, real);
+  }
+}
+
+// A list of e entries cut into S nearly equal slices: the entry slice s
+// starts at.
+struct Cut {
+  u32 base, rest;
+  __device__ __forceinline__ Cut(u32 e, u32 S) : base(e / S), rest(e % S) {}
+  __device__ __forceinline__ u32 at(u32 s) const { return base * s + min(s, rest); }
+  __device__ __forceinline__ u32 longest() const { return base + (rest ? 1u : 0u); }
+};
+
+// a / b for a below 2^12, from r = 1 / b: (a + 1/2) / b is at least 1 / 2b from
+// a whole number, far more than the roundings.
+__device__ __forceinline__ u32 small_div(u32 a, float r) {
+  return static_cast<u32>((static_cast<float>(a) + 0.5f) * r);
+}
+
+__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
+__device__ __forceinline__ float2 dup(float a) { return make_float2(a, a); }
+
+// A lane's two targets, one in each half of the pairs, and what has been
+// summed onto them.
+struct Targets {
+  float2 px, py, pz;
+  float2 ax, ay, az, pot;
+};
+
+// One staged body (or monopole) against the lane's targets, without the
+// factor -G (applied once to the sums): d = source - target; without
+// softening, self0 / self1 leave the target itself out.
+template <bool kSoft>
+__device__ __forceinline__ void add_body(Targets &a, const float4 b, const float2 e2,
+                                         bool self0 = false, bool self1 = false) {
+  const float2 dx = __fadd2_rn(dup(b.x), a.px), dy = __fadd2_rn(dup(b.y), a.py),
+               dz = __fadd2_rn(dup(b.z), a.pz);
+  float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+  float2 m = dup(b.w);
+  if (!kSoft) {
+    r2 = f2(self0 ? 1.f : r2.x, self1 ? 1.f : r2.y);
+    m = f2(self0 ? 0.f : m.x, self1 ? 0.f : m.y);
+  }
+  const float2 inv = kSoft ? f2(rsqrt_normal(r2.x), rsqrt_normal(r2.y))
+                           : f2(rsqrtf(r2.x), rsqrtf(r2.y));
+  const float2 mr = __fmul2_rn(m, inv);                     // m / r
+  const float2 mr3 = __fmul2_rn(mr, __fmul2_rn(inv, inv));  // m / r^3
+  a.ax = __ffma2_rn(mr3, dx, a.ax);
+  a.ay = __ffma2_rn(mr3, dy, a.ay);
+  a.az = __ffma2_rn(mr3, dz, a.az);
+  a.pot = __fadd2_rn(a.pot, mr);
+}
+
+// One staged cell with its quadrupole (q: Qxx, Qyy, Qzz, Qxy; w: Qxz, Qyz),
+// d = source - target: a / G = m d / r^3 - Q d / r^5 + 5/2 (d.Q.d) d / r^7, phi
+// / -G = m / r + 1/2 d.Q.d / r^5; r.Q.r / r^5 once for both.
+template <bool kSoft>
+__device__ __forceinline__ void add_cell(Targets &a, const float4 c, const float4 q,
+                                         const float2 w, const float2 e2) {
+  const float2 dx = __fadd2_rn(dup(c.x), a.px), dy = __fadd2_rn(dup(c.y), a.py),
+               dz = __fadd2_rn(dup(c.z), a.pz);
+  const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
+  const float2 inv = kSoft ? f2(rsqrt_normal(r2.x), rsqrt_normal(r2.y))
+                           : f2(rsqrtf(r2.x), rsqrtf(r2.y));
+  const float2 m = dup(c.w), qxy = dup(q.w), qxz = dup(w.x), qyz = dup(w.y);
+  const float2 inv2 = __fmul2_rn(inv, inv), inv3 = __fmul2_rn(inv, inv2);
+  const float2 qx = __ffma2_rn(dup(q.x), dx, __ffma2_rn(qxy, dy, __fmul2_rn(qxz, dz)));
+  const float2 qy = __ffma2_rn(qxy, dx, __ffma2_rn(dup(q.y), dy, __fmul2_rn(qyz, dz)));
+  const float2 qz = __ffma2_rn(qxz, dx, __ffma2_rn(qyz, dy, __fmul2_rn(dup(q.z), dz)));
+  const float2 rqr = __ffma2_rn(dx, qx, __ffma2_rn(dy, qy, __fmul2_rn(dz, qz)));
+  const float2 inv5 = __fmul2_rn(inv3, inv2), rqr5 = __fmul2_rn(rqr, inv5);
+  const float2 along = __ffma2_rn(__fmul2_rn(dup(2.5f), rqr5), inv2, __fmul2_rn(m, inv3));
+  const float2 n5 = f2(-inv5.x, -inv5.y);
+  a.ax = __ffma2_rn(along, dx, __ffma2_rn(qx, n5, a.ax));
+  a.ay = __ffma2_rn(along, dy, __ffma2_rn(qy, n5, a.ay));
+  a.az = __ffma2_rn(along, dz, __ffma2_rn(qz, n5, a.az));
+  a.pot = __ffma2_rn(dup(0.5f), rqr5, __ffma2_rn(m, inv, a.pot));
+}
+
+// kSoft: eps2 at least kSoftEps2. Every target appears exactly once in
+// its own group's body list (each body is covered once and no accepted cell
+// holds a target), and with softening its self term adds exactly zero
+// acceleration (d = 0) and a known -G m_i / eps to the potential, so the
+// loop needs no self test and the self potential is taken back out at the
+// end; nor do the zeros past a list's end need one. Otherwise the self term
+// is singular, or powers of 1/eps overflow: each entry is tested as in the
+// reference, and only real entries are worked (kU = 1).
+// kTeam: the block's warps share a group's passes (else a warp per group).
+// kU: staged entries a lane works per inner-loop iteration (1 or 2, a
+// context option searched by gtc_autotune_eval): their arithmetic is
+// independent up to the accumulation, which stays in list order, so results
+// do not depend on it.
+template <bool kQuad, bool kSoft, bool kTeam, int kU>
+__global__ void __launch_bounds__(kT, kBlocksPerSm)
     k_eval(const float4 *__restrict__ bodies, const float4 *__restrict__ cells,
            const u32 *__restrict__ cell_list, const u32 *__restrict__ body_list,
            const uint4 *__restrict__ groups, u32 ngroups, float G, float eps2, EvalOut eo,
-           u32 *next_group, const u32 *ng_dev = nullptr, const u32 *abort = nullptr) {
-  // Staged entries, per warp: slice k's W entries start at float4 k (3W + 1)
-  // (cells) and k (W + 1) (bodies); the 16-byte gap puts the slices on
-  // different shared-memory banks, so their broadcast loads do not conflict.
-  __shared__ float4 sc[kWarpsPerBlock][3 * 32 + 4];
-  __shared__ float4 sb[kWarpsPerBlock][32 + 4];
-  __shared__ u32 sj[kWarpsPerBlock][kSoft ? 1 : 32 + 4];  // staged body indices (self test)
+           u32 *next_group, const u32 *ng_dev, const u32 *abort, u32 pass_cost) {
+  // Staged entries, per warp and round parity: slice area a of the pass holds
+  // W entries from float4 a (kF4 W + 1) on (3 float4 per quadrupole cell, else
+  // 1); W is even and the 16-byte gap puts the areas on different banks.
+  constexpr u32 kF4 = kQuad ? 3 : 1;
+  __shared__ float4 stage[kWarpsPerBlock][2][kStage * kF4 + 32];
+  __shared__ u32 sj[kWarpsPerBlock][2][kSoft ? 1 : kStage + 32];  // staged body indices (self test)
+  // per target: the running sum (a, potential); per slice and target in a team
+  __shared__ float4 sums[kTeam ? kMaxSlices : kWarpsPerBlock][32];
+  __shared__ u32 team_group;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  // a graph replay: the group count from the device, nothing after an abort
   if (abort && *abort) return;
   if (ng_dev) ngroups = min(ngroups, *ng_dev);
+  const float2 e2 = dup(eps2);
   for (;;) {
     u32 g = 0;
-    if (lane == 0) g = atomicAdd(next_group, 1u);
-    g = __shfl_sync(kFullMask, g, 0);
+    if (kTeam) {
+      if (threadIdx.x == 0) team_group = atomicAdd(next_group, 1u);
+      __syncthreads();
+      g = team_group;
+    } else {
+      if (lane == 0) g = atomicAdd(next_group, 1u);
+      g = __shfl_sync(kFullMask, g, 0);
+    }
     if (g >= ngroups) return;
     const uint4 q0 = groups[4ull * g], q1 = groups[4ull * g + 1], q2 = groups[4ull * g + 2],
                 q3 = groups[4ull * g + 3];
     const SegView cs = cell_segs(q1, q2), bs = body_segs(q2, q3);  // list entry -> index
-    // A group of T <= 16 targets splits its lists into ns = min(4, 32 / T)
-    // slices: lane l takes target l % T of slice l / T, each slice stages
-    // W = 32 / ns entries per round, and the slices' sums are added up by
-    // shuffles at the end (larger groups: one slice, W = 32).
-    const u32 T = q0.y - q0.x;
-    const u32 ns = T == 0 ? 1u : min(4u, 32u / T);
-    const u32 W = 32u / ns;
-    const u32 slice = T ? static_cast<u32>(lane) / T : 0u;
-    const u32 t = T ? static_cast<u32>(lane) % T : 0u;
-    const bool computes = slice < ns;  // lanes past ns * T only stage
-    const u32 i = q0.x + t;
-    const float4 bi = computes ? bodies[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const u32 stage_slice = static_cast<u32>(lane) / W, stage_pos = static_cast<u32>(lane) % W;
-    float ax = 0.f, ay = 0.f, az = 0.f, pot = 0.f;
-
-    {
-      const u32 e = q0.z;  // cells, slice k: entries [e k / ns, e (k + 1) / ns)
-      const u32 c0 = e * stage_slice / ns, c1 = e * (stage_slice + 1) / ns;
-      const u32 m0 = e * slice / ns, m1 = e * (slice + 1) / ns;
-      const u32 rounds = (((e + ns - 1) / ns) + W - 1) / W;
-      for (u32 r = 0; r < rounds; ++r) {
-        const u32 k = c0 + r * W + stage_pos;
-        if (stage_slice < ns && k < c1) {
-          const u64 c = cell_list[cs.at(k)];
-          const float4 q = __ldg(&cells[3 * c]);
-          float4 *dst = &sc[warp][stage_slice * (3 * W + 1) + 3 * stage_pos];
-          dst[0] = make_float4(q.x, q.y, q.z, G * q.w);
-          if (kQuad) {
-            const float4 c1v = __ldg(&cells[3 * c + 1]), c2v = __ldg(&cells[3 * c + 2]);
-            dst[1] = make_float4(G * c1v.x, G * c1v.y, G * c1v.z, G * c1v.w);
-            dst[2] = make_float4(G * c2v.x, G * c2v.y, 0.f, 0.f);
-          }
-        }
-        __syncwarp();
-        const u32 base = m0 + r * W;
-        const u32 cnt = computes && base < m1 ? min(W, m1 - base) : 0u;
-        const float4 *mine = &sc[warp][slice * (3 * W + 1)];
-        for (u32 j = 0; j < cnt; ++j) {
-          Staged st;
-          st.cm = mine[3 * j];
-          if (kQuad) {
-            st.q0 = mine[3 * j + 1];
-            st.q1 = mine[3 * j + 2];
-          }
-          add_cell<kQuad>(bi.x, bi.y, bi.z, st, eps2, ax, ay, az, pot);
-        }
-        __syncwarp();
-      }
-    }
-
-    {
-      const u32 e = q0.w;
-      const u32 c0 = e * stage_slice / ns, c1 = e * (stage_slice + 1) / ns;
-      const u32 m0 = e * slice / ns, m1 = e * (slice + 1) / ns;
-      const u32 rounds = (((e + ns - 1) / ns) + W - 1) / W;
-      for (u32 r = 0; r < rounds; ++r) {
-        const u32 k = c0 + r * W + stage_pos;
-        if (stage_slice < ns && k < c1) {
-          const u32 j = body_list[bs.at(k)];
-          const float4 b = __ldg(&bodies[j]);
-          sb[warp][stage_slice * (W + 1) + stage_pos] = make_float4(b.x, b.y, b.z, G * b.w);
-          if (!kSoft) sj[warp][stage_slice * (W + 1) + stage_pos] = j;
-        }
-        __syncwarp();
-        const u32 base = m0 + r * W;
-        const u32 cnt = computes && base < m1 ? min(W, m1 - base) : 0u;
-        const float4 *mine = &sb[warp][slice * (W + 1)];
-        for (u32 q = 0; q < cnt; ++q) {
-          const float4 b = mine[q];
-          const float dx = bi.x - b.x, dy = bi.y - b.y, dz = bi.z - b.z;
-          float r2 = fmaf(dx, dx, fmaf(dy, dy, fmaf(dz, dz, eps2)));
-          float w = b.w;
-          if (!kSoft) {
-            const bool self = sj[warp][kSoft ? 0 : slice * (W + 1) + q] == i;
-            r2 = self ? 1.0f : r2;
-            w = self ? 0.0f : w;
-          }
-          const float inv = rsqrtf(r2);
-          const float gm = w * inv;
-          const float gm3 = gm * inv * inv;
-          ax = fmaf(-gm3, dx, ax);
-          ay = fmaf(-gm3, dy, ay);
-          az = fmaf(-gm3, dz, az);
-          pot -= gm;
-        }
-        __syncwarp();
-      }
-    }
-    // the slices' partial sums onto slice 0
-    for (u32 k = 1; k < ns; ++k) {
-      const int src = min(lane + static_cast<int>(k * T), 31);
-      const float sx = __shfl_sync(kFullMask, ax, src), sy = __shfl_sync(kFullMask, ay, src),
-                  sz = __shfl_sync(kFullMask, az, src), sp = __shfl_sync(kFullMask, pot, src);
-      if (slice == 0) {
-        ax += sx;
-        ay += sy;
-        az += sz;
-        pot += sp;
-      }
-    }
-    if (kSoft) pot += G * bi.w * rsqrtf(eps2);  // the self term, added once above
-    if (slice == 0 && t < T) write_target(eo, i, make_float4(ax, ay, az, pot));
-  }
-}
-
-// The softened quadrupole evaluation (the benchmark configuration) with
-// Blackwell's packed FP32 instructions: each lane works two staged entries
-// at once, one in each half of a float2, so every FFMA2/FMUL2/FADD2 does two
-// interactions' arithmetic and the issue count per interaction halves.
-// Entries are staged as interleaved pairs (x_a, x_b, y_a, y_b, ...), with
-// coordinates and G m negated so that d = p + (-c) is one FADD2; a slot
-// past the list holds a dummy far away with zero mass and quadrupole, which
-// adds exactly zero (its r^2 overflows to inf and rsqrt(inf) = 0).
-//
-// Lane fill: a group of T targets splits both lists into ns slices and
-// numbers its (slice k, target t) slots v = k T + t; pass p gives slot
-// 32 p + l to lane l, so ceil(ns T / 32) passes keep nearly every lane busy
-// whatever T is (ns T / 32 lanes' worth of work per pass, against T of 32
-// with one slice). ns is picked per group from the list lengths. A pass
-// holds at most 4 slices (T >= 11: a 32-slot window spans at most
-// floor(31 / T) + 2 of them; T <= 10: one pass of min(4, 32 / T) slices),
-// each staged in its own shared-memory area. After a pass the lanes add
-// their partial sums (even plus odd entries) onto the target's running sum
-// in shared memory, slice by slice in increasing order, so the summation
-// order is fixed.
-constexpr float kFar = 1.0e30f;
-constexpr int kPairCellF4 = 5;   // float4 per staged cell pair
-constexpr int kPairBodyF4 = 2;   // float4 per staged body pair
-constexpr u32 kMaxSlices = 16;   // slices per group at most
-// The tile shape (EvalShape, a context option each and searched by
-// gtc_autotune_eval): the staged pairs a lane works per inner-loop
-// iteration (kU, 1 or 2) -- the pairs' arithmetic is independent up to the
-// accumulation, which stays in list order, so results do not depend on it;
-// more pairs per iteration give each warp more independent work to hide the
-// rsqrt and shared-load latencies; a round's 2W staged entries (2W a
-// multiple of 4) are padded with far dummies, so an iteration never reads
-// past them -- and a pass's fixed cost in staged entries per lane, which
-// sets how many slices a group's lists are cut into (below).
-
-__device__ __forceinline__ float2 f2(float a, float b) { return make_float2(a, b); }
-
-__device__ __forceinline__ u32 even_up(u32 x) { return (x + 1u) & ~1u; }
-
-// Slices for a group of T targets with ec cells and eb bodies (warp-uniform):
-// the ns in 1..16 that minimises passes x (pair steps per pass + pass_cost).
-__device__ __forceinline__ u32 choose_slices(u32 T, u32 ec, u32 eb, int lane, u32 pass_cost) {
-  if (T <= 10) return T == 0 ? 1u : min(4u, 32u / T);
-  const u32 ns = static_cast<u32>(lane) % kMaxSlices + 1u;
-  const u32 passes = (ns * T + 31u) / 32u;
-  const u64 cost = static_cast<u64>(passes) *
-                   (even_up((ec + ns - 1) / ns) + even_up((eb + ns - 1) / ns) + pass_cost);
-  const u32 key = static_cast<u32>(cost < (1ull << 27) ? cost : (1ull << 27) - 1) << 4 | (ns - 1u);
-  return (__reduce_min_sync(kFullMask, key) & 15u) + 1u;
-}
-
-template <int kU>
-__global__ void __launch_bounds__(kT)
-    k_eval_pairs(const float4 *__restrict__ bodies, const float4 *__restrict__ cells,
-                 const u32 *__restrict__ cell_list, const u32 *__restrict__ body_list,
-                 const uint4 *__restrict__ groups, u32 ngroups, float G, float eps2,
-                 EvalOut eo, u32 *next_group, const u32 *ng_dev, const u32 *abort,
-                 u32 pass_cost) {
-  // per warp, staged pairs: each lane stages two entries per round, so area
-  // a (2W entries) starts at float4 a * (W * per-pair + 1) (at most 4 areas:
-  // 164 and 68 float4); the 16-byte gap puts the areas on different
-  // shared-memory banks
-  __shared__ float4 sc[kWarpsPerBlock][164];
-  __shared__ float4 sb[kWarpsPerBlock][68];
-  __shared__ float4 sacc[kWarpsPerBlock][32];  // per target: a and potential
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (abort && *abort) return;
-  if (ng_dev) ngroups = min(ngroups, *ng_dev);
-  const float2 e2 = f2(eps2, eps2), m25 = f2(-2.5f, -2.5f), mhalf = f2(-0.5f, -0.5f);
-  for (;;) {
-    u32 g = 0;
-    if (lane == 0) g = atomicAdd(next_group, 1u);
-    g = __shfl_sync(kFullMask, g, 0);
-    if (g >= ngroups) return;
-    const uint4 q0 = groups[4ull * g], q1 = groups[4ull * g + 1], q2 = groups[4ull * g + 2],
-                q3 = groups[4ull * g + 3];
-    const SegView cs = cell_segs(q1, q2), bs = body_segs(q2, q3);  // list entry -> index
-    const u32 T = q0.y - q0.x;
-    if (T == 0) continue;
+    const u32 T = q0.y - q0.x, P = (T + 1) / 2;
     const u32 ec = q0.z, eb = q0.w;
-    const u32 ns = choose_slices(T, ec, eb, lane, pass_cost);
-    const u32 slots = ns * T;
-    const u32 passes = (slots + 31u) / 32u;
-    if (static_cast<u32>(lane) < T) sacc[warp][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-    __syncwarp();
-
-    for (u32 p = 0; p < passes; ++p) {
-      const u32 v = 32u * p + static_cast<u32>(lane);
-      const bool computes = v < slots;
-      const u32 slice = v / T, t = v % T;
-      const u32 k_lo = (32u * p) / T;
-      const u32 nsp = min(ns - 1u, (32u * p + 31u) / T) - k_lo + 1u;  // 1..4
-      const u32 W = nsp == 1u ? 32u : (nsp == 2u ? 16u : (nsp == 3u ? 10u : 8u));
-      const u32 area = slice - k_lo;
-      const u32 stage_area = static_cast<u32>(lane) / W, stage_pos = static_cast<u32>(lane) % W;
-      const u32 stage_slice = k_lo + stage_area;
-      const bool stages = stage_area < nsp;
-      const u32 half = stage_pos & 1u, pair = stage_pos >> 1;
-      const float4 bi = computes ? bodies[q0.x + t] : make_float4(0.f, 0.f, 0.f, 0.f);
-      const float2 px = f2(bi.x, bi.x), py = f2(bi.y, bi.y), pz = f2(bi.z, bi.z);
-      float2 ax = f2(0.f, 0.f), ay = ax, az = ax, pot = ax;
-
-      {  // cells
-        const u32 cstride = W * kPairCellF4 + 1;
-        const u32 c0 = ec * stage_slice / ns, c1 = ec * (stage_slice + 1) / ns;
-        const u32 m0 = ec * slice / ns, m1 = ec * (slice + 1) / ns;
-        const u32 rounds = ((ec + ns - 1) / ns + 2 * W - 1) / (2 * W);
-        for (u32 r = 0; r < rounds; ++r) {
-          if (stages) {
-            // two entries per lane: positions stage_pos and stage_pos + W
-            float v[2][10];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const u32 k = c0 + 2 * r * W + h * W + stage_pos;
-              if (k < c1) {
-                const u64 c = cell_list[cs.at(k)];
-                const float4 a = __ldg(&cells[3 * c]), b = __ldg(&cells[3 * c + 1]),
-                             q = __ldg(&cells[3 * c + 2]);
-                v[h][0] = -a.x; v[h][1] = -a.y; v[h][2] = -a.z; v[h][3] = -G * a.w;
-                v[h][4] = G * b.x; v[h][5] = G * b.y; v[h][6] = G * b.z; v[h][7] = G * b.w;
-                v[h][8] = G * q.x; v[h][9] = G * q.y;
-              } else {
-                v[h][0] = v[h][1] = v[h][2] = -kFar;
-                v[h][3] = v[h][4] = v[h][5] = v[h][6] = v[h][7] = v[h][8] = v[h][9] = 0.f;
-              }
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float *f = reinterpret_cast<float *>(
-                  &sc[warp][stage_area * cstride + (pair + h * (W / 2)) * kPairCellF4]);
-#pragma unroll
-              for (int q = 0; q < 10; ++q) f[2 * q + half] = v[h][q];
-            }
-          }
-          __syncwarp();
-          const u32 base = m0 + 2 * r * W;
-          const u32 cnt = computes && base < m1 ? min(2 * W, m1 - base) : 0u;
-          const float4 *mine = &sc[warp][area * cstride];
-          for (u32 j = 0; j < cnt; j += 2 * kU) {
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-            const float4 s0 = mine[5 * u], s1 = mine[5 * u + 1], s2 = mine[5 * u + 2],
-                         s3 = mine[5 * u + 3], s4 = mine[5 * u + 4];
-            // s0 = -cx, -cy  s1 = -cz, -Gm  s2 = Qxx, Qyy  s3 = Qzz, Qxy  s4 = Qxz, Qyz (pairs)
-            const float2 dx = __fadd2_rn(px, f2(s0.x, s0.y)), dy = __fadd2_rn(py, f2(s0.z, s0.w)),
-                         dz = __fadd2_rn(pz, f2(s1.x, s1.y));
-            const float2 ngm = f2(s1.z, s1.w);
-            const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-            const float2 inv = f2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
-            const float2 inv2 = __fmul2_rn(inv, inv), inv3 = __fmul2_rn(inv, inv2);
-            const float2 qxx = f2(s2.x, s2.y), qyy = f2(s2.z, s2.w), qzz = f2(s3.x, s3.y),
-                         qxy = f2(s3.z, s3.w), qxz = f2(s4.x, s4.y), qyz = f2(s4.z, s4.w);
-            const float2 qx = __ffma2_rn(qxx, dx, __ffma2_rn(qxy, dy, __fmul2_rn(qxz, dz)));
-            const float2 qy = __ffma2_rn(qxy, dx, __ffma2_rn(qyy, dy, __fmul2_rn(qyz, dz)));
-            const float2 qz = __ffma2_rn(qxz, dx, __ffma2_rn(qyz, dy, __fmul2_rn(qzz, dz)));
-            const float2 rqr = __ffma2_rn(dx, qx, __ffma2_rn(dy, qy, __fmul2_rn(dz, qz)));
-            // r.Q.r / r^5 once, for both the acceleration along d and the potential
-            const float2 inv5 = __fmul2_rn(inv3, inv2), rqr5 = __fmul2_rn(rqr, inv5);
-            const float2 along = __ffma2_rn(__fmul2_rn(m25, rqr5), inv2, __fmul2_rn(ngm, inv3));
-            ax = __ffma2_rn(along, dx, __ffma2_rn(qx, inv5, ax));
-            ay = __ffma2_rn(along, dy, __ffma2_rn(qy, inv5, ay));
-            az = __ffma2_rn(along, dz, __ffma2_rn(qz, inv5, az));
-            pot = __ffma2_rn(mhalf, rqr5, __ffma2_rn(ngm, inv, pot));
-            }
-            mine += kPairCellF4 * kU;
-          }
-          __syncwarp();
-        }
-      }
-
-      {  // bodies
-        const u32 bstride = W * kPairBodyF4 + 1;
-        const u32 c0 = eb * stage_slice / ns, c1 = eb * (stage_slice + 1) / ns;
-        const u32 m0 = eb * slice / ns, m1 = eb * (slice + 1) / ns;
-        const u32 rounds = ((eb + ns - 1) / ns + 2 * W - 1) / (2 * W);
-        for (u32 r = 0; r < rounds; ++r) {
-          if (stages) {
-            float v[2][4];
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              const u32 k = c0 + 2 * r * W + h * W + stage_pos;
-              if (k < c1) {
-                const float4 b = __ldg(&bodies[body_list[bs.at(k)]]);
-                v[h][0] = -b.x; v[h][1] = -b.y; v[h][2] = -b.z; v[h][3] = -G * b.w;
-              } else {
-                v[h][0] = v[h][1] = v[h][2] = -kFar;
-                v[h][3] = 0.f;
-              }
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              float *f = reinterpret_cast<float *>(
-                  &sb[warp][stage_area * bstride + (pair + h * (W / 2)) * kPairBodyF4]);
-#pragma unroll
-              for (int q = 0; q < 4; ++q) f[2 * q + half] = v[h][q];
-            }
-          }
-          __syncwarp();
-          const u32 base = m0 + 2 * r * W;
-          const u32 cnt = computes && base < m1 ? min(2 * W, m1 - base) : 0u;
-          const float4 *mine = &sb[warp][area * bstride];
-          for (u32 j = 0; j < cnt; j += 2 * kU) {
-#pragma unroll
-            for (int u = 0; u < kU; ++u) {
-            const float4 s0 = mine[2 * u], s1 = mine[2 * u + 1];
-            const float2 dx = __fadd2_rn(px, f2(s0.x, s0.y)), dy = __fadd2_rn(py, f2(s0.z, s0.w)),
-                         dz = __fadd2_rn(pz, f2(s1.x, s1.y));
-            const float2 r2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __ffma2_rn(dz, dz, e2)));
-            const float2 inv = f2(rsqrt_normal(r2.x), rsqrt_normal(r2.y));
-            const float2 gm = __fmul2_rn(f2(s1.z, s1.w), inv);       // -G m / r
-            const float2 gm3 = __fmul2_rn(gm, __fmul2_rn(inv, inv));  // -G m / r^3
-            ax = __ffma2_rn(gm3, dx, ax);
-            ay = __ffma2_rn(gm3, dy, ay);
-            az = __ffma2_rn(gm3, dz, az);
-            pot = __fadd2_rn(pot, gm);
-            }
-            mine += kPairBodyF4 * kU;
-          }
-          __syncwarp();
-        }
-      }
-      // this pass's partial sums onto the targets', slice by slice
-      const float sx = ax.x + ax.y, sy = ay.x + ay.y, sz = az.x + az.y, sp = pot.x + pot.y;
-      for (u32 a = 0; a < nsp; ++a) {
-        if (computes && area == a) {
-          float4 &acc = sacc[warp][t];
-          acc.x += sx;
-          acc.y += sy;
-          acc.z += sz;
-          acc.w += sp;
-        }
+    u32 S = 0;
+    if (T > 0) {
+      S = choose_slices(T, ec, eb, lane, pass_cost);
+      const u32 slots = S * P;
+      const u32 passes = (slots + 31u) / 32u;
+      const float per_P = 1.f / static_cast<float>(P);
+      const Cut cut_c(ec, S), cut_b(eb, S);
+      if (!kTeam) {
+        sums[warp][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
         __syncwarp();
       }
+      for (u32 p = kTeam ? warp : 0u; p < passes; p += kTeam ? kWarpsPerBlock : 1u) {
+        const u32 v = 32u * p + static_cast<u32>(lane);
+        const bool computes = v < slots;
+        const u32 slice = small_div(v, per_P), t0 = 2u * (v - slice * P),
+                  t1 = min(t0 + 1u, T - 1u);
+        // the slices of the pass, and each one's share of the staging area
+        const u32 s_lo = __shfl_sync(kFullMask, slice, 0);
+        const u32 nsp = min(S - 1u, __shfl_sync(kFullMask, slice, 31)) - s_lo + 1u;
+        const u32 W = small_div(kStage, 1.f / static_cast<float>(nsp)) & ~1u;  // 2..64
+        const float per_W = 1.f / static_cast<float>(W);
+        const u32 area = slice - s_lo;
+        const float4 b0 = bodies[q0.x + (computes ? t0 : 0u)],
+                     b1 = bodies[q0.x + (computes ? t1 : 0u)];
+        Targets tg{f2(-b0.x, -b1.x), f2(-b0.y, -b1.y), f2(-b0.z, -b1.z),
+                   dup(0.f), dup(0.f), dup(0.f), dup(0.f)};
+        // The lane's two staging places (slice area and position in it) and
+        // the list entries that go there round by round: cells, then bodies.
+        u32 to_c[kPer], to_b[kPer], next[2][kPer], last[2][kPer];
+#pragma unroll
+        for (int h = 0; h < kPer; ++h) {
+          const u32 e = static_cast<u32>(lane) + 32u * h, a = small_div(e, per_W), pos = e - a * W;
+          to_c[h] = a < nsp ? a * (kF4 * W + 1u) + kF4 * pos : kNone;
+          to_b[h] = a * (W + 1u) + pos;
+#pragma unroll
+          for (int l = 0; l < 2; ++l) {
+            const Cut &cut = l ? cut_b : cut_c;
+            next[l][h] = cut.at(s_lo + a) + pos;
+            last[l][h] = a < nsp ? cut.at(s_lo + a + 1u) : 0u;
+          }
+        }
+        const u32 cell_rounds = (cut_c.longest() + W - 1u) / W;
+        const u32 rounds = cell_rounds + (cut_b.longest() + W - 1u) / W;
+        // the list indices of round r, kNone past the slice's end
+        u32 idx[kPer];
+        auto load_indices = [&](u32 r) {
+#pragma unroll
+          for (int h = 0; h < kPer; ++h) {
+            idx[h] = kNone;
+            if (r < cell_rounds) {
+              if (next[0][h] < last[0][h]) idx[h] = cell_list[cs.at(next[0][h])];
+              next[0][h] += W;
+            } else if (r < rounds) {
+              if (next[1][h] < last[1][h]) idx[h] = body_list[bs.at(next[1][h])];
+              next[1][h] += W;
+            }
+          }
+        };
+        // starts the copies of the entries idx names into round r's buffer
+        auto stage_round = [&](u32 r) {
+          if (r < rounds) {
+            float4 *buf = stage[warp][r & 1u];
+#pragma unroll
+            for (int h = 0; h < kPer; ++h) {
+              if (to_c[h] == kNone) continue;
+              if (r < cell_rounds) {
+                copy_cell<kQuad>(buf + to_c[h], cells, idx[h]);
+              } else {
+                copy_async16(buf + to_b[h], bodies + (idx[h] == kNone ? 0u : idx[h]),
+                             idx[h] != kNone);
+                if (!kSoft) sj[warp][r & 1u][to_b[h]] = idx[h];
+              }
+            }
+          }
+          asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        load_indices(0);
+        stage_round(0);
+        load_indices(1);
+        u32 left_c = cut_c.base + (slice < cut_c.rest ? 1u : 0u),
+            left_b = cut_b.base + (slice < cut_b.rest ? 1u : 0u);
+        if (!computes) left_c = left_b = 0u;
+        for (u32 r = 0; r < rounds; ++r) {
+          asm volatile("cp.async.wait_group 0;" ::: "memory");
+          __syncwarp();  // every lane's copies of round r; round r - 1 read
+          stage_round(r + 1u);
+          load_indices(r + 2u);
+          const float4 *buf = stage[warp][r & 1u];
+          if (r < cell_rounds) {
+            const u32 cnt = min(W, left_c);
+            left_c -= cnt;
+            const float4 *mine = buf + area * (kF4 * W + 1u);
+            for (u32 j = 0; j < cnt; j += kU) {
+#pragma unroll
+              for (int u = 0; u < kU; ++u) {
+                const float4 c = mine[kF4 * u];
+                if (kQuad) {
+                  const float4 q = mine[kF4 * u + 1];
+                  const float2 w = *reinterpret_cast<const float2 *>(&mine[kF4 * u + 2]);
+                  add_cell<kSoft>(tg, c, q, w, e2);
+                } else {
+                  add_body<kSoft>(tg, c, e2);
+                }
+              }
+              mine += kF4 * kU;
+            }
+          } else {
+            const u32 cnt = min(W, left_b);
+            left_b -= cnt;
+            const float4 *mine = buf + area * (W + 1u);
+            for (u32 j = 0; j < cnt; j += kU) {
+#pragma unroll
+              for (int u = 0; u < kU; ++u) {
+                const float4 b = mine[u];
+                u32 self = kNone;  // the entry's target, if it is one
+                if (!kSoft) self = sj[warp][r & 1u][kSoft ? 0u : area * (W + 1u) + j + u] - q0.x;
+                add_body<kSoft>(tg, b, e2, !kSoft && self == t0, !kSoft && self == t1);
+              }
+              mine += kU;
+            }
+          }
+        }
+        __syncwarp();  // the last round is read before the next pass stages
+        // this pass's partial sums onto the targets', slice by slice
+        const float4 r0 = make_float4(tg.ax.x, tg.ay.x, tg.az.x, tg.pot.x),
+                     r1 = make_float4(tg.ax.y, tg.ay.y, tg.az.y, tg.pot.y);
+        if (kTeam) {
+          if (computes) {
+            sums[slice][t0] = r0;
+            if (t1 != t0) sums[slice][t1] = r1;
+          }
+        } else {
+          for (u32 a = 0; a < nsp; ++a) {
+            if (computes && area == a) {
+              float4 &u = sums[warp][t0];
+              u = make_float4(u.x + r0.x, u.y + r0.y, u.z + r0.z, u.w + r0.w);
+              if (t1 != t0) {
+                float4 &w = sums[warp][t1];
+                w = make_float4(w.x + r1.x, w.y + r1.y, w.z + r1.z, w.w + r1.w);
+              }
+            }
+            __syncwarp();
+          }
+        }
+      }
     }
-    if (static_cast<u32>(lane) < T) {
+    if (kTeam) __syncthreads();
+    if (static_cast<u32>(lane) < T && (!kTeam || warp == 0)) {
       const u32 i = q0.x + static_cast<u32>(lane);
-      float4 acc = sacc[warp][lane];
-      acc.w += G * bodies[i].w * rsqrtf(eps2);  // the self term (softened), taken back once
-      write_target(eo, i, acc);
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (kTeam) {
+        for (u32 s = 0; s < S; ++s) {
+          const float4 u = sums[s][lane];
+          acc = make_float4(acc.x + u.x, acc.y + u.y, acc.z + u.z, acc.w + u.w);
+        }
+      } else {
+        acc = sums[warp][lane];
+      }
+      // the self term (softened), taken back once
+      if (kSoft) acc.w -= __fmul_rn(bodies[i].w, rsqrtf(eps2));
+      write_target(eo, i, make_float4(G * acc.x, G * acc.y, G * acc.z, -G * acc.w));
     }
+    if (kTeam) __syncthreads();  // the sums are read before the next group's
   }
 }
 
-template <int kU>
-void launch_pairs(const float4 *bodies, const float4 *cells, const u32 *cell_list,
-                  const u32 *body_list, const uint4 *groups, u64 n_groups, float G, float eps2,
-                  const EvalOut &eo, u32 *counter, cudaStream_t s, const Scalars *sc,
-                  u32 pass_cost, u64 want, int sms) {
+// What evaluate_lists' launches share.
+struct EvalArgs {
+  const float4 *bodies, *cells;
+  const u32 *cell_list, *body_list;
+  const uint4 *groups;
+  u64 n_groups;  // groups at most
+  float G, eps2;
+  EvalOut eo;
+  u32 *counter;
+  EvalShape shape;
+  const Scalars *sc;  // a graph replay: the group count and the abort word
+};
+
+template <bool kQuad, bool kSoft, bool kTeam, int kU>
+void launch_shape(const EvalArgs &a, int sms, cudaStream_t s) {
   int per_sm = 0;
-  GTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eval_pairs<kU>, kT, 0));
-  const u32 grid = static_cast<u32>(std::min<u64>(want, static_cast<u64>(sms) * std::max(1, per_sm)));
-  k_eval_pairs<kU><<<grid, kT, 0, s>>>(bodies, cells, cell_list, body_list, groups,
-                                       static_cast<u32>(n_groups), G, eps2, eo, counter,
-                                       sc ? &sc->n_groups : nullptr, sc ? &sc->abort : nullptr,
-                                       pass_cost);
+  GTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &per_sm, k_eval<kQuad, kSoft, kTeam, kU>, kT, 0));
+  const u64 want = kTeam ? a.n_groups : (a.n_groups + kWarpsPerBlock - 1) / kWarpsPerBlock;
+  const u32 grid =
+      static_cast<u32>(std::min<u64>(want, static_cast<u64>(sms) * std::max(1, per_sm)));
+  k_eval<kQuad, kSoft, kTeam, kU><<<grid, kT, 0, s>>>(
+      a.bodies, a.cells, a.cell_list, a.body_list, a.groups, static_cast<u32>(a.n_groups), a.G,
+      a.eps2, a.eo, a.counter, a.sc ? &a.sc->n_groups : nullptr, a.sc ? &a.sc->abort : nullptr,
+      a.shape.pass_cost);
+  GTC_LAUNCH_CHECK();
 }
+
+// Groups below which a block's warps share a group.
+constexpr u64 kTeamGroups = 6000;
 
 template <bool kQuad, bool kSoft>
-void launch_eval(const float4 *bodies, const float4 *cells, const u32 *cell_list,
-                 const u32 *body_list, const uint4 *groups, u64 n_groups, float G, float eps2,
-                 const EvalOut &eo, u32 *counter, cudaStream_t s, const EvalShape &shape,
-                 const Scalars *sc = nullptr) {
-  int dev = 0, sms = 0, per_sm = 0;
+void launch_eval(const EvalArgs &a, u64 groups_hint, cudaStream_t s) {
+  constexpr int kTwo = kSoft ? 2 : 1;  // (an unsoftened slice is worked without padding)
+  int dev = 0, sms = 0;
   GTC_CUDA(cudaGetDevice(&dev));
   GTC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  GTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eval<kQuad, kSoft>, kT, 0));
-  const u64 want = (n_groups + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  if (kQuad && kSoft) {
-    if (shape.pairs == 1)
-      launch_pairs<1>(bodies, cells, cell_list, body_list, groups, n_groups, G, eps2, eo, counter,
-                      s, sc, shape.pass_cost, want, sms);
-    else
-      launch_pairs<2>(bodies, cells, cell_list, body_list, groups, n_groups, G, eps2, eo, counter,
-                      s, sc, shape.pass_cost, want, sms);
+  GTC_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(u32), s));
+  if (groups_hint < kTeamGroups) {
+    if (a.shape.pairs == 1) launch_shape<kQuad, kSoft, true, 1>(a, sms, s);
+    else launch_shape<kQuad, kSoft, true, kTwo>(a, sms, s);
   } else {
-    const u32 grid = static_cast<u32>(std::min<u64>(want, static_cast<u64>(sms) * std::max(1, per_sm)));
-    k_eval<kQuad, kSoft><<<grid, kT, 0, s>>>(bodies, cells, cell_list, body_list, groups,
-                                             static_cast<u32>(n_groups), G, eps2, eo, counter,
-                                             sc ? &sc->n_groups : nullptr,
-                                             sc ? &sc->abort : nullptr);
+    if (a.shape.pairs == 1) launch_shape<kQuad, kSoft, false, 1>(a, sms, s);
+    else launch_shape<kQuad, kSoft, false, kTwo>(a, sms, s);
   }
-  GTC_LAUNCH_CHECK();
+}
+
+void launch_any(const EvalArgs &a, bool quadrupole, u64 groups_hint, cudaStream_t s) {
+  if (a.n_groups == 0) return;
+  const bool soft = a.eps2 >= kSoftEps2;
+  if (quadrupole && soft) launch_eval<true, true>(a, groups_hint, s);
+  else if (quadrupole) launch_eval<true, false>(a, groups_hint, s);
+  else if (soft) launch_eval<false, true>(a, groups_hint, s);
+  else launch_eval<false, false>(a, groups_hint, s);
 }
 
 }  // namespace
@@ -504,35 +467,19 @@ void evaluate_lists(const float4 *bodies, const float4 *cells, const u32 *cell_l
                     const u32 *body_list, const uint4 *groups, u64 n_groups, float G, float eps2,
                     bool quadrupole, const EvalOut &eo, u32 *counter, cudaStream_t s,
                     const EvalShape &shape) {
-  if (n_groups == 0) return;
-  GTC_CUDA(cudaMemsetAsync(counter, 0, sizeof(u32), s));
-  const bool soft = eps2 > 0.0f;
-  if (quadrupole && soft)
-    launch_eval<true, true>(bodies, cells, cell_list, body_list, groups, n_groups, G, eps2, eo, counter, s, shape);
-  else if (quadrupole)
-    launch_eval<true, false>(bodies, cells, cell_list, body_list, groups, n_groups, G, eps2, eo, counter, s, shape);
-  else if (soft)
-    launch_eval<false, true>(bodies, cells, cell_list, body_list, groups, n_groups, G, eps2, eo, counter, s, shape);
-  else
-    launch_eval<false, false>(bodies, cells, cell_list, body_list, groups, n_groups, G, eps2, eo, counter, s, shape);
+  launch_any(EvalArgs{bodies, cells, cell_list, body_list, groups, n_groups, G, eps2, eo, counter,
+                      shape, nullptr},
+             quadrupole, n_groups, s);
 }
 
 void evaluate_lists_graph(const float4 *bodies, const float4 *cells, const u32 *cell_list,
                           const u32 *body_list, const uint4 *groups, u64 max_groups,
-                          const Scalars *sc, float G, float eps2, bool quadrupole,
-                          const EvalOut &eo, u32 *counter, cudaStream_t s,
+                          u64 groups_hint, const Scalars *sc, float G, float eps2,
+                          bool quadrupole, const EvalOut &eo, u32 *counter, cudaStream_t s,
                           const EvalShape &shape) {
-  if (max_groups == 0) return;
-  GTC_CUDA(cudaMemsetAsync(counter, 0, sizeof(u32), s));
-  const bool soft = eps2 > 0.0f;
-  if (quadrupole && soft)
-    launch_eval<true, true>(bodies, cells, cell_list, body_list, groups, max_groups, G, eps2, eo, counter, s, shape, sc);
-  else if (quadrupole)
-    launch_eval<true, false>(bodies, cells, cell_list, body_list, groups, max_groups, G, eps2, eo, counter, s, shape, sc);
-  else if (soft)
-    launch_eval<false, true>(bodies, cells, cell_list, body_list, groups, max_groups, G, eps2, eo, counter, s, shape, sc);
-  else
-    launch_eval<false, false>(bodies, cells, cell_list, body_list, groups, max_groups, G, eps2, eo, counter, s, shape, sc);
+  launch_any(EvalArgs{bodies, cells, cell_list, body_list, groups, max_groups, G, eps2, eo,
+                      counter, shape, sc},
+             quadrupole, groups_hint, s);
 }
 
 }  // namespace gtc

@@ -58,10 +58,10 @@ struct alignas(16) WalkRec64 {
   double mx, my, mz, crit2;  // crit = 2 half / theta + delta (group_lists.cpp:59-60)
 };
 
-// Tile shape of the softened quadrupole list evaluation: staged pairs a
-// lane works per inner-loop iteration (1 or 2; the forces do not depend on
-// it), and a pass's fixed cost in staged entries per lane, which sets how
-// many slices a group's lists are cut into (summation order).
+// Tile shape of the list evaluation: staged entries a lane works per
+// inner-loop iteration (1 or 2; the forces do not depend on it), and a
+// pass's fixed cost in staged entries per lane, which sets how many slices a
+// group's lists are cut into (summation order).
 struct EvalShape {
   int pairs = 2;
   u32 pass_cost = 24;
@@ -396,10 +396,11 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
 // The single walk task of a graph replay (the root), written before capture.
 void write_root_task(Workspace &ws, cudaStream_t s);
 // The evaluation of a replay: the group count from the device, nothing
-// after an abort.
+// after an abort. `groups_hint`: the group count the launch is shaped for
+// (the results do not depend on it).
 void evaluate_lists_graph(const float4 *bodies, const float4 *cells, const u32 *cell_list,
                           const u32 *body_list, const uint4 *groups, u64 max_groups,
-                          const Scalars *sc, float G, float eps2, bool quadrupole,
+                          u64 groups_hint, const Scalars *sc, float G, float eps2, bool quadrupole,
                           const EvalOut &eo, u32 *counter, cudaStream_t s,
                           const EvalShape &shape = EvalShape{});
 
