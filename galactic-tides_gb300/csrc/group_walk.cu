@@ -12,8 +12,8 @@
 // the marks into the group array, which comes out in tree order as in the
 // reference.
 //
-// Walk. One thread per group traverses the nodes in their stored order
-// (the order the reference's stack pops them): accept -> record and jump to
+// Walk. By warps (below) or by threads: one thread per group traverses the
+// nodes in their stored order (the order the reference's stack pops them): accept -> record and jump to
 // the node's skip link, leaf -> record its bodies and jump, otherwise step
 // to the next node (its last child). A counting pass sizes the lists; after
 // the offsets are scanned a second pass writes them. Once a walk has
@@ -115,10 +115,12 @@ __global__ void k_last_end(const Scalars *sc, u32 n, u32 *gend) {
 }
 
 // A graph replay's checks around the one-pass walk (bit 8): more groups
-// than the captured slots cover (before), overflow pools too small for the
-// lists that outgrew their slots (after).
-__global__ void k_check_groups_graph(Scalars *sc, u32 groups) {
+// than the captured slots cover, or so many that a warp walks more or fewer
+// together than the captured walk (before; walk_super 0: any), overflow pools
+// too small for the lists that outgrew their slots (after).
+__global__ void k_check_groups_graph(Scalars *sc, u32 groups, int walk_super) {
   if (sc->n_groups > groups) sc->abort |= 8u;
+  if (walk_super != 0 && walk_super_for(sc->n_groups) != walk_super) sc->abort |= 8u;
 }
 __global__ void k_check_slots_graph(Scalars *sc) {
   if (sc->list_overflow) sc->abort |= 8u;
@@ -501,25 +503,36 @@ __global__ void __launch_bounds__(kWalkThreads)
     atomicAdd(&sc->walk_nodes, static_cast<unsigned long long>(sum));
 }
 
-// The walk by warps: one warp per group, 32 node tests per step. The
+// The walk by warps: a warp walks the tree for kSuper (1, 2 or 4) neighbouring
+// groups at once, 32 nodes per step. Neighbouring groups meet mostly the same nodes
+// (two share about 90% of their tests), so a node's record is loaded once for
+// all of them, and a step's 32 lanes make 32 kSuper tests between loads. The
 // warp keeps the nodes still to visit as a stack of index ranges in shared
-// memory, each a run of whole subtrees [i, end) (i, skip[i], ... before
-// end). Each step the lanes take the ranges on top, test each range's first
-// node, and push back the rest of its range and, when the node is opened,
-// its children's range (children on top: depth first). The same nodes are
-// tested, with the same verdicts, as by the reference's walk; only the order
-// the entries reach the lists differs (step order, lane order within a
-// step; fixed for given inputs). Exports put each group's lists back in the
-// reference's order (increasing node and body index, which is its visiting
-// order). Modes: count the lists (kCount); write them at scanned offsets
-// (kFill); write them into per-group slots, counting past a slot that
+// memory, each a run of whole subtrees [i, end) (i, skip[i], ... before end)
+// with a mask of the groups that opened its parent. Each step the lanes take
+// the ranges on top, test each range's first node against every group of its
+// mask, and push back the rest of the range and, for the groups that opened
+// the node, its children's range (children on top: depth first). Every group
+// tests exactly the nodes of the reference's walk, with the same verdicts;
+// only the order the entries reach its lists differs (step order, lane order
+// within a step). That order is fixed by the kSuper groups walked together,
+// which are those at places kSuper j .. kSuper j + kSuper - 1 of their own
+// system, whatever else a launch walks. Exports put each group's lists back
+// in increasing order. Modes: count the lists (kCount); write them at scanned
+// offsets (kFill); write them into per-group slots, counting past a slot that
 // overflows (kSlots, the one-pass walk, whose counts and records then go
 // through the split walk's spill and record kernels as one part); write the
 // lists of the groups that outgrew their slots again, whole, into their
-// places in the overflow pools (kSpill).
+// places in the overflow pools (kSpill: the others of their kSuper are walked
+// along unwritten).
+//
+// Bound: instruction issue (75% of the issue slots busy at 1M bodies, four
+// groups to a warp; 190 instructions per 32 tests, the test itself 33). 2M
+// bodies 0.96 ms against 1.63 ms by threads (bound by their chains of
+// scattered record loads). kSuper: walk_super_for.
 constexpr int kSlots = 2;
 constexpr int kWarpWalkWarps = 4;
-constexpr int kWarpStack = 1024;  // ranges per warp
+constexpr u32 kWarpStack = 640;   // ranges per warp
 constexpr u32 kWarpWalkThreads = kWarpWalkWarps * 32;
 
 struct WarpWalkOut {
@@ -532,181 +545,328 @@ struct WarpWalkOut {
   const uint4 *plan = nullptr;    // kSlots, a forest: per-group slots (starts, sizes)
 };
 
-__device__ __forceinline__ u32 warp_excl_scan(u32 v, int lane, u32 &total) {
-  u32 s = v;
+// Where a forest's groups belong: the first group and the group count of
+// each system come from the group choice's scan at its first body.
+struct GroupSystems {
+  const u32 *gbegin = nullptr;
+  const u16 *sys = nullptr;      // null: one system
+  const u32 *start = nullptr;
+  const u32 *mscan = nullptr;
+  u32 systems = 0;
+};
+
+// What a warp keeps in shared memory.
+template <int kSuper>
+struct WarpWalk {
+  uint2 stk[kWarpStack];
+  float4 box[kSuper][2];         // the groups' FP32 boxes
+  uint4 out[kSuper];             // cell list start and room, body list start and room
+  u32 q_begin[64], q_count[64];  // body runs met, to be written 32 at a time
+  u8 q_mask[64];
+  u8 mask[kWarpStack];
+};
+
+__device__ __noinline__ int decide64(const WalkRec64 *walk64, u32 i, const double *gbox, u32 g) {
+  double gc[3], gh[3];
+  for (int a = 0; a < 3; ++a) {
+    gc[a] = gbox[6ull * g + a];
+    gh[a] = gbox[6ull * g + 3 + a];
+  }
+  return accept64(load64(walk64, i), gc, gh) ? 1 : 0;
+}
+
+// Appends the first `runs` (at most 32) queued body runs to the lists of the
+// groups in their masks, in queue order. Every lane of the warp calls it.
+template <bool kWrite, int kSuper>
+__device__ __forceinline__ void append_runs(const WarpWalk<kSuper> &w, u32 runs, u32 (&nb)[kSuper],
+                                            u32 *body_list) {
+  const u32 lane = threadIdx.x & 31u;
+  const bool has = lane < runs;
+  const u32 begin = has ? w.q_begin[lane] : 0u, count = has ? w.q_count[lane] : 0u;
+  const u32 mask = has ? w.q_mask[lane] : 0u;
+  u32 at[kSuper];
+  if (__any_sync(kFullMask, count > 2047u)) {  // a sum may pass 16 bits
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const u32 y = __shfl_up_sync(kFullMask, s, o);
-    if (lane >= o) s += y;
-  }
-  total = __shfl_sync(kFullMask, s, 31);
-  return s - v;
-}
-
-// Walks the ranges on a warp's stack (stk[0..top), each a run of whole
-// subtrees [i, end)) to the end for group g: each step the lanes take the
-// ranges on top, test each range's first node, and push back the rest of
-// its range and, when the node is opened, its children's range (children
-// on top). Cells and bodies go to cl / bl from nc / nb on (kWrite; counting
-// past cap_c / cap_b), in step order, lane order within a step. When the
-// stack is nearly full, lane 0 walks the top range alone, so no step can
-// overflow it. Every lane of the warp calls it; nc and nb are warp-uniform.
-template <bool kWrite>
-__device__ __forceinline__ void walk_ranges_warp(uint2 *stk, u32 top, const WalkRec32 *walk32,
-                                                 const WalkRec64 *walk64, const float *gf,
-                                                 const float *hf, float gbound,
-                                                 const double *gbox, u32 g, u32 *cl, u32 *bl,
-                                                 u64 cap_c, u64 cap_b, u64 &nc, u64 &nb,
-                                                 u32 &exact, u32 &visits, Scalars *sc) {
-  const int lane = threadIdx.x & 31;
-  const unsigned below = (1u << lane) - 1u;
-  while (top > 0) {
-    if (top > kWarpStack - 2 * 32) {
-      // nearly full: lane 0 walks the top range alone, without a stack
-      const uint2 e = stk[top - 1];
-      --top;
-      __syncwarp();
-      if (lane == 0) {
-        u32 i = e.x;
-        while (i < e.y) {
-          const WalkRec32 r = load32(walk32, i);
-          ++visits;
-          const int verdict = decide(r, walk64, i, gf, hf, gbound, gbox, g, exact);
-          const u32 nbody = r.nbody_leaf & 0x7fffffffu;
-          const bool leaf = (r.nbody_leaf >> 31) != 0;
-          if (verdict == 1 && nbody > kFewBodies) {
-            if (kWrite && nc < cap_c) cl[nc] = i;
-            ++nc;
-          } else if (verdict == 1 || leaf) {
-            for (u32 j = 0; j < nbody; ++j)
-              if (kWrite && nb + j < cap_b) bl[nb + j] = r.begin + j;
-            nb += nbody;
-          }
-          if (verdict == 1 || leaf) {
-            if (r.skip <= i) {  // malformed tree: never loop
-              atomicOr(&sc->error, 1u);
-              break;
-            }
-            i = r.skip;
-          } else {
-            ++i;
-          }
-        }
+    for (int k = 0; k < kSuper; ++k) {
+      const u32 c = (mask >> k) & 1u ? count : 0u;
+      u32 s = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u32 y = __shfl_up_sync(kFullMask, s, o);
+        if (lane >= static_cast<u32>(o)) s += y;
       }
-      nc = __shfl_sync(kFullMask, nc, 0);
-      nb = __shfl_sync(kFullMask, nb, 0);
-      continue;
+      at[k] = nb[k] + s - c;
+      nb[k] += __shfl_sync(kFullMask, s, 31);
     }
-    const u32 take = min(32u, top);
-    const bool has = static_cast<u32>(lane) < take;
-    const uint2 e = has ? stk[top - 1 - lane] : make_uint2(0u, 0u);
-    top -= take;
-    __syncwarp();
-    WalkRec32 r{};
-    int verdict = 0;
-    if (has) {
-      r = load32(walk32, e.x);
-      ++visits;
-      verdict = decide(r, walk64, e.x, gf, hf, gbound, gbox, g, exact);
+  } else {  // four groups' sums in the 16-bit fields of one scan
+#pragma unroll
+    for (int q = 0; q < kSuper; q += 4) {
+      u64 c = 0;
+#pragma unroll
+      for (int k = 0; k < 4 && q + k < kSuper; ++k)
+        c |= static_cast<u64>((mask >> (q + k)) & 1u ? count : 0u) << (16 * k);
+      u64 s = c;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u64 y = __shfl_up_sync(kFullMask, s, o);
+        if (lane >= static_cast<u32>(o)) s += y;
+      }
+      const u64 total = __shfl_sync(kFullMask, s, 31);
+      s -= c;
+#pragma unroll
+      for (int k = 0; k < 4 && q + k < kSuper; ++k) {
+        at[q + k] = nb[q + k] + static_cast<u32>((s >> (16 * k)) & 0xffffull);
+        nb[q + k] += static_cast<u32>((total >> (16 * k)) & 0xffffull);
+      }
     }
-    const u32 nbody = r.nbody_leaf & 0x7fffffffu;
-    const bool leaf = (r.nbody_leaf >> 31) != 0;
-    const bool bad = has && r.skip <= e.x;  // malformed tree: never loop
-    if (bad) atomicOr(&sc->error, 1u);
-    const bool cell = has && verdict == 1 && nbody > kFewBodies;
-    const bool bod = has && !cell && (verdict == 1 || leaf);
-    const bool kids = has && !bad && verdict == 0 && !leaf;
-    const bool rest = has && !bad && r.skip < e.y;
-    // cells: one slot per accepting lane, in lane order
-    const unsigned mc = __ballot_sync(kFullMask, cell);
-    if (kWrite && cell) {
-      const u64 pos = nc + __popc(mc & below);
-      if (pos < cap_c) cl[pos] = e.x;
+  }
+  if (kWrite) {
+#pragma unroll
+    for (int k = 0; k < kSuper; ++k) {
+      if (!((mask >> k) & 1u)) continue;
+      const uint4 o = w.out[k];
+      for (u32 j = 0; j < count; ++j)
+        if (at[k] + j < o.w) body_list[static_cast<u64>(o.z) + at[k] + j] = begin + j;
     }
-    nc += __popc(mc);
-    // bodies: each lane's run after the runs of the lanes before it
-    u32 bt = 0;
-    const u32 boff = warp_excl_scan(bod ? nbody : 0u, lane, bt);
-    if (kWrite && bod)
-      for (u32 j = 0; j < nbody; ++j)
-        if (nb + boff + j < cap_b) bl[nb + boff + j] = r.begin + j;
-    nb += bt;
-    // pushes: each lane its rest, then its children's range (on top)
-    u32 pt = 0;
-    const u32 poff = warp_excl_scan(static_cast<u32>(rest) + static_cast<u32>(kids), lane, pt);
-    if (rest) stk[top + poff] = make_uint2(r.skip, e.y);
-    if (kids) stk[top + poff + (rest ? 1u : 0u)] = make_uint2(e.x + 1, r.skip);
-    top += pt;
-    __syncwarp();
   }
 }
 
-template <int kMode>
+template <int kMode, int kSuper>
 __global__ void __launch_bounds__(kWarpWalkThreads)
     k_walk_warp(const WalkRec32 *walk32, const WalkRec64 *walk64, const double *gbox,
-                const float *gboxf, u32 ng_cap, WarpWalkOut out, u32 *next_group, Scalars *sc,
-                const u32 *ng_dev, const u32 *abort, const u32 *group_root) {
-  __shared__ uint2 stack_all[kWarpWalkWarps][kWarpStack];
+                const float *gboxf, u32 ng_cap, WarpWalkOut out, u32 *next_chunk, Scalars *sc,
+                const u32 *ng_dev, const u32 *abort, const u32 *group_root, GroupSystems gs,
+                bool own_size) {
+  constexpr bool kWrite = kMode != kCount;
+  __shared__ WarpWalk<kSuper> walks[kWarpWalkWarps];
   if (aborted(abort)) return;
   const u32 ng = bounded(ng_cap, ng_dev);
-  const int lane = threadIdx.x & 31;
-  uint2 *stk = stack_all[threadIdx.x >> 5];
+  const u32 lane = threadIdx.x & 31u;
+  const u32 below = (1u << lane) - 1u;
+  WarpWalk<kSuper> &w = walks[threadIdx.x >> 5];
   u32 exact = 0, visits = 0;
+  u32 g = 0, chunk_end = 0;  // groups of the taken chunk still to look at
   for (;;) {
-    u32 g = 0;
-    if (lane == 0) g = atomicAdd(next_group, 1u);
-    g = __shfl_sync(kFullMask, g, 0);
-    if (g >= ng) break;
-    u32 *cl = nullptr, *bl = nullptr;
-    u64 cap_c = ~0ull, cap_b = ~0ull;
-    if (kMode == kFill) {
-      cl = out.cell_list + out.cell_off[g];
-      bl = out.body_list + out.body_off[g];
-    } else if (kMode == kSlots) {
-      if (out.plan) {
-        const uint4 st = out.plan[2ull * g], cp = out.plan[2ull * g + 1];
-        cap_c = cp.x;
-        cap_b = cp.y;
-        cl = out.cell_list + st.x;
-        bl = out.body_list + st.y;
-      } else {
-        cap_c = out.slot_cells;
-        cap_b = out.slot_bodies;
-        cl = out.cell_list + static_cast<u64>(g) * cap_c;
-        bl = out.body_list + static_cast<u64>(g) * cap_b;
-      }
-    } else if (kMode == kSpill) {
-      if (out.spill_cells[g] == kNoSpill) continue;
-      cl = out.cell_list + out.spill_cells[g];
-      bl = out.body_list + out.spill_bodies[g];
+    if (g >= chunk_end) {
+      u32 c = 0;
+      if (lane == 0) c = atomicAdd(next_chunk, 1u);
+      c = __shfl_sync(kFullMask, c, 0);
+      if (static_cast<u64>(c) * kSuper >= ng) break;
+      g = c * kSuper;
+      chunk_end = min(ng, g + kSuper);
     }
-    const float4 b0 = reinterpret_cast<const float4 *>(gboxf)[2ull * g],
-                 b1 = reinterpret_cast<const float4 *>(gboxf)[2ull * g + 1];
-    const float gf[3] = {b0.x, b0.y, b0.z}, hf[3] = {b0.w, b1.x, b1.y};
-    const float gbound = b1.z;
-    u64 nc = 0, nb = 0;  // warp-uniform
-    // the root contains every group and is opened, unless it is a leaf
-    const u32 root = group_root ? group_root[g] : 0u;
-    const WalkRec32 rr = load32(walk32, root);
-    const bool root_leaf = (rr.nbody_leaf >> 31) != 0;
-    if (lane == 0) stk[0] = make_uint2(root_leaf ? root : root + 1, rr.skip);
-    u32 top = 1;
-    __syncwarp();
-    walk_ranges_warp<kMode != kCount>(stk, top, walk32, walk64, gf, hf, gbound, gbox, g, cl, bl,
-                                      cap_c, cap_b, nc, nb, exact, visits, sc);
-    if (lane == 0) {
-      if (kMode == kCount) {
-        out.ncells[g] = nc;
-        out.nbodies[g] = nb;
+    // the chunk's next group at a place kSuper j of its system leads its kSuper
+    const u32 lead = g++;
+    u32 first = 0, end = ng;
+    if (gs.sys) {
+      const u32 k = gs.sys[gs.gbegin[lead]];
+      first = gs.mscan[gs.start[k]];
+      if (k + 1 < gs.systems) end = gs.mscan[gs.start[k + 1]];
+    }
+    // (own_size: the systems that walk kSuper groups at a time only)
+    if ((lead - first) % kSuper != 0 || (own_size && walk_super_for(end - first) != kSuper))
+      continue;
+    const u32 count = min(static_cast<u32>(kSuper), end - lead);
+    if (lane < kSuper) {  // lane k readies group k
+      const u32 q = lead + min(lane, count - 1u);
+      w.box[lane][0] = reinterpret_cast<const float4 *>(gboxf)[2ull * q];
+      w.box[lane][1] = reinterpret_cast<const float4 *>(gboxf)[2ull * q + 1];
+      uint4 o = make_uint4(0u, 0u, 0u, 0u);
+      if (kMode == kFill) {
+        o = make_uint4(static_cast<u32>(out.cell_off[q]), 0xffffffffu,
+                       static_cast<u32>(out.body_off[q]), 0xffffffffu);
       } else if (kMode == kSlots) {
-        out.ncells[g] = nc;
-        out.nbodies[g] = nb;
-        out.ncells[static_cast<u64>(out.cap) + g] = 0;
-        out.nbodies[static_cast<u64>(out.cap) + g] = 0;
-        out.split[2ull * g] = static_cast<u32>(nc < 0xffffffffull ? nc : 0xffffffffull);
-        out.split[2ull * g + 1] = static_cast<u32>(nb < 0xffffffffull ? nb : 0xffffffffull);
+        if (out.plan) {
+          const uint4 st = out.plan[2ull * q], cp = out.plan[2ull * q + 1];
+          o = make_uint4(st.x, cp.x, st.y, cp.y);
+        } else {
+          o = make_uint4(q * out.slot_cells, out.slot_cells, q * out.slot_bodies,
+                         out.slot_bodies);
+        }
+      } else if (kMode == kSpill) {
+        if (out.spill_cells[q] != kNoSpill)
+          o = make_uint4(out.spill_cells[q], 0xffffffffu, out.spill_bodies[q], 0xffffffffu);
+      }
+      w.out[lane] = o;
+    }
+    if (kMode == kSpill) {
+      const bool spilled = lane < count && out.spill_cells[lead + lane] != kNoSpill;
+      if (!__any_sync(kFullMask, spilled)) continue;
+    }
+    u32 nc[kSuper], nb[kSuper];  // warp-uniform
+#pragma unroll
+    for (int k = 0; k < kSuper; ++k) nc[k] = nb[k] = 0u;
+    // the root contains every group and is opened, unless it is a leaf
+    const u32 root = group_root ? group_root[lead] : 0u;
+    const WalkRec32 rr = load32(walk32, root);
+    if (lane == 0) {
+      w.stk[0] = make_uint2((rr.nbody_leaf >> 31) != 0 ? root : root + 1, rr.skip);
+      w.mask[0] = static_cast<u8>((1u << count) - 1u);
+    }
+    u32 top = 1, queued = 0;
+    __syncwarp();
+    while (top > 0) {
+      if (top > kWarpStack - 2 * 32) {
+        // nearly full: lane k walks the top range for group k alone, without
+        // a stack
+        append_runs<kWrite>(w, queued, nb, out.body_list);
+        queued = 0;
+        --top;
+        const uint2 e = w.stk[top];
+        const u32 m = w.mask[top];
+        u32 c = 0, b = 0;
+#pragma unroll
+        for (int k = 0; k < kSuper; ++k)
+          if (lane == k) {
+            c = nc[k];
+            b = nb[k];
+          }
+        if (lane < kSuper && (m >> lane) & 1u) {
+          const float4 b0 = w.box[lane][0], b1 = w.box[lane][1];
+          const float gf[3] = {b0.x, b0.y, b0.z}, hf[3] = {b0.w, b1.x, b1.y};
+          const uint4 o = w.out[lane];
+          u32 i = e.x;
+          while (i < e.y) {
+            const WalkRec32 r = load32(walk32, i);
+            ++visits;
+            int verdict = accept32(r, gf, hf, b1.z);
+            if (verdict == 2) {
+              verdict = decide64(walk64, i, gbox, lead + lane);
+              ++exact;
+            }
+            const u32 nbody = r.nbody_leaf & 0x7fffffffu;
+            const bool leaf = (r.nbody_leaf >> 31) != 0;
+            if (verdict == 1 && nbody > kFewBodies) {
+              if (kWrite && c < o.y) out.cell_list[static_cast<u64>(o.x) + c] = i;
+              ++c;
+            } else if (verdict == 1 || leaf) {
+              for (u32 j = 0; j < nbody; ++j)
+                if (kWrite && b + j < o.w) out.body_list[static_cast<u64>(o.z) + b + j] = r.begin + j;
+              b += nbody;
+            }
+            if (verdict == 1 || leaf) {
+              if (r.skip <= i) {  // malformed tree: never loop
+                atomicOr(&sc->error, 1u);
+                break;
+              }
+              i = r.skip;
+            } else {
+              ++i;
+            }
+          }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < kSuper; ++k) {
+          nc[k] = __shfl_sync(kFullMask, c, k);
+          nb[k] = __shfl_sync(kFullMask, b, k);
+        }
+        continue;
+      }
+      const u32 take = min(32u, top);
+      const bool has = lane < take;
+      const uint2 e = has ? w.stk[top - 1u - lane] : make_uint2(0u, 0u);
+      const u32 m = has ? w.mask[top - 1u - lane] : 0u;
+      top -= take;
+      __syncwarp();
+      WalkRec32 r{};
+      u32 accepted = 0;
+      if (has) {
+        r = load32(walk32, e.x);
+        visits += __popc(m);
+#pragma unroll
+        for (int k = 0; k < kSuper; ++k) {
+          const float4 b0 = w.box[k][0], b1 = w.box[k][1];
+          const float gf[3] = {b0.x, b0.y, b0.z}, hf[3] = {b0.w, b1.x, b1.y};
+          int verdict = accept32(r, gf, hf, b1.z);
+          if (verdict == 2 && (m >> k) & 1u) {
+            verdict = decide64(walk64, e.x, gbox, lead + k);
+            ++exact;
+          }
+          accepted |= (verdict == 1 ? 1u : 0u) << k;
+        }
+        accepted &= m;
+      }
+      const u32 nbody = r.nbody_leaf & 0x7fffffffu;
+      const bool leaf = (r.nbody_leaf >> 31) != 0;
+      const bool bad = has && r.skip <= e.x;  // malformed tree: never loop
+      if (bad) atomicOr(&sc->error, 1u);
+      const u32 cells = nbody > kFewBodies ? accepted : 0u;
+      const u32 runs = (leaf ? m : accepted) & ~cells;
+      const u32 opened = leaf || bad ? 0u : m & ~accepted;
+      const bool rest = has && !bad && r.skip < e.y;
+      // cells: one place per accepting lane, in lane order
+#pragma unroll
+      for (int k = 0; k < kSuper; ++k) {
+        const bool mine = (cells >> k) & 1u;
+        const u32 all = __ballot_sync(kFullMask, mine);
+        if (kWrite && mine) {
+          const u32 at = nc[k] + __popc(all & below);
+          const uint2 o = *reinterpret_cast<const uint2 *>(&w.out[k]);
+          if (at < o.y) out.cell_list[static_cast<u64>(o.x) + at] = e.x;
+        }
+        nc[k] += __popc(all);
+      }
+      // body runs, queued in lane order and appended 32 at a time
+      const u32 with_runs = __ballot_sync(kFullMask, runs != 0u);
+      if (runs) {
+        const u32 at = queued + __popc(with_runs & below);
+        w.q_begin[at] = r.begin;
+        w.q_count[at] = nbody;
+        w.q_mask[at] = static_cast<u8>(runs);
+      }
+      queued += __popc(with_runs);
+      // pushes: each lane its rest, then its children's range (on top)
+      const u32 rests = __ballot_sync(kFullMask, rest),
+                kids = __ballot_sync(kFullMask, opened != 0u);
+      u32 at = top + __popc(rests & below) + __popc(kids & below);
+      if (rest) {
+        w.stk[at] = make_uint2(r.skip, e.y);
+        w.mask[at] = static_cast<u8>(m);
+        ++at;
+      }
+      if (opened) {
+        w.stk[at] = make_uint2(e.x + 1u, r.skip);
+        w.mask[at] = static_cast<u8>(opened);
+      }
+      top += __popc(rests) + __popc(kids);
+      __syncwarp();
+      if (queued >= 32u) {
+        append_runs<kWrite>(w, 32u, nb, out.body_list);
+        queued -= 32u;
+        __syncwarp();
+        if (lane < queued) {
+          const u32 b = w.q_begin[32u + lane], c = w.q_count[32u + lane];
+          const u8 k = w.q_mask[32u + lane];
+          w.q_begin[lane] = b;
+          w.q_count[lane] = c;
+          w.q_mask[lane] = k;
+        }
+        __syncwarp();
       }
     }
+    append_runs<kWrite>(w, queued, nb, out.body_list);
+    if (kMode == kCount || kMode == kSlots) {
+      u32 c = 0, b = 0;
+#pragma unroll
+      for (int k = 0; k < kSuper; ++k)
+        if (lane == k) {
+          c = nc[k];
+          b = nb[k];
+        }
+      if (lane < count) {
+        const u32 q = lead + lane;
+        out.ncells[q] = c;
+        out.nbodies[q] = b;
+        if (kMode == kSlots) {
+          out.ncells[static_cast<u64>(out.cap) + q] = 0;
+          out.nbodies[static_cast<u64>(out.cap) + q] = 0;
+          out.split[2ull * q] = c;
+          out.split[2ull * q + 1] = b;
+        }
+      }
+    }
+    __syncwarp();  // the shared memory is free for the next groups
   }
   if (kMode == kCount || kMode == kSlots) {
     const u32 ex = __reduce_add_sync(kFullMask, exact), vs = __reduce_add_sync(kFullMask, visits);
@@ -879,23 +1039,44 @@ void size_slots(Workspace &ws, const Scalars &h, bool split) {
   ws.slot_near_bodies = slot(ws.walk_warps ? 0 : split ? h.max_near_bodies : h.max_bodies);
 }
 
-// The warp walk over ng groups: enough warps to fill the GPU, groups taken
-// from a counter.
-template <int kMode>
-void launch_warp_walk(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scalars *sc,
-                      cudaStream_t s, const u32 *ng_dev = nullptr, const u32 *abort = nullptr) {
-  int dev = 0, sms = 0;
+// The warp walk over ng groups: enough warps to fill the GPU, kSuper groups at
+// a time taken from a counter.
+template <int kMode, int kSuper>
+void launch_warp_walk_of(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scalars *sc,
+                         cudaStream_t s, const u32 *ng_dev, const u32 *abort) {
+  int dev = 0, sms = 0, per_sm = 0;
   GTC_CUDA(cudaGetDevice(&dev));
   GTC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  GTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_warp<kMode, kSuper>,
+                                                         kWarpWalkThreads, 0));
   ws.walk_next.ensure(sizeof(u32));
   GTC_CUDA(cudaMemsetAsync(ws.walk_next.ptr, 0, sizeof(u32), s));
   const u32 blocks = static_cast<u32>(std::max<u64>(
-      1, std::min<u64>(ceil_div(ng_cap, kWarpWalkWarps), 8ull * static_cast<u64>(sms))));
-  k_walk_warp<kMode><<<blocks, kWarpWalkThreads, 0, s>>>(
+      1, std::min<u64>(ceil_div(ng_cap, kWarpWalkWarps * kSuper),
+                       static_cast<u64>(std::max(1, per_sm)) * static_cast<u64>(sms))));
+  GroupSystems gs;
+  if (ws.forest)
+    gs = GroupSystems{ws.gbegin.as<u32>(), ws.forest.sys, ws.forest.start,
+                      ws.flags_scan.as<u32>(), ws.forest.systems};
+  k_walk_warp<kMode, kSuper><<<blocks, kWarpWalkThreads, 0, s>>>(
       ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), ws.gbox.as<double>(),
       ws.gboxf.as<float>(), ng_cap, out, ws.walk_next.as<u32>(), sc, ng_dev, abort,
-      ws.forest.group_root);
+      ws.forest.group_root, gs, ws.walk_super == 0);
   GTC_LAUNCH_CHECK();
+}
+
+template <int kMode>
+void launch_warp_walk(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scalars *sc,
+                      cudaStream_t s, const u32 *ng_dev = nullptr, const u32 *abort = nullptr) {
+  switch (ws.walk_super) {
+    case 1: return launch_warp_walk_of<kMode, 1>(ws, out, ng_cap, sc, s, ng_dev, abort);
+    case 2: return launch_warp_walk_of<kMode, 2>(ws, out, ng_cap, sc, s, ng_dev, abort);
+    case 4: return launch_warp_walk_of<kMode, 4>(ws, out, ng_cap, sc, s, ng_dev, abort);
+    default:  // a forest: each system in the launch of its size
+      launch_warp_walk_of<kMode, 4>(ws, out, ng_cap, sc, s, ng_dev, abort);
+      launch_warp_walk_of<kMode, 2>(ws, out, ng_cap, sc, s, ng_dev, abort);
+      launch_warp_walk_of<kMode, 1>(ws, out, ng_cap, sc, s, ng_dev, abort);
+  }
 }
 
 // The node arrays the group choice reads (a forest's per-system fields too).
@@ -976,7 +1157,7 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   read_scalars(ws, host, s);
   const u32 ng = host->n_groups, ntasks = fv ? 1u : host->aux;
   ws.n_groups = ng;
-  ws.walk_warps = ws.warps_for(ng);
+  ws.choose_walk(ng);
   const u32 gb = ceil_div(ng, kT);
   k_group_box<<<gb, kT, 0, s>>>(gbegin, gend, ng, ws.tpos.as<double>(),
                                 fv ? fv.roots : ws.root.as<TreeRoot>(), ws.gbox.as<double>(),
@@ -1178,7 +1359,7 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
   // one pass into the captured slots (near field and rest), outgrown groups
   // again into the pools
   if (!caps.sys_slots) {  // (per-system slots: a system past its capacity spills)
-    k_check_groups_graph<<<1, 1, 0, s>>>(sc, caps.groups);
+    k_check_groups_graph<<<1, 1, 0, s>>>(sc, caps.groups, ws.walk_mode < 0 ? ws.walk_super : 0);
     GTC_LAUNCH_CHECK();
   }
   GTC_CUDA(cudaMemsetAsync(&sc->n_cell_list, 0, 2 * sizeof(u64), s));
@@ -1188,7 +1369,7 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
   GTC_CUDA(cudaMemsetAsync(&sc->spilled, 0, sizeof(u32), s));
   GTC_CUDA(cudaMemsetAsync(&sc->walk_nodes, 0, sizeof(unsigned long long), s));
   u32 *spill_c = ws.spill.as<u32>(), *spill_b = spill_c + n;
-  ws.walk_warps = ws.warps_for(caps.groups);  // the replays' walk, chosen at capture
+  // (the replays' walk: the choice of the eager solve before the capture)
   const u64 near_c = static_cast<u64>(caps.groups) * caps.slot_cells;
   const u64 near_b = static_cast<u64>(caps.groups) * caps.slot_bodies;
   u64 pool_at_c = near_c + static_cast<u64>(caps.groups) * caps.slot_near_cells;

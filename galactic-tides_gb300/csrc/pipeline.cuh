@@ -117,6 +117,20 @@ struct ForestView {
   explicit operator bool() const { return systems > 0; }
 };
 
+// Neighbouring groups of a system of `groups` groups that a warp walks
+// together: more the more there are, since few groups leave most of the GPU
+// idle and want a warp each, and many are bound by instructions and share node
+// records and steps. The walk's time by groups per warp 1 / 2 / 4 (with the
+// spill and record kernels): 240 groups 71 / 82 / 110 us, 2.2k 98 / 100 / 143,
+// 4.4k 127 / 114 / 161, 8.8k 192 / 174 / 235, 17.6k 364 / 282 / 307 (the solve
+// 1.74 / 1.69 ms by 2 / 4: fewer warps beside the side stream), 87k 1720 / 1142 /
+// 962; by threads 1.63 ms at 87k, a warp each with two scans a step 276 us at
+// 8.8k. It depends on the system's own groups only, as does the order of
+// their lists: a forest's systems keep the order each has alone.
+__host__ __device__ inline int walk_super_for(u64 groups) {
+  return groups < 3000 ? 1 : groups < 15000 ? 2 : 4;
+}
+
 struct Workspace {
   ForestView forest;
   // bodies
@@ -148,18 +162,20 @@ struct Workspace {
   int sort_levels = 0;        // key levels the next eager build sorts first (0: all 21)
   int tree_depth = 0;         // the last eager build's deepest leaf
   int walk_split_depth = 0;   // tuning: subtree depth of the walk tasks (0..2)
-  // The plain walk by warps (one warp per group, 32 node tests per step) or
-  // by threads (two per group in the one pass, one in count + fill). Mode
-  // -1 (default) picks warps below kWarpWalkGroups groups: with fewer, the
-  // thread walk leaves most of the GPU idle; with more, its neighbouring
-  // groups walking the same nodes together make it the faster. walk_warps:
-  // the choice of the current lists.
+  // The plain walk by warps or by threads (two per group in the one pass, one
+  // in count + fill). Mode -1 (default): by warps, each walking
+  // walk_super_for(its system's groups) groups; 1: by warps, two groups each
+  // always; 0: by threads. walk_warps, walk_super (0 in a forest's default:
+  // per system): the choice of the current lists; a captured step keeps the
+  // choice of the eager solve before it, and aborts when another applies.
   int walk_mode = -1;
   bool walk_warps = true;
-  static constexpr u64 kWarpWalkGroups = 40000;
-  bool warps_for(u64 groups) const {
-    return walk_mode > 0 || (walk_mode < 0 && groups < kWarpWalkGroups);
+  int walk_super = 1;
+  void choose_walk(u64 groups) {
+    walk_warps = walk_mode != 0;
+    walk_super = walk_mode > 0 ? 2 : forest ? 0 : walk_super_for(groups);
   }
+  static constexpr u64 kWarpWalkGroups = 40000;  // learned walk: rounds by warps below
   // The current lists hold each group's entries in walk-step order rather
   // than the reference's visiting order (exports sort them back).
   bool lists_unordered = false;

@@ -28,39 +28,39 @@ __device__ __forceinline__ bool accept64(const WalkRec64 &r, const double *gc, c
 // The same test in FP32 with a rigorous error band. Every FP32 input is the
 // FP64 quantity (relative to the root centre) rounded once; the node record
 // carries B_n >= all its |values| + slack and the group B_g >= max|centre| +
-// max half-extent, so every quantity compared below is at most ~2 (B_n + B_g)
-// in size and each FP32 result is within 5 * 2^-24 (B_n + B_g) of the value
-// from the exact inputs (more than the FP64 roundings too). The band
-// E = 2^-20 (B_n + B_g) is over three times that: a comparison whose sides
-// differ by more than E has the FP64 outcome; otherwise the caller runs the
-// FP64 test. Returns 1 accept, 0 open, 2 undecided (NaNs end up undecided).
+// max half-extent, so with B = B_n + B_g every FP32 difference formed below is
+// within 8 * 2^-24 B of the value from the exact inputs (three rounded inputs,
+// two or three operations on values up to 2 B), half of E = 2^-20 B:
+// * overlap: on every axis |c - g| - gh <= slack (group_lists.cpp:147), so the
+//   largest of the three decides, outside a band of E;
+// * the distance from the box to the centre of mass (:150-151): d^2 is the sum
+//   of squares of v_a = max(|m - g| - gh, 0), each within E / 2 of its exact
+//   value, so d^2 is within E (v_x + v_y + v_z) + E^2 of the exact one, plus a few
+//   2^-24 of itself, which the factors (1 +- 2^-18) cover with the rounding of
+//   crit^2. (A lower and an upper bound per axis took half as many
+//   instructions again.)
+// A comparison outside its band has the FP64 outcome; otherwise the caller
+// runs the FP64 test. Returns 1 accept, 0 open, 2 undecided (NaNs end up
+// undecided).
 constexpr float kBand = 1.0f / (1 << 20);
 
 __device__ __forceinline__ int accept32(const WalkRec32 &r, const float *gf, const float *hf,
                                         float gbound) {
   const float e = kBand * (r.bound + gbound);
-  bool separated = false, within = true;
-  float lo2 = 0.f, hi2 = 0.f;
-  const float c[3] = {r.cx, r.cy, r.cz}, mm[3] = {r.mx, r.my, r.mz};
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    // overlap: on every axis |c - g| <= slack + gh (group_lists.cpp:147)
-    const float x = fabsf(c[a] - gf[a]), y = r.slack + hf[a];
-    separated |= x > y + e;
-    within &= x < y - e;
-    // distance from the box to the centre of mass (group_lists.cpp:150-151)
-    const float d = fabsf(mm[a] - gf[a]) - hf[a];
-    const float dl = fmaxf(d - e, 0.f), dh = fmaxf(d + e, 0.f);
-    lo2 = fmaf(dl, dl, lo2);
-    hi2 = fmaf(dh, dh, hi2);
-  }
+  const float over = fmaxf(fmaxf(fabsf(r.cx - gf[0]) - hf[0], fabsf(r.cy - gf[1]) - hf[1]),
+                           fabsf(r.cz - gf[2]) - hf[2]) - r.slack;
+  const float vx = fmaxf(fabsf(r.mx - gf[0]) - hf[0], 0.f),
+              vy = fmaxf(fabsf(r.my - gf[1]) - hf[1], 0.f),
+              vz = fmaxf(fabsf(r.mz - gf[2]) - hf[2], 0.f);
+  const float d2 = fmaf(vx, vx, fmaf(vy, vy, vz * vz));
+  const float tol = e * (vx + vy + vz + e);
   const float c2 = r.crit2;
+  const bool apart = d2 - tol > c2 * (1.f + 4.f * kBand);   // farther than crit for sure
+  const bool close = d2 + tol < c2 * (1.f - 4.f * kBand);   // nearer for sure
+  int verdict = over < -e || close ? 0 : (over > e && apart ? 1 : 2);
   // scales where a rounding above may be a subnormal's: left to FP64
-  if (e < 1e-36f || (hi2 < 1e-35f && c2 < 1e-35f)) return 2;
-  if (within) return 0;                                      // overlaps: opened
-  if (hi2 * (1.f + 4.f * kBand) < c2 * (1.f - 4.f * kBand)) return 0;  // too close
-  if (separated && lo2 * (1.f - 4.f * kBand) > c2 * (1.f + 4.f * kBand)) return 1;
-  return 2;
+  if (e < 1e-36f || fmaxf(d2 + tol, c2) < 1e-35f) verdict = 2;
+  return verdict;
 }
 
 __device__ __forceinline__ WalkRec32 load32(const WalkRec32 *w, u32 i) {

@@ -402,19 +402,17 @@ gtc_status gtc_autotune_eval(gtc_context *ctx, const double *pos, const double *
  *                        back how many pairs the last one deferred (more
  *                        rounds follow one read back each); 1 reads back
  *                        after every round. Results do not depend on it.
- *   "walk_warps"         -1 (default), 0 or 1: the plain walk by warps, one
- *                        per group, 32 node tests per step (1), or by
- *                        threads, two per group in the one-pass walk (0),
- *                        whose lists keep the reference's order; -1 takes
- *                        warps below 40000 groups (the thread walk leaves
- *                        the GPU idle there) and threads above (neighbouring
- *                        groups share their record loads). Lists hold the
- *                        same entries.
+ *   "walk_warps"         -1 (default), 0 or 1: the plain walk by warps, 32
+ *                        nodes per step for one, two or four neighbouring
+ *                        groups (-1: by the number of groups; 1: always two),
+ *                        or by threads, two per group in the one-pass walk
+ *                        (0), whose lists keep the reference's order. Lists
+ *                        hold the same entries.
  *   "learned_warps"      -1 (default), 0 or 1: the learned walk's rounds by
  *                        warps, one per group (1), or by three threads per
  *                        group with the long walks handed to warps (0, the
- *                        budgets below); -1 picks as "walk_warps" does.
- *   "eval_pairs"         2 (default) or 1: staged pairs each lane of the list
+ *                        budgets below); -1 takes warps below 40000 groups.
+ *   "eval_pairs"         2 (default) or 1: staged entries each lane of the list
  *                        evaluation works per inner iteration (the forces do
  *                        not depend on it; gtc_autotune_eval picks it).
  *   "eval_pass_cost"     whole number 1..256 (default 24): a pass's fixed cost

@@ -241,3 +241,27 @@ def test_tree_solver_galaxy_and_coincident(ctx, oracle, gtc):
     acc, pot = ctx.tree_force(pos, mass, theta=0.75, eps=0.01)
     want, wpot, _ = oracle.tree_force(pos, mass, theta=0.75, eps=0.01)
     assert np.array_equal(acc, want) and np.array_equal(pot, wpot)
+
+
+@pytest.mark.parametrize("theta", [0.05, 0.7])
+@pytest.mark.parametrize("gs", [32, 5, 1])
+@pytest.mark.parametrize("walk", [-1, 1])
+def test_warp_walk_groups_per_warp(gtc, oracle, gs, theta, walk):
+    """About 1200, 5000 and 17003 groups: one, two and four groups to a warp
+    (two always with walk_warps 1), the last ones short of that; theta 0.05 opens
+    nearly everything (long lists, full stacks). Count and fill, then one pass:
+    the oracle's lists and counters both times."""
+    n = 17003 if theta > 0.1 else 3001
+    pos, mass = lopsided_sphere(n, 21)
+    nodes, order, lists = oracle.lists(pos, mass, theta=theta, group_size=gs, leaf_size=4,
+                                       pack=True)
+    with gtc.Context(0) as c:
+        c.set_option("walk_warps", walk)
+        for passes in (2, 1):
+            c.group_force(pos, mass, G=1.0, theta=theta, eps=0.01, group_size=gs, leaf_size=4,
+                          pack=True)
+            dev, st = c.export(), c.stats()
+            assert st["list_passes"] == passes
+            assert compare_lists(dev, dev["nodes"], lists, nodes) == []
+            assert st["cell_interactions"] == lists.stats.cell_interactions
+            assert st["body_interactions"] == lists.stats.body_interactions
