@@ -65,7 +65,7 @@ void Workspace::release_all() {
                          &key2, &tiny, &lcp, &leafdepth, &count, &count_scan, &flags,
                          &flags_scan, &tpos, &tmass, &bodies, &out, &dpos, &dkey, &dkey_alt,
                          &drec, &drec_alt, &dseg, &dtmp, &geom, &mom, &quad, &delta, &nbegin,
-                         &nend, &skip, &parent, &depth, &nchild, &isleaf, &kids, &arrive, &bucket, &walk32, &walk64, &cells,
+                         &nend, &skip, &parent, &depth, &nchild, &isleaf, &kids, &arrive, &bucket, &climb, &qterm, &walk32, &walk64, &cells,
                          &tasks, &gbegin, &gend, &gbox, &gboxf, &gcells, &gbodies, &gcell_off, &gbody_off,
                          &groups, &cell_list, &body_list, &spill, &splitpt, &root, &bbox_part, &scalars, &split, &scan_tmp,
                          &direct_part, &up_arrive, &walk_next, &radix.counts, &radix.scan_tmp};
@@ -333,6 +333,8 @@ void reserve_graph(gtc::Workspace &ws, const gtc::Scalars &hs, double headroom, 
   ws.kids.ensure(m * 8 * sizeof(u32));
   ws.isleaf.ensure(m);
   ws.bucket.ensure(m * 4);
+  ws.climb.ensure(2 * m * sizeof(u32));
+  ws.qterm.ensure(m * 6 * sizeof(double));
   ws.walk32.ensure(m * sizeof(gtc::WalkRec32));
   ws.walk64.ensure(m * sizeof(gtc::WalkRec64));
   ws.cells.ensure(m * 3 * sizeof(float4));

@@ -143,7 +143,7 @@ struct Workspace {
   DeviceBuffer dpos, dkey, dkey_alt, drec, drec_alt, dseg, dtmp;
   // nodes
   DeviceBuffer geom, mom, quad, delta, nbegin, nend, skip, parent, depth, nchild, isleaf, kids,
-      arrive, bucket, walk32, walk64, cells;
+      arrive, bucket, climb, qterm, walk32, walk64, cells;
   // groups and lists
   DeviceBuffer tasks, gbegin, gend, gbox, gboxf, gcells, gbodies, gcell_off, gbody_off, groups, cell_list,
       body_list, spill, splitpt;

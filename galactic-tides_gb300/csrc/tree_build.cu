@@ -962,6 +962,7 @@ struct MomentArrays {
   double2 *mom;     // 2 per node: (mx, my), (mz, mass)
   double2 *quad;    // 3 x double2 per node: xx yy | zz xy | xz yz
   double *delta;
+  double *term;     // 6 per node: what it adds to its parent's quadrupole beside its own
 };
 
 __device__ __forceinline__ Dbl4 load_pair(const double2 *a, u32 p) {
@@ -969,39 +970,91 @@ __device__ __forceinline__ Dbl4 load_pair(const double2 *a, u32 p) {
   return make_dbl4(u.x, u.y, v.x, v.y);
 }
 
-__device__ __forceinline__ void store_pair(double2 *a, u32 p, double x, double y, double z,
-                                           double w) {
-  a[2 * p] = make_double2(x, y);
-  a[2 * p + 1] = make_double2(z, w);
+// The moments in two passes, with the reference's operations in its order:
+// the centres of mass first (all the walk's records need), the quadrupoles
+// after them, from the stored centres of mass. The walk starts after the
+// first pass while the second one runs beside it.
+//
+// FP64 sets the time: the pipe issues one warp instruction in 16 cycles
+// whatever its lanes, with a latency of 64, a division takes 560. So one lane
+// works one component of a node (a centre of mass: x, y, z, mass; a
+// quadrupole: six): the components of a node advance together, and a node's
+// chain is its children's additions and one division.
+//
+// A team of lanes starts from each leaf; the last child of a node to finish
+// hands the node to its own block's queue (a count per node, no waiting), and
+// the block's teams work the queue together, so that the lanes of a warp are
+// full while a block has work. One launch builds the whole tree: with a launch
+// per depth each depth took 9 us (centres of mass) and 15 us (quadrupoles)
+// however few its nodes. Centres of mass with the walk records, then the
+// quadrupoles and cells: 5k bodies 113 -> 40 and 180 -> 53 us, 50k 130 -> 48 and
+// 254 -> 70 us, 2M 358 -> 311 us and, beside the walk, 1.63 -> 1.10 ms.
+__device__ __forceinline__ double *mom_d(const MomentArrays &a) {
+  return reinterpret_cast<double *>(a.mom);
 }
 
-// The moments in two passes, with the reference's operations in its order:
-// the centre of mass and delta first (all the walk's records need), the
-// quadrupole after it, from the stored centre of mass. The walk starts
-// after the first pass while the second one runs beside it.
-__device__ void leaf_com(const MomentArrays &a, u32 p) {  // octree.cpp:46-54, 71
-  const Dbl4 g = load_pair(a.geom, p);
+// A centre of mass and mass by a team of four lanes (component c: x, y, z,
+// mass) from their sums: the mass in lane 3, sums of mass times position in
+// the others (octree.cpp:46-54, 75-85).
+__device__ __forceinline__ void finish_com(const MomentArrays &a, u32 p, int c, double sum,
+                                           u32 team_mask) {
+  const double m = __shfl_sync(team_mask, sum, 3, 4);
+  double v = sum;
+  if (c < 3) v = m > 0 ? sum / m : reinterpret_cast<const double *>(a.geom)[4ull * p + c];
+  mom_d(a)[4ull * p + c] = v;
+}
+
+__device__ __forceinline__ void leaf_com(const MomentArrays &a, u32 p, int c, u32 team_mask) {
   const u32 b0 = a.nbegin[p], b1 = a.nend[p];
-  double m = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
+  double sum = 0.0;
   for (u32 k = b0; k < b1; ++k) {
     const double mi = a.tmass[k];
-    m += mi;
-    cx += mi * a.tpos[3ull * k];
-    cy += mi * a.tpos[3ull * k + 1];
-    cz += mi * a.tpos[3ull * k + 2];
+    const double t = c < 3 ? mi * a.tpos[3ull * k + c] : mi;
+    sum += t;
   }
-  if (m > 0) {
-    cx = cx / m;
-    cy = cy / m;
-    cz = cz / m;
-  } else {
-    cx = g.x;
-    cy = g.y;
-    cz = g.z;
-  }
-  store_pair(a.mom, p, cx, cy, cz, m);
-  const double ex = cx - g.x, ey = cy - g.y, ez = cz - g.z;
-  a.delta[p] = sqrt(ex * ex + ey * ey + ez * ez);
+  finish_com(a, p, c, sum, team_mask);
+}
+
+// A node's children, first octant first (kids lists them last octant first),
+// as many as it has.
+__device__ __forceinline__ int load_kids(const MomentArrays &a, u32 p, u32 ch[8]) {
+  const uint4 k0 = a.kids[2ull * p], k1 = a.kids[2ull * p + 1];
+  ch[0] = k0.x;
+  ch[1] = k0.y;
+  ch[2] = k0.z;
+  ch[3] = k0.w;
+  ch[4] = k1.x;
+  ch[5] = k1.y;
+  ch[6] = k1.z;
+  ch[7] = k1.w;
+  return a.nchild[p];
+}
+
+// Children finished by other blocks of the same launch are read from L2: an
+// SM's L1 may hold an older copy of the line.
+__device__ __forceinline__ void node_com(const MomentArrays &a, u32 p, int c, u32 team_mask) {
+  u32 ch[8];
+  const int nc = load_kids(a, p, ch);
+  double v[8], w[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (j < nc) {
+      w[j] = __ldcg(mom_d(a) + 4ull * ch[j] + 3);
+      v[j] = __ldcg(mom_d(a) + 4ull * ch[j] + c);
+    }
+  double sum = 0.0;
+#pragma unroll
+  for (int j = 7; j >= 0; --j)
+    if (j < nc) {
+      const double t = c < 3 ? w[j] * v[j] : w[j];
+      sum += t;
+    }
+  finish_com(a, p, c, sum, team_mask);
+}
+
+__device__ __forceinline__ double delta_of(const Dbl4 &com, const Dbl4 &g) {  // octree.cpp:71, 101
+  const double ex = com.x - g.x, ey = com.y - g.y, ez = com.z - g.z;
+  return sqrt(ex * ex + ey * ey + ez * ez);
 }
 
 __device__ void leaf_quad(const MomentArrays &a, u32 p) {  // octree.cpp:55-70
@@ -1026,60 +1079,42 @@ __device__ void leaf_quad(const MomentArrays &a, u32 p) {  // octree.cpp:55-70
   a.quad[3 * p + 2] = make_double2(q4, q5);
 }
 
-__device__ void node_com(const MomentArrays &a, u32 p) {  // octree.cpp:75-85, 101
-  const Dbl4 g = load_pair(a.geom, p);
-  const uint4 k0 = a.kids[2ull * p], k1 = a.kids[2ull * p + 1];
-  const u32 ch[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};  // last octant first
-  const int nc = a.nchild[p];
-  double m = 0.0, cx = 0.0, cy = 0.0, cz = 0.0;
-  for (int j = nc - 1; j >= 0; --j) {
-    const Dbl4 c = load_pair(a.mom, ch[j]);
-    m += c.w;
-    cx += c.w * c.x;
-    cy += c.w * c.y;
-    cz += c.w * c.z;
-  }
-  if (m > 0) {
-    cx = cx / m;
-    cy = cy / m;
-    cz = cz / m;
-  } else {
-    cx = g.x;
-    cy = g.y;
-    cz = g.z;
-  }
-  store_pair(a.mom, p, cx, cy, cz, m);
-  const double ex = cx - g.x, ey = cy - g.y, ez = cz - g.z;
-  a.delta[p] = sqrt(ex * ex + ey * ey + ez * ez);
+// What node p adds to its parent's quadrupole beside its own (octree.cpp:86-100:
+// the parallel-axis terms). They need centres of mass only, so every node's
+// are formed at once, and a node's chain is additions.
+__device__ __forceinline__ void quad_term(const MomentArrays &a, u32 p) {
+  const u32 q = a.parent[p];
+  if (q == 0xffffffffu) return;
+  const Dbl4 c = load_pair(a.mom, p), pc = load_pair(a.mom, q);
+  const double dx = c.x - pc.x, dy = c.y - pc.y, dz = c.z - pc.z;
+  const double r2 = dx * dx + dy * dy + dz * dz;
+  double2 *t = reinterpret_cast<double2 *>(a.term + 6ull * p);
+  t[0] = make_double2(c.w * (3 * dx * dx - r2), c.w * (3 * dy * dy - r2));
+  t[1] = make_double2(c.w * (3 * dz * dz - r2), c.w * 3 * dx * dy);
+  t[2] = make_double2(c.w * 3 * dx * dz, c.w * 3 * dy * dz);
 }
 
-__device__ void node_quad(const MomentArrays &a, u32 p) {  // octree.cpp:86-100
-  const Dbl4 pc = load_pair(a.mom, p);
-  const double cx = pc.x, cy = pc.y, cz = pc.z;
-  const uint4 k0 = a.kids[2ull * p], k1 = a.kids[2ull * p + 1];
-  const u32 ch[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
-  const int nc = a.nchild[p];
-  double q0 = 0, q1 = 0, q2 = 0, q3 = 0, q4 = 0, q5 = 0;
-  for (int j = nc - 1; j >= 0; --j) {
-    const Dbl4 c = load_pair(a.mom, ch[j]);
-    const double2 qa = a.quad[3 * ch[j]], qb = a.quad[3 * ch[j] + 1], qc = a.quad[3 * ch[j] + 2];
-    const double dx = c.x - cx, dy = c.y - cy, dz = c.z - cz;
-    const double r2 = dx * dx + dy * dy + dz * dz;
-    q0 += qa.x + c.w * (3 * dx * dx - r2);
-    q1 += qa.y + c.w * (3 * dy * dy - r2);
-    q2 += qb.x + c.w * (3 * dz * dz - r2);
-    q3 += qb.y + c.w * 3 * dx * dy;
-    q4 += qc.x + c.w * 3 * dx * dz;
-    q5 += qc.y + c.w * 3 * dy * dz;
-  }
-  a.quad[3 * p] = make_double2(q0, q1);
-  a.quad[3 * p + 1] = make_double2(q2, q3);
-  a.quad[3 * p + 2] = make_double2(q4, q5);
+// Component c (below 6) of a node's quadrupole from its children's.
+__device__ __forceinline__ void node_quad(const MomentArrays &a, u32 p, int c) {
+  u32 ch[8];
+  const int nc = load_kids(a, p, ch);
+  double *quad = reinterpret_cast<double *>(a.quad);
+  double v[8], t[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (j < nc) {
+      v[j] = __ldcg(quad + 6ull * ch[j] + c);
+      t[j] = a.term[6ull * ch[j] + c];
+    }
+  double sum = 0.0;
+#pragma unroll
+  for (int j = 7; j >= 0; --j)
+    if (j < nc) sum += v[j] + t[j];
+  quad[6ull * p + c] = sum;
 }
 
 // FP32 estimates of the moments, for the learned walk's decisions only: the
-// same sums as the FP64 passes (leaf_com and leaf_quad, node_com and
-// node_quad), in FP32 on the FP32 bodies (relative to the root centre),
+// same sums as the FP64 passes, in FP32 on the FP32 bodies (relative to the root centre),
 // written as GTCell-layout cells plus delta.
 // They take a few tens of microseconds where the FP64 moments take most of a
 // millisecond, so the learned walk starts while the FP64 moments -- which
@@ -1196,156 +1231,177 @@ __device__ void node_moments32(const Moment32Arrays &a, u32 p) {
   finish_moments32(a, p, m, cx, cy, cz, q);
 }
 
-// Moments bottom-up, one launch per depth: leaves first (any depth), then
-// the inner nodes of each depth from the deepest up, so every node's
-// children are complete when it is combined. Nodes are bucketed by depth
-// (bucket kLeafBucket holds the leaves); the order inside a bucket does not
-// matter, each node's sums run in the reference's order.
-// Buckets also split by size -- inner nodes by child count, leaves by body
-// count -- so that the nodes a warp combines loop the same number of times:
-// the FP64 pipe, the bound here, then issues full warps.
-constexpr int kSizeClasses = 8;                          // 1..8 children
+// Leaves are bucketed by body count, so that the leaves a warp sums loop the
+// same number of times: the FP64 pipe, the bound here, then issues full
+// warps. The order inside a bucket does not matter, each leaf's sums run in
+// the reference's order. Small trees go without (kBucketNodes).
 constexpr int kLeafClasses = 9;                          // 1..8 bodies, more
-constexpr int kLeafBucket = (kMaxDepth + 1) * kSizeClasses;  // first leaf bucket
-constexpr int kBuckets = kLeafBucket + kLeafClasses;
+constexpr int kBuckets = kLeafClasses;
 
 struct BucketView {
-  const u8 *depth, *isleaf, *nchild;
+  const u8 *isleaf;
   const u32 *nbegin, *nend;
 };
 
+// A leaf's bucket, -1 for an inner node.
 __device__ __forceinline__ int bucket_of(const BucketView &v, u32 p) {
-  if (v.isleaf[p]) {
-    const u32 nb = v.nend[p] - v.nbegin[p];
-    return kLeafBucket + static_cast<int>(nb < 1 ? 0u : min(nb, static_cast<u32>(kLeafClasses)) - 1);
-  }
-  const int c = v.nchild[p];
-  return v.depth[p] * kSizeClasses + (c < 1 ? 0 : min(c, kSizeClasses) - 1);
+  if (!v.isleaf[p]) return -1;
+  const u32 nb = v.nend[p] - v.nbegin[p];
+  return static_cast<int>(nb < 1 ? 0u : min(nb, static_cast<u32>(kLeafClasses)) - 1);
 }
 
 // Per-block histograms in shared memory, one global atomic per bucket.
 __global__ void __launch_bounds__(kT)
     k_bucket_count(BucketView v, u32 m, u32 *count, const u32 *m_dev = nullptr,
-                   u32 *abort = nullptr, int depth_cap = kMaxDepth) {
+                   const u32 *abort = nullptr) {
   __shared__ u32 h[kBuckets];
   if (aborted(abort)) return;
-  for (int b = threadIdx.x; b < kBuckets; b += kT) h[b] = 0;
+  if (threadIdx.x < kBuckets) h[threadIdx.x] = 0;
   __syncthreads();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (p < bounded(m, m_dev)) {
-    if (abort && !v.isleaf[p] && v.depth[p] > depth_cap) atomicOr(abort, 4u);
-    atomicAdd(&h[bucket_of(v, p)], 1u);
+    const int b = bucket_of(v, p);
+    if (b >= 0) atomicAdd(&h[b], 1u);
   }
   __syncthreads();
-  for (int b = threadIdx.x; b < kBuckets; b += kT)
-    if (h[b]) atomicAdd(&count[b], h[b]);
+  if (threadIdx.x < kBuckets && h[threadIdx.x]) atomicAdd(&count[threadIdx.x], h[threadIdx.x]);
 }
 
-// offsets[b] = start of bucket b; also clears the fill counters.
-constexpr int kBucketThreads = 512;  // one bucket per thread
-static_assert(kBuckets <= kBucketThreads, "bucket scan covers every bucket");
-__global__ void __launch_bounds__(kBucketThreads)
-    k_bucket_offsets(const u32 *count, u32 *offset, u32 *fill, const u32 *abort = nullptr) {
-  __shared__ u32 part[kBucketThreads / 32];
-  if (aborted(abort)) return;  // the same flag for every thread
-  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-  const u32 c = t < kBuckets ? count[t] : 0u;
-  u32 incl = c;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const u32 v = __shfl_up_sync(kFullMask, incl, o);
-    if (lane >= o) incl += v;
-  }
-  if (lane == 31) part[w] = incl;
-  __syncthreads();
-  if (w == 0) {
-    const u32 v = lane < kBucketThreads / 32 ? part[lane] : 0u;
-    u32 pi = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const u32 x = __shfl_up_sync(kFullMask, pi, o);
-      if (lane >= o) pi += x;
-    }
-    if (lane < kBucketThreads / 32) part[lane] = pi - v;
-  }
-  __syncthreads();
-  if (t < kBuckets) {
-    offset[t] = part[w] + incl - c;
-    fill[t] = 0;
-  }
-}
-
-// Each block reserves one range per bucket, then places its nodes in it.
+// Each block reserves one range per bucket behind the buckets before it, then
+// places its leaves there. meta: the counts, then the places taken.
 __global__ void __launch_bounds__(kT)
-    k_bucket_fill(BucketView v, u32 m, const u32 *offset, u32 *fill, u32 *bucket,
-                  const u32 *m_dev = nullptr, const u32 *abort = nullptr) {
+    k_bucket_fill(BucketView v, u32 m, u32 *meta, u32 *bucket, const u32 *m_dev = nullptr,
+                  const u32 *abort = nullptr) {
   __shared__ u32 h[kBuckets], base[kBuckets];
   if (aborted(abort)) return;
-  for (int b = threadIdx.x; b < kBuckets; b += kT) h[b] = 0;
+  if (threadIdx.x < kBuckets) h[threadIdx.x] = 0;
   __syncthreads();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   int b = -1;
   u32 local = 0;
   if (p < bounded(m, m_dev)) {
     b = bucket_of(v, p);
-    local = atomicAdd(&h[b], 1u);
+    if (b >= 0) local = atomicAdd(&h[b], 1u);
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < kBuckets; k += kT)
-    base[k] = h[k] ? offset[k] + atomicAdd(&fill[k], h[k]) : 0;
+  if (threadIdx.x < kBuckets) {
+    u32 first = 0;
+    for (u32 k = 0; k < threadIdx.x; ++k) first += meta[k];
+    base[threadIdx.x] =
+        h[threadIdx.x] ? first + atomicAdd(&meta[kBuckets + threadIdx.x], h[threadIdx.x]) : 0u;
+  }
   __syncthreads();
   if (b >= 0) bucket[base[b] + local] = p;
 }
 
-// kQuad: the quadrupole pass, else the centre-of-mass pass.
-template <bool kQuad>
-__global__ void __launch_bounds__(kT)
-    k_leaf_moments(MomentArrays a, const u32 *bucket, const u32 *meta) {
-  // the leaf buckets' count and first place, from the bucket scan
+__device__ __forceinline__ u32 leaf_count(const u32 *meta) {
   u32 count = 0;
-  for (int b = kLeafBucket; b < kLeafBucket + kLeafClasses; ++b) count += meta[b];
-  const u32 k = blockIdx.x * kT + threadIdx.x;
-  if (k >= count) return;
-  const u32 p = bucket[meta[kBuckets + kLeafBucket] + k];
-  if (kQuad) leaf_quad(a, p);
-  else leaf_com(a, p);
+  for (int b = 0; b < kLeafClasses; ++b) count += meta[b];
+  return count;
 }
 
-// Inner-node moments of one depth: one warp per block, `per` nodes to a
-// warp (lanes past it idle). A depth with few nodes spreads them over many
-// SMs: the sums are FP64-bound, and one SM's FP64 rate took ~40 us for a
-// block of 256 nodes whatever the depth.
-constexpr int kMomentWarps = 1216;  // warps a depth is spread over (8 per SM)
-
-__host__ __device__ __forceinline__ u32 nodes_per_warp(u32 count) {
-  const u32 per = (count + kMomentWarps - 1) / kMomentWarps;
-  return per < 1 ? 1u : (per > 32 ? 32u : per);
+// The k-th leaf: from the buckets, or (bucket null) node k when it is a leaf.
+// kNoNode past the last.
+constexpr u32 kNoNode = 0xffffffffu;
+__device__ __forceinline__ u32 nth_leaf(u64 k, const u32 *bucket, const u32 *meta,
+                                        const u8 *isleaf, u32 m) {
+  if (bucket) return k < leaf_count(meta) ? bucket[k] : kNoNode;
+  return k < m && isleaf[k] ? static_cast<u32>(k) : kNoNode;
 }
 
-// Over the device counts of buckets [b0, b0 + nb) (leaves or one depth's
-// inner nodes), grid-stride over kMomentWarps warps: no count is read back,
-// so the launches of every depth queue at once (eager and graph replays).
+// One more of node q's children is finished (by this thread's warp, whose
+// lanes' values a __syncwarp put before this): its values are visible to
+// whoever counts the last one, and the others' to this thread if it does.
+__device__ __forceinline__ u32 count_arrival(u32 *arrive) {
+  u32 before;
+  asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
+               : "=r"(before)
+               : "l"(arrive)
+               : "memory");
+  return before;
+}
+
+// Bottom-up over the whole tree in one launch (above), by teams of kLanes
+// lanes: the centres of mass (kQuad false) or, the leaves' quadrupoles and the
+// terms being there, the quadrupoles. A block takes per_block leaves (at most
+// kMostLeaves), then the nodes its queue holds, turn by turn; a turn hands over
+// at most as many nodes as it worked. `arrive` counts each node's finished
+// children (zero at the start).
+constexpr u32 kUpThreads = 128;
+constexpr u32 kMostLeaves = 128;
 template <bool kQuad>
-__global__ void __launch_bounds__(32)
-    k_node_moments(MomentArrays a, const u32 *bucket, const u32 *meta, int b0, int nb,
-                   const u32 *abort) {
-  if (*abort) return;
-  u32 count = 0;
-  for (int b = b0; b < b0 + nb; ++b) count += meta[b];
-  const u32 off = meta[kBuckets + b0];
-  const u32 per = nodes_per_warp(count);
-  if (threadIdx.x >= per) return;
-  for (u64 k = static_cast<u64>(blockIdx.x) * per + threadIdx.x; k < count;
-       k += static_cast<u64>(gridDim.x) * per) {
-    const u32 p = bucket[off + k];
-    if (b0 >= kLeafBucket) {
-      if (kQuad) leaf_quad(a, p);
-      else leaf_com(a, p);
-    } else {
-      if (kQuad) node_quad(a, p);
-      else node_com(a, p);
+__global__ void __launch_bounds__(kUpThreads)
+    k_moments_up(MomentArrays a, const u32 *bucket, const u32 *meta, const u8 *isleaf, u32 m,
+                 u32 per_block, u32 *arrive, const u32 *m_dev, const u32 *abort) {
+  constexpr u32 kLanes = kQuad ? 8 : 4;
+  __shared__ u32 queue[2][kMostLeaves];
+  __shared__ u32 queued[2];
+  if (aborted(abort)) return;
+  m = bounded(m, m_dev);
+  const u32 teams = blockDim.x / kLanes, team = threadIdx.x / kLanes;
+  const int c = static_cast<int>(threadIdx.x % kLanes);
+  const u32 team_mask = ((1u << kLanes) - 1u) << (threadIdx.x & 31u & ~(kLanes - 1u));
+  if (threadIdx.x < 2) queued[threadIdx.x] = 0u;
+  __syncthreads();
+  auto hand_over = [&](int next, u32 q, u32 children) {
+    if (q != kNoNode && count_arrival(&arrive[q]) + 1u == children)
+      queue[next][atomicAdd(&queued[next], 1u)] = q;
+  };
+  const u64 first = static_cast<u64>(blockIdx.x) * per_block;
+  if (kQuad) {  // the leaves only count
+    for (u32 i = threadIdx.x; i < per_block; i += blockDim.x) {
+      const u32 p = nth_leaf(first + i, bucket, meta, isleaf, m);
+      if (p == kNoNode) continue;
+      const u32 q = a.parent[p];
+      hand_over(0, q, q != kNoNode ? a.nchild[q] : 0u);
+    }
+  } else {
+    for (u32 i = team; i < per_block; i += teams) {
+      const u32 p = nth_leaf(first + i, bucket, meta, isleaf, m);
+      if (p == kNoNode) continue;
+      const u32 q = a.parent[p], children = q != kNoNode ? a.nchild[q] : 0u;
+      leaf_com(a, p, c, team_mask);
+      __syncwarp(team_mask);
+      if (c == 0) hand_over(0, q, children);
     }
   }
+  for (int turn = 0; turn <= kMaxDepth; ++turn) {
+    const int cur = turn & 1;
+    __syncthreads();  // this turn's queue is complete, the next one's counter clear
+    const u32 count = queued[cur];
+    if (count == 0) return;
+    for (u32 i = team; i < count; i += teams) {
+      const u32 p = queue[cur][i];
+      const u32 q = a.parent[p], children = q != kNoNode ? a.nchild[q] : 0u;
+      if (!kQuad) node_com(a, p, c, team_mask);
+      else if (c < 6) node_quad(a, p, c);
+      __syncwarp(team_mask);
+      if (c == 0) hand_over(cur ^ 1, q, children);
+    }
+    __syncthreads();  // read by all before the counter is used again
+    if (threadIdx.x == 0) queued[cur] = 0u;
+  }
+}
+
+// The leaves' quadrupoles, a thread each.
+constexpr u32 kLeafThreads = 64;  // small blocks: small trees spread over the SMs
+__global__ void __launch_bounds__(kLeafThreads)
+    k_leaf_quads(MomentArrays a, const u32 *bucket, const u32 *meta, const u8 *isleaf, u32 m,
+                 const u32 *m_dev, const u32 *abort) {
+  if (aborted(abort)) return;
+  const u32 p = nth_leaf(static_cast<u64>(blockIdx.x) * kLeafThreads + threadIdx.x, bucket, meta,
+                         isleaf, bounded(m, m_dev));
+  if (p != kNoNode) leaf_quad(a, p);
+}
+
+// Every node's term in its parent's quadrupole; with `deltas` (no walk
+// records, which hold them otherwise) its delta too.
+__global__ void __launch_bounds__(kLeafThreads)
+    k_quad_terms(MomentArrays a, u32 m, bool deltas, const u32 *m_dev, const u32 *abort) {
+  const u32 p = blockIdx.x * kLeafThreads + threadIdx.x;
+  if (aborted(abort) || p >= bounded(m, m_dev)) return;
+  quad_term(a, p);
+  if (deltas) a.delta[p] = delta_of(load_pair(a.mom, p), load_pair(a.geom, p));
 }
 
 // All of the FP32 moments in one launch, bottom-up: a thread per leaf (in
@@ -1358,11 +1414,9 @@ __global__ void __launch_bounds__(32)
 __global__ void __launch_bounds__(kT)
     k_moments32_up(Moment32Arrays a, const u32 *bucket, const u32 *meta, const u32 *parent,
                    u32 *arrive) {
-  u32 count = 0;
-  for (int b = kLeafBucket; b < kLeafBucket + kLeafClasses; ++b) count += meta[b];
   const u32 k = blockIdx.x * kT + threadIdx.x;
-  if (k >= count) return;
-  u32 p = bucket[meta[kBuckets + kLeafBucket] + k];
+  if (k >= leaf_count(meta)) return;
+  u32 p = bucket[k];
   leaf_moments32(a, p);
   for (int step = 0; step <= kMaxDepth; ++step) {
     const u32 q = parent[p];
@@ -1390,11 +1444,11 @@ __global__ void k_check_tree_graph(Scalars *sc, u32 cap, int sorted_levels) {
 
 // --------------------------------------------------------------- packing
 
-// Walk records (FP32 and FP64) of every node (group_lists.cpp:59-61): they
-// need the centres of mass and deltas only, so they are packed after the
+// Walk records (FP32 and FP64) of every node (group_lists.cpp:59-61) and the
+// deltas: they need the centres of mass only, so they are packed after the
 // first moment pass.
 __global__ void __launch_bounds__(kT)
-    k_pack_walk(const double2 *geom, const double2 *mom, const double *delta, const u32 *nbegin,
+    k_pack_walk(const double2 *geom, const double2 *mom, double *delta, const u32 *nbegin,
                 const u32 *nend, const u32 *skip, const u8 *isleaf, u32 m, const TreeRoot *root,
                 double inv_theta, WalkRec32 *walk32, WalkRec64 *walk64,
                 const u32 *m_dev = nullptr, const u32 *abort = nullptr,
@@ -1403,7 +1457,9 @@ __global__ void __launch_bounds__(kT)
   if (aborted(abort) || p >= bounded(m, m_dev)) return;
   if (sys) root += sys[nbegin[p]];  // a forest: relative to the node's system's root
   const Dbl4 g = load_pair(geom, p), c = load_pair(mom, p);
-  const double crit = 2.0 * g.w * inv_theta + delta[p];
+  const double d = delta_of(c, g);
+  delta[p] = d;
+  const double crit = 2.0 * g.w * inv_theta + d;
   WalkRec64 r;
   r.cx = g.x;
   r.cy = g.y;
@@ -1670,6 +1726,90 @@ void pack_bodies_tree(Workspace &ws, u32 n, const TreeRoot *root, const u32 *abo
   }
   GTC_LAUNCH_CHECK();
 }
+
+// A build's moment launches: m nodes (a replay: at most; the count and the
+// abort word on the device).
+struct MomentPlan {
+  MomentArrays ma;
+  const u32 *bucket, *meta;  // null: small trees take their leaves in node order
+  u32 m;
+  u32 *arrive;               // two counts per node, one for each pass
+  const u32 *m_dev, *abort;
+};
+
+// Below this many nodes the three launches that sort the leaves by size cost
+// more than the warps' uneven loops.
+constexpr u32 kBucketNodes = 65536;
+
+u64 arrive_bytes(u64 m) { return 2 * m * sizeof(u32); }
+
+MomentPlan plan_moments(Workspace &ws, u32 m, bool buckets, cudaStream_t s,
+                        const u32 *m_dev = nullptr, const u32 *abort = nullptr) {
+  MomentPlan p{};
+  p.m = m;
+  p.m_dev = m_dev;
+  p.abort = abort;
+  p.ma = MomentArrays{ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
+                      ws.skip.as<u32>(), ws.parent.as<u32>(), ws.nchild.as<u8>(),
+                      ws.kids.as<uint4>(), ws.tpos.as<double>(), ws.tmass.as<double>(),
+                      ws.mom.as<double2>(), ws.quad.as<double2>(), ws.delta.as<double>(),
+                      ws.qterm.as<double>()};
+  p.arrive = ws.climb.as<u32>();
+  GTC_CUDA(cudaMemsetAsync(p.arrive, 0, arrive_bytes(m), s));
+  if (buckets || m >= kBucketNodes) {
+    u32 *meta = ws.arrive.as<u32>(), *bucket = ws.bucket.as<u32>();
+    GTC_CUDA(cudaMemsetAsync(meta, 0, 2 * kBuckets * sizeof(u32), s));
+    const BucketView bv{ws.isleaf.as<u8>(), ws.nbegin.as<u32>(), ws.nend.as<u32>()};
+    k_bucket_count<<<ceil_div(m, kT), kT, 0, s>>>(bv, m, meta, m_dev, abort);
+    GTC_LAUNCH_CHECK();
+    k_bucket_fill<<<ceil_div(m, kT), kT, 0, s>>>(bv, m, meta, bucket, m_dev, abort);
+    GTC_LAUNCH_CHECK();
+    p.bucket = bucket;
+    p.meta = meta;
+  }
+  return p;
+}
+
+// Many leaves to a block keep its queue full on the way up; few spread a
+// small tree over the SMs. (2M: blocks of 512, 256, 128 threads with a leaf per
+// thread take 0.39, 0.33, 0.31 ms for the centres of mass and walk records.)
+template <bool kQuad>
+void launch_up(const Workspace &ws, const MomentPlan &p, u32 *arrive, cudaStream_t s) {
+  const u32 per_block = p.m >= kBucketNodes ? kMostLeaves : 32u;
+  k_moments_up<kQuad><<<ceil_div(p.m, per_block), kUpThreads, 0, s>>>(
+      p.ma, p.bucket, p.meta, ws.isleaf.as<u8>(), p.m, per_block, arrive, p.m_dev, p.abort);
+  GTC_LAUNCH_CHECK();
+}
+
+void launch_coms(const Workspace &ws, const MomentPlan &p, cudaStream_t s) {
+  launch_up<false>(ws, p, p.arrive, s);
+}
+
+void launch_pack_walk(Workspace &ws, const MomentPlan &p, const TreeRoot *root, double theta,
+                      cudaStream_t s) {
+  k_pack_walk<<<ceil_div(p.m, kT), kT, 0, s>>>(
+      ws.geom.as<double2>(), ws.mom.as<double2>(), ws.delta.as<double>(), ws.nbegin.as<u32>(),
+      ws.nend.as<u32>(), ws.skip.as<u32>(), ws.isleaf.as<u8>(), p.m, root, 1.0 / theta,
+      ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), p.m_dev, p.abort, ws.forest.sys);
+  GTC_LAUNCH_CHECK();
+}
+
+// The quadrupoles, from the centres of mass, and the FP32 cells.
+void launch_quads(Workspace &ws, const MomentPlan &p, const TreeRoot *root, bool deltas,
+                  cudaStream_t s) {
+  const u32 blocks = ceil_div(p.m, kLeafThreads);
+  k_leaf_quads<<<blocks, kLeafThreads, 0, s>>>(p.ma, p.bucket, p.meta, ws.isleaf.as<u8>(), p.m,
+                                               p.m_dev, p.abort);
+  GTC_LAUNCH_CHECK();
+  k_quad_terms<<<blocks, kLeafThreads, 0, s>>>(p.ma, p.m, deltas, p.m_dev, p.abort);
+  GTC_LAUNCH_CHECK();
+  launch_up<true>(ws, p, p.arrive + p.m, s);
+  k_pack_cells<<<ceil_div(p.m, kT), kT, 0, s>>>(ws.mom.as<double2>(), ws.quad.as<double2>(),
+                                                ws.nbegin.as<u32>(), p.m, root,
+                                                ws.cells.as<float4>(), p.m_dev, p.abort,
+                                                ws.forest.sys);
+  GTC_LAUNCH_CHECK();
+}
 }  // namespace
 
 void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
@@ -1818,7 +1958,9 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   ws.depth.ensure(m);
   ws.nchild.ensure(m);
   ws.isleaf.ensure(m);
-  ws.arrive.ensure(3 * kBuckets * sizeof(u32));
+  ws.arrive.ensure(2 * kBuckets * sizeof(u32));
+  ws.climb.ensure(arrive_bytes(m));
+  ws.qterm.ensure(m * 6 * sizeof(double));
   ws.bucket.ensure(m * 4ull);
   ws.walk32.ensure(m * sizeof(WalkRec32));
   ws.walk64.ensure(m * sizeof(WalkRec64));
@@ -1842,59 +1984,17 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   GTC_LAUNCH_CHECK();
   ws.stage(Workspace::kStTopo, s);
 
-  // moments, one depth at a time from the leaves up
-  u32 *meta = ws.arrive.as<u32>();  // count[kBuckets], offset[kBuckets], fill[kBuckets]
-  u32 *bucket = ws.bucket.as<u32>();
-  GTC_CUDA(cudaMemsetAsync(meta, 0, kBuckets * sizeof(u32), s));
-  const BucketView bv{ws.depth.as<u8>(), ws.isleaf.as<u8>(), ws.nchild.as<u8>(),
-                      ws.nbegin.as<u32>(), ws.nend.as<u32>()};
-  k_bucket_count<<<mb, kT, 0, s>>>(bv, m, meta);
-  GTC_LAUNCH_CHECK();
-  k_bucket_offsets<<<1, kBucketThreads, 0, s>>>(meta, meta + kBuckets, meta + 2 * kBuckets);
-  GTC_LAUNCH_CHECK();
-  k_bucket_fill<<<mb, kT, 0, s>>>(bv, m, meta + kBuckets, meta + 2 * kBuckets, bucket);
-  GTC_LAUNCH_CHECK();
-  MomentArrays ma{ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
-                  ws.skip.as<u32>(), ws.parent.as<u32>(), ws.nchild.as<u8>(),
-                  ws.kids.as<uint4>(), ws.tpos.as<double>(), ws.tmass.as<double>(),
-                  ws.mom.as<double2>(),
-                  ws.quad.as<double2>(), ws.delta.as<double>()};
-  // the moments and node records on the side stream: the FP64 moments'
-  // small depths leave most SMs idle, and the group choice needs none of
-  // it. Bucket sizes are read on the device: leaves (at most m), then each
-  // depth's inner nodes from the deepest possible one up.
-  // The centres of mass first and the walk records from them (the walk
-  // waits for these only), then the quadrupoles and the cells beside the
-  // walk.
+  // the moments and node records on the side stream, beside the group choice
+  // (which needs none of it): the centres of mass first and the walk records
+  // from them (the walk waits for these only), then the quadrupoles and the
+  // cells beside the walk
+  const MomentPlan mp = plan_moments(ws, m, !walk_records, s);
   cudaStream_t ms = fork_side(ws, s);
   ws.stage(Workspace::kStMom0, ms);
-  k_leaf_moments<false><<<mb, kT, 0, ms>>>(ma, bucket, meta);
-  GTC_LAUNCH_CHECK();
-  for (int d = static_cast<int>(host->depth) - 1; d >= 0; --d) {
-    k_node_moments<false><<<kMomentWarps, 32, 0, ms>>>(ma, bucket, meta, d * kSizeClasses,
-                                                        kSizeClasses, &sc->abort);
-    GTC_LAUNCH_CHECK();
-  }
-  if (walk_records) {
-    k_pack_walk<<<mb, kT, 0, ms>>>(ws.geom.as<double2>(), ws.mom.as<double2>(),
-                                   ws.delta.as<double>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
-                                   ws.skip.as<u32>(), ws.isleaf.as<u8>(), m, root,
-                                   1.0 / sp.theta, ws.walk32.as<WalkRec32>(),
-                                   ws.walk64.as<WalkRec64>(), nullptr, nullptr, fv.sys);
-    GTC_LAUNCH_CHECK();
-  }
+  launch_coms(ws, mp, ms);
+  if (walk_records) launch_pack_walk(ws, mp, root, sp.theta, ms);
   mark_walk_ready(ws, ms);
-  k_leaf_moments<true><<<mb, kT, 0, ms>>>(ma, bucket, meta);
-  GTC_LAUNCH_CHECK();
-  for (int d = static_cast<int>(host->depth) - 1; d >= 0; --d) {
-    k_node_moments<true><<<kMomentWarps, 32, 0, ms>>>(ma, bucket, meta, d * kSizeClasses,
-                                                       kSizeClasses, &sc->abort);
-    GTC_LAUNCH_CHECK();
-  }
-  k_pack_cells<<<mb, kT, 0, ms>>>(ws.mom.as<double2>(), ws.quad.as<double2>(),
-                                  ws.nbegin.as<u32>(), m, root, ws.cells.as<float4>(), nullptr,
-                                  nullptr, fv.sys);
-  GTC_LAUNCH_CHECK();
+  launch_quads(ws, mp, root, !walk_records, ms);
   ws.stage(Workspace::kStMom1, ms);
   pack_bodies_tree(ws, n32, root, nullptr, s);
 }
@@ -1964,53 +2064,13 @@ void build_tree_graph(Workspace &ws, const double *pos, const double *mass, u64 
   k_tree_order<<<nb, kT, 0, s>>>(pos, mass, idx, n32, ws.tpos.as<double>(), ws.tmass.as<double>(),
                                  abort);
   GTC_LAUNCH_CHECK();
-  u32 *meta = ws.arrive.as<u32>();
-  u32 *bucket = ws.bucket.as<u32>();
-  GTC_CUDA(cudaMemsetAsync(meta, 0, kBuckets * sizeof(u32), s));
-  const BucketView bv{ws.depth.as<u8>(), ws.isleaf.as<u8>(), ws.nchild.as<u8>(),
-                      ws.nbegin.as<u32>(), ws.nend.as<u32>()};
-  k_bucket_count<<<mb, kT, 0, s>>>(bv, mcap, meta, m_dev, abort, caps.depth);
-  GTC_LAUNCH_CHECK();
-  k_bucket_offsets<<<1, kBucketThreads, 0, s>>>(meta, meta + kBuckets, meta + 2 * kBuckets, abort);
-  GTC_LAUNCH_CHECK();
-  k_bucket_fill<<<mb, kT, 0, s>>>(bv, mcap, meta + kBuckets, meta + 2 * kBuckets, bucket, m_dev,
-                                  abort);
-  GTC_LAUNCH_CHECK();
-  MomentArrays ma{ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
-                  ws.skip.as<u32>(), ws.parent.as<u32>(), ws.nchild.as<u8>(),
-                  ws.kids.as<uint4>(), ws.tpos.as<double>(), ws.tmass.as<double>(),
-                  ws.mom.as<double2>(),
-                  ws.quad.as<double2>(), ws.delta.as<double>()};
   // the centres of mass and the walk records in line; the quadrupoles and
   // the cells on the side stream, beside the group choice and the walk (the
   // caller joins it before the evaluation)
-  k_node_moments<false><<<kMomentWarps, 32, 0, s>>>(ma, bucket, meta, kLeafBucket, kLeafClasses,
-                                                     abort);
-  GTC_LAUNCH_CHECK();
-  for (int d = std::min(caps.depth, kMaxDepth); d >= 0; --d) {
-    k_node_moments<false><<<kMomentWarps, 32, 0, s>>>(ma, bucket, meta, d * kSizeClasses,
-                                                       kSizeClasses, abort);
-    GTC_LAUNCH_CHECK();
-  }
-  k_pack_walk<<<mb, kT, 0, s>>>(ws.geom.as<double2>(), ws.mom.as<double2>(),
-                                ws.delta.as<double>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
-                                ws.skip.as<u32>(), ws.isleaf.as<u8>(), mcap, root, 1.0 / sp.theta,
-                                ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), m_dev,
-                                abort, fv.sys);
-  GTC_LAUNCH_CHECK();
-  cudaStream_t ms = fork_side(ws, s);
-  k_node_moments<true><<<kMomentWarps, 32, 0, ms>>>(ma, bucket, meta, kLeafBucket, kLeafClasses,
-                                                     abort);
-  GTC_LAUNCH_CHECK();
-  for (int d = std::min(caps.depth, kMaxDepth); d >= 0; --d) {
-    k_node_moments<true><<<kMomentWarps, 32, 0, ms>>>(ma, bucket, meta, d * kSizeClasses,
-                                                      kSizeClasses, abort);
-    GTC_LAUNCH_CHECK();
-  }
-  k_pack_cells<<<mb, kT, 0, ms>>>(ws.mom.as<double2>(), ws.quad.as<double2>(),
-                                  ws.nbegin.as<u32>(), mcap, root, ws.cells.as<float4>(), m_dev,
-                                  abort, fv.sys);
-  GTC_LAUNCH_CHECK();
+  const MomentPlan mp = plan_moments(ws, mcap, false, s, m_dev, abort);
+  launch_coms(ws, mp, s);
+  launch_pack_walk(ws, mp, root, sp.theta, s);
+  launch_quads(ws, mp, root, false, fork_side(ws, s));
   pack_bodies_tree(ws, n32, root, abort, s);
 }
 
