@@ -67,7 +67,7 @@ void Workspace::release_all() {
                          &drec, &drec_alt, &dseg, &dtmp, &geom, &mom, &quad, &delta, &nbegin,
                          &nend, &skip, &parent, &depth, &nchild, &isleaf, &kids, &arrive, &bucket, &climb, &qterm, &walk32, &walk64, &cells,
                          &tasks, &gbegin, &gend, &gbox, &gboxf, &gcells, &gbodies, &gcell_off, &gbody_off,
-                         &groups, &cell_list, &body_list, &spill, &splitpt, &root, &bbox_part, &scalars, &split, &scan_tmp,
+                         &groups, &cell_list, &body_list, &spill, &splitpt, &root, &bbox_part, &bbox_ticket, &scalars, &split, &scan_tmp,
                          &direct_part, &up_arrive, &walk_next, &radix.counts, &radix.scan_tmp};
   for (DeviceBuffer *b : all) b->release();
   if (side) {
@@ -338,7 +338,6 @@ void reserve_graph(gtc::Workspace &ws, const gtc::Scalars &hs, double headroom, 
   ws.walk32.ensure(m * sizeof(gtc::WalkRec32));
   ws.walk64.ensure(m * sizeof(gtc::WalkRec64));
   ws.cells.ensure(m * 3 * sizeof(float4));
-  if (!ws.forest) ws.split.ensure(3ull * gtc::kSplitSize * sizeof(double));  // (a forest steps)
   ws.flags.ensure(std::max<u64>(n, m) * 4);
   ws.flags_scan.ensure(std::max<u64>(n, m) * 4);
   ws.gcells.ensure(2 * n * 8);

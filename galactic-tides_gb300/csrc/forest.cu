@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kT)
 ForestRun::~ForestRun() {
   ws.release_all();
   DeviceBuffer *own[] = {&tables, &sysid, &roots, &root_node, &group_root, &apos, &amass, &stats,
-                         &counter, &split_flags, &sys_groups, &sys_max, &slot_plan, &graph_slots};
+                         &counter, &sys_groups, &sys_max, &slot_plan, &graph_slots};
   for (DeviceBuffer *b : own) b->release();
   if (host_sc) cudaFreeHost(host_sc);
   if (host_lists) cudaFreeHost(host_lists);
@@ -183,7 +183,6 @@ void ForestRun::setup(const std::vector<ForestSystem> &systems, cudaStream_t s) 
   apos.ensure(std::max<u64>(1, n) * 24);
   amass.ensure(std::max<u64>(1, n) * 8);
   stats.ensure(k * sizeof(ForestSystemStats));
-  split_flags.ensure(k * sizeof(u32));
   sys_groups.ensure(k * sizeof(u32));
   sys_max.ensure(4ull * k * sizeof(u32));
   slot_plan.ensure(std::max<u64>(1, n) * 2 * sizeof(uint4));
@@ -195,7 +194,7 @@ void ForestRun::setup(const std::vector<ForestSystem> &systems, cudaStream_t s) 
     GTC_CUDA(cudaMallocHost(reinterpret_cast<void **>(&host_lists), 5ull * k * sizeof(u32)));
     host_systems = k;
   }
-  int T = kLevelsPerWord;
+  int T = kSplitLevels;
   while (T > 1 && 3ull * k * (1ull << T) * sizeof(double) > kSplitBudget) --T;
   counter.ensure(sizeof(u32));
   if (!host_sc) GTC_CUDA(cudaMallocHost(reinterpret_cast<void **>(&host_sc), sizeof(Scalars)));
@@ -213,7 +212,6 @@ void ForestRun::setup(const std::vector<ForestSystem> &systems, cudaStream_t s) 
   fv.sys_blocks = reinterpret_cast<const uint2 *>(t + off_sblk);
   fv.bbox_nblocks = static_cast<u32>(blk.size());
   fv.split_levels = T;
-  fv.split_unsorted = split_flags.as<u32>();
   fv.sys_groups = sys_groups.as<u32>();
   fv.sys_max = sys_max.as<u32>();
   fv.host_groups = host_lists;

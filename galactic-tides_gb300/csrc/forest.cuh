@@ -32,11 +32,11 @@ struct ForestRun {
   SolverParams sp{};            // the shared parameters (group size and packing per system)
   u64 n = 0;                    // bodies in all
   DeviceBuffer tables, sysid, roots, root_node, group_root, apos, amass, stats, counter,
-      split_flags, sys_groups, sys_max, slot_plan, graph_slots;
+      sys_groups, sys_max, slot_plan, graph_slots;
   u32 *host_lists = nullptr;    // pinned: per-system group counts, then list maxima
   u32 host_systems = 0;         // systems host_lists holds
   // Memory for the systems' split tables: each gets levels 0..T-1 (3 x 2^T
-  // doubles), T the most levels (up to the 21 of one key word) within it.
+  // doubles), T the most levels (up to kSplitLevels) within it.
   static constexpr u64 kSplitBudget = 256ull << 20;
   const ForestSystemPtrs *ptrs_dev = nullptr;
   Scalars *host_sc = nullptr;   // pinned

@@ -8,7 +8,7 @@
 //              delta), range [begin, end), skip, parent, depth, children, and
 //              the packed FP32 cell (48 B), FP32 walk record (48 B) and FP64
 //              walk record (64 B) the kernels read.
-//   per axis   the split table: the centres of key levels 0..20, heap order.
+//   per axis   the split table: the centres of levels 0..10, heap order.
 //   per group  target range, FP64 and FP32 boxes, and the 64 B group record
 //              (counts and up to three segments of each list).
 //   lists      cell_list / body_list, uint32 node / body indices: back to
@@ -24,9 +24,9 @@ namespace gtc {
 
 constexpr int kMaxDepth = 60;     // depth cap of the reference octree (octree.cpp:18)
 constexpr int kLevelsPerWord = 21;
-// Levels of the per-axis split-value table of the key kernel (all of the
-// first key word's), and its size per axis (heap order, index 0 unused).
-constexpr int kSplitLevels = kLevelsPerWord;
+// Levels of the per-axis split table node centres are taken from, and its size
+// per axis (heap order, index 0 unused).
+constexpr int kSplitLevels = 11;
 constexpr u32 kSplitSize = 1u << kSplitLevels;
 constexpr u32 kFewBodies = 2;     // accepted cells this small go on the body list (group_lists.h:58)
 constexpr int kMaxGroupSize = 32;
@@ -40,6 +40,10 @@ struct TreeRoot {
   // first level whose node may be "tiny" for some body (from the box: no
   // body's own bound is larger), kMaxDepth + 1 when none is
   int tiny_from;
+  // the keys' grid: 2^20 / half, and how near to a whole number (in 2^-31 cells)
+  // the comparisons with the centres decide instead (~0: always)
+  u32 grid_band;
+  double grid;
 };
 
 // What the grouped walk reads per node. The FP32 record decides almost every
@@ -109,8 +113,7 @@ struct ForestView {
   u32 *host_groups = nullptr;      // pinned copies of both, read back by eager builds
   u32 *host_max = nullptr;
   uint4 *slot_plan = nullptr;      // per group: slot starts, then sizes (per-system slots)
-  int split_levels = 0;            // levels T of each system's split table (2^T per axis)
-  u32 *split_unsorted = nullptr;   // per system: its table's in-order values decrease somewhere
+  int split_levels = 0;            // levels of each system's split table
   const uint4 *bbox_blocks = nullptr;  // bounding-box blocks: (system, rank, blocks, 0)
   const uint2 *sys_blocks = nullptr;   // per system: (first bounding-box block, blocks)
   u32 bbox_nblocks = 0;
@@ -148,7 +151,7 @@ struct Workspace {
   DeviceBuffer tasks, gbegin, gend, gbox, gboxf, gcells, gbodies, gcell_off, gbody_off, groups, cell_list,
       body_list, spill, splitpt;
   // scalars and reductions
-  DeviceBuffer root, bbox_part, scalars, split;
+  DeviceBuffer root, bbox_part, bbox_ticket, scalars, split;
   DeviceBuffer scan_tmp;
   DeviceBuffer direct_part;               // direct sum: per-slice partial sums
   DeviceBuffer up_arrive;                 // bottom-up FP32 moments: children finished, per node
@@ -237,7 +240,6 @@ struct Scalars {
   unsigned long long spill_used[2];  // one-pass walk: overflow pool entries taken (cells, bodies)
   u32 spilled;            // one-pass walk: groups that outgrew their slots
   unsigned long long walk_nodes;  // node records the walk tested
-  u32 split_unsorted;     // the split table's in-order values decrease somewhere (keys step by level)
 };
 
 // The list statistics of one group per lane (valid lanes), summed and
@@ -454,7 +456,8 @@ void launch_fp64_sample(const double *pos, const double *mass, u64 n, const u64 
 // float4 bodies relative to the bounding-box centre (gravity_backends.cpp:15-23, :62).
 void pack_bodies_bbox(Workspace &ws, const double *pos, const double *mass, u64 n,
                       cudaStream_t s);
-void bbox_root(Workspace &ws, const double *pos, u64 n, cudaStream_t s);
+// `split`: the root's split table too.
+void bbox_root(Workspace &ws, const double *pos, u64 n, cudaStream_t s, bool split);
 
 // Throws for a device-detected failure code (Scalars::error; 0: none): bit 4
 // non-finite positions (InvalidArgument), 8 the learned walk's count and fill

@@ -109,10 +109,116 @@ __device__ __forceinline__ double from_order_key(u64 k) {
   return __longlong_as_double(static_cast<long long>((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
 }
 
-// Per-block boxes. Min and max are taken on the order-preserving integer
+// The split table: along an axis the centres of the tree's levels form a binary
+// tree (heap order, node 1 the root centre, the children of node k at level d
+// the centre stepped down and up by half_at[d + 1], with the reference's FP64
+// addition). Node centres (k_nodes) come from the first kSplitLevels levels and
+// are stepped below them (a forest of very many systems: fewer levels each).
+// Built by one block, level by level.
+__device__ void build_split(const double *centre, const double *half_at, int levels,
+                            double *split) {
+  for (int a = static_cast<int>(threadIdx.x); a < 3; a += kT) split[(a << levels) + 1] = centre[a];
+  for (int d = 1; d < levels; ++d) {
+    __syncthreads();
+    const double h = half_at[d];
+    for (u32 j = threadIdx.x; j < 3u << d; j += kT) {
+      double *t = split + (static_cast<u64>(j >> d) << levels);
+      const u32 k = (1u << d) + (j & ((1u << d) - 1u));
+      t[k] = t[k >> 1] + ((k & 1u) ? h : -h);  // step_centre's operation
+    }
+  }
+}
+
+// Root cube from the partial boxes (octree.cpp:184-198; min/max are exact in any
+// order), by one block, and its split table (null: none wanted).
+__device__ void root_from_parts(const double *part, int nparts, TreeRoot *root, int levels,
+                                double *split) {
+  __shared__ double s[kT / 32][6];
+  __shared__ double half_at[kMaxDepth + 1], centre[3], half_s;
+  __shared__ long long tiny_bound;
+  __shared__ int not_tiny[2];
+  double v[6];
+  for (int a = 0; a < 3; ++a) {
+    v[a] = INFINITY;
+    v[3 + a] = -INFINITY;
+  }
+  for (int p = threadIdx.x; p < nparts; p += kT)
+    for (int a = 0; a < 3; ++a) {
+      v[a] = fmin(v[a], __ldcg(part + 6 * p + a));
+      v[3 + a] = fmax(v[3 + a], __ldcg(part + 6 * p + 3 + a));
+    }
+  for (int a = 0; a < 3; ++a)
+    for (int o = 16; o > 0; o >>= 1) {
+      v[a] = fmin(v[a], __shfl_xor_sync(kFullMask, v[a], o));
+      v[3 + a] = fmax(v[3 + a], __shfl_xor_sync(kFullMask, v[3 + a], o));
+    }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0)
+    for (int a = 0; a < 6; ++a) s[warp][a] = v[a];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) {
+      lo[a] = s[0][a];
+      hi[a] = s[0][3 + a];
+      for (int w = 1; w < kT / 32; ++w) {
+        lo[a] = fmin(lo[a], s[w][a]);
+        hi[a] = fmax(hi[a], s[w][3 + a]);
+      }
+    }
+    double half = 0.0, reach = 0.0;
+    for (int a = 0; a < 3; ++a) {
+      root->lo[a] = lo[a];
+      root->hi[a] = hi[a];
+      centre[a] = (lo[a] + hi[a]) * 0.5;
+      root->center[a] = centre[a];
+      const double e = 0.5 * (hi[a] - lo[a]);
+      half = half < e ? e : half;
+      reach = fmax(reach, fabs(centre[a]));
+    }
+    half = half * (1.0 + 1e-9) + 1e-300;
+    half_s = half;
+    // the grid of the keys (grid_rank): its band covers the roundings of the
+    // reference's centres, at most 20 of 2^-53 (|centre| + half) each, and of
+    // the rank itself, in units of 2^-31 cells: 5 (|centre| + half) / half + 1
+    root->grid = static_cast<double>(1 << (kLevelsPerWord - 1)) / half;
+    const double band = 8.0 * ((reach + half) / half) + 8.0;
+    root->grid_band = band < 1e9 && half > 1e-280 ? static_cast<u32>(band) : ~0u;
+    // every body's |x| + |y| + |z| is at most this sum (rounding is monotone),
+    // so no body's tiny bound in k_keys exceeds this one
+    double m1 = 0.0;
+    for (int a = 0; a < 3; ++a) m1 = m1 + fmax(fabs(lo[a]), fabs(hi[a]));
+    tiny_bound = __double_as_longlong(2e-12 * (m1 + 1e-300));
+  }
+  __syncthreads();
+  if (threadIdx.x < 64) {  // (half falls with depth: the levels above the bound come first)
+    const int d = static_cast<int>(threadIdx.x);
+    double h = half_s;
+    if (h > 1e-280) {  // exact: the exponent less d
+      h = __longlong_as_double(__double_as_longlong(h) - (static_cast<long long>(d) << 52));
+    } else {
+      for (int k = 0; k < d; ++k) h = 0.5 * h;
+    }
+    if (d <= kMaxDepth) {
+      half_at[d] = h;
+      root->half_at[d] = h;
+    }
+    const unsigned above =
+        __ballot_sync(kFullMask, d <= kMaxDepth && __double_as_longlong(h) >= tiny_bound);
+    if (lane == 0) not_tiny[warp] = __popc(above);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) root->tiny_from = not_tiny[0] + not_tiny[1];
+  if (split) build_split(centre, half_at, levels, split);
+}
+
+// The bounding box, and from it (the last block to finish) the root cube and
+// its split table. Min and max are taken on the order-preserving integer
 // images (exact, and off the FP64 pipe); with 16-byte aligned positions a
-// thread loads two bodies as three 16-byte words.
-__global__ void __launch_bounds__(kT) k_bbox_partial(const double *pos, u64 n, double *part) {
+// thread loads two bodies as three 16-byte words. `ticket` counts finished
+// blocks and wraps to zero by itself.
+__global__ void __launch_bounds__(kT)
+    k_bbox(const double *pos, u64 n, double *part, u32 *ticket, TreeRoot *root, double *split) {
   const u64 inf_lo = order_key(INFINITY), inf_hi = order_key(-INFINITY);
   u64 lo[3] = {inf_lo, inf_lo, inf_lo}, hi[3] = {inf_hi, inf_hi, inf_hi};
   auto take = [&](int a, double v) {
@@ -161,65 +267,15 @@ __global__ void __launch_bounds__(kT) k_bbox_partial(const double *pos, u64 n, d
       v = threadIdx.x < 3 ? (x < v ? x : v) : (x > v ? x : v);
     }
     part[6 * blockIdx.x + threadIdx.x] = from_order_key(v);
+    __threadfence();
   }
-}
-
-// Root cube from the reduced box (octree.cpp:184-198); min/max are exact in
-// any order, so the partial boxes are reduced by the whole block.
-__device__ void root_from_parts(const double *part, int nparts, TreeRoot *root) {
-  double v[6];
-  for (int a = 0; a < 3; ++a) {
-    v[a] = INFINITY;
-    v[3 + a] = -INFINITY;
-  }
-  for (int p = threadIdx.x; p < nparts; p += kT)
-    for (int a = 0; a < 3; ++a) {
-      v[a] = fmin(v[a], part[6 * p + a]);
-      v[3 + a] = fmax(v[3 + a], part[6 * p + 3 + a]);
-    }
-  for (int a = 0; a < 3; ++a)
-    for (int o = 16; o > 0; o >>= 1) {
-      v[a] = fmin(v[a], __shfl_xor_sync(kFullMask, v[a], o));
-      v[3 + a] = fmax(v[3 + a], __shfl_xor_sync(kFullMask, v[3 + a], o));
-    }
-  __shared__ double s[kT / 32][6];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  if (lane == 0)
-    for (int a = 0; a < 6; ++a) s[warp][a] = v[a];
+  __shared__ bool last;
   __syncthreads();
-  if (threadIdx.x != 0) return;
-  double lo[3], hi[3];
-  for (int a = 0; a < 3; ++a) {
-    lo[a] = s[0][a];
-    hi[a] = s[0][3 + a];
-    for (int w = 1; w < kT / 32; ++w) {
-      lo[a] = fmin(lo[a], s[w][a]);
-      hi[a] = fmax(hi[a], s[w][3 + a]);
-    }
-  }
-  double half = 0.0;
-  for (int a = 0; a < 3; ++a) {
-    root->lo[a] = lo[a];
-    root->hi[a] = hi[a];
-    root->center[a] = (lo[a] + hi[a]) * 0.5;
-    const double e = 0.5 * (hi[a] - lo[a]);
-    half = half < e ? e : half;
-  }
-  half = half * (1.0 + 1e-9) + 1e-300;
-  root->half_at[0] = half;
-  for (int d = 0; d < kMaxDepth; ++d) root->half_at[d + 1] = 0.5 * root->half_at[d];
-  // every body's |x| + |y| + |z| is at most this sum (rounding is monotone),
-  // so no body's tiny bound in k_keys exceeds this one
-  double m1 = 0.0;
-  for (int a = 0; a < 3; ++a) m1 = m1 + fmax(fabs(lo[a]), fabs(hi[a]));
-  const long long bound = __double_as_longlong(2e-12 * (m1 + 1e-300));
-  int d = 0;
-  while (d <= kMaxDepth && __double_as_longlong(root->half_at[d]) >= bound) ++d;
-  root->tiny_from = d;
-}
-
-__global__ void __launch_bounds__(kT) k_root(const double *part, int nparts, TreeRoot *root) {
-  root_from_parts(part, nparts, root);
+  if (threadIdx.x == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  root_from_parts(part, static_cast<int>(gridDim.x), root, kSplitLevels, split);
 }
 
 // A forest's boxes: block b covers part of system blk[b].x (rank blk[b].y of
@@ -265,94 +321,15 @@ __global__ void __launch_bounds__(kT)
 }
 
 __global__ void __launch_bounds__(kT)
-    k_root_forest(const double *part, const uint2 *sys_blk, TreeRoot *roots) {
+    k_root_forest(const double *part, const uint2 *sys_blk, TreeRoot *roots, int levels,
+                  double *split) {
   const uint2 q = sys_blk[blockIdx.x];
-  root_from_parts(part + 6ull * q.x, static_cast<int>(q.y), roots + blockIdx.x);
+  root_from_parts(part + 6ull * q.x, static_cast<int>(q.y), roots + blockIdx.x, levels,
+                  split + (static_cast<u64>(3u * blockIdx.x) << levels));
 }
 
 // ------------------------------------------------------------------- keys
 
-
-// Split values. Along one axis the centre a body's walk compares against at
-// level d depends only on the body's first d bits on that axis: the centres
-// of all levels form a binary tree per axis (heap order, node 1 the root
-// centre, the children of node k at level d the centre stepped down and up
-// by half_at[d + 1], with the reference's FP64 addition). A body's key bits
-// on an axis are then a binary search in that tree. The table holds levels
-// 0..kSplitLevels - 1 (2^kSplitLevels - 1 values per axis), built once per
-// tree instead of once per body; the levels below are stepped per body.
-constexpr int kSplitTop = 11;                    // levels one block per axis builds
-
-// Levels 0..kSplitTop - 1, one block per axis, level by level.
-__global__ void __launch_bounds__(1024) k_split_top(const TreeRoot *root, double *split) {
-  const int axis = blockIdx.x;
-  double *t = split + static_cast<u64>(axis) * kSplitSize;
-  if (threadIdx.x == 0) t[1] = root->center[axis];
-  __syncthreads();
-  for (int d = 1; d < kSplitTop; ++d) {
-    const double h = root->half_at[d];
-    for (u32 j = threadIdx.x; j < (1u << d); j += blockDim.x) {
-      const u32 k = (1u << d) + j;
-      const double c = t[k >> 1];
-      t[k] = c + ((k & 1u) ? h : -h);  // step_centre's operation
-    }
-    __syncthreads();
-  }
-}
-
-// `Levels` levels below level `from`: one thread per node of level `from`
-// builds its subtree in registers, level by level, and stores it.
-template <int Levels>
-__global__ void __launch_bounds__(kT) k_split_sub(const TreeRoot *root, double *split, int from) {
-  const u32 per_axis = 1u << from;
-  const u32 tid = blockIdx.x * kT + threadIdx.x;
-  if (tid >= 3 * per_axis) return;
-  double *t = split + static_cast<u64>(tid / per_axis) * kSplitSize;
-  const u32 base = per_axis + tid % per_axis;  // heap index at level `from`
-  double v[2 << Levels];                        // v[1] the subtree's root, heap order below
-  v[1] = t[base];
-#pragma unroll
-  for (int l = 1; l <= Levels; ++l) {
-    const double h = root->half_at[from + l];
-#pragma unroll
-    for (int j = 0; j < (1 << l); ++j) {
-      const int k = (1 << l) + j;
-      v[k] = v[k >> 1] + ((k & 1) ? h : -h);
-      t[(static_cast<u64>(base) << l) + j] = v[k];
-    }
-  }
-}
-
-// The table in order. Along an axis, the split values in in-order (heap
-// node 2^d + m of level d at in-order position (2m + 1) 2^(kSplitLevels - 1
-// - d) - 1). When they never decrease, a body's path through the table is
-// the rank of its coordinate among them: the number of values <= x, whose
-// kSplitLevels bits are the path's level-0.. bits (up iff x >= the centre),
-// the path's deepest centre being the value at the rank with its last bit
-// cleared.
-constexpr u32 kSplitValues = kSplitSize - 1;  // per axis: heap nodes 1..kSplitSize - 1
-
-// Heap index of in-order position p.
-__device__ __forceinline__ u32 split_heap(u32 p) {
-  const u32 q = p + 1;
-  const int tz = __ffs(q) - 1;
-  return (1u << (kSplitLevels - 1 - tz)) + (q >> (tz + 1));
-}
-
-// In-order neighbours come in (leaf, inner node) pairs, leaves at the even
-// positions: each leaf against the values on either side of it.
-__global__ void __launch_bounds__(kT) k_split_check(const double *split, u32 *unsorted) {
-  constexpr u32 kLeaves = 1u << (kSplitLevels - 1);
-  const u32 t = blockIdx.x * kT + threadIdx.x;
-  if (t >= 3 * kLeaves) return;
-  const double *s = split + static_cast<u64>(t / kLeaves) * kSplitSize;
-  const u32 j = t % kLeaves, p = 2 * j;
-  const u64 v = order_key(s[kLeaves + j]);
-  bool bad = false;
-  if (j > 0) bad |= order_key(s[split_heap(p - 1)]) > v;
-  if (p + 1 < kSplitValues) bad |= v > order_key(s[split_heap(p + 1)]);
-  if (bad) atomicOr(unsorted, 1u);
-}
 
 // Bits b of v at bit 3b (v < 2^21).
 __device__ __forceinline__ u64 spread3(u64 v) {
@@ -365,31 +342,33 @@ __device__ __forceinline__ u64 spread3(u64 v) {
   return v;
 }
 
-// Rank of kx among an axis's in-order values: a guess from the grid the
-// values lie on (1 / inv_w apart), then moved until the values on either
-// side bracket kx. False if that takes more than a few steps.
-__device__ __forceinline__ bool split_rank(const double *table, u64 kx, double x,
-                                           double lo_edge, float inv_w, u32 &r) {
-  const float g = static_cast<float>(x - lo_edge) * inv_w;
-  int v = g > 0.f ? static_cast<int>(fminf(g, static_cast<float>(kSplitValues))) : 0;
-  for (int it = 0; it < 4; ++it) {
-    if (v > 0 && kx < order_key(__ldg(table + split_heap(v - 1)))) {
-      --v;
-    } else if (v < static_cast<int>(kSplitValues) && kx >= order_key(__ldg(table + split_heap(v)))) {
-      ++v;
-    } else {
-      r = static_cast<u32>(v);
-      return true;
-    }
-  }
-  return false;
+// The first kLevelsPerWord path bits of coordinate x on an axis: up at level d
+// iff x >= the centre of level d on the path. But for the roundings of the
+// centres, all 2^21 - 1 of them lie on a grid of spacing half / 2^20 about the
+// root centre, so the bits are those of x's place on it, the whole part of
+// (x - centre) / spacing + 2^20; adding 2^21 puts that into the top 21 mantissa
+// bits, with 31 bits of fraction below. Where the fraction is nearer to a
+// whole number than the roundings reach (grid_band), the answer is left open.
+__device__ __forceinline__ bool grid_rank(double x, double centre, double grid, u32 band,
+                                          u64 &bits) {
+  constexpr int kFraction = 52 - kLevelsPerWord;
+  const double t = __fma_rn(x - centre, grid, static_cast<double>(3u << (kLevelsPerWord - 1)));
+  const u64 b = static_cast<u64>(__double_as_longlong(t));
+  const u32 f = static_cast<u32>(b) & ((1u << kFraction) - 1u);
+  bits = (b >> kFraction) & ((1ull << kLevelsPerWord) - 1ull);
+  return (b >> 52) == 1023u + kLevelsPerWord && f >= band && f <= (1u << kFraction) - band;
 }
 
 // First key word: levels 1..21 from the root; records the first depth whose
 // node is "tiny" (a leaf whatever its count). Digits below a tiny node are 0,
-// so bodies of such a leaf stay in input order through the sort. The centres
-// of the first kSplitLevels levels come from the split table; the rest are
-// stepped as the reference does.
+// so bodies of such a leaf stay in input order through the sort.
+//
+// Two FP64 operations per axis (grid_rank) where no level can be tiny and no
+// coordinate lies within the roundings of a centre; else, about one body in
+// 10^7 for a box near the origin, the reference's comparisons level by level.
+// (A table of all 2^21 centres per axis took four launches and 60 us a call
+// to build and check, and 67 us to look up at 2M bodies: box, table and keys
+// 90 -> 22 us at 5k, 161 -> 71 us at 2M.)
 //
 // A node holding body p has |centre|_1 <= |p|_1 + 3 half (plus rounding), so
 // it can only be tiny once half < 1e-12 (|p|_1 + 3 half + 1e-300), i.e. once
@@ -397,244 +376,45 @@ __device__ __forceinline__ bool split_rank(const double *table, u64 kx, double x
 // twice that bound skip the exact FP64 test; the comparison of two positive
 // doubles is done on their bit patterns.
 __global__ void __launch_bounds__(kT)
-    k_keys(const double *pos, u32 n, const TreeRoot *root, const double *split,
-           const u32 *unsorted, u64 *key, u32 *idx, u8 *tiny, u32 *error) {
-  __shared__ double half_at[kLevelsPerWord + 1];
-  __shared__ float inv_spacing;  // 1 / the spacing of the table's deepest values
-  if (threadIdx.x <= kLevelsPerWord) half_at[threadIdx.x] = root->half_at[threadIdx.x];
-  if (threadIdx.x == 0) inv_spacing = static_cast<float>(1.0 / root->half_at[kSplitLevels - 1]);
-  __syncthreads();
-  const bool by_rank = *unsorted == 0;
+    k_keys(const double *pos, u32 n, const u16 *sys, const TreeRoot *roots, u64 *key, u32 *idx,
+           u8 *tiny, u32 *error) {
   const u32 i = blockIdx.x * kT + threadIdx.x;
   if (i >= n) return;
+  const TreeRoot *root = roots + (sys ? sys[i] : 0);  // (a forest: the body's system's)
   const double x = pos[3ull * i], y = pos[3ull * i + 1], z = pos[3ull * i + 2];
   if (!isfinite(x) || !isfinite(y) || !isfinite(z)) atomicOr(error, 4u);
-  const u64 kx = order_key(x), ky = order_key(y), kz = order_key(z);
-  // the first level whose node could be tiny for this body (half_at falls
-  // with depth): the levels above it need no tiny test at all
-  int dt = root->tiny_from;
-  if (dt <= kLevelsPerWord) {
+  const double ox = root->center[0], oy = root->center[1], oz = root->center[2];
+  const double grid = root->grid;
+  const u32 band = root->grid_band;
+  u64 k = 0, rx, ry, rz;
+  int t = kNoTiny;
+  if (root->tiny_from > kLevelsPerWord && band != ~0u && grid_rank(x, ox, grid, band, rx) &&
+      grid_rank(y, oy, grid, band, ry) && grid_rank(z, oz, grid, band, rz)) {
+    k = spread3(rx) | (spread3(ry) << 1) | (spread3(rz) << 2);
+  } else {
+    // the first level whose node could be tiny for this body (half_at falls
+    // with depth): the levels above it need no tiny test at all
     const long long maybe_tiny =
         __double_as_longlong(2e-12 * (fabs(x) + fabs(y) + fabs(z) + 1e-300));
-    dt = 0;
-    while (dt <= kLevelsPerWord && __double_as_longlong(half_at[dt]) >= maybe_tiny) ++dt;
+    int dt = root->tiny_from;
+    if (dt <= kLevelsPerWord) {
+      dt = 0;
+      while (dt <= kLevelsPerWord && __double_as_longlong(root->half_at[dt]) >= maybe_tiny) ++dt;
+    }
+    const u64 kx = order_key(x), ky = order_key(y), kz = order_key(z);
+    double cx = ox, cy = oy, cz = oz;
+    for (int d = 0; d < kLevelsPerWord; ++d) {
+      if (d >= dt && t == kNoTiny && tiny_node(root->half_at[d], cx, cy, cz)) t = d;
+      int o = (kx >= order_key(cx) ? 1 : 0) | (ky >= order_key(cy) ? 2 : 0) |
+              (kz >= order_key(cz) ? 4 : 0);
+      if (t != kNoTiny) o = 0;
+      k = (k << 3) | static_cast<u64>(o);
+      step_centre(cx, cy, cz, o, root->half_at[d + 1]);
+    }
+    if (dt <= kLevelsPerWord && t == kNoTiny &&
+        tiny_node(root->half_at[kLevelsPerWord], cx, cy, cz))
+      t = kLevelsPerWord;
   }
-  const double *tx = split, *ty = split + kSplitSize, *tz = split + 2ull * kSplitSize;
-  u32 ix = 1, iy = 1, iz = 1;
-  double cx = 0.0, cy = 0.0, cz = 0.0;
-  u64 k = 0;
-  int t = kNoTiny;
-  // level d: its centre (table, or stepped below the table), the tiny test
-  // where it can apply, the digit, and the next level's index or centre
-  auto level = [&](int d, bool test) {
-    if (d < kSplitLevels) {
-      cx = __ldg(tx + ix);
-      cy = __ldg(ty + iy);
-      cz = __ldg(tz + iz);
-    }
-    if (test && t == kNoTiny && tiny_node(half_at[d], cx, cy, cz)) t = d;
-    int o = (kx >= order_key(cx) ? 1 : 0) | (ky >= order_key(cy) ? 2 : 0) |
-            (kz >= order_key(cz) ? 4 : 0);
-    if (t != kNoTiny) o = 0;
-    k = (k << 3) | static_cast<u64>(o);
-    if (d + 1 < kSplitLevels) {
-      ix = 2 * ix + (o & 1);
-      iy = 2 * iy + ((o >> 1) & 1);
-      iz = 2 * iz + (o >> 2);
-    } else {
-      step_centre(cx, cy, cz, o, half_at[d + 1]);
-    }
-  };
-  int d = 0;
-  if (by_rank && dt >= kSplitLevels) {
-    // no tiny test within the table's levels: its levels by rank
-    const float inv_w = inv_spacing;
-    u32 rx, ry, rz;
-    if (split_rank(tx, kx, x, root->center[0] - half_at[0], inv_w, rx) &&
-        split_rank(ty, ky, y, root->center[1] - half_at[0], inv_w, ry) &&
-        split_rank(tz, kz, z, root->center[2] - half_at[0], inv_w, rz)) {
-      k = spread3(rx) | (spread3(ry) << 1) | (spread3(rz) << 2);
-      if (dt <= kLevelsPerWord) {  // the centre below the table, for the last tiny test
-        constexpr u32 kLeaves = 1u << (kSplitLevels - 1);
-        cx = __ldg(tx + kLeaves + (rx >> 1));
-        cy = __ldg(ty + kLeaves + (ry >> 1));
-        cz = __ldg(tz + kLeaves + (rz >> 1));
-        const int o = static_cast<int>((rx & 1u) | ((ry & 1u) << 1) | ((rz & 1u) << 2));
-        step_centre(cx, cy, cz, o, half_at[kSplitLevels]);
-      }
-      d = kSplitLevels;
-    }
-  }
-  for (; d < kLevelsPerWord && d < dt; ++d) level(d, false);
-  for (; d < kLevelsPerWord; ++d) level(d, true);
-  if (dt <= kLevelsPerWord && t == kNoTiny && tiny_node(half_at[kLevelsPerWord], cx, cy, cz))
-    t = kLevelsPerWord;
-  key[i] = k;
-  idx[i] = i;
-  tiny[i] = static_cast<u8>(t);
-}
-
-// A forest's split tables: per system and axis, levels 0..T-1 of the same
-// table as above (heap order, 2^T entries, the system's own root), T set by
-// the forest's memory budget. Built by the same operations as the
-// single-system table: levels 0..min(T, kSplitTop)-1 by one block per
-// (system, axis), the rest by subtrees of 4, 2 or 1 levels.
-__global__ void __launch_bounds__(1024)
-    k_split_top_forest(const TreeRoot *roots, double *split, u32 size, int top) {
-  const u32 sa = blockIdx.x;  // system * 3 + axis
-  const TreeRoot *root = roots + sa / 3;
-  double *t = split + static_cast<u64>(sa) * size;
-  if (threadIdx.x == 0) t[1] = root->center[sa % 3];
-  __syncthreads();
-  for (int d = 1; d < top; ++d) {
-    const double h = root->half_at[d];
-    for (u32 j = threadIdx.x; j < (1u << d); j += blockDim.x) {
-      const u32 k = (1u << d) + j;
-      const double c = t[k >> 1];
-      t[k] = c + ((k & 1u) ? h : -h);  // step_centre's operation
-    }
-    __syncthreads();
-  }
-}
-
-template <int Levels>
-__global__ void __launch_bounds__(kT)
-    k_split_sub_forest(const TreeRoot *roots, double *split, u32 size, u32 tables, int from) {
-  const u32 per_axis = 1u << from;
-  const u64 tid = static_cast<u64>(blockIdx.x) * kT + threadIdx.x;
-  if (tid >= static_cast<u64>(tables) * per_axis) return;
-  const u32 sa = static_cast<u32>(tid / per_axis);
-  const TreeRoot *root = roots + sa / 3;
-  double *t = split + static_cast<u64>(sa) * size;
-  const u32 base = per_axis + static_cast<u32>(tid % per_axis);
-  double v[2 << Levels];
-  v[1] = t[base];
-#pragma unroll
-  for (int l = 1; l <= Levels; ++l) {
-    const double h = root->half_at[from + l];
-#pragma unroll
-    for (int j = 0; j < (1 << l); ++j) {
-      const int k = (1 << l) + j;
-      v[k] = v[k >> 1] + ((k & 1) ? h : -h);
-      t[(static_cast<u64>(base) << l) + j] = v[k];
-    }
-  }
-}
-
-// Heap index of in-order position p in a table of `levels` levels.
-__device__ __forceinline__ u32 split_heap_at(u32 p, int levels) {
-  const u32 q = p + 1;
-  const int tz = __ffs(q) - 1;
-  return (1u << (levels - 1 - tz)) + (q >> (tz + 1));
-}
-
-// k_split_check per (system, axis) table; a system whose in-order values
-// decrease somewhere gets its flag set (its keys then walk the table level
-// by level).
-__global__ void __launch_bounds__(kT)
-    k_split_check_forest(const double *split, u32 size, int levels, u32 tables, u32 *unsorted) {
-  const u32 leaves = 1u << (levels - 1);
-  const u64 t = static_cast<u64>(blockIdx.x) * kT + threadIdx.x;
-  if (t >= static_cast<u64>(tables) * leaves) return;
-  const u32 sa = static_cast<u32>(t / leaves);
-  const double *s = split + static_cast<u64>(sa) * size;
-  const u32 j = static_cast<u32>(t % leaves), p = 2 * j, values = size - 1;
-  const u64 v = order_key(s[leaves + j]);
-  bool bad = false;
-  if (j > 0) bad |= order_key(s[split_heap_at(p - 1, levels)]) > v;
-  if (p + 1 < values) bad |= v > order_key(s[split_heap_at(p + 1, levels)]);
-  if (bad) atomicOr(unsorted + sa / 3, 1u);
-}
-
-// split_rank on a table of `levels` levels (values = 2^levels - 1).
-__device__ __forceinline__ bool split_rank_at(const double *table, u64 kx, double x,
-                                              double lo_edge, float inv_w, int levels,
-                                              u32 &r) {
-  const u32 values = (1u << levels) - 1;
-  const float g = static_cast<float>(x - lo_edge) * inv_w;
-  int v = g > 0.f ? static_cast<int>(fminf(g, static_cast<float>(values))) : 0;
-  for (int it = 0; it < 4; ++it) {
-    if (v > 0 && kx < order_key(__ldg(table + split_heap_at(v - 1, levels)))) {
-      --v;
-    } else if (v < static_cast<int>(values) &&
-               kx >= order_key(__ldg(table + split_heap_at(v, levels)))) {
-      ++v;
-    } else {
-      r = static_cast<u32>(v);
-      return true;
-    }
-  }
-  return false;
-}
-
-// A forest's first key word: k_keys with each body's own system's root and
-// table of T levels (levels below T stepped as the reference does).
-__global__ void __launch_bounds__(kT)
-    k_keys_forest(const double *pos, u32 n, const u16 *sys, const TreeRoot *roots,
-                  const double *split, u32 size, int T, const u32 *unsorted, u64 *key, u32 *idx,
-                  u8 *tiny, u32 *error) {
-  const u32 i = blockIdx.x * kT + threadIdx.x;
-  if (i >= n) return;
-  const u32 s = sys[i];
-  const TreeRoot *root = roots + s;
-  const double *half_at = root->half_at;
-  const double x = pos[3ull * i], y = pos[3ull * i + 1], z = pos[3ull * i + 2];
-  if (!isfinite(x) || !isfinite(y) || !isfinite(z)) atomicOr(error, 4u);
-  const u64 kx = order_key(x), ky = order_key(y), kz = order_key(z);
-  int dt = root->tiny_from;
-  if (dt <= kLevelsPerWord) {
-    const long long maybe_tiny =
-        __double_as_longlong(2e-12 * (fabs(x) + fabs(y) + fabs(z) + 1e-300));
-    dt = 0;
-    while (dt <= kLevelsPerWord && __double_as_longlong(half_at[dt]) >= maybe_tiny) ++dt;
-  }
-  const double *tx = split + 3ull * s * size, *ty = tx + size, *tz = ty + size;
-  u32 ix = 1, iy = 1, iz = 1;
-  double cx = 0.0, cy = 0.0, cz = 0.0;
-  u64 k = 0;
-  int t = kNoTiny;
-  auto level = [&](int d, bool test) {
-    if (d < T) {
-      cx = __ldg(tx + ix);
-      cy = __ldg(ty + iy);
-      cz = __ldg(tz + iz);
-    }
-    if (test && t == kNoTiny && tiny_node(half_at[d], cx, cy, cz)) t = d;
-    int o = (kx >= order_key(cx) ? 1 : 0) | (ky >= order_key(cy) ? 2 : 0) |
-            (kz >= order_key(cz) ? 4 : 0);
-    if (t != kNoTiny) o = 0;
-    k = (k << 3) | static_cast<u64>(o);
-    if (d + 1 < T) {
-      ix = 2 * ix + (o & 1);
-      iy = 2 * iy + ((o >> 1) & 1);
-      iz = 2 * iz + (o >> 2);
-    } else {
-      step_centre(cx, cy, cz, o, half_at[d + 1]);
-    }
-  };
-  int d = 0;
-  if (unsorted[s] == 0 && dt >= T) {
-    // no tiny test within the table's levels: its levels by rank, then the
-    // centre of level T (the path's deepest table centre, stepped once)
-    const float inv_w = 1.0f / static_cast<float>(half_at[T - 1]);
-    u32 rx, ry, rz;
-    if (split_rank_at(tx, kx, x, root->center[0] - half_at[0], inv_w, T, rx) &&
-        split_rank_at(ty, ky, y, root->center[1] - half_at[0], inv_w, T, ry) &&
-        split_rank_at(tz, kz, z, root->center[2] - half_at[0], inv_w, T, rz)) {
-      k = spread3(rx) | (spread3(ry) << 1) | (spread3(rz) << 2);
-      const u32 leaves = 1u << (T - 1);
-      cx = __ldg(tx + leaves + (rx >> 1));
-      cy = __ldg(ty + leaves + (ry >> 1));
-      cz = __ldg(tz + leaves + (rz >> 1));
-      const int o = static_cast<int>((rx & 1u) | ((ry & 1u) << 1) | ((rz & 1u) << 2));
-      step_centre(cx, cy, cz, o, half_at[T]);
-      d = T;
-    }
-  }
-  for (; d < kLevelsPerWord && d < dt; ++d) level(d, false);
-  for (; d < kLevelsPerWord; ++d) level(d, true);
-  if (dt <= kLevelsPerWord && t == kNoTiny && tiny_node(half_at[kLevelsPerWord], cx, cy, cz))
-    t = kLevelsPerWord;
   key[i] = k;
   idx[i] = i;
   tiny[i] = static_cast<u8>(t);
@@ -665,10 +445,11 @@ __global__ void __launch_bounds__(kT)
   idx[k] = idx_copy[j];
 }
 
-// Per sorted position: levels shared with the next body, and the leaf depth.
+// Per sorted position: levels shared with the next body, the leaf depth, and
+// the number of nodes that end there.
 __global__ void __launch_bounds__(kT)
     k_levels(KeyView kv, const u32 *idx, const u8 *tiny, u32 n, int L, signed char *lcp_next,
-             u8 *leafdepth, Scalars *sc) {
+             u8 *leafdepth, u32 *count, Scalars *sc) {
   // win[i] = lcp(i, i + L) for the block's positions and the L before them,
   // each computed once; a body's w is the largest over its windows
   constexpr int kMaxWin = 64;
@@ -685,7 +466,8 @@ __global__ void __launch_bounds__(kT)
   }
   int ld = 0;
   if (b < n) {
-    lcp_next[b] = static_cast<signed char>(b + 1 < n ? lcp(kv, b, b + 1) : -1);
+    const int next = b + 1 < n ? lcp(kv, b, b + 1) : -1;
+    lcp_next[b] = static_cast<signed char>(next);
     int w = -1;
     if (n > static_cast<u32>(L)) {
       const u32 lo = b >= static_cast<u32>(L) ? b - L : 0;
@@ -696,6 +478,7 @@ __global__ void __launch_bounds__(kT)
     ld = min(w + 1, kMaxDepth);
     ld = min(ld, static_cast<int>(tiny[idx[b]]));
     leafdepth[b] = static_cast<u8>(ld);
+    count[b] = static_cast<u32>(max(0, ld - next));  // the nodes that end at b
   }
   // one atomic per warp for each counter
   const u32 deep = __popc(__ballot_sync(kFullMask, b < n && ld > kLevelsPerWord * kv.words));
@@ -790,21 +573,13 @@ __global__ void __launch_bounds__(kT)
 
 // ------------------------------------------------------------------ nodes
 
-__global__ void __launch_bounds__(kT)
-    k_node_count(const signed char *lcp_next, const u8 *leafdepth, u32 n, u32 *count,
-                 const u32 *abort = nullptr) {
-  const u32 b = blockIdx.x * kT + threadIdx.x;
-  if (aborted(abort)) return;
-  if (b < n) count[b] = static_cast<u32>(max(0, static_cast<int>(leafdepth[b]) - lcp_next[b]));
-}
-
 // Writes the nodes ending at sorted position b, shallowest first.
 __global__ void __launch_bounds__(kT)
     k_nodes(KeyView kv, const signed char *lcp_next, const u8 *leafdepth, const u32 *count,
             const u32 *count_scan, u32 n, const Scalars *sc, const TreeRoot *root,
             const double *split, double2 *geom, u32 *nbegin, u32 *nend, u32 *skip, u8 *depth,
-            u8 *isleaf, const u32 *abort = nullptr, u32 table_size = kSplitSize,
-            int table_levels = kSplitLevels) {
+            u8 *isleaf, int table_levels, const u32 *abort = nullptr) {
+  const u32 table_size = 1u << table_levels;
   const u32 b = blockIdx.x * kT + threadIdx.x;
   if (b >= n || aborted(abort)) return;
   const u32 c = count[b];
@@ -1545,19 +1320,23 @@ void read_scalars(Workspace &ws, Scalars *host, cudaStream_t s) {
 
 }  // namespace
 
-void bbox_root(Workspace &ws, const double *pos, u64 n, cudaStream_t s) {
+void bbox_root(Workspace &ws, const double *pos, u64 n, cudaStream_t s, bool split) {
   const u32 nparts = std::min<u32>(1024, std::max<u32>(1, ceil_div(n, kT)));
   ws.bbox_part.ensure(6 * sizeof(double) * nparts);
   ws.root.ensure(sizeof(TreeRoot));
-  k_bbox_partial<<<nparts, kT, 0, s>>>(pos, n, ws.bbox_part.as<double>());
-  GTC_LAUNCH_CHECK();
-  k_root<<<1, kT, 0, s>>>(ws.bbox_part.as<double>(), static_cast<int>(nparts), ws.root.as<TreeRoot>());
+  if (!ws.bbox_ticket.ptr) {
+    ws.bbox_ticket.ensure(sizeof(u32));
+    GTC_CUDA(cudaMemsetAsync(ws.bbox_ticket.ptr, 0, sizeof(u32), s));
+  }
+  if (split) ws.split.ensure(3ull * kSplitSize * sizeof(double));
+  k_bbox<<<nparts, kT, 0, s>>>(pos, n, ws.bbox_part.as<double>(), ws.bbox_ticket.as<u32>(),
+                               ws.root.as<TreeRoot>(), split ? ws.split.as<double>() : nullptr);
   GTC_LAUNCH_CHECK();
 }
 
 void pack_bodies_bbox(Workspace &ws, const double *pos, const double *mass, u64 n,
                       cudaStream_t s) {
-  bbox_root(ws, pos, n, s);
+  bbox_root(ws, pos, n, s, false);
   ws.bodies.ensure(n * sizeof(float4));
   const TreeRoot *root = ws.root.as<TreeRoot>();
   k_pack_bodies<<<ceil_div(n, kT), kT, 0, s>>>(pos, mass, static_cast<u32>(n),
@@ -1606,33 +1385,14 @@ void join_walk(Workspace &ws, cudaStream_t s) {
 }
 
 namespace {
-// The split table, its in-order copy and check, and the first key word of
-// every body.
-void make_keys(Workspace &ws, const double *pos, u32 n, cudaStream_t s) {
-  const TreeRoot *root = ws.root.as<TreeRoot>();
-  Scalars *sc = ws.scalars.as<Scalars>();
-  ws.split.ensure(3ull * kSplitSize * sizeof(double));
-  k_split_top<<<3, 1024, 0, s>>>(root, ws.split.as<double>());
-  GTC_LAUNCH_CHECK();
-  // levels kSplitTop..20: subtrees of 4, 4 and 2 levels
-  static_assert(kSplitTop - 1 + 4 + 4 + 2 == kSplitLevels - 1, "split table levels");
-  double *split = ws.split.as<double>();
-  k_split_sub<4><<<ceil_div(3u << (kSplitTop - 1), kT), kT, 0, s>>>(root, split, kSplitTop - 1);
-  GTC_LAUNCH_CHECK();
-  k_split_sub<4><<<ceil_div(3u << (kSplitTop + 3), kT), kT, 0, s>>>(root, split, kSplitTop + 3);
-  GTC_LAUNCH_CHECK();
-  k_split_sub<2><<<ceil_div(3u << (kSplitTop + 7), kT), kT, 0, s>>>(root, split, kSplitTop + 7);
-  GTC_LAUNCH_CHECK();
-  k_split_check<<<ceil_div(3u << (kSplitLevels - 1), kT), kT, 0, s>>>(split, &sc->split_unsorted);
-  GTC_LAUNCH_CHECK();
-  k_keys<<<ceil_div(n, kT), kT, 0, s>>>(pos, n, root, split, &sc->split_unsorted,
-                                        ws.key0.as<u64>(), ws.idx.as<u32>(), ws.tiny.as<u8>(),
-                                        &sc->error);
+// The first key word of every body.
+void make_keys(Workspace &ws, const double *pos, u32 n, const TreeRoot *root, cudaStream_t s) {
+  k_keys<<<ceil_div(n, kT), kT, 0, s>>>(pos, n, ws.forest.sys, root, ws.key0.as<u64>(),
+                                        ws.idx.as<u32>(), ws.tiny.as<u8>(),
+                                        &ws.scalars.as<Scalars>()->error);
   GTC_LAUNCH_CHECK();
 }
-}  // namespace
 
-namespace {
 // Sorts the (key, body) pairs on the first `levels` levels of the first key
 // word, rounded up to whole 8-bit passes (21 or more: the whole word), and
 // returns the levels the order is exact for. Bodies that share those levels
@@ -1670,39 +1430,16 @@ int sort_top_levels(Workspace &ws, u32 n, int levels, cudaStream_t s,
   return low == 0 ? kLevelsPerWord : (3 * kLevelsPerWord - low) / 3;
 }
 
-// A forest's root cubes (one per system), split tables and first key words.
-void forest_keys(Workspace &ws, const double *pos, u32 n, cudaStream_t s) {
+// A forest's root cubes and split tables (one per system).
+void forest_roots_and_tables(Workspace &ws, const double *pos, cudaStream_t s) {
   const ForestView &fv = ws.forest;
   ws.bbox_part.ensure(6 * sizeof(double) * fv.bbox_nblocks);
+  ws.split.ensure((3ull * fv.systems << fv.split_levels) * sizeof(double));
   k_bbox_forest<<<fv.bbox_nblocks, kT, 0, s>>>(pos, fv.bbox_blocks, fv.start,
                                                ws.bbox_part.as<double>());
   GTC_LAUNCH_CHECK();
-  k_root_forest<<<fv.systems, kT, 0, s>>>(ws.bbox_part.as<double>(), fv.sys_blocks, fv.roots);
-  GTC_LAUNCH_CHECK();
-  const int T = fv.split_levels;
-  const u32 size = 1u << T, tables = 3 * fv.systems;
-  ws.split.ensure(static_cast<u64>(tables) * size * sizeof(double));
-  double *split = ws.split.as<double>();
-  const int top = std::min(T, kSplitTop);
-  k_split_top_forest<<<tables, 1024, 0, s>>>(fv.roots, split, size, top);
-  GTC_LAUNCH_CHECK();
-  for (int lv = top; lv < T;) {  // levels lv.. below the nodes of level lv - 1
-    const int L = T - lv >= 4 ? 4 : (T - lv >= 2 ? 2 : 1);
-    const u32 blocks = ceil_div(static_cast<u64>(tables) << (lv - 1), kT);
-    if (L == 4) k_split_sub_forest<4><<<blocks, kT, 0, s>>>(fv.roots, split, size, tables, lv - 1);
-    else if (L == 2) k_split_sub_forest<2><<<blocks, kT, 0, s>>>(fv.roots, split, size, tables, lv - 1);
-    else k_split_sub_forest<1><<<blocks, kT, 0, s>>>(fv.roots, split, size, tables, lv - 1);
-    GTC_LAUNCH_CHECK();
-    lv += L;
-  }
-  GTC_CUDA(cudaMemsetAsync(fv.split_unsorted, 0, fv.systems * sizeof(u32), s));
-  k_split_check_forest<<<ceil_div(static_cast<u64>(tables) << (T - 1), kT), kT, 0, s>>>(
-      split, size, T, tables, fv.split_unsorted);
-  GTC_LAUNCH_CHECK();
-  k_keys_forest<<<ceil_div(n, kT), kT, 0, s>>>(pos, n, fv.sys, fv.roots, split, size, T,
-                                               fv.split_unsorted, ws.key0.as<u64>(),
-                                               ws.idx.as<u32>(), ws.tiny.as<u8>(),
-                                               &ws.scalars.as<Scalars>()->error);
+  k_root_forest<<<fv.systems, kT, 0, s>>>(ws.bbox_part.as<double>(), fv.sys_blocks, fv.roots,
+                                          fv.split_levels, ws.split.as<double>());
   GTC_LAUNCH_CHECK();
 }
 
@@ -1841,13 +1578,13 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
 
   ws.stage(Workspace::kStBuild, s);
   const ForestView &fv = ws.forest;
-  if (fv) forest_keys(ws, pos, n32, s);
-  else bbox_root(ws, pos, n, s);
+  if (fv) forest_roots_and_tables(ws, pos, s);
+  else bbox_root(ws, pos, n, s, true);
   const TreeRoot *root = fv ? fv.roots : ws.root.as<TreeRoot>();
   u64 *key0 = ws.key0.as<u64>();
   u32 *idx = ws.idx.as<u32>();
   u8 *tiny = ws.tiny.as<u8>();
-  if (!fv) make_keys(ws, pos, n32, s);
+  make_keys(ws, pos, n32, root, s);
   // the levels the last tree needed first; all of them when a leaf lies
   // deeper (sorting the partly sorted pairs again gives the full order)
   ws.stage(Workspace::kStSort0, s);
@@ -1861,11 +1598,9 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   // the levels, so that one read back serves both).
   u32 *count = ws.count.as<u32>(), *cscan = ws.count_scan.as<u32>();
   auto count_nodes = [&] {
-    k_node_count<<<nb, kT, 0, s>>>(lcp_next, leafdepth, n32, count);
-    GTC_LAUNCH_CHECK();
     exclusive_scan_u32(count, cscan, n, &sc->n_nodes, ws.scan_tmp, s);
   };
-  k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, sc);
+  k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
   GTC_LAUNCH_CHECK();
   count_nodes();
   read_scalars(ws, host, s);
@@ -1874,7 +1609,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     sort_top_levels(ws, n32, kLevelsPerWord, s);
     GTC_CUDA(cudaMemsetAsync(&sc->deep, 0, sizeof(u32), s));
     GTC_CUDA(cudaMemsetAsync(&sc->depth, 0, sizeof(u32), s));
-    k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, sc);
+    k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
     GTC_LAUNCH_CHECK();
     count_nodes();
     read_scalars(ws, host, s);
@@ -1933,7 +1668,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     else kv.w2 = ws.key2.as<u64>();
     kv.words += 1;
     GTC_CUDA(cudaMemsetAsync(&sc->deep, 0, sizeof(u32), s));
-    k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, sc);
+    k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
     GTC_LAUNCH_CHECK();
     read_scalars(ws, host, s);
   }
@@ -1969,9 +1704,8 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
 
   k_nodes<<<nb, kT, 0, s>>>(kv, lcp_next, leafdepth, count, cscan, n32, sc, root,
                             ws.split.as<double>(), ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
-                            ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(), nullptr,
-                            fv ? 1u << fv.split_levels : kSplitSize,
-                            fv ? fv.split_levels : kSplitLevels);
+                            ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(),
+                            fv ? fv.split_levels : kSplitLevels, nullptr);
   GTC_LAUNCH_CHECK();
   ws.kids.ensure(static_cast<u64>(m) * 8 * sizeof(u32));
   k_children<<<mb, kT, 0, s>>>(ws.skip.as<u32>(), ws.isleaf.as<u8>(), m, ws.parent.as<u32>(),
@@ -2027,22 +1761,20 @@ void build_tree_graph(Workspace &ws, const double *pos, const double *mass, u64 
   u32 *abort = &sc->abort;
   GTC_CUDA(cudaMemsetAsync(sc, 0, sizeof(Scalars), s));
   const ForestView &fv = ws.forest;
-  if (fv) forest_keys(ws, pos, n32, s);
-  else bbox_root(ws, pos, n, s);
+  if (fv) forest_roots_and_tables(ws, pos, s);
+  else bbox_root(ws, pos, n, s, true);
   const TreeRoot *root = fv ? fv.roots : ws.root.as<TreeRoot>();
   u64 *key0 = ws.key0.as<u64>();
   u32 *idx = ws.idx.as<u32>();
   u8 *tiny = ws.tiny.as<u8>();
-  if (!fv) make_keys(ws, pos, n32, s);
+  make_keys(ws, pos, n32, root, s);
   // the levels the captured depth allows: a deeper tree aborts the replay
   const int sorted = sort_top_levels(ws, n32, caps.depth + 1, s);
   const KeyView kv{key0, nullptr, nullptr, 1, fv.sys};
   signed char *lcp_next = ws.lcp.as<signed char>();
   u8 *leafdepth = ws.leafdepth.as<u8>();
-  k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, sc);
-  GTC_LAUNCH_CHECK();
   u32 *count = ws.count.as<u32>(), *cscan = ws.count_scan.as<u32>();
-  k_node_count<<<nb, kT, 0, s>>>(lcp_next, leafdepth, n32, count);
+  k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
   GTC_LAUNCH_CHECK();
   exclusive_scan_u32(count, cscan, n, &sc->n_nodes, ws.scan_tmp, s);
   k_check_tree_graph<<<1, 1, 0, s>>>(sc, mcap, sorted);
@@ -2050,9 +1782,8 @@ void build_tree_graph(Workspace &ws, const double *pos, const double *mass, u64 
   const u32 *m_dev = &sc->n_nodes;
   k_nodes<<<nb, kT, 0, s>>>(kv, lcp_next, leafdepth, count, cscan, n32, sc, root,
                             ws.split.as<double>(), ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
-                            ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(), abort,
-                            fv ? 1u << fv.split_levels : kSplitSize,
-                            fv ? fv.split_levels : kSplitLevels);
+                            ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(),
+                            fv ? fv.split_levels : kSplitLevels, abort);
   GTC_LAUNCH_CHECK();
   k_children<<<mb, kT, 0, s>>>(ws.skip.as<u32>(), ws.isleaf.as<u8>(), mcap, ws.parent.as<u32>(),
                                ws.nchild.as<u8>(), ws.kids.as<uint4>(), m_dev, abort);

@@ -265,3 +265,46 @@ def test_warp_walk_groups_per_warp(gtc, oracle, gs, theta, walk):
             assert compare_lists(dev, dev["nodes"], lists, nodes) == []
             assert st["cell_interactions"] == lists.stats.cell_interactions
             assert st["body_interactions"] == lists.stats.body_interactions
+
+
+def _lattice(rng, n, step):
+    """Bodies on a dyadic lattice, the box's corners among them: many
+    coordinates lie exactly on the centres' grid or a half's 1e-9 beside it."""
+    pos = rng.integers(-64, 65, (n, 3)) * step
+    pos[0], pos[1] = -64 * step, 64 * step
+    return pos
+
+
+@pytest.mark.parametrize("offset", [0.0, 1.0, -3e4, 1e9, 1e14])
+@pytest.mark.parametrize("kind", ["sphere", "lattice", "flat"])
+def test_keys_on_and_off_the_grid(ctx, oracle, kind, offset):
+    """Key bits from the grid's ranks and, near a centre or far from the origin
+    (where roundings reach many cells, or the tiny-node rule applies), by the
+    reference's comparisons: the oracle's tree and order, bit for bit."""
+    rng = np.random.default_rng(3)
+    n = 4001
+    if kind == "sphere":
+        pos, mass = lopsided_sphere(n, 13)
+    else:
+        mass = rng.random(n) + 0.5
+        pos = _lattice(rng, n, 0.03125 if kind == "lattice" else 1.0 / 3.0)
+        if kind == "flat":
+            pos[:, 2] = 0.0
+    pos = np.ascontiguousarray(pos + offset)
+    ctx.group_force(pos, mass, theta=0.7, eps=0.05)
+    dev = ctx.export()
+    nodes, order, lists = oracle.lists(pos, mass, theta=0.7)
+    assert np.array_equal(dev["order"], order)
+    assert compare_trees(dev["nodes"], nodes) == []
+
+
+@pytest.mark.parametrize("scale", [1e-290, 1e-150, 1e120])
+def test_keys_of_extreme_lengths(ctx, oracle, scale):
+    pos, mass = lopsided_sphere(1500, 17)
+    pos = np.ascontiguousarray(pos * scale)
+    ctx.tree_force(pos, mass, theta=0.7, eps=0.05 * scale)
+    ctx.group_force(pos, mass, theta=0.7, eps=1.0)
+    dev = ctx.export()
+    nodes, order, lists = oracle.lists(pos, mass, theta=0.7)
+    assert np.array_equal(dev["order"], order)
+    assert compare_trees(dev["nodes"], nodes) == []
