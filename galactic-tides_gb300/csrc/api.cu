@@ -90,7 +90,7 @@ void check_device_error(u32 code) {
   if (code == 0) return;
   if (code & 4u) throw InvalidArgument("cuda: positions must be finite");
   if (code & 8u) throw RuntimeError("cuda: the learned walk's count and fill passes disagree");
-  if (code & 16u) throw RuntimeError("cuda: the radix sort's look-back outwaited its bound");
+  if (code & 16u) throw RuntimeError("cuda: a sort's or scan's look-back outwaited its bound");
   throw RuntimeError("cuda: inconsistent tree detected on the device (code " +
                      std::to_string(code) + ")");
 }
@@ -237,7 +237,6 @@ void group_force(gtc_context *ctx, const double *pos, const double *mass, u64 n,
   GTC_CUDA(cudaEventRecord(ctx->ev[2], s));
   if (n > 0) {
     ws.out.ensure(n * sizeof(float4));
-    ctx->counter.ensure(sizeof(u32));
     if (ctx->have_model) ctx->prev_amag.ensure(n * sizeof(float));  // |a| for the next learned solve
     const gtc::EvalOut eo{ws.out.as<float4>(), ws.idx.as<u32>(), acc, pot,
                           ctx->have_model ? ctx->prev_amag.as<float>() : nullptr};
@@ -245,7 +244,8 @@ void group_force(gtc_context *ctx, const double *pos, const double *mass, u64 n,
     gtc::evaluate_lists(ws.bodies.as<float4>(), ws.cells.as<float4>(), ws.cell_list.as<u32>(),
                         ws.body_list.as<u32>(), ws.groups.as<uint4>(), ws.n_groups,
                         static_cast<float>(sp.G), static_cast<float>(sp.eps * sp.eps),
-                        sp.quadrupole != 0, eo, ctx->counter.as<u32>(), s, ws.eval_shape);
+                        sp.quadrupole != 0, eo, &ws.scalars.as<gtc::Scalars>()->eval_next, s,
+                        ws.eval_shape);
     GTC_CUDA(cudaEventRecord(ctx->ev[5], s));
   }
   GTC_CUDA(cudaEventRecord(ctx->ev[3], s));
@@ -377,9 +377,7 @@ struct GraphStep {
   void reserve() {
     gtc::Workspace &ws = ctx->ws;
     reserve_graph(ws, *ctx->host_sc, ctx->graph_headroom, n, caps);
-    ctx->counter.ensure(sizeof(u32));
     if (ctx->have_model) ctx->prev_amag.ensure(n * sizeof(float));
-    gtc::write_root_task(ws, ctx->stream);
   }
 
   // Events are recorded as external nodes so that their times can be read.
@@ -405,7 +403,7 @@ struct GraphStep {
                               ws.cell_list.as<u32>(), ws.body_list.as<u32>(),
                               ws.groups.as<uint4>(), n, caps.groups, sc, static_cast<float>(sp.G),
                               static_cast<float>(sp.eps * sp.eps), sp.quadrupole != 0, eo,
-                              ctx->counter.as<u32>(), s, ws.eval_shape);
+                              &sc->eval_next, s, ws.eval_shape);
     mark(5, s);
     gtc::kick(vel, acc, n, h, s, &sc->abort);
     mark(3, s);
@@ -732,7 +730,7 @@ struct ForestGraph {
                               ws.cell_list.as<u32>(), ws.body_list.as<u32>(),
                               ws.groups.as<uint4>(), f->n, caps.groups, sc, static_cast<float>(f->sp.G),
                               static_cast<float>(f->sp.eps * f->sp.eps), f->sp.quadrupole != 0,
-                              gtc::EvalOut{ws.out.as<float4>()}, f->counter.as<u32>(), s,
+                              gtc::EvalOut{ws.out.as<float4>()}, &sc->eval_next, s,
                               ws.eval_shape);
     f->scatter(1, h, &sc->abort, s);
     GTC_CUDA(cudaMemcpyAsync(f->host_sc, sc, sizeof(gtc::Scalars), cudaMemcpyDeviceToHost, s));
@@ -1054,6 +1052,7 @@ gtc_status gtc_tree(gtc_context *ctx, const gtc_float4 *bodies, const gtc_cell *
     GTC_CUDA(cudaStreamSynchronize(s));  // rec is released at the end of scope
     GTC_CUDA(cudaMemsetAsync(ws.out.ptr, 0, n * 16, s));
     ctx->counter.ensure(sizeof(u32));
+    GTC_CUDA(cudaMemsetAsync(ctx->counter.ptr, 0, sizeof(u32), s));
     GTC_CUDA(cudaEventRecord(ctx->ev[2], s));
     gtc::evaluate_lists(ws.bodies.as<float4>(), ws.cells.as<float4>(), ws.cell_list.as<u32>(),
                         ws.body_list.as<u32>(), ws.groups.as<uint4>(), ng, p->G, p->eps2,

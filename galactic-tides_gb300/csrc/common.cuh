@@ -78,11 +78,12 @@ __device__ __forceinline__ float rsqrt_normal(float x) {
 
 // --------------------------------------------------------------- scans
 // Exclusive prefix sums over n elements on `s`. `tmp` is grown as needed.
-// The total is written to *total_dev (device memory, may be null).
+// The total is written to *total_dev (device memory, may be null). A wait past
+// its bound sets bit 16 of *error (device word; null: a word of the scratch).
 void exclusive_scan_u32(const u32 *in, u32 *out, u64 n, u32 *total_dev, DeviceBuffer &tmp,
-                        cudaStream_t s);
+                        cudaStream_t s, u32 *error = nullptr);
 void exclusive_scan_u64(const u64 *in, u64 *out, u64 n, u64 *total_dev, DeviceBuffer &tmp,
-                        cudaStream_t s);
+                        cudaStream_t s, u32 *error = nullptr);
 // Grows tmp to what scans of up to n elements need (none allocates after).
 void reserve_scans(DeviceBuffer &tmp, u64 n);
 

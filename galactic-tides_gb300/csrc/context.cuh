@@ -15,7 +15,7 @@ struct gtc_context {
   gtc_stats stats{};
   gtc::Workspace ws;
   gtc::Scalars *host_sc = nullptr;  // pinned
-  gtc::DeviceBuffer counter;        // evaluator work queue
+  gtc::DeviceBuffer counter;        // evaluator work queue of gtc_tree
   gtc::DeviceBuffer sample_scratch; // FP64 sample partial sums
   bool have_group = false;
   gtc::SolverParams last{};

@@ -442,7 +442,6 @@ void launch_eval(const EvalArgs &a, u64 groups_hint, cudaStream_t s) {
   int dev = 0, sms = 0;
   GTC_CUDA(cudaGetDevice(&dev));
   GTC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  GTC_CUDA(cudaMemsetAsync(a.counter, 0, sizeof(u32), s));
   if (groups_hint < kTeamGroups) {
     if (a.shape.pairs == 1) launch_shape<kQuad, kSoft, true, 1>(a, sms, s);
     else launch_shape<kQuad, kSoft, true, kTwo>(a, sms, s);

@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(kT)
 ForestRun::~ForestRun() {
   ws.release_all();
   DeviceBuffer *own[] = {&tables, &sysid, &roots, &root_node, &group_root, &apos, &amass, &stats,
-                         &counter, &sys_groups, &sys_max, &slot_plan, &graph_slots};
+                         &sys_groups, &sys_max, &slot_plan, &graph_slots};
   for (DeviceBuffer *b : own) b->release();
   if (host_sc) cudaFreeHost(host_sc);
   if (host_lists) cudaFreeHost(host_lists);
@@ -196,7 +196,6 @@ void ForestRun::setup(const std::vector<ForestSystem> &systems, cudaStream_t s) 
   }
   int T = kSplitLevels;
   while (T > 1 && 3ull * k * (1ull << T) * sizeof(double) > kSplitBudget) --T;
-  counter.ensure(sizeof(u32));
   if (!host_sc) GTC_CUDA(cudaMallocHost(reinterpret_cast<void **>(&host_sc), sizeof(Scalars)));
   char *t = tables.as<char>();
   ForestView &fv = ws.forest;
@@ -262,8 +261,8 @@ void ForestRun::solve(int kick, double h, cudaStream_t s, bool write) {
   evaluate_lists(ws.bodies.as<float4>(), ws.cells.as<float4>(), ws.cell_list.as<u32>(),
                  ws.body_list.as<u32>(), ws.groups.as<uint4>(), ws.n_groups,
                  static_cast<float>(sp.G), static_cast<float>(sp.eps * sp.eps),
-                 sp.quadrupole != 0, EvalOut{ws.out.as<float4>()}, counter.as<u32>(), s,
-                 ws.eval_shape);
+                 sp.quadrupole != 0, EvalOut{ws.out.as<float4>()},
+                 &ws.scalars.as<Scalars>()->eval_next, s, ws.eval_shape);
   if (write) scatter(kick, h, nullptr, s);
   GTC_CUDA(cudaMemcpyAsync(host_sc, ws.scalars.ptr, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
   GTC_CUDA(cudaStreamSynchronize(s));

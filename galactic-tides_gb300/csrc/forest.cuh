@@ -31,7 +31,7 @@ struct ForestRun {
   std::vector<ForestSystem> sys;
   SolverParams sp{};            // the shared parameters (group size and packing per system)
   u64 n = 0;                    // bodies in all
-  DeviceBuffer tables, sysid, roots, root_node, group_root, apos, amass, stats, counter,
+  DeviceBuffer tables, sysid, roots, root_node, group_root, apos, amass, stats,
       sys_groups, sys_max, slot_plan, graph_slots;
   u32 *host_lists = nullptr;    // pinned: per-system group counts, then list maxima
   u32 host_systems = 0;         // systems host_lists holds

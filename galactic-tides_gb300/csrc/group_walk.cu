@@ -99,19 +99,18 @@ __global__ void __launch_bounds__(kT)
   if (open) mark[run_begin] = 1;
 }
 
+// The groups' first bodies and ends; the last group ends with the bodies.
 __global__ void __launch_bounds__(kT)
     k_group_ranges(const u32 *mark, const u32 *scan, u32 n, u32 *gbegin, u32 *gend,
                    const u32 *abort = nullptr) {
   const u32 b = blockIdx.x * kT + threadIdx.x;
-  if (b >= n || aborted(abort) || !mark[b]) return;
-  const u32 g = scan[b];
-  gbegin[g] = b;
-  if (g > 0) gend[g - 1] = b;
-}
-
-__global__ void k_last_end(const Scalars *sc, u32 n, u32 *gend) {
-  if (sc->abort) return;
-  if (sc->n_groups > 0 && sc->n_groups <= n) gend[sc->n_groups - 1] = n;
+  if (b >= n || aborted(abort)) return;
+  const u32 g = scan[b];  // groups that start before b
+  if (mark[b]) {
+    gbegin[g] = b;
+    if (g > 0) gend[g - 1] = b;
+  }
+  if (b == n - 1 && g + mark[b] > 0) gend[g + mark[b] - 1] = n;
 }
 
 // A graph replay's checks around the one-pass walk (bit 8): more groups
@@ -126,9 +125,6 @@ __global__ void k_check_slots_graph(Scalars *sc) {
   if (sc->list_overflow) sc->abort |= 8u;
 }
 
-// Group bounding box (group_lists.cpp:125-131): centre and half-extent in
-// FP64, and the same in FP32 with the centre taken relative to the root
-// centre (the frame of the FP32 walk records).
 // Order-preserving image of a finite double with +0 and -0 equal: a < b as
 // doubles exactly when key(a) < key(b).
 __device__ __forceinline__ u64 zero_equal_key(double v) {
@@ -136,45 +132,53 @@ __device__ __forceinline__ u64 zero_equal_key(double v) {
   if (b == 0x8000000000000000ull) b = 0;
   return (b >> 63) ? ~b : (b | 0x8000000000000000ull);
 }
+__device__ __forceinline__ double of_key(u64 k) {
+  return __longlong_as_double(static_cast<long long>((k >> 63) ? (k & 0x7fffffffffffffffull) : ~k));
+}
 
+// Group bounding box (group_lists.cpp:125-131): centre and half-extent in
+// FP64, and the same in FP32 with the centre taken relative to the root
+// centre (the frame of the FP32 walk records). Eight lanes share a group's
+// bodies, a few loads each, and its smallest and largest coordinates, taken on
+// integer images of the doubles off the FP64 pipe (a zero comes out as +0; its
+// sign changes no distance). One thread per group walked up to 32 bodies in
+// series: 21 us however few the groups.
+constexpr u32 kBoxLanes = 8;
 __global__ void __launch_bounds__(kT)
     k_group_box(const u32 *gbegin, const u32 *gend, u32 ng, const double *tpos,
                 const TreeRoot *root, double *gbox, float *gboxf, const u32 *ng_dev,
                 const u32 *abort, ForestView fv) {
   // gboxf per group: centre (3), half-extent (3), magnitude bound, pad
-  const u32 g = blockIdx.x * kT + threadIdx.x;
-  if (aborted(abort) || g >= bounded(ng, ng_dev)) return;
+  const u32 g = (blockIdx.x * kT + threadIdx.x) / kBoxLanes;
+  const u32 lane = threadIdx.x % kBoxLanes;
+  if (aborted(abort) || g >= bounded(ng, ng_dev)) return;  // (the same for a group's lanes)
+  const u32 lanes = 0xffu << (threadIdx.x & 31u & ~(kBoxLanes - 1u));
   const u32 b0 = gbegin[g], b1 = gend[g];
   if (fv.sys) {  // a forest: the group's system's root
     const u16 k = fv.sys[b0];
     root += k;
-    fv.group_root[g] = fv.root_node[k];
+    if (lane == 0) fv.group_root[g] = fv.root_node[k];
   }
-  // the reference's running min and max (v < lo, hi < v: the first of equal
-  // values stays), compared on integer images of the doubles (+0 and -0
-  // equal) instead of on the FP64 pipe
-  double lo[3], hi[3];
-  u64 klo[3], khi[3];
-  for (int a = 0; a < 3; ++a) {
-    lo[a] = hi[a] = tpos[3ull * b0 + a];
-    klo[a] = khi[a] = zero_equal_key(lo[a]);
-  }
-  for (u32 k = b0; k < b1; ++k)
+  u64 lo[3] = {~0ull, ~0ull, ~0ull}, hi[3] = {0ull, 0ull, 0ull};
+  for (u32 k = b0 + lane; k < b1; k += kBoxLanes)
     for (int a = 0; a < 3; ++a) {
-      const double v = tpos[3ull * k + a];
-      const u64 kv = zero_equal_key(v);
-      if (kv < klo[a]) {
-        klo[a] = kv;
-        lo[a] = v;
-      }
-      if (khi[a] < kv) {
-        khi[a] = kv;
-        hi[a] = v;
-      }
+      const u64 v = zero_equal_key(tpos[3ull * k + a]);
+      lo[a] = v < lo[a] ? v : lo[a];
+      hi[a] = v > hi[a] ? v : hi[a];
     }
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+#pragma unroll
+    for (u32 o = kBoxLanes / 2; o > 0; o >>= 1) {
+      const u64 l = __shfl_xor_sync(lanes, lo[a], o), h = __shfl_xor_sync(lanes, hi[a], o);
+      lo[a] = l < lo[a] ? l : lo[a];
+      hi[a] = h > hi[a] ? h : hi[a];
+    }
+  if (lane != 0) return;
   float gmax = 0.f, hmax = 0.f;
   for (int a = 0; a < 3; ++a) {
-    const double c = (lo[a] + hi[a]) * 0.5, h = (hi[a] - lo[a]) * 0.5;
+    const double l = of_key(lo[a]), u = of_key(hi[a]);
+    const double c = (l + u) * 0.5, h = (u - l) * 0.5;
     gbox[6ull * g + a] = c;
     gbox[6ull * g + 3 + a] = h;
     const float cf = static_cast<float>(c - root->center[a]), hf = static_cast<float>(h);
@@ -253,8 +257,8 @@ __global__ void __launch_bounds__(kT)
     bl = out.body_list + out.spill_bodies[g];
   }
   u32 nc = 0, nb = 0, exact = 0, visits = 0;
-  // (a forest has one task, its group's own root)
-  const Task task = group_root ? Task{group_root[g], kNone, 0u, 0u} : tasks[t];
+  // one task (tasks null): the root, a forest's the group's own
+  const Task task = tasks ? tasks[t] : Task{group_root ? group_root[g] : 0u, kNone, 0u, 0u};
   auto take = [&](const WalkRec32 &r, u32 i, int verdict) {
     const u32 nbody = r.nbody_leaf & 0x7fffffffu;
     if (verdict == 1 && nbody > kFewBodies) {
@@ -520,11 +524,10 @@ __global__ void __launch_bounds__(kWalkThreads)
 // system, whatever else a launch walks. Exports put each group's lists back
 // in increasing order. Modes: count the lists (kCount); write them at scanned
 // offsets (kFill); write them into per-group slots, counting past a slot that
-// overflows (kSlots, the one-pass walk, whose counts and records then go
-// through the split walk's spill and record kernels as one part); write the
-// lists of the groups that outgrew their slots again, whole, into their
-// places in the overflow pools (kSpill: the others of their kSuper are walked
-// along unwritten).
+// overflows (kSlots, the one-pass walk): a group that outgrew its slot gets a
+// place in the overflow pools and the warp walks its kSuper once more, the
+// others into their slots again; then the warp writes the groups' records and
+// keeps the statistics.
 //
 // Bound: instruction issue (75% of the issue slots busy at 1M bodies, four
 // groups to a warp; 190 instructions per 32 tests, the test itself 33). 2M
@@ -536,13 +539,16 @@ constexpr u32 kWarpStack = 640;   // ranges per warp
 constexpr u32 kWarpWalkThreads = kWarpWalkWarps * 32;
 
 struct WarpWalkOut {
-  u64 *ncells, *nbodies;          // kCount: per group; kSlots: SplitOut's part 0 (cap: its stride)
-  const u64 *cell_off, *body_off; // kFill
   u32 *cell_list, *body_list;
-  const u32 *spill_cells, *spill_bodies;  // kSpill
-  u32 *split;                     // kSlots: the split walk's split points (all lists: part 0)
-  u32 slot_cells, slot_bodies, cap;
-  const uint4 *plan = nullptr;    // kSlots, a forest: per-group slots (starts, sizes)
+  u64 *ncells, *nbodies;          // kCount
+  const u64 *cell_off, *body_off; // kFill
+  // kSlots
+  u32 slot_cells, slot_bodies;
+  const uint4 *plan;              // a forest: per-group slots (starts, sizes)
+  u64 pool_cells_at, pool_cells, pool_bodies_at, pool_bodies;
+  const u32 *gbegin, *gend;
+  uint4 *groups;
+  u32 *sys_max;                   // a forest: per-system maxima of the list lengths
 };
 
 // Where a forest's groups belong: the first group and the group count of
@@ -555,6 +561,38 @@ struct GroupSystems {
   u32 systems = 0;
 };
 
+// A share of the list statistics (group_stats_warp's, whole lists): of the
+// groups that were group k of a warp's kSuper.
+struct WalkStats {
+  u64 ci, bi, tc, tb, ml;
+  u32 mg, mc, mb;
+  __device__ void flush(Scalars *sc) {  // every lane of the warp
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ci += __shfl_xor_sync(kFullMask, ci, o);
+      bi += __shfl_xor_sync(kFullMask, bi, o);
+      tc += __shfl_xor_sync(kFullMask, tc, o);
+      tb += __shfl_xor_sync(kFullMask, tb, o);
+      const u64 m = __shfl_xor_sync(kFullMask, ml, o);
+      ml = m > ml ? m : ml;
+    }
+    mg = __reduce_max_sync(kFullMask, mg);
+    mc = __reduce_max_sync(kFullMask, mc);
+    mb = __reduce_max_sync(kFullMask, mb);
+    if ((threadIdx.x & 31) != 0 || mg == 0) return;  // (a warp that had no group)
+    atomicAdd(&sc->cell_interactions, static_cast<unsigned long long>(ci));
+    atomicAdd(&sc->body_interactions, static_cast<unsigned long long>(bi));
+    atomicAdd(reinterpret_cast<unsigned long long *>(&sc->n_cell_list),
+              static_cast<unsigned long long>(tc));
+    atomicAdd(reinterpret_cast<unsigned long long *>(&sc->n_body_list),
+              static_cast<unsigned long long>(tb));
+    atomicMax(&sc->max_list, static_cast<unsigned long long>(ml));
+    atomicMax(&sc->max_group, mg);
+    atomicMax(&sc->max_cells, mc);
+    atomicMax(&sc->max_bodies, mb);
+  }
+};
+
 // What a warp keeps in shared memory.
 template <int kSuper>
 struct WarpWalk {
@@ -562,6 +600,7 @@ struct WarpWalk {
   float4 box[kSuper][2];         // the groups' FP32 boxes
   uint4 out[kSuper];             // cell list start and room, body list start and room
   u32 q_begin[64], q_count[64];  // body runs met, to be written 32 at a time
+  WalkStats stats[kSuper];
   u8 q_mask[64];
   u8 mask[kWarpStack];
 };
@@ -645,6 +684,7 @@ __global__ void __launch_bounds__(kWarpWalkThreads)
   const u32 below = (1u << lane) - 1u;
   WarpWalk<kSuper> &w = walks[threadIdx.x >> 5];
   u32 exact = 0, visits = 0;
+  if (kMode == kSlots && lane < kSuper) w.stats[lane] = WalkStats{};
   u32 g = 0, chunk_end = 0;  // groups of the taken chunk still to look at
   for (;;) {
     if (g >= chunk_end) {
@@ -683,22 +723,18 @@ __global__ void __launch_bounds__(kWarpWalkThreads)
           o = make_uint4(q * out.slot_cells, out.slot_cells, q * out.slot_bodies,
                          out.slot_bodies);
         }
-      } else if (kMode == kSpill) {
-        if (out.spill_cells[q] != kNoSpill)
-          o = make_uint4(out.spill_cells[q], 0xffffffffu, out.spill_bodies[q], 0xffffffffu);
       }
       w.out[lane] = o;
     }
-    if (kMode == kSpill) {
-      const bool spilled = lane < count && out.spill_cells[lead + lane] != kNoSpill;
-      if (!__any_sync(kFullMask, spilled)) continue;
-    }
     u32 nc[kSuper], nb[kSuper];  // warp-uniform
-#pragma unroll
-    for (int k = 0; k < kSuper; ++k) nc[k] = nb[k] = 0u;
     // the root contains every group and is opened, unless it is a leaf
     const u32 root = group_root ? group_root[lead] : 0u;
     const WalkRec32 rr = load32(walk32, root);
+    const u32 visits0 = visits, exact0 = exact;
+    bool rewalk = false;  // (kSlots: some group's lists go to the pools)
+  again:
+#pragma unroll
+    for (int k = 0; k < kSuper; ++k) nc[k] = nb[k] = 0u;
     if (lane == 0) {
       w.stk[0] = make_uint2((rr.nbody_leaf >> 31) != 0 ? root : root + 1, rr.skip);
       w.mask[0] = static_cast<u8>((1u << count) - 1u);
@@ -854,15 +890,56 @@ __global__ void __launch_bounds__(kWarpWalkThreads)
           c = nc[k];
           b = nb[k];
         }
-      if (lane < count) {
-        const u32 q = lead + lane;
+      const u32 q = lead + lane;
+      if (kMode == kCount && lane < count) {
         out.ncells[q] = c;
         out.nbodies[q] = b;
-        if (kMode == kSlots) {
-          out.ncells[static_cast<u64>(out.cap) + q] = 0;
-          out.nbodies[static_cast<u64>(out.cap) + q] = 0;
-          out.split[2ull * q] = c;
-          out.split[2ull * q + 1] = b;
+      }
+      if (kMode == kSlots) {
+        if (!rewalk) {
+          const bool over = lane < count && (c > w.out[lane].y || b > w.out[lane].w);
+          if (__any_sync(kFullMask, over)) {
+            if (over) {
+              const u64 ac = atomicAdd(&sc->spill_used[0], static_cast<unsigned long long>(c));
+              const u64 ab = atomicAdd(&sc->spill_used[1], static_cast<unsigned long long>(b));
+              if (ac + c <= out.pool_cells && ab + b <= out.pool_bodies)
+                w.out[lane] = make_uint4(static_cast<u32>(out.pool_cells_at + ac), c,
+                                         static_cast<u32>(out.pool_bodies_at + ab), b);
+              else
+                atomicOr(&sc->list_overflow, 1u);
+              atomicAdd(&sc->spilled, 1u);
+            }
+            rewalk = true;
+            visits = visits0;  // the second walk's count stands for both
+            exact = exact0;
+            __syncwarp();
+            goto again;
+          }
+        }
+        if (lane < count) {
+          const u32 first_body = out.gbegin[q], end_body = out.gend[q];
+          const uint4 o = w.out[lane];
+          store_group_rec(out.groups, q, first_body, end_body, one_segment(o.x, c),
+                          one_segment(o.z, b));
+          const u64 t = end_body - first_body;
+          WalkStats &st = w.stats[lane];
+          st.ci += t * c;
+          st.bi += t * b - t;
+          st.tc += c;
+          st.tb += b;
+          st.ml = max(st.ml, static_cast<u64>(c) + b);
+          st.mg = max(st.mg, static_cast<u32>(t));
+          st.mc = max(st.mc, c);
+          st.mb = max(st.mb, b);
+        }
+        if (out.sys_max) {
+          const u32 mc = __reduce_max_sync(kFullMask, lane < count ? c : 0u),
+                    mb = __reduce_max_sync(kFullMask, lane < count ? b : 0u);
+          if (lane == 0) {
+            const u32 k = gs.sys[gs.gbegin[lead]];
+            atomicMax(&out.sys_max[4ull * k], mc);
+            atomicMax(&out.sys_max[4ull * k + 1], mb);
+          }
         }
       }
     }
@@ -872,8 +949,12 @@ __global__ void __launch_bounds__(kWarpWalkThreads)
     const u32 ex = __reduce_add_sync(kFullMask, exact), vs = __reduce_add_sync(kFullMask, visits);
     if (lane == 0) {
       if (ex) atomicAdd(&sc->fp64_tests, static_cast<unsigned long long>(ex));
-      atomicAdd(&sc->walk_nodes, static_cast<unsigned long long>(vs));
+      if (vs) atomicAdd(&sc->walk_nodes, static_cast<unsigned long long>(vs));
     }
+  }
+  if (kMode == kSlots) {
+    WalkStats st = lane < kSuper ? w.stats[lane] : WalkStats{};
+    st.flush(sc);
   }
 }
 
@@ -1049,8 +1130,13 @@ void launch_warp_walk_of(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scal
   GTC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   GTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_warp<kMode, kSuper>,
                                                          kWarpWalkThreads, 0));
-  ws.walk_next.ensure(sizeof(u32));
-  GTC_CUDA(cudaMemsetAsync(ws.walk_next.ptr, 0, sizeof(u32), s));
+  // the one-pass walk's counters are zeroed with the scalars
+  u32 *next = kMode == kSlots ? &sc->walk_next[kSuper >> 1] : nullptr;
+  if (!next) {
+    ws.walk_next.ensure(sizeof(u32));
+    next = ws.walk_next.as<u32>();
+    GTC_CUDA(cudaMemsetAsync(next, 0, sizeof(u32), s));
+  }
   const u32 blocks = static_cast<u32>(std::max<u64>(
       1, std::min<u64>(ceil_div(ng_cap, kWarpWalkWarps * kSuper),
                        static_cast<u64>(std::max(1, per_sm)) * static_cast<u64>(sms))));
@@ -1060,8 +1146,8 @@ void launch_warp_walk_of(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scal
                       ws.flags_scan.as<u32>(), ws.forest.systems};
   k_walk_warp<kMode, kSuper><<<blocks, kWarpWalkThreads, 0, s>>>(
       ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), ws.gbox.as<double>(),
-      ws.gboxf.as<float>(), ng_cap, out, ws.walk_next.as<u32>(), sc, ng_dev, abort,
-      ws.forest.group_root, gs, ws.walk_super == 0);
+      ws.gboxf.as<float>(), ng_cap, out, next, sc, ng_dev, abort, ws.forest.group_root, gs,
+      ws.walk_super == 0);
   GTC_LAUNCH_CHECK();
 }
 
@@ -1105,24 +1191,22 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   const u32 n32 = static_cast<u32>(n), m = static_cast<u32>(ws.n_nodes);
   const u32 gs = static_cast<u32>(sp.group_size);
   Scalars *sc = ws.scalars.as<Scalars>();
-  ws.walk_next.ensure(sizeof(u32));  // before any graph capture reuses the walk
-  GTC_CUDA(cudaMemsetAsync(&sc->spilled, 0, sizeof(u32), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->walk_nodes, 0, sizeof(unsigned long long), s));
   ws.flags.ensure(std::max<u64>(n, m) * 4);
   ws.flags_scan.ensure(std::max<u64>(n, m) * 4);
   u32 *mark = ws.flags.as<u32>(), *mscan = ws.flags_scan.as<u32>();
   const u32 mb = ceil_div(m, kT);
 
-  // walk tasks (their count is read back with the group count)
-  ws.tasks.ensure(m * sizeof(Task));
-  // (the learned walk splits each group's walk along its own path instead;
-  // a forest's groups walk their own system's tree whole, one task each)
+  // walk tasks of a split walk (their count is read back with the group
+  // count); the learned walk splits each group's walk along its own path
+  // instead, a forest's groups walk their own system's tree whole
   const ForestView &fv = ws.forest;
-  if (!lw && !fv) {
+  const bool split_tasks = !lw && !fv && ws.walk_split_depth > 0;
+  if (split_tasks) {
+    ws.tasks.ensure(m * sizeof(Task));
     k_task_flags<<<mb, kT, 0, s>>>(ws.depth.as<u8>(), ws.isleaf.as<u8>(), m, ws.walk_split_depth,
                                    mark);
     GTC_LAUNCH_CHECK();
-    exclusive_scan_u32(mark, mscan, m, &sc->aux, ws.scan_tmp, s);
+    exclusive_scan_u32(mark, mscan, m, &sc->aux, ws.scan_tmp, s, &sc->error);
     k_task_fill<<<mb, kT, 0, s>>>(mark, mscan, ws.depth.as<u8>(), ws.parent.as<u32>(), m,
                                   ws.tasks.as<Task>());
     GTC_LAUNCH_CHECK();
@@ -1133,7 +1217,7 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   const NodeView nv = node_view(ws);
   k_group_marks<<<mb, kT, 0, s>>>(nv, m, gs, sp.pack, mark);
   GTC_LAUNCH_CHECK();
-  exclusive_scan_u32(mark, mscan, n, &sc->n_groups, ws.scan_tmp, s);
+  exclusive_scan_u32(mark, mscan, n, &sc->n_groups, ws.scan_tmp, s, &sc->error);
   ws.gbegin.ensure(n * 4);
   ws.gend.ensure(n * 4);
   ws.gbox.ensure(n * 48);
@@ -1142,8 +1226,6 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   u32 *gbegin = ws.gbegin.as<u32>(), *gend = ws.gend.as<u32>();
   k_group_ranges<<<ceil_div(n, kT), kT, 0, s>>>(mark, mscan, n32, gbegin, gend);
   GTC_LAUNCH_CHECK();
-  k_last_end<<<1, 1, 0, s>>>(sc, n32, gend);
-  GTC_LAUNCH_CHECK();
   if (fv) {  // each system's group count, read back with the total
     k_sys_groups<<<ceil_div(fv.systems, kT), kT, 0, s>>>(mscan, fv.start, fv.systems, sc,
                                                          fv.sys_groups);
@@ -1151,15 +1233,12 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
     GTC_CUDA(cudaMemcpyAsync(fv.host_groups, fv.sys_groups, fv.systems * sizeof(u32),
                              cudaMemcpyDeviceToHost, s));
   }
-  GTC_CUDA(cudaMemsetAsync(&sc->cell_interactions, 0, 3 * sizeof(unsigned long long), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->max_group, 0, sizeof(u32), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->fp64_tests, 0, 3 * sizeof(unsigned long long), s));
   read_scalars(ws, host, s);
-  const u32 ng = host->n_groups, ntasks = fv ? 1u : host->aux;
+  const u32 ng = host->n_groups, ntasks = split_tasks ? host->aux : 1u;
   ws.n_groups = ng;
   ws.choose_walk(ng);
   const u32 gb = ceil_div(ng, kT);
-  k_group_box<<<gb, kT, 0, s>>>(gbegin, gend, ng, ws.tpos.as<double>(),
+  k_group_box<<<ceil_div(static_cast<u64>(ng) * kBoxLanes, kT), kT, 0, s>>>(gbegin, gend, ng, ws.tpos.as<double>(),
                                 fv ? fv.roots : ws.root.as<TreeRoot>(), ws.gbox.as<double>(),
                                 ws.gboxf.as<float>(), nullptr, nullptr, fv);
   GTC_LAUNCH_CHECK();
@@ -1181,11 +1260,10 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   const WalkRec64 *w64 = ws.walk64.as<WalkRec64>();
   const double *gbox = ws.gbox.as<double>();
   const float *gboxf = ws.gboxf.as<float>();
-  const Task *tasks = ws.tasks.as<Task>();
+  const Task *tasks = split_tasks ? ws.tasks.as<Task>() : nullptr;
   const u64 slots = static_cast<u64>(ng) * ntasks;
   ws.gcells.ensure(slots * 8);
   ws.gbodies.ensure(slots * 8);
-  GTC_CUDA(cudaMemsetAsync(&sc->max_cells, 0, 4 * sizeof(u32), s));
   const u32 tb = ceil_div(slots, kT);
   // a forest's per-system maxima of the lists, read back after the walk
   auto clear_sys_max = [&] {
@@ -1217,46 +1295,48 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
       ext_c + ext_b <= std::max<u64>(16 * prev_entries, 1ull << 28)) {
     ws.cell_list.ensure(ext_c * 4);
     ws.body_list.ensure(ext_b * 4);
-    ws.spill.ensure(2ull * ng * sizeof(u32));
-    ws.splitpt.ensure(2ull * ng * sizeof(u32));
-    ws.gcells.ensure(2ull * ng * 8);
-    ws.gbodies.ensure(2ull * ng * 8);
-    u32 *spill_c = ws.spill.as<u32>(), *spill_b = spill_c + ng;
-    GTC_CUDA(cudaMemsetAsync(&sc->n_cell_list, 0, 2 * sizeof(u64), s));
-    GTC_CUDA(cudaMemsetAsync(&sc->list_overflow, 0, sizeof(u32), s));
-    GTC_CUDA(cudaMemsetAsync(sc->spill_used, 0, 2 * sizeof(unsigned long long), s));
-    GTC_CUDA(cudaMemsetAsync(&sc->spilled, 0, sizeof(u32), s));
-    GTC_CUDA(cudaMemsetAsync(&sc->max_cells, 0, 4 * sizeof(u32), s));
-    SplitOut so{ws.gcells.as<u64>(), ws.gbodies.as<u64>(), ws.splitpt.as<u32>(),
-                ws.cell_list.as<u32>(), ws.body_list.as<u32>(), near_c, near_b,
-                sl_c, sl_b, sn_c, sn_b, ng};
-    so.sys = fv.sys;
-    so.sys_max = fv.sys_max;
-    const WarpWalkOut wwo{so.ncells, so.nbodies, nullptr, nullptr, ws.cell_list.as<u32>(),
-                          ws.body_list.as<u32>(), spill_c, spill_b, so.split, sl_c, sl_b, ng};
     if (ws.walk_warps) {
+      WarpWalkOut wwo{};
+      wwo.cell_list = ws.cell_list.as<u32>();
+      wwo.body_list = ws.body_list.as<u32>();
+      wwo.slot_cells = sl_c;
+      wwo.slot_bodies = sl_b;
+      wwo.pool_cells_at = pool_at_c;
+      wwo.pool_cells = pool_c;
+      wwo.pool_bodies_at = pool_at_b;
+      wwo.pool_bodies = pool_b;
+      wwo.gbegin = gbegin;
+      wwo.gend = gend;
+      wwo.groups = ws.groups.as<uint4>();
+      wwo.sys_max = fv.sys_max;
       launch_warp_walk<kSlots>(ws, wwo, ng, sc, s);
     } else {
+      ws.spill.ensure(2ull * ng * sizeof(u32));
+      ws.splitpt.ensure(2ull * ng * sizeof(u32));
+      ws.gcells.ensure(2ull * ng * 8);
+      ws.gbodies.ensure(2ull * ng * 8);
+      u32 *spill_c = ws.spill.as<u32>(), *spill_b = spill_c + ng;
+      SplitOut so{ws.gcells.as<u64>(), ws.gbodies.as<u64>(), ws.splitpt.as<u32>(),
+                  ws.cell_list.as<u32>(), ws.body_list.as<u32>(), near_c, near_b,
+                  sl_c, sl_b, sn_c, sn_b, ng};
+      so.sys = fv.sys;
+      so.sys_max = fv.sys_max;
       k_walk_split<<<ceil_div(2ull * ng, kWalkThreads), kWalkThreads, 0, s>>>(
           w32, w64, gbox, gboxf, gbegin, gend, ws.kids.as<uint4>(), ws.nchild.as<u8>(),
           ws.nbegin.as<u32>(), ws.nend.as<u32>(), ng, so, sc, nullptr, nullptr, fv.group_root);
       GTC_LAUNCH_CHECK();
-    }
-    k_split_spill<<<gb, kT, 0, s>>>(so, ng, pool_at_c, pool_c, pool_at_b, pool_b, spill_c, spill_b,
-                                    sc);
-    GTC_LAUNCH_CHECK();
-    if (ws.walk_warps) {
-      launch_warp_walk<kSpill>(ws, wwo, ng, sc, s);
-    } else {
+      k_split_spill<<<gb, kT, 0, s>>>(so, ng, pool_at_c, pool_c, pool_at_b, pool_b, spill_c,
+                                      spill_b, sc);
+      GTC_LAUNCH_CHECK();
       WalkOut wo{ws.gcells.as<u64>(), ws.gbodies.as<u64>(), nullptr, nullptr,
                  ws.cell_list.as<u32>(), ws.body_list.as<u32>(), spill_c, spill_b};
       k_walk<kSpill><<<tb, kT, 0, s>>>(w32, w64, gbox, gboxf, ng, tasks, 1, wo, sc, nullptr,
                                        nullptr, fv.group_root);
       GTC_LAUNCH_CHECK();
+      k_split_records<<<gb, kT, 0, s>>>(gbegin, gend, ng, so, spill_c, spill_b,
+                                        ws.groups.as<uint4>(), sc);
+      GTC_LAUNCH_CHECK();
     }
-    k_split_records<<<gb, kT, 0, s>>>(gbegin, gend, ng, so, spill_c, spill_b,
-                                      ws.groups.as<uint4>(), sc);
-    GTC_LAUNCH_CHECK();
     ws.stage(Workspace::kStWalk1, s);
     read_sys_max();
     read_scalars(ws, host, s);
@@ -1286,8 +1366,11 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   WalkOut wo{ws.gcells.as<u64>(), ws.gbodies.as<u64>(), cell_off, body_off, nullptr, nullptr,
              nullptr, nullptr};
   const bool warps = ws.walk_warps && ntasks == 1;
-  WarpWalkOut wwo{ws.gcells.as<u64>(), ws.gbodies.as<u64>(), cell_off, body_off, nullptr, nullptr,
-                  nullptr, nullptr, nullptr, 0u, 0u, ng};
+  WarpWalkOut wwo{};
+  wwo.ncells = ws.gcells.as<u64>();
+  wwo.nbodies = ws.gbodies.as<u64>();
+  wwo.cell_off = cell_off;
+  wwo.body_off = body_off;
   if (warps) {
     launch_warp_walk<kCount>(ws, wwo, ng, sc, s);
   } else {
@@ -1295,8 +1378,8 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
                                      nullptr, fv.group_root);
     GTC_LAUNCH_CHECK();
   }
-  exclusive_scan_u64(ws.gcells.as<u64>(), cell_off, slots, cell_off + slots, ws.scan_tmp, s);
-  exclusive_scan_u64(ws.gbodies.as<u64>(), body_off, slots, body_off + slots, ws.scan_tmp, s);
+  exclusive_scan_u64(ws.gcells.as<u64>(), cell_off, slots, cell_off + slots, ws.scan_tmp, s, &sc->error);
+  exclusive_scan_u64(ws.gbodies.as<u64>(), body_off, slots, body_off + slots, ws.scan_tmp, s, &sc->error);
   GTC_CUDA(cudaMemcpyAsync(&sc->n_cell_list, cell_off + slots, 8, cudaMemcpyDeviceToDevice, s));
   GTC_CUDA(cudaMemcpyAsync(&sc->n_body_list, body_off + slots, 8, cudaMemcpyDeviceToDevice, s));
   k_group_records<<<gb, kT, 0, s>>>(gbegin, gend, ng, ntasks, cell_off, body_off,
@@ -1343,16 +1426,12 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
   const NodeView nv = node_view(ws);
   k_group_marks<<<mb, kT, 0, s>>>(nv, mcap, gs, sp.pack, mark, &sc->n_nodes, abort);
   GTC_LAUNCH_CHECK();
-  exclusive_scan_u32(mark, mscan, n, &sc->n_groups, ws.scan_tmp, s);
+  exclusive_scan_u32(mark, mscan, n, &sc->n_groups, ws.scan_tmp, s, &sc->error);
   u32 *gbegin = ws.gbegin.as<u32>(), *gend = ws.gend.as<u32>();
   k_group_ranges<<<nb, kT, 0, s>>>(mark, mscan, n32, gbegin, gend, abort);
   GTC_LAUNCH_CHECK();
-  k_last_end<<<1, 1, 0, s>>>(sc, n32, gend);
-  GTC_LAUNCH_CHECK();
-  GTC_CUDA(cudaMemsetAsync(&sc->cell_interactions, 0, 3 * sizeof(unsigned long long), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->max_group, 0, sizeof(u32), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->fp64_tests, 0, 3 * sizeof(unsigned long long), s));
-  k_group_box<<<nb, kT, 0, s>>>(gbegin, gend, n32, ws.tpos.as<double>(),
+  const u64 boxes = std::min<u64>(n, fv ? n : caps.groups);
+  k_group_box<<<ceil_div(boxes * kBoxLanes, kT), kT, 0, s>>>(gbegin, gend, static_cast<u32>(boxes), ws.tpos.as<double>(),
                                 fv ? fv.roots : ws.root.as<TreeRoot>(), ws.gbox.as<double>(),
                                 ws.gboxf.as<float>(), &sc->n_groups, abort, fv);
   GTC_LAUNCH_CHECK();
@@ -1362,12 +1441,6 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
     k_check_groups_graph<<<1, 1, 0, s>>>(sc, caps.groups, ws.walk_mode < 0 ? ws.walk_super : 0);
     GTC_LAUNCH_CHECK();
   }
-  GTC_CUDA(cudaMemsetAsync(&sc->n_cell_list, 0, 2 * sizeof(u64), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->list_overflow, 0, sizeof(u32), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->max_cells, 0, 4 * sizeof(u32), s));
-  GTC_CUDA(cudaMemsetAsync(sc->spill_used, 0, 2 * sizeof(unsigned long long), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->spilled, 0, sizeof(u32), s));
-  GTC_CUDA(cudaMemsetAsync(&sc->walk_nodes, 0, sizeof(unsigned long long), s));
   u32 *spill_c = ws.spill.as<u32>(), *spill_b = spill_c + n;
   // (the replays' walk: the choice of the eager solve before the capture)
   const u64 near_c = static_cast<u64>(caps.groups) * caps.slot_cells;
@@ -1378,9 +1451,15 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
               ws.cell_list.as<u32>(), ws.body_list.as<u32>(), near_c, near_b,
               caps.slot_cells, caps.slot_bodies, caps.slot_near_cells,
               caps.slot_near_bodies, n32};
-  WarpWalkOut wwo{so.ncells, so.nbodies, nullptr, nullptr, ws.cell_list.as<u32>(),
-                  ws.body_list.as<u32>(), spill_c, spill_b, so.split, caps.slot_cells,
-                  caps.slot_bodies, n32};
+  WarpWalkOut wwo{};
+  wwo.cell_list = ws.cell_list.as<u32>();
+  wwo.body_list = ws.body_list.as<u32>();
+  wwo.slot_cells = caps.slot_cells;
+  wwo.slot_bodies = caps.slot_bodies;
+  wwo.gbegin = gbegin;
+  wwo.gend = gend;
+  wwo.groups = ws.groups.as<uint4>();
+  wwo.sys_max = fv.sys_max;
   if (fv) {
     so.sys = fv.sys;
     so.sys_max = fv.sys_max;
@@ -1396,7 +1475,11 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
     }
   }
   if (ws.walk_warps) {
-    launch_warp_walk<kSlots>(ws, wwo, n32, sc, s, &sc->n_groups, abort);
+    wwo.pool_cells_at = pool_at_c;
+    wwo.pool_cells = caps.pool_cells;
+    wwo.pool_bodies_at = pool_at_b;
+    wwo.pool_bodies = caps.pool_bodies;
+    launch_warp_walk<kSlots>(ws, wwo, static_cast<u32>(boxes), sc, s, &sc->n_groups, abort);
   } else {
     k_walk_split<<<ceil_div(2ull * n, kWalkThreads), kWalkThreads, 0, s>>>(
         ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), ws.gbox.as<double>(),
@@ -1404,33 +1487,21 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
         ws.nbegin.as<u32>(), ws.nend.as<u32>(), n32, so, sc, &sc->n_groups, abort,
         fv.group_root);
     GTC_LAUNCH_CHECK();
-  }
-  k_split_spill<<<nb, kT, 0, s>>>(so, n32, pool_at_c, caps.pool_cells, pool_at_b,
-                                  caps.pool_bodies, spill_c, spill_b, sc, &sc->n_groups, abort);
-  GTC_LAUNCH_CHECK();
-  if (ws.walk_warps) {
-    launch_warp_walk<kSpill>(ws, wwo, n32, sc, s, &sc->n_groups, abort);
-  } else {
+    k_split_spill<<<nb, kT, 0, s>>>(so, n32, pool_at_c, caps.pool_cells, pool_at_b,
+                                    caps.pool_bodies, spill_c, spill_b, sc, &sc->n_groups, abort);
+    GTC_LAUNCH_CHECK();
     WalkOut wo{ws.gcells.as<u64>(), ws.gbodies.as<u64>(), nullptr, nullptr,
                ws.cell_list.as<u32>(), ws.body_list.as<u32>(), spill_c, spill_b};
-    const Task *tasks = ws.tasks.as<Task>();
     k_walk<kSpill><<<nb, kT, 0, s>>>(ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(),
-                                     ws.gbox.as<double>(), ws.gboxf.as<float>(), n32, tasks, 1,
+                                     ws.gbox.as<double>(), ws.gboxf.as<float>(), n32, nullptr, 1,
                                      wo, sc, &sc->n_groups, abort, fv.group_root);
     GTC_LAUNCH_CHECK();
+    k_split_records<<<nb, kT, 0, s>>>(gbegin, gend, n32, so, spill_c, spill_b,
+                                      ws.groups.as<uint4>(), sc, &sc->n_groups, abort);
+    GTC_LAUNCH_CHECK();
   }
-  k_split_records<<<nb, kT, 0, s>>>(gbegin, gend, n32, so, spill_c, spill_b,
-                                    ws.groups.as<uint4>(), sc, &sc->n_groups, abort);
-  GTC_LAUNCH_CHECK();
   k_check_slots_graph<<<1, 1, 0, s>>>(sc);
   GTC_LAUNCH_CHECK();
-}
-
-void write_root_task(Workspace &ws, cudaStream_t s) {
-  ws.tasks.ensure(sizeof(Task));
-  const Task t{0u, kNone, 0u, 0u};
-  GTC_CUDA(cudaMemcpyAsync(ws.tasks.ptr, &t, sizeof(Task), cudaMemcpyHostToDevice, s));
-  GTC_CUDA(cudaStreamSynchronize(s));
 }
 
 }  // namespace gtc

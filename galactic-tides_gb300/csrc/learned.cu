@@ -463,7 +463,8 @@ void learned_add_samples(gtc_context *ctx, const double *pos, const double *mass
   k_finite_flags<<<ceil_div(np, kT), kT, 0, s>>>(label.as<float>(), np, flag.as<u32>());
   GTC_LAUNCH_CHECK();
   u32 *kept_dev = scan.as<u32>() + np;
-  exclusive_scan_u32(flag.as<u32>(), scan.as<u32>(), np, kept_dev, ws.scan_tmp, s);
+  exclusive_scan_u32(flag.as<u32>(), scan.as<u32>(), np, kept_dev, ws.scan_tmp, s,
+                         &ws.scalars.as<Scalars>()->error);
   u32 kept = 0;
   read_back(&kept, kept_dev, sizeof(u32), s);
   if (kept == 0) return;

@@ -1111,7 +1111,8 @@ void learned_build_lists(Workspace &ws, const LearnedWalk &lw, u32 ng, Scalars *
         k_lcont<<<cont_blocks, kContWarps * 32, 0, s>>>(a, r > 0);
         GTC_LAUNCH_CHECK();
       }
-      exclusive_scan_u32(a.pcount, roff, nparts, roff + nparts, ws.scan_tmp, s);
+      exclusive_scan_u32(a.pcount, roff, nparts, roff + nparts, ws.scan_tmp, s,
+                         &ws.scalars.as<Scalars>()->error);
     };
     // the round's deferred pairs as rows, and the network's decisions on
     // them: `launch_rows` rows' worth of blocks, the count read on the device

@@ -182,7 +182,7 @@ struct Workspace {
   // The current lists hold each group's entries in walk-step order rather
   // than the reference's visiting order (exports sort them back).
   bool lists_unordered = false;
-  DeviceBuffer walk_next;     // the warp walk's group counter
+  DeviceBuffer walk_next;     // the warp walk's group counter (count and fill)
   // One-pass walk: group g's lists start at g * slot_cells and g *
   // slot_bodies (capacities sized from the previous walk's longest lists);
   // 0 until a walk has measured them. `gapped`: the current lists use that
@@ -240,6 +240,8 @@ struct Scalars {
   unsigned long long spill_used[2];  // one-pass walk: overflow pool entries taken (cells, bodies)
   u32 spilled;            // one-pass walk: groups that outgrew their slots
   unsigned long long walk_nodes;  // node records the walk tested
+  u32 walk_next[3];       // the warp walk's group counters (one-pass walk: its launches)
+  u32 eval_next;          // the evaluation's group counter
 };
 
 // The list statistics of one group per lane (valid lanes), summed and
@@ -361,7 +363,8 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
 
 struct LearnedWalk;
 
-// Stage 2: groups (with sibling packing) and the grouped walk; fills groups,
+// Stage 2 (on the scalars stage 1 zeroed): groups (with sibling packing) and
+// the grouped walk; fills groups,
 // cell_list and body_list and the interaction counters. With `lw` the walk
 // decides by the learned criterion instead of the opening angle.
 void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars *host,
@@ -380,8 +383,8 @@ struct EvalOut {
 };
 
 // Stage 3: warp-per-group evaluation of the lists into eo.
-// `counter` is one device word the kernel's work queue uses; `shape` the
-// tile shape of the softened quadrupole evaluation.
+// `counter` is one device word the kernel's work queue uses, zero at the start;
+// `shape` the tile shape.
 void evaluate_lists(const float4 *bodies, const float4 *cells, const u32 *cell_list,
                     const u32 *body_list, const uint4 *groups, u64 n_groups, float G, float eps2,
                     bool quadrupole, const EvalOut &eo, u32 *counter, cudaStream_t s,
@@ -411,8 +414,6 @@ void build_tree_graph(Workspace &ws, const double *pos, const double *mass, u64 
                       const SolverParams &sp, const GraphCaps &caps, cudaStream_t s);
 void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &caps,
                        cudaStream_t s);
-// The single walk task of a graph replay (the root), written before capture.
-void write_root_task(Workspace &ws, cudaStream_t s);
 // The evaluation of a replay: the group count from the device, nothing
 // after an abort. `groups_hint`: the group count the launch is shaped for
 // (the results do not depend on it).
@@ -461,7 +462,7 @@ void bbox_root(Workspace &ws, const double *pos, u64 n, cudaStream_t s, bool spl
 
 // Throws for a device-detected failure code (Scalars::error; 0: none): bit 4
 // non-finite positions (InvalidArgument), 8 the learned walk's count and fill
-// passes disagree, 16 a radix-sort look-back outwaited its bound, 1 (and any
+// passes disagree, 16 a sort's or scan's look-back outwaited its bound, 1 (and any
 // other) an inconsistent tree.
 void check_device_error(u32 code);
 

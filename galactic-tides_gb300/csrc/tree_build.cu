@@ -1598,7 +1598,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   // the levels, so that one read back serves both).
   u32 *count = ws.count.as<u32>(), *cscan = ws.count_scan.as<u32>();
   auto count_nodes = [&] {
-    exclusive_scan_u32(count, cscan, n, &sc->n_nodes, ws.scan_tmp, s);
+    exclusive_scan_u32(count, cscan, n, &sc->n_nodes, ws.scan_tmp, s, &sc->error);
   };
   k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
   GTC_LAUNCH_CHECK();
@@ -1627,7 +1627,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     u32 *flag = ws.flags.as<u32>(), *fscan = ws.flags_scan.as<u32>();
     k_deep_flags<<<nb, kT, 0, s>>>(leafdepth, n32, limit, flag);
     GTC_LAUNCH_CHECK();
-    exclusive_scan_u32(flag, fscan, n, &sc->deep, ws.scan_tmp, s);
+    exclusive_scan_u32(flag, fscan, n, &sc->deep, ws.scan_tmp, s, &sc->error);
     read_scalars(ws, host, s);
     const u32 nd = host->deep;
     ws.dpos.ensure(nd * 4ull);
@@ -1654,7 +1654,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     u32 *sflag = ws.flags.as<u32>(), *sscan = ws.flags_scan.as<u32>();
     k_deep_segments<<<ndb, kT, 0, s>>>(kv, dpos, nd, sflag);
     GTC_LAUNCH_CHECK();
-    exclusive_scan_u32(sflag, sscan, nd, &sc->aux, ws.scan_tmp, s);
+    exclusive_scan_u32(sflag, sscan, nd, &sc->aux, ws.scan_tmp, s, &sc->error);
     read_scalars(ws, host, s);
     int seg_bits = 1;
     while (seg_bits < 32 && (1ull << seg_bits) <= host->aux) ++seg_bits;
@@ -1776,7 +1776,7 @@ void build_tree_graph(Workspace &ws, const double *pos, const double *mass, u64 
   u32 *count = ws.count.as<u32>(), *cscan = ws.count_scan.as<u32>();
   k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
   GTC_LAUNCH_CHECK();
-  exclusive_scan_u32(count, cscan, n, &sc->n_nodes, ws.scan_tmp, s);
+  exclusive_scan_u32(count, cscan, n, &sc->n_nodes, ws.scan_tmp, s, &sc->error);
   k_check_tree_graph<<<1, 1, 0, s>>>(sc, mcap, sorted);
   GTC_LAUNCH_CHECK();
   const u32 *m_dev = &sc->n_nodes;
