@@ -1441,6 +1441,7 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
     k_check_groups_graph<<<1, 1, 0, s>>>(sc, caps.groups, ws.walk_mode < 0 ? ws.walk_super : 0);
     GTC_LAUNCH_CHECK();
   }
+  join_walk(ws, s);  // the walk reads the node records (the cells follow on the side stream)
   u32 *spill_c = ws.spill.as<u32>(), *spill_b = spill_c + n;
   // (the replays' walk: the choice of the eager solve before the capture)
   const u64 near_c = static_cast<u64>(caps.groups) * caps.slot_cells;

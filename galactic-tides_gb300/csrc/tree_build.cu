@@ -1795,13 +1795,14 @@ void build_tree_graph(Workspace &ws, const double *pos, const double *mass, u64 
   k_tree_order<<<nb, kT, 0, s>>>(pos, mass, idx, n32, ws.tpos.as<double>(), ws.tmass.as<double>(),
                                  abort);
   GTC_LAUNCH_CHECK();
-  // the centres of mass and the walk records in line; the quadrupoles and
-  // the cells on the side stream, beside the group choice and the walk (the
-  // caller joins it before the evaluation)
+  // the moments on the side stream, as in the eager build (the walk waits for
+  // the walk records, the caller joins the rest before the evaluation)
   const MomentPlan mp = plan_moments(ws, mcap, false, s, m_dev, abort);
-  launch_coms(ws, mp, s);
-  launch_pack_walk(ws, mp, root, sp.theta, s);
-  launch_quads(ws, mp, root, false, fork_side(ws, s));
+  cudaStream_t ms = fork_side(ws, s);
+  launch_coms(ws, mp, ms);
+  launch_pack_walk(ws, mp, root, sp.theta, ms);
+  mark_walk_ready(ws, ms);
+  launch_quads(ws, mp, root, false, ms);
   pack_bodies_tree(ws, n32, root, abort, s);
 }
 
