@@ -171,119 +171,6 @@ struct LearnedJoin {
   }
 };
 
-// The grouped solver on device arrays (caller order in and out).
-void group_force(gtc_context *ctx, const double *pos, const double *mass, u64 n,
-                 const gtc::SolverParams &sp, double *acc, double *pot) {
-  if (n > 0xffffffffull) throw gtc::RuntimeError("too many particles for the 32 bit GPU indices");
-  cudaStream_t s = ctx->stream;
-  gtc::Workspace &ws = ctx->ws;
-  ctx->have_group = false;
-  ctx->stats = gtc_stats{};
-  const unsigned long long launches0 = gtc::launches_so_far();
-  if (n == 0) {
-    ws.n = ws.n_nodes = ws.n_groups = ws.n_cell_list = ws.n_body_list = 0;
-    ctx->have_group = true;
-    ctx->last = sp;
-    return;
-  }
-  // The learned walk needs a model and |a| of a previous solve of the same
-  // bodies; otherwise the theta walk runs (the fallback).
-  const bool learned = sp.criterion == GTC_CRITERION_LEARNED && ctx->have_model &&
-                       ctx->prev_n == n;
-  for (bool &h : ws.stage_hit) h = false;
-  GTC_CUDA(cudaEventRecord(ctx->ev[0], s));
-  const gtc::SideJoin side_join{ws, s};
-  gtc::build_tree(ws, pos, mass, n, sp, s, ctx->host_sc, !learned);
-  GTC_CUDA(cudaEventRecord(ctx->ev[1], s));
-  LearnedJoin learned_join{ctx, s, false};
-  if (learned) {
-    // the walk's inputs from FP32 moment estimates, on their own stream
-    // beside the group choice (the walk waits for them); the walk then runs
-    // while the side stream accumulates the FP64 moments the evaluation reads
-    if (!ctx->lstream) {
-      int least = 0, greatest = 0;
-      GTC_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-      GTC_CUDA(cudaStreamCreateWithPriority(&ctx->lstream, cudaStreamNonBlocking, greatest));
-      GTC_CUDA(cudaEventCreateWithFlags(&ctx->lfork, cudaEventDisableTiming));
-      GTC_CUDA(cudaEventCreateWithFlags(&ctx->ldone, cudaEventDisableTiming));
-    }
-    GTC_CUDA(cudaEventRecord(ctx->lfork, s));
-    GTC_CUDA(cudaStreamWaitEvent(ctx->lstream, ctx->lfork, 0));
-    learned_join.active = true;
-    gtc::learned_walk_inputs(ws, ctx->lscratch, ctx->cfeat,
-                             static_cast<float>(1.0 / ctx->guard_theta), ctx->model_ymean,
-                             ctx->lstream);
-    GTC_CUDA(cudaEventRecord(ctx->ldone, ctx->lstream));
-    gtc::LearnedWalk lw;
-    lw.inputs_ready = ctx->ldone;
-    lw.net = ctx->net.as<gtc::LearnedNet>();
-    lw.cfeat = ctx->cfeat.as<gtc::CellFeat>();
-    lw.gtol = &ctx->gtol;
-    lw.scratch = &ctx->lscratch;
-    lw.y_mean = ctx->model_ymean;
-    lw.prev_amag = ctx->prev_amag.as<float>();
-    lw.alpha = sp.alpha;
-    lw.G = sp.G;
-    lw.inv_theta_guard = static_cast<float>(1.0 / ctx->guard_theta);
-    lw.band = ctx->band_override >= 0 ? static_cast<float>(ctx->band_override) : ctx->model_band;
-    lw.walk_budget = ctx->walk_budget == 0 ? ~0u : ctx->walk_budget;
-    lw.pair_budget = ctx->pair_budget == 0 ? ~0u : ctx->pair_budget;
-    lw.plan_rounds = !ctx->read_every_round;
-    lw.warps_mode = ctx->learned_warps;
-    gtc::build_lists(ws, sp, s, ctx->host_sc, &lw);
-  } else {
-    gtc::build_lists(ws, sp, s, ctx->host_sc);
-  }
-  GTC_CUDA(cudaEventRecord(ctx->ev[2], s));
-  if (n > 0) {
-    ws.out.ensure(n * sizeof(float4));
-    if (ctx->have_model) ctx->prev_amag.ensure(n * sizeof(float));  // |a| for the next learned solve
-    const gtc::EvalOut eo{ws.out.as<float4>(), ws.idx.as<u32>(), acc, pot,
-                          ctx->have_model ? ctx->prev_amag.as<float>() : nullptr};
-    GTC_CUDA(cudaEventRecord(ctx->ev[4], s));
-    gtc::evaluate_lists(ws.bodies.as<float4>(), ws.cells.as<float4>(), ws.cell_list.as<u32>(),
-                        ws.body_list.as<u32>(), ws.groups.as<uint4>(), ws.n_groups,
-                        static_cast<float>(sp.G), static_cast<float>(sp.eps * sp.eps),
-                        sp.quadrupole != 0, eo, &ws.scalars.as<gtc::Scalars>()->eval_next, s,
-                        ws.eval_shape);
-    GTC_CUDA(cudaEventRecord(ctx->ev[5], s));
-  }
-  GTC_CUDA(cudaEventRecord(ctx->ev[3], s));
-  GTC_CUDA(cudaMemcpyAsync(ctx->host_sc, ws.scalars.ptr, sizeof(gtc::Scalars),
-                           cudaMemcpyDeviceToHost, s));
-  GTC_CUDA(cudaStreamSynchronize(s));
-  gtc::check_device_error(ctx->host_sc->error);
-  gtc_stats &st = ctx->stats;
-  st.tree_ms = elapsed(ctx->ev[0], ctx->ev[1]);
-  st.lists_ms = elapsed(ctx->ev[1], ctx->ev[2]);
-  st.evaluate_ms = elapsed(ctx->ev[2], ctx->ev[3]);
-  st.total_ms = elapsed(ctx->ev[0], ctx->ev[3]);
-  st.eval_kernel_ms = elapsed(ctx->ev[4], ctx->ev[5]);
-  st.kernel_launches = gtc::launches_so_far() - launches0;
-  if (n > 0) {
-    const gtc::Scalars &h = *ctx->host_sc;
-    st.cell_interactions = h.cell_interactions;
-    st.body_interactions = h.body_interactions;
-    st.max_list = h.max_list;
-    st.max_group = h.max_group;
-    st.depth = h.depth;
-    st.walk_tests_fp64 = h.fp64_tests;
-    st.mlp_rows = h.mlp_rows;
-    st.mlp_batches = h.mlp_batches;
-  }
-  st.criterion_used = learned ? GTC_CRITERION_LEARNED : GTC_CRITERION_THETA;
-  st.list_passes = ws.list_passes;
-  st.spilled_groups = n > 0 ? ctx->host_sc->spilled : 0;
-  st.walk_nodes = n > 0 ? ctx->host_sc->walk_nodes : 0;
-  ctx->prev_n = ctx->have_model ? n : 0;
-  st.n_cell_list = ws.n_cell_list;
-  st.n_body_list = ws.n_body_list;
-  st.n_nodes = static_cast<u32>(ws.n_nodes);
-  st.n_groups = static_cast<u32>(ws.n_groups);
-  ctx->have_group = true;
-  ctx->last = sp;
-}
-
 // The capacities of a captured solve of n bodies and the buffers they need:
 // the last eager solve's sizes (hs, ws) with headroom (list slots with
 // twice the headroom: the longest of many lists moves more than the totals
@@ -294,7 +181,8 @@ void reserve_graph(gtc::Workspace &ws, const gtc::Scalars &hs, double headroom, 
   const double f = 1.0 + headroom;
   const u64 pad = headroom > 0 ? 1024 : 0;
   caps.nodes = static_cast<u32>(std::min<u64>(static_cast<u64>(ws.n_nodes * f) + pad, 0xfffffff0ull));
-  caps.depth = std::min<int>(gtc::kMaxDepth, static_cast<int>(hs.depth) + (pad ? 2 : 0));
+  // (levels sorted: this and one more, rounded up to whole passes)
+  caps.depth = std::min<int>(gtc::kMaxDepth, static_cast<int>(hs.depth));
   // list slots: the last walk's group count, and its longest lists with
   // twice the headroom (the longest of many lists moves more than the
   // totals do); offsets stay below 2^32 (a replay that needs more aborts)
@@ -310,8 +198,9 @@ void reserve_graph(gtc::Workspace &ws, const gtc::Scalars &hs, double headroom, 
   const bool split = ws.list_passes == 1;
   caps.slot_cells = slot(hs.max_cells);
   caps.slot_bodies = slot(hs.max_bodies);
-  caps.slot_near_cells = slot(split ? hs.max_near_cells : hs.max_cells);
-  caps.slot_near_bodies = slot(split ? hs.max_near_bodies : hs.max_bodies);
+  // (the warp walk writes whole lists into the first slots)
+  caps.slot_near_cells = ws.walk_warps ? 0 : slot(split ? hs.max_near_cells : hs.max_cells);
+  caps.slot_near_bodies = ws.walk_warps ? 0 : slot(split ? hs.max_near_bodies : hs.max_bodies);
   auto pool = [&](u32 rest, u32 near) {
     const u64 used = static_cast<u64>(caps.groups) * (static_cast<u64>(rest) + near);
     const u64 room = used < 0xffffffffull ? 0xffffffffull - used : 0;
@@ -356,6 +245,229 @@ void reserve_graph(gtc::Workspace &ws, const gtc::Scalars &hs, double headroom, 
   ws.splitpt.ensure(2 * n * sizeof(u32));
   ws.out.ensure(n * sizeof(float4));
   gtc::reserve_scans(ws.scan_tmp, std::max<u64>(n, m));
+}
+
+// Reads a solve's scalars back and fills the context's statistics.
+void finish_solve(gtc_context *ctx, u64 n, const gtc::SolverParams &sp, bool learned) {
+  const gtc::Workspace &ws = ctx->ws;
+  const gtc::Scalars &h = *ctx->host_sc;
+  gtc_stats &st = ctx->stats;
+  st.tree_ms = elapsed(ctx->ev[0], ctx->ev[1]);
+  st.lists_ms = elapsed(ctx->ev[1], ctx->ev[2]);
+  st.evaluate_ms = elapsed(ctx->ev[2], ctx->ev[3]);
+  st.total_ms = elapsed(ctx->ev[0], ctx->ev[3]);
+  st.eval_kernel_ms = elapsed(ctx->ev[4], ctx->ev[5]);
+  st.cell_interactions = h.cell_interactions;
+  st.body_interactions = h.body_interactions;
+  st.max_list = h.max_list;
+  st.max_group = h.max_group;
+  st.depth = h.depth;
+  st.walk_tests_fp64 = h.fp64_tests;
+  st.mlp_rows = h.mlp_rows;
+  st.mlp_batches = h.mlp_batches;
+  st.criterion_used = learned ? GTC_CRITERION_LEARNED : GTC_CRITERION_THETA;
+  st.list_passes = ws.list_passes;
+  st.spilled_groups = h.spilled;
+  st.walk_nodes = h.walk_nodes;
+  ctx->prev_n = ctx->have_model ? n : 0;
+  st.n_cell_list = ws.n_cell_list;
+  st.n_body_list = ws.n_body_list;
+  st.n_nodes = static_cast<u32>(ws.n_nodes);
+  st.n_groups = static_cast<u32>(ws.n_groups);
+  ctx->have_group = true;
+  ctx->last = sp;
+}
+
+void read_scalars(gtc_context *ctx, cudaStream_t s) {
+  GTC_CUDA(cudaMemcpyAsync(ctx->host_sc, ctx->ws.scalars.ptr, sizeof(gtc::Scalars),
+                           cudaMemcpyDeviceToHost, s));
+  GTC_CUDA(cudaStreamSynchronize(s));
+}
+
+// The evaluation's outputs of a solve (|a| too for the next learned one).
+gtc::EvalOut solve_out(gtc_context *ctx, u64 n, double *acc, double *pot) {
+  gtc::Workspace &ws = ctx->ws;
+  ws.out.ensure(n * sizeof(float4));
+  if (ctx->have_model) ctx->prev_amag.ensure(n * sizeof(float));
+  return gtc::EvalOut{ws.out.as<float4>(), ws.idx.as<u32>(), acc, pot,
+                      ctx->have_model ? ctx->prev_amag.as<float>() : nullptr};
+}
+
+bool same_lists(const gtc::SolverParams &a, const gtc::SolverParams &b) {
+  return a.theta == b.theta && a.group_size == b.group_size && a.leaf_size == b.leaf_size &&
+         a.pack == b.pack;
+}
+
+// Remembers a theta solve's sizes for the next one.
+void plan_quick(gtc_context *ctx, u64 n, const gtc::SolverParams &sp) {
+  const gtc::Workspace &ws = ctx->ws;
+  gtc_context::QuickPlan &q = ctx->quick;
+  const gtc::Scalars &h = *ctx->host_sc;
+  // the buffers reserved before serve on while the sizes stay well inside them
+  const bool fits = q.valid && q.reserved && q.n == n && same_lists(q.sp, sp) && h.spilled == 0 &&
+                    q.walk_super == ws.walk_super && ws.n_nodes < q.caps.nodes - q.caps.nodes / 16 &&
+                    ws.n_groups < q.caps.groups - q.caps.groups / 16;
+  q.valid = ws.key_words == 1 && ws.walk_warps && ws.walk_split_depth == 0;
+  q.reserved = fits;
+  q.n = n;
+  q.n_nodes = ws.n_nodes;
+  q.n_groups = ws.n_groups;
+  q.list_passes = ws.list_passes;
+  q.walk_mode = ws.walk_mode;
+  q.walk_super = ws.walk_super;
+  q.sp = sp;
+  q.sizes = h;
+}
+
+// A theta solve launched whole from the last one's sizes, with nothing read
+// back before its end: the kernels of a captured step, grids and buffers sized
+// by those with headroom, counts read on the device. False when it outgrew
+// them (its kernels then stopped where that showed): solve by reading sizes.
+// Without the two read backs 50k bodies take 0.44 instead of 0.47 ms, 200k 0.83
+// instead of 0.86 (2M: the same).
+bool group_force_quick(gtc_context *ctx, const double *pos, const double *mass, u64 n,
+                       const gtc::SolverParams &sp, double *acc, double *pot) {
+  cudaStream_t s = ctx->stream;
+  gtc::Workspace &ws = ctx->ws;
+  gtc_context::QuickPlan &q = ctx->quick;
+  if (!q.reserved) {
+    ws.n_nodes = q.n_nodes;
+    ws.n_groups = q.n_groups;
+    ws.list_passes = q.list_passes;
+    ws.walk_warps = true;
+    reserve_graph(ws, q.sizes, 0.25, n, q.caps);
+    q.reserved = true;
+  }
+  ws.walk_warps = true;
+  ws.walk_super = q.walk_super;
+  const gtc::Scalars *sc = ws.scalars.as<gtc::Scalars>();
+  {
+    const gtc::SideJoin side_join{ws, s};
+    gtc::join_side(ws, s);  // nothing of an earlier call may still write the buffers
+    GTC_CUDA(cudaEventRecord(ctx->ev[0], s));
+    gtc::build_tree_graph(ws, pos, mass, n, sp, q.caps, s);
+    GTC_CUDA(cudaEventRecord(ctx->ev[1], s));
+    gtc::build_lists_graph(ws, sp, q.caps, s);
+    gtc::join_side(ws, s);  // the cells
+    GTC_CUDA(cudaEventRecord(ctx->ev[2], s));
+    GTC_CUDA(cudaEventRecord(ctx->ev[4], s));
+    gtc::evaluate_lists_graph(ws.bodies.as<float4>(), ws.cells.as<float4>(),
+                              ws.cell_list.as<u32>(), ws.body_list.as<u32>(),
+                              ws.groups.as<uint4>(), q.caps.groups, q.n_groups, sc,
+                              static_cast<float>(sp.G), static_cast<float>(sp.eps * sp.eps),
+                              sp.quadrupole != 0, solve_out(ctx, n, acc, pot),
+                              &ws.scalars.as<gtc::Scalars>()->eval_next, s, ws.eval_shape);
+    GTC_CUDA(cudaEventRecord(ctx->ev[5], s));
+    GTC_CUDA(cudaEventRecord(ctx->ev[3], s));
+  }
+  read_scalars(ctx, s);
+  gtc::check_device_error(ctx->host_sc->error);
+  if (ctx->host_sc->abort) return false;
+  const gtc::Scalars &h = *ctx->host_sc;
+  ws.n_nodes = h.n_nodes;
+  ws.n_groups = h.n_groups;
+  ws.n_cell_list = h.n_cell_list;
+  ws.n_body_list = h.n_body_list;
+  ws.tree_depth = static_cast<int>(h.depth);
+  ws.sort_levels = static_cast<int>(h.depth) + 1;
+  ws.gapped = true;
+  ws.lists_unordered = true;
+  ws.list_passes = 1;
+  return true;
+}
+
+// Below this many bodies a solve reads its sizes back.
+constexpr u64 kQuickBodies = 256;
+
+// The grouped solver on device arrays (caller order in and out).
+void group_force(gtc_context *ctx, const double *pos, const double *mass, u64 n,
+                 const gtc::SolverParams &sp, double *acc, double *pot) {
+  if (n > 0xffffffffull) throw gtc::RuntimeError("too many particles for the 32 bit GPU indices");
+  cudaStream_t s = ctx->stream;
+  gtc::Workspace &ws = ctx->ws;
+  ctx->have_group = false;
+  ctx->stats = gtc_stats{};
+  const unsigned long long launches0 = gtc::launches_so_far();
+  if (n == 0) {
+    ws.n = ws.n_nodes = ws.n_groups = ws.n_cell_list = ws.n_body_list = 0;
+    ctx->have_group = true;
+    ctx->last = sp;
+    return;
+  }
+  // The learned walk needs a model and |a| of a previous solve of the same
+  // bodies; otherwise the theta walk runs (the fallback).
+  const bool learned = sp.criterion == GTC_CRITERION_LEARNED && ctx->have_model &&
+                       ctx->prev_n == n;
+  for (bool &h : ws.stage_hit) h = false;
+  if (!learned && ctx->quick.valid && ctx->quick.n == n && same_lists(ctx->quick.sp, sp) &&
+      ctx->quick.walk_mode == ws.walk_mode && !ws.stage_on && n >= kQuickBodies) {
+    if (group_force_quick(ctx, pos, mass, n, sp, acc, pot)) {
+      finish_solve(ctx, n, sp, false);
+      ctx->stats.kernel_launches = gtc::launches_so_far() - launches0;
+      plan_quick(ctx, n, sp);
+      return;
+    }
+    ctx->quick.valid = false;
+  }
+  GTC_CUDA(cudaEventRecord(ctx->ev[0], s));
+  const gtc::SideJoin side_join{ws, s};
+  gtc::build_tree(ws, pos, mass, n, sp, s, ctx->host_sc, !learned);
+  GTC_CUDA(cudaEventRecord(ctx->ev[1], s));
+  LearnedJoin learned_join{ctx, s, false};
+  if (learned) {
+    // the walk's inputs from FP32 moment estimates, on their own stream
+    // beside the group choice (the walk waits for them); the walk then runs
+    // while the side stream accumulates the FP64 moments the evaluation reads
+    if (!ctx->lstream) {
+      int least = 0, greatest = 0;
+      GTC_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+      GTC_CUDA(cudaStreamCreateWithPriority(&ctx->lstream, cudaStreamNonBlocking, greatest));
+      GTC_CUDA(cudaEventCreateWithFlags(&ctx->lfork, cudaEventDisableTiming));
+      GTC_CUDA(cudaEventCreateWithFlags(&ctx->ldone, cudaEventDisableTiming));
+    }
+    GTC_CUDA(cudaEventRecord(ctx->lfork, s));
+    GTC_CUDA(cudaStreamWaitEvent(ctx->lstream, ctx->lfork, 0));
+    learned_join.active = true;
+    gtc::learned_walk_inputs(ws, ctx->lscratch, ctx->cfeat,
+                             static_cast<float>(1.0 / ctx->guard_theta), ctx->model_ymean,
+                             ctx->lstream);
+    GTC_CUDA(cudaEventRecord(ctx->ldone, ctx->lstream));
+    gtc::LearnedWalk lw;
+    lw.inputs_ready = ctx->ldone;
+    lw.net = ctx->net.as<gtc::LearnedNet>();
+    lw.cfeat = ctx->cfeat.as<gtc::CellFeat>();
+    lw.gtol = &ctx->gtol;
+    lw.scratch = &ctx->lscratch;
+    lw.y_mean = ctx->model_ymean;
+    lw.prev_amag = ctx->prev_amag.as<float>();
+    lw.alpha = sp.alpha;
+    lw.G = sp.G;
+    lw.inv_theta_guard = static_cast<float>(1.0 / ctx->guard_theta);
+    lw.band = ctx->band_override >= 0 ? static_cast<float>(ctx->band_override) : ctx->model_band;
+    lw.walk_budget = ctx->walk_budget == 0 ? ~0u : ctx->walk_budget;
+    lw.pair_budget = ctx->pair_budget == 0 ? ~0u : ctx->pair_budget;
+    lw.plan_rounds = !ctx->read_every_round;
+    lw.warps_mode = ctx->learned_warps;
+    gtc::build_lists(ws, sp, s, ctx->host_sc, &lw);
+  } else {
+    gtc::build_lists(ws, sp, s, ctx->host_sc);
+  }
+  GTC_CUDA(cudaEventRecord(ctx->ev[2], s));
+  const gtc::EvalOut eo = solve_out(ctx, n, acc, pot);
+  GTC_CUDA(cudaEventRecord(ctx->ev[4], s));
+  gtc::evaluate_lists(ws.bodies.as<float4>(), ws.cells.as<float4>(), ws.cell_list.as<u32>(),
+                      ws.body_list.as<u32>(), ws.groups.as<uint4>(), ws.n_groups,
+                      static_cast<float>(sp.G), static_cast<float>(sp.eps * sp.eps),
+                      sp.quadrupole != 0, eo, &ws.scalars.as<gtc::Scalars>()->eval_next, s,
+                      ws.eval_shape);
+  GTC_CUDA(cudaEventRecord(ctx->ev[5], s));
+  GTC_CUDA(cudaEventRecord(ctx->ev[3], s));
+  read_scalars(ctx, s);
+  gtc::check_device_error(ctx->host_sc->error);
+  finish_solve(ctx, n, sp, learned);
+  ctx->stats.kernel_launches = gtc::launches_so_far() - launches0;
+  if (learned) ctx->quick.valid = false;
+  else plan_quick(ctx, n, sp);
 }
 
 // One system's leapfrog step inside a captured CUDA graph: kick and drift,
@@ -1210,6 +1322,7 @@ gtc_status gtc_set_option(gtc_context *ctx, const char *name, double value) {
   return guarded(ctx, [&] {
     const std::string key = name ? name : "";
     if (!std::isfinite(value)) throw gtc::InvalidArgument("option values must be finite");
+    ctx->quick.valid = false;
     if (key == "walk_split_depth") {
       if (value != std::floor(value) || value < 0 || value > 2)
         throw gtc::InvalidArgument("walk_split_depth must be 0, 1 or 2");

@@ -264,3 +264,33 @@ def test_warp_walk_matches_thread_walk(gtc, oracle):
         err = rel_errors(aw, at)
         assert np.median(err) < 1e-6 and err.max() < 1e-4
         assert np.abs(pw / pt - 1).max() < 1e-5
+
+
+def test_solves_from_the_last_sizes(gtc):
+    """A repeated solve launches from the last one's sizes. Its results are a
+    fresh context's, bit for bit: on the same bodies, on others of as many with
+    a tree that outgrows them (redone by reading its sizes), and after other
+    calls on the context."""
+    kw = dict(G=1.0, eps=0.025, quadrupole=True, theta=0.75, group_size=32, leaf_size=8,
+              pack=True)
+    a, _, ma, _ = gtc.make_galaxy(30_000, seed=6)
+    b, _, mb, _ = gtc.make_galaxy(30_000, seed=7)
+    rng = np.random.default_rng(2)
+    c = rng.normal(size=(30_000, 3))           # many more nodes, longer lists
+    c[:2000] = 0.3 + 1e-4 * rng.normal(size=(2000, 3))
+    d = np.concatenate([rng.normal(size=(29_000, 3)) * 10.0,      # deeper than a key word
+                        1.0 + rng.normal(size=(1000, 3)) * 1e-7])
+    want = {}
+    for name, (pos, mass) in dict(a=(a, ma), b=(b, mb), c=(c, ma), d=(d, ma)).items():
+        with gtc.Context(0) as fresh:
+            want[name] = fresh.group_force(pos, mass, **kw)
+    with gtc.Context(0) as ctx:
+        for name in ("a", "a", "b", "b", "c", "c", "d", "a", "a", "tree", "a", "a"):
+            if name == "tree":
+                ctx.tree_force(c[:5000], ma[:5000])
+                continue
+            pos, mass = dict(a=(a, ma), b=(b, mb), c=(c, ma), d=(d, ma))[name]
+            acc, pot = ctx.group_force(pos, mass, **kw)
+            assert np.array_equal(acc, want[name][0]) and np.array_equal(pot, want[name][1]), name
+            st = ctx.stats()
+            assert st["n_nodes"] == len(ctx.export()["nodes"])
