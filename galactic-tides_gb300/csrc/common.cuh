@@ -95,6 +95,7 @@ void reserve_scans(DeviceBuffer &tmp, u64 n);
 // of the scratch).
 struct RadixScratch {
   DeviceBuffer counts, scan_tmp;
+  int cluster_ctas = -1;  // CTAs a cluster may have here (-1: not asked yet)
 };
 void radix_sort_pairs(u64 *keys, u32 *vals, u64 *alt_keys, u32 *alt_vals, u32 n, int bits,
                       RadixScratch &scratch, cudaStream_t s, int low_bit = 0,

@@ -16,10 +16,23 @@
 // a digit's run). Per pass a pair is read once and written once (12 B each
 // way); the former per-pass histogram read (8 B) and scan launches are gone.
 //
+// (Time at 2M, six passes: 248 us with __match_any_sync and each load beside its
+// ranking, 238 with the loads first, 215 with ballots; 35 us a pass, bound by
+// the latencies of a tile's stages. Look-backs of 1 to 16 words a time measure
+// the same.)
+//
 // A look-back waits only on tiles taken earlier from the counter, whose
 // blocks are running or done and publish their counts before waiting
 // themselves, so the waits end. Each wait is bounded all the same: past the
 // limit the kernel records error bit 16 (and the pass's output is garbage).
+//
+// Up to kClusterItems pairs a CTA of one thread-block cluster (16 CTAs where the
+// GPU takes such clusters, else 8) the whole sort is one launch: the pairs stay
+// in registers, a pass ranks them as above, the CTAs write their digit counts
+// into each other's shared memory, and each pair goes straight to its place in
+// the shared memory of the CTA that will hold it. Two cluster barriers a pass
+// replace the counting launches, the look-back and a launch per pass: five
+// passes of 5k pairs 64 -> 22 us, of 50k 68 -> 53 us.
 
 #include <utility>
 
@@ -41,6 +54,7 @@ static_assert(kThreads == kBins, "the scatter gives each thread one digit");
 constexpr u64 kAggregate = 1ull << 62;       // this tile's own count
 constexpr u64 kInclusive = 2ull << 62;       // the count of this and every earlier tile
 constexpr u64 kCountMask = (1ull << 62) - 1;
+constexpr int kBack = 4;                     // words a look-back loads at once
 constexpr u32 kSpinLimit = 1u << 22;         // polls of one word before giving up
 constexpr u32 kSortTimeout = 16u;            // error bit
 
@@ -51,6 +65,20 @@ __device__ __forceinline__ u64 load_relaxed(const u64 *p) {
 }
 __device__ __forceinline__ void store_relaxed(u64 *p, u64 v) {
   asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+
+// The lanes with digit d among those with a key: one ballot per bit. (Eight
+// ballots and their logic are some 24 instructions of a few cycles each;
+// __match_any_sync works through the warp's distinct values in turn.)
+__device__ __forceinline__ unsigned peers_of(u32 d, bool ok) {
+  unsigned peers = __ballot_sync(kFullMask, ok);
+#pragma unroll
+  for (int b = 0; b < 8; ++b) {
+    const bool bit = (d >> b) & 1u;
+    const unsigned m = __ballot_sync(kFullMask, bit);
+    peers &= bit ? m : ~m;
+  }
+  return peers;
 }
 
 // Digit counts of every pass: hist[p][d] += pairs whose digit p is d.
@@ -110,14 +138,18 @@ __global__ void __launch_bounds__(kThreads)
   u64 key[kPerLane];
   u32 val[kPerLane];
   u32 rank[kPerLane];
+  // (all loads first: the ranking's warp barriers would put them in series)
 #pragma unroll
   for (int c = 0; c < kPerLane; ++c) {
     const u64 i = base + static_cast<u64>(c) * 32 + lane;
-    const bool ok = i < n;
-    key[c] = ok ? keys[i] : 0;
-    val[c] = ok ? vals[i] : 0;
-    const u32 d = ok ? static_cast<u32>((key[c] >> shift) & 0xff) : kBins;  // kBins: no key
-    const unsigned peers = __match_any_sync(kFullMask, d);
+    key[c] = i < n ? keys[i] : 0;
+    val[c] = i < n ? vals[i] : 0;
+  }
+#pragma unroll
+  for (int c = 0; c < kPerLane; ++c) {
+    const bool ok = base + static_cast<u64>(c) * 32 + lane < n;
+    const u32 d = static_cast<u32>((key[c] >> shift) & 0xff);
+    const unsigned peers = peers_of(d, ok);
     u32 before = 0;
     if (ok) before = wh[warp][d];
     __syncwarp();
@@ -137,21 +169,32 @@ __global__ void __launch_bounds__(kThreads)
     // this tile's count of digit d, then the earlier tiles' by looking back
     u64 *mine = status + static_cast<u64>(tile) * kBins + d;
     store_relaxed(mine, (tile == 0 ? kInclusive : kAggregate) | run);
+    // Back over the earlier tiles, kBack words at a time: a hop costs an L2 round
+    // trip, and the first wave's tiles find few running totals.
     u64 excl = 0;
-    for (u32 t = tile; t > 0;) {
-      const u64 *w = status + static_cast<u64>(t - 1) * kBins + d;
-      u64 v = load_relaxed(w);
-      for (u32 spin = 0; (v >> 62) == 0; ++spin) {
-        if (spin == kSpinLimit) {
-          atomicOr(error, kSortTimeout);
-          v = kInclusive;  // give up: count 0, stop
-          break;
+    bool stop = false;
+    for (u32 t = tile; t > 0 && !stop;) {
+      u64 v[kBack];
+#pragma unroll
+      for (int k = 0; k < kBack; ++k)
+        v[k] = static_cast<u32>(k) < t
+                   ? load_relaxed(status + static_cast<u64>(t - 1 - k) * kBins + d)
+                   : kInclusive;
+#pragma unroll
+      for (int k = 0; k < kBack; ++k) {
+        if (stop) continue;
+        for (u32 spin = 0; (v[k] >> 62) == 0; ++spin) {
+          if (spin == kSpinLimit) {
+            atomicOr(error, kSortTimeout);
+            v[k] = kInclusive;  // give up: count 0, stop
+            break;
+          }
+          v[k] = load_relaxed(status + static_cast<u64>(t - 1 - k) * kBins + d);
         }
-        v = load_relaxed(w);
+        excl += v[k] & kCountMask;
+        stop = (v[k] >> 62) == 2;  // a running total: done
       }
-      excl += v & kCountMask;
-      if ((v >> 62) == 2) break;  // a running total: done
-      --t;
+      t = t > kBack ? t - kBack : 0;
     }
     if (tile > 0) store_relaxed(mine, kInclusive | (excl + run));
     gout[d] = digit_start[d] + excl;
@@ -191,6 +234,215 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// ------------------------------------------- one cluster, all passes
+
+constexpr int kCT = 1024;
+constexpr int kCWarps = kCT / 32;
+constexpr int kMaxCtas = 16;
+constexpr int kMostPerThread = 8;
+constexpr u32 kClusterItems = kCT * kMostPerThread;  // pairs per CTA at most
+
+__device__ __forceinline__ u32 cluster_rank() {
+  u32 r;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
+               ::: "memory");
+}
+// Address of this CTA's shared `p` in CTA `rank` of the cluster.
+__device__ __forceinline__ u32 remote(const void *p, u32 rank) {
+  u32 a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;"
+      : "=r"(a)
+      : "r"(static_cast<u32>(__cvta_generic_to_shared(p))), "r"(rank));
+  return a;
+}
+__device__ __forceinline__ void put(u32 addr, u32 v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ void put(u32 addr, u64 v) {
+  asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(addr), "l"(v) : "memory");
+}
+
+template <int kPer>
+struct ClusterSort {
+  u64 key[kCT * kPer];
+  u32 val[kCT * kPer];
+  u32 wh[kCWarps][kBins];      // per-warp digit counts, then starts within a quarter
+  u32 quarter[4][kBins];       // eight warps' counts, then starts within the CTA
+  u32 table[kMaxCtas][kBins];  // every CTA's digit counts
+  u32 start[kBins];            // where this CTA's pairs of each digit go
+  u32 wsum[kBins / 32];
+};
+
+// CTA r holds the pairs [r kCT kPer, (r + 1) kCT kPer) at the start of every
+// pass, item c of a lane at warp * 32 kPer + 32 c + lane of them.
+template <int kPer>
+__global__ void __launch_bounds__(kCT)
+    k_sort_cluster(u64 *keys, u32 *vals, u32 n, u32 ctas, int low_bit, int passes) {
+  extern __shared__ __align__(16) unsigned char raw[];
+  ClusterSort<kPer> &sm = *reinterpret_cast<ClusterSort<kPer> *>(raw);
+  constexpr u32 kShare = kCT * kPer;
+  const u32 rank = cluster_rank();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lt = (1u << lane) - 1u;
+  const u32 local0 = static_cast<u32>(warp) * 32 * kPer + lane;
+  const u32 base = rank * kShare + local0;
+  u64 key[kPer];
+  u32 val[kPer], place[kPer];
+#pragma unroll
+  for (int c = 0; c < kPer; ++c) {
+    const u32 i = base + 32 * c;
+    key[c] = i < n ? keys[i] : 0;
+    val[c] = i < n ? vals[i] : 0;
+  }
+  for (int p = 0; p < passes; ++p) {
+    const int shift = low_bit + 8 * p;
+    for (int b = lane; b < kBins; b += 32) sm.wh[warp][b] = 0;
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      const bool ok = base + 32 * c < n;
+      const u32 d = static_cast<u32>(key[c] >> shift) & 0xff;
+      const unsigned peers = peers_of(d, ok);
+      u32 before = 0;
+      if (ok) before = sm.wh[warp][d];
+      __syncwarp();
+      if (ok && (peers & lt) == 0) sm.wh[warp][d] = before + __popc(peers);
+      __syncwarp();
+      place[c] = before + __popc(peers & lt);
+    }
+    __syncthreads();
+    {  // starts of each warp's pairs of digit d: within eight warps ...
+      const u32 d = threadIdx.x & (kBins - 1), q = threadIdx.x / kBins;
+      u32 run = 0;
+#pragma unroll
+      for (int k = 0; k < kCWarps / 4; ++k) {
+        const u32 v = sm.wh[q * (kCWarps / 4) + k][d];
+        sm.wh[q * (kCWarps / 4) + k][d] = run;
+        run += v;
+      }
+      sm.quarter[q][d] = run;
+    }
+    __syncthreads();
+    if (threadIdx.x < kBins) {  // ... within the CTA, whose counts all CTAs get
+      const u32 d = threadIdx.x;
+      u32 run = 0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const u32 v = sm.quarter[q][d];
+        sm.quarter[q][d] = run;
+        run += v;
+      }
+      for (u32 r = 0; r < ctas; ++r) put(remote(&sm.table[rank][d], r), run);
+    }
+    cluster_sync();
+    u32 total = 0, before = 0, incl = 0;
+    if (threadIdx.x < kBins) {  // digit starts over the cluster
+      for (u32 r = 0; r < ctas; ++r) {
+        const u32 v = sm.table[r][threadIdx.x];
+        if (r < rank) before += v;
+        total += v;
+      }
+      incl = total;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u32 v = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= o) incl += v;
+      }
+      if (lane == 31) sm.wsum[warp] = incl;
+    }
+    __syncthreads();
+    if (threadIdx.x < kBins) {
+      for (int w = 0; w < warp; ++w) before += sm.wsum[w];
+      sm.start[threadIdx.x] = before + incl - total;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      if (base + 32 * c >= n) continue;
+      const u32 d = static_cast<u32>(key[c] >> shift) & 0xff;
+      const u32 to = sm.start[d] + sm.quarter[warp / (kCWarps / 4)][d] + sm.wh[warp][d] + place[c];
+      const u32 cta = to / kShare, at = to % kShare;
+      put(remote(&sm.key[at], cta), key[c]);
+      put(remote(&sm.val[at], cta), val[c]);
+    }
+    cluster_sync();
+    // (the pairs are read before the next barrier, behind which the next pass
+    // writes)
+#pragma unroll
+    for (int c = 0; c < kPer; ++c) {
+      key[c] = sm.key[local0 + 32 * c];
+      val[c] = sm.val[local0 + 32 * c];
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < kPer; ++c) {
+    const u32 i = base + 32 * c;
+    if (i < n) {
+      keys[i] = key[c];
+      vals[i] = val[c];
+    }
+  }
+}
+
+template <int kPer>
+cudaLaunchConfig_t cluster_config(u32 ctas, cudaLaunchAttribute *attr, cudaStream_t s) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = ctas;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(kCT);
+  cfg.dynamicSmemBytes = sizeof(ClusterSort<kPer>);
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+template <int kPer>
+void allow_cluster(bool sixteen) {
+  GTC_CUDA(cudaFuncSetAttribute(k_sort_cluster<kPer>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                static_cast<int>(sizeof(ClusterSort<kPer>))));
+  if (sixteen)
+    GTC_CUDA(cudaFuncSetAttribute(k_sort_cluster<kPer>,
+                                  cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+}
+
+// The CTAs a cluster of the largest kind may have here: 16, 8, or 0 (no such
+// cluster fits the GPU).
+int cluster_ctas() {
+  for (int ctas : {16, 8}) {
+    allow_cluster<kMostPerThread>(ctas == 16);
+    cudaLaunchAttribute attr;
+    const cudaLaunchConfig_t cfg =
+        cluster_config<kMostPerThread>(static_cast<u32>(ctas), &attr, nullptr);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k_sort_cluster<kMostPerThread>, &cfg) ==
+            cudaSuccess &&
+        clusters > 0)
+      return ctas;
+    (void)cudaGetLastError();
+  }
+  return 0;
+}
+
+template <int kPer>
+void launch_cluster(u64 *keys, u32 *vals, u32 n, int low_bit, int passes, bool sixteen,
+                    cudaStream_t s) {
+  allow_cluster<kPer>(sixteen);
+  u32 ctas = 1;
+  while (ctas * kCT * kPer < n) ctas *= 2;
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config<kPer>(ctas, &attr, s);
+  GTC_CUDA(cudaLaunchKernelEx(&cfg, k_sort_cluster<kPer>, keys, vals, n, ctas, low_bit, passes));
+  GTC_LAUNCH_CHECK();
+}
+
 }  // namespace
 
 void radix_sort_pairs(u64 *keys, u32 *vals, u64 *alt_keys, u32 *alt_vals, u32 n, int bits,
@@ -199,6 +451,16 @@ void radix_sort_pairs(u64 *keys, u32 *vals, u64 *alt_keys, u32 *alt_vals, u32 n,
   const u32 ntiles = ceil_div(n, kTile);
   const int passes = (bits + 7) / 8;
   if (passes > kMaxPasses) throw InvalidArgument("radix sort: more than 64 key bits");
+  if (scratch.cluster_ctas < 0) scratch.cluster_ctas = cluster_ctas();
+  const u32 ctas = static_cast<u32>(scratch.cluster_ctas);
+  if (n <= ctas * kClusterItems) {  // the fewest pairs per thread that fit
+    const bool wide = ctas == 16;
+    if (n <= ctas * kCT) launch_cluster<1>(keys, vals, n, low_bit, passes, wide, s);
+    else if (n <= ctas * kCT * 2) launch_cluster<2>(keys, vals, n, low_bit, passes, wide, s);
+    else if (n <= ctas * kCT * 4) launch_cluster<4>(keys, vals, n, low_bit, passes, wide, s);
+    else launch_cluster<8>(keys, vals, n, low_bit, passes, wide, s);
+    return;
+  }
   // scratch, sized for the most passes whatever this call needs (so that a
   // captured sort of more levels than the eager one finds it allocated):
   // per pass the status words of every tile, then the digit counts, digit

@@ -308,3 +308,16 @@ def test_keys_of_extreme_lengths(ctx, oracle, scale):
     nodes, order, lists = oracle.lists(pos, mass, theta=0.7)
     assert np.array_equal(dev["order"], order)
     assert compare_trees(dev["nodes"], nodes) == []
+
+
+@pytest.mark.parametrize("n", [2, 33, 1024, 1025, 4097, 16384, 16385, 32769, 65537, 131072,
+                               131073, 150001])
+def test_tree_order_over_sort_sizes(ctx, oracle, n):
+    """The sort by one cluster (up to 131072 pairs, one to eight a thread) and by
+    tiles (beyond): the oracle's order, equal keys in input order."""
+    pos, mass = lopsided_sphere(n, 23)
+    pos[n // 3:n // 3 + n // 50] = pos[n // 2]          # many equal keys
+    ctx.group_force(pos, mass, theta=1.0, eps=0.05)
+    order = ctx.export()["order"]
+    nodes, want, _ = oracle.lists(pos, mass, theta=1.0)
+    assert np.array_equal(order, want)
