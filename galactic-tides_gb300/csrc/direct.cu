@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "pipeline.cuh"
+#include "wide.cuh"
 
 namespace gtc {
 namespace {
@@ -146,13 +147,9 @@ struct Body64 {
 // of the third-order (Halley) iteration: with e = 1 - x y^2 exactly the
 // relative deficit of y^2, 1/sqrt(x) = y (1 - e)^(-1/2) = y (1 + e/2 + 3/8 e^2
 // + O(e^3)). An estimate good to 2^-18 leaves 5/16 e^3 < 2^-52 / 8, so the
-// result is within about one unit in the last place (the sqrt and the
-// division it replaces round twice). Five FP64 operations where sqrt and
-// division issue about fifteen, on the pipe that bounds the kernel: 4096
-// targets x 500k bodies 102.4 -> 66.1 ms (16.7 SM cycles per FP64 warp
-// instruction, 18 of them per interaction; the pipe's rate is 16). Zero,
-// subnormal, negative, infinite and NaN inputs take the plain division, as
-// before.
+// result is within about one unit in the last place (sqrt and a division
+// round twice). Zero, subnormal, negative, infinite and NaN inputs take the
+// plain division. For the distances inverse_powers does not take.
 __device__ __forceinline__ double rsqrt64(double x) {
   const u32 hi = static_cast<u32>(__double2hiint(x));
   if (hi - 0x00100000u >= 0x7fe00000u) return 1.0 / sqrt(x);
@@ -164,6 +161,12 @@ __device__ __forceinline__ double rsqrt64(double x) {
 
 // Partial sums of targets idx[blockIdx.x*kST + t] over the source slice
 // blockIdx.y; slices are reduced in order afterwards (deterministic).
+//
+// Bound: the FP64 pipe (16 cycles of an SM per warp instruction). An
+// interaction issues 8 of them: the three differences, G m / r^3 and the four
+// additions; the distance's inverse powers come from the integer pipes
+// (wide.cuh). 4096 targets x 500k bodies: 102.4 ms with sqrt and division (26
+// instructions), 66.1 ms with rsqrt64 (18), 30.1 ms so (29.5 at the pipe's rate).
 __global__ void __launch_bounds__(kST)
     k_direct64(const double *__restrict__ pos, const double *__restrict__ mass, u64 n,
                const u64 *__restrict__ idx, u64 m, u64 slice, double G, double eps2,
@@ -179,6 +182,7 @@ __global__ void __launch_bounds__(kST)
     pz = pos[3 * i + 2];
   }
   double ax = 0, ay = 0, az = 0, phi = 0;
+  const Softening soft(eps2);
   const u64 j0 = static_cast<u64>(blockIdx.y) * slice;
   const u64 j1 = min_u64(n, j0 + slice);
   for (u64 base = j0; base < j1; base += kST) {
@@ -188,18 +192,20 @@ __global__ void __launch_bounds__(kST)
     __syncthreads();
     const u32 cnt = static_cast<u32>(min_u64(kST, j1 - base));
     const u64 self = i - base;  // the target's place in this tile (past it: none)
-#pragma unroll 2
     for (u32 k = 0; k < cnt; ++k) {
       if (k == self) continue;
       const Body64 b = tile[k];
       const double dx = px - b.x, dy = py - b.y, dz = pz - b.z;
-      const double inv = rsqrt64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
-      const double gm = b.m * inv;
-      const double gm3 = gm * (inv * inv);
+      double w, w3;  // 1/r, 1/r^3
+      if (!inverse_powers(dx, dy, dz, soft, w, w3)) {
+        w = rsqrt64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
+        w3 = w * w * w;
+      }
+      const double gm3 = b.m * w3;
       ax = fma(-gm3, dx, ax);
       ay = fma(-gm3, dy, ay);
       az = fma(-gm3, dz, az);
-      phi -= gm;
+      phi = fma(-b.m, w, phi);
     }
     __syncthreads();
   }
