@@ -30,6 +30,20 @@ __device__ __forceinline__ u64 mantissa(double v, int &exponent) {
   return exponent ? (b << 11) | 0x8000000000000000ull : 0ull;
 }
 
+// 2^62 / sqrt(a 2^-62) for a in [2^62, 2^64), within 2^-59 of itself and below
+// 2^62: the SFU's estimate and one third-order step (as rsqrt64 in FP64), in
+// fixed point.
+__device__ __forceinline__ u64 inverse_sqrt(u64 a) {
+  const float f = static_cast<float>(static_cast<u32>(a >> 32)) * (1.f / (1 << 30));
+  const u32 y0 = __float2uint_rz(rsqrt_normal(f) * 4294967296.f);
+  const long long e = (1ll << 62) - static_cast<long long>(mulhi(a, static_cast<u64>(y0) * y0));
+  const long long t = static_cast<long long>(static_cast<u64>(y0) * static_cast<u32>(e) >> 32) +
+                      static_cast<long long>(static_cast<int>(e >> 32)) * y0;
+  const long long t2 = static_cast<long long>(static_cast<int>(t >> 12)) * static_cast<int>(e >> 12);
+  const u64 y = (static_cast<u64>(y0) << 30) + static_cast<u64>((t >> 1) + ((t2 >> 40) * 3 >> 1));
+  return y < (1ull << 62) ? y : (1ull << 62) - 1ull;
+}
+
 // A softening length squared, taken apart once per thread.
 struct Softening {
   u64 m;
@@ -57,16 +71,7 @@ __device__ __forceinline__ bool inverse_powers(double dx, double dy, double dz,
   const int s = lead - ((top - lead) & 1);                // h is whole
   const u64 a = s >= 0 ? sum << s : sum >> 1;
   const int h = (top - 2044 - s) / 2;
-  // y = 2^62 / sqrt(a 2^-62): the SFU's estimate and one third-order step, as
-  // rsqrt64 in FP64, in fixed point
-  const float f = static_cast<float>(static_cast<u32>(a >> 32)) * (1.f / (1 << 30));
-  const u32 y0 = __float2uint_rz(rsqrt_normal(f) * 4294967296.f);
-  const long long e = (1ll << 62) - static_cast<long long>(mulhi(a, static_cast<u64>(y0) * y0));
-  const long long t = static_cast<long long>(static_cast<u64>(y0) * static_cast<u32>(e) >> 32) +
-                      static_cast<long long>(static_cast<int>(e >> 32)) * y0;
-  const long long t2 = static_cast<long long>(static_cast<int>(t >> 12)) * static_cast<int>(e >> 12);
-  const u64 y = min((static_cast<u64>(y0) << 30) + (t >> 1) + ((t2 >> 40) * 3 >> 1),
-                    (1ull << 62) - 1ull);
+  const u64 y = inverse_sqrt(a);
   w = __longlong_as_double((static_cast<long long>(1021 - h) << 52) +
                            static_cast<long long>((y + (1ull << 8)) >> 9));
   const u64 y1 = y << 2, cube = mulhi(mulhi(y1, y1), y1);
@@ -75,6 +80,85 @@ __device__ __forceinline__ bool inverse_powers(double dx, double dy, double dz,
   w3 = __longlong_as_double((static_cast<long long>(1021 - lz - 3 * h) << 52) +
                             static_cast<long long>((c >> 11) + ((c >> 10) & 1ull)));
   return true;
+}
+
+// ------------------------------------------- the same roundings as FP64's
+//
+// Products and 1/sqrt rounded as FP64 rounds them (to nearest, ties to even),
+// bit for bit, on the integer pipes: about 22 instructions for a product and
+// 80 for the root and the quotient, against the time of 64 and of some 1600 on
+// the FP64 pipe. For normal numbers and zeros (whose products are +0); the
+// caller sees to it that no product leaves the normal range. Factors are kept
+// as 53-bit mantissas: their product's point then moves by 11 or 12 places,
+// one funnel shift a word, and signs and exponents add up in one word.
+
+struct Factor {
+  u32 hi, lo;  // 53-bit mantissa; 0 for zero
+  u32 se;      // sign and exponent where a double has them, less the leading bit
+};
+
+template <bool kNonZero = false>
+__device__ __forceinline__ Factor factor(double v) {
+  const u32 hi = static_cast<u32>(__double2hiint(v)), lo = static_cast<u32>(__double2loint(v));
+  const u32 m = (hi & 0xfffffu) | 0x100000u;
+  // (a comparison of all 64 bits with zero would be made on the FP64 pipe)
+  return Factor{kNonZero || (hi << 1) != 0u ? m : 0u, lo, hi - m};
+}
+
+template <bool kNonZero = false>
+__device__ __forceinline__ double product(const Factor &a, const Factor &b) {
+  const u64 t0 = static_cast<u64>(a.lo) * b.lo;
+  const u64 t1 = static_cast<u64>(a.hi) * b.lo + (t0 >> 32);
+  const u64 t2 = static_cast<u64>(a.lo) * b.hi + t1;
+  const u64 t3 = static_cast<u64>(a.hi) * b.hi + (t2 >> 32);
+  const u32 p0 = static_cast<u32>(t0), p1 = static_cast<u32>(t2), p2 = static_cast<u32>(t3),
+            p3 = static_cast<u32>(t3 >> 32);  // leading bit at 8 or 9, unless zero
+  const u32 up = p3 >> 9, s = 12u - up;
+  u32 hi = __funnelshift_l(p2, p3, s), lo = __funnelshift_l(p1, p2, s);
+  const u32 rest = __funnelshift_l(p0, p1, s);
+  // ties to even: behind an odd number the half counts as more
+  const u32 more = p0 << s | (lo & 1u);
+  const u32 carry = rest > 0x80000000u - (more != 0u ? 1u : 0u) ? 1u : 0u;
+  lo += carry;
+  hi += lo < carry ? 1u : 0u;
+  hi += a.se + b.se + ((up - 1022u) << 20);
+  if (!kNonZero && p3 == 0u) hi = 0u;
+  return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
+}
+
+// The high word of 2^kExp, its sign shifted out. above<kExp> gathers how far |v|'s
+// lies above it, the largest of several: 0 <= v < 2^(kExp + n) or v = 0 for all
+// of them if that is below kWord<kExp + n> - kWord<kExp>.
+template <int kExp>
+constexpr u32 kWord = static_cast<u32>(kExp + 1023) << 21;
+template <int kExp>
+__device__ __forceinline__ u32 above(double v, u32 most) {
+  const u32 k = static_cast<u32>(__double2hiint(v)) << 1, l =
+      static_cast<u32>(__double2loint(v));
+  return (k | l) == 0u ? most : max(most, k - kWord<kExp>);
+}
+
+// 1 / sqrt(x), the root and the quotient each rounded, for a normal x > 0. Each rounding takes the
+// candidate below an estimate good to 2^-58 and compares it with the midpoint
+// above it exactly, in the low 64 bits of a difference that is known to be small.
+__device__ __forceinline__ double recip_sqrt(double x) {
+  int ex;
+  const u64 m = mantissa(x, ex);
+  const int odd = (ex - 1023) & 1;
+  const u64 a = odd ? m : m >> 1;  // x = a 2^-62 4^h
+  const int h = (ex - 1023 - odd) / 2;
+  const u64 y = inverse_sqrt(a);
+  // s = sqrt(a 2^-62) in units of 2^-52
+  const u64 f = mulhi(a, y << 2) >> 10, mid = 2ull * f + 1ull;
+  const u64 s = f + (static_cast<long long>((a << 44) - mid * mid) > 0 ? 1ull : 0ull);
+  // 1 / s in units of 2^-53: y and the Newton step that turns 1/sqrt into 1/s
+  const long long d = -static_cast<long long>(s * y);
+  const u64 r = y + static_cast<u64>(static_cast<long long>(y >> 32) *
+                                     static_cast<int>(d >> 32) >> 50);
+  const u64 g = r >> 9, mid2 = 2ull * g + 1ull;
+  const u64 i = g + (-static_cast<long long>(s * mid2) > 0 ? 1ull : 0ull);
+  return __longlong_as_double((static_cast<long long>(1021 - h) << 52) +
+                              static_cast<long long>(i));
 }
 
 }  // namespace gtc

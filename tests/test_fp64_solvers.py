@@ -35,6 +35,30 @@ def test_tree_walk_leaf_longer_than_a_list_bitwise(ctx, oracle, big):
     assert np.array_equal(acc, want) and np.array_equal(pot, wpot)
 
 
+@pytest.mark.parametrize("quadrupole", [False, True])
+@pytest.mark.parametrize("case", ["planar", "line", "window", "massless", "G"])
+def test_tree_walk_products_bitwise(ctx, oracle, case, quadrupole):
+    """Products worked on the integer pipes: zero components and zero moments
+    (with their signs), lengths whose high powers leave the products' window
+    for some of a warp's interactions, bodies without mass, G other than 1."""
+    pos, mass = lopsided_sphere(2000, 12)
+    G, eps = 1.0, 0.01
+    if case == "planar":
+        pos[:, 2] = 0.0
+    elif case == "line":
+        pos[:, 1:] = -0.0
+    elif case == "window":
+        pos, eps = pos * 1e-22, 0.0
+    elif case == "massless":
+        mass[::3] = 0.0
+    else:
+        G = 6.674e-11
+    kw = dict(G=G, theta=0.6, eps=eps, quadrupole=quadrupole)
+    acc, pot = ctx.tree_force(pos, mass, **kw)
+    want, wpot, _ = oracle.tree_force(pos, mass, **kw)
+    assert np.array_equal(acc, want, equal_nan=True) and np.array_equal(pot, wpot, equal_nan=True)
+
+
 @pytest.mark.parametrize("n,m", [(1, 1), (127, 5), (128, 128), (129, 129), (3001, 257)])
 @pytest.mark.parametrize("scale", [1.0, 1e-160, 1e140])
 def test_fp64_sample_sizes_and_scales(ctx, oracle, n, m, scale):
