@@ -28,9 +28,9 @@
 // galaxy took 63 ms; in turns 32 ms (87 FP64 instructions per 32
 // interactions, the pipe 84% busy). Their products, the root and the quotient
 // then went to the integer pipes (wide.cuh), rounded alike, which leaves the
-// 25 sums: 12.3 ms, the FP64 pipe near 70% busy, the integer and multiply
-// pipes near 60%. Ten blocks an SM (96 registers, none spilled) 12.3 ms,
-// unbounded (114) 13.1; blocks of 128 and lists of 16 to 48 measure the same.
+// 25 sums: 11.7 ms, the FP64 pipe near 70% busy, the integer and multiply
+// pipes near 60%. Ten blocks an SM (96 registers, none spilled) 11.7 ms,
+// unbounded (114) 12.4; blocks of 128 and lists of 16 to 48 measure the same.
 
 #include "pipeline.cuh"
 #include "walk_test.cuh"

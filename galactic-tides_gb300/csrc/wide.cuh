@@ -114,14 +114,18 @@ __device__ __forceinline__ double product(const Factor &a, const Factor &b) {
   const u32 p0 = static_cast<u32>(t0), p1 = static_cast<u32>(t2), p2 = static_cast<u32>(t3),
             p3 = static_cast<u32>(t3 >> 32);  // leading bit at 8 or 9, unless zero
   const u32 up = p3 >> 9, s = 12u - up;
-  u32 hi = __funnelshift_l(p2, p3, s), lo = __funnelshift_l(p1, p2, s);
+  const u32 high = __funnelshift_l(p2, p3, s), low = __funnelshift_l(p1, p2, s);
   const u32 rest = __funnelshift_l(p0, p1, s);
   // ties to even: behind an odd number the half counts as more
-  const u32 more = p0 << s | (lo & 1u);
-  const u32 carry = rest > 0x80000000u - (more != 0u ? 1u : 0u) ? 1u : 0u;
-  lo += carry;
-  hi += lo < carry ? 1u : 0u;
-  hi += a.se + b.se + ((up - 1022u) << 20);
+  const u32 more = p0 << s | (low & 1u);
+  u32 hi, lo;
+  asm("{\n\t.reg .u32 t;\n\t"
+      "add.cc.u32 t, %2, 0xffffffff;\n\t"    // carry: more != 0
+      "addc.cc.u32 t, %3, 0x7fffffff;\n\t"   // carry: above the half
+      "addc.cc.u32 %0, %4, 0;\n\t"
+      "addc.u32 %1, %5, %6;\n\t}"
+      : "=r"(lo), "=r"(hi)
+      : "r"(more), "r"(rest), "r"(low), "r"(high), "r"(a.se + b.se + ((up - 1022u) << 20)));
   if (!kNonZero && p3 == 0u) hi = 0u;
   return __hiloint2double(static_cast<int>(hi), static_cast<int>(lo));
 }
