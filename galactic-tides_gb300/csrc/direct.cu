@@ -139,8 +139,10 @@ constexpr int kST = 128;   // sample targets per block
 
 __device__ __forceinline__ u64 min_u64(u64 a, u64 b) { return a < b ? a : b; }
 
-struct Body64 {
-  double x, y, z, m;  // m: G times the mass
+struct alignas(16) Body64 {
+  Fixed p[3];
+  Mass mass;  // G times the mass, taken apart; e = 0: not worked in fixed point
+  double m;
 };
 
 // 1/sqrt(x) in FP64: the SFU's estimate (rsqrt.approx.ftz.f64) and one step
@@ -159,19 +161,42 @@ __device__ __forceinline__ double rsqrt64(double x) {
   return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
+// What a source adds to its target, in FP64 coordinates: for tiles and bodies
+// that their tile's fixed point does not hold.
+struct Pair64 {
+  double dx, dy, dz, w, gm3;
+};
+__device__ __noinline__ void pair64(const double *__restrict__ source, double px, double py,
+                                    double pz, double m, const Softening &soft, double eps2,
+                                    Pair64 &o) {
+  o.dx = px - source[0];
+  o.dy = py - source[1];
+  o.dz = pz - source[2];
+  double w3;  // 1/r^3
+  if (!inverse_powers(o.dx, o.dy, o.dz, soft, o.w, w3)) {
+    o.w = rsqrt64(fma(o.dx, o.dx, fma(o.dy, o.dy, fma(o.dz, o.dz, eps2))));
+    w3 = o.w * o.w * o.w;
+  }
+  o.gm3 = m * w3;
+}
+
 // Partial sums of targets idx[blockIdx.x*kST + t] over the source slice
 // blockIdx.y; slices are reduced in order afterwards (deterministic).
 //
-// Bound: the FP64 pipe (16 cycles of an SM per warp instruction). An
-// interaction issues 8 of them: the three differences, G m / r^3 and the four
-// additions; the distance's inverse powers come from the integer pipes
-// (wide.cuh). 4096 targets x 500k bodies: 102.4 ms with sqrt and division (26
-// instructions), 66.1 ms with rsqrt64 (18), 30.1 ms so (29.5 at the pipe's rate).
+// A tile's coordinates and the targets' are kept as 96-bit integers of the
+// tile's largest exponent; an interaction is worked in integers from the
+// differences to G m / r^3 and issues four FP64 instructions, its additions
+// (wide.cuh). Bound: the FP64 pipe (16 cycles of an SM per warp instruction)
+// and the integer pipes. 4096 targets x 500k bodies: 102.4 ms with sqrt and
+// division (26 FP64 instructions), 66.1 ms with rsqrt64 (18), 30.1 ms with
+// 1/r and 1/r^3 in integers (8), 21.1 ms so: both pipes about 65% busy. Fewer
+// registers (48) 22.2 ms; the loop unrolled measures the same.
 __global__ void __launch_bounds__(kST)
     k_direct64(const double *__restrict__ pos, const double *__restrict__ mass, u64 n,
                const u64 *__restrict__ idx, u64 m, u64 slice, double G, double eps2,
                double2 *part) {
   __shared__ Body64 tile[kST];
+  __shared__ u32 largest[kST / 32];
   const u64 s = static_cast<u64>(blockIdx.x) * kST + threadIdx.x;
   const bool active = s < m;
   const u64 i = active ? idx[s] : ~0ull;
@@ -181,31 +206,68 @@ __global__ void __launch_bounds__(kST)
     py = pos[3 * i + 1];
     pz = pos[3 * i + 2];
   }
+  auto exponent = [](double v) { return static_cast<u32>(__double2hiint(v)) >> 20 & 0x7ffu; };
+  const u32 own = max(exponent(px), max(exponent(py), exponent(pz)));
   double ax = 0, ay = 0, az = 0, phi = 0;
   const Softening soft(eps2);
   const u64 j0 = static_cast<u64>(blockIdx.y) * slice;
   const u64 j1 = min_u64(n, j0 + slice);
   for (u64 base = j0; base < j1; base += kST) {
     const u64 j = base + threadIdx.x;
-    tile[threadIdx.x] = j < j1 ? Body64{pos[3 * j], pos[3 * j + 1], pos[3 * j + 2], G * mass[j]}
-                               : Body64{0, 0, 0, 0};
+    double bx = 0, by = 0, bz = 0, bm = 0;
+    if (j < j1) {
+      bx = pos[3 * j];
+      by = pos[3 * j + 1];
+      bz = pos[3 * j + 2];
+      bm = G * mass[j];
+    }
+    const u32 e = max(own, max(exponent(bx), max(exponent(by), exponent(bz))));
+    const u32 wide = __reduce_max_sync(kFullMask, e);
+    if ((threadIdx.x & 31) == 0) largest[threadIdx.x >> 5] = wide;
+    __syncthreads();  // (the tile is free: the last one's end is behind a barrier)
+    u32 most = largest[0];
+#pragma unroll
+    for (int k = 1; k < kST / 32; ++k) most = max(most, largest[k]);
+    const int scale = static_cast<int>(most);
+    Body64 own_body;
+    own_body.mass = to_mass(bm);
+    own_body.m = bm;
+    const bool held = to_fixed(bx, scale, own_body.p[0]) & to_fixed(by, scale, own_body.p[1]) &
+                      to_fixed(bz, scale, own_body.p[2]);
+    if (!held) own_body.mass.e = 0u;
+    tile[threadIdx.x] = own_body;
+    Fixed tx, ty, tz;
+    const FixedSoftening fs(soft, scale);
+    const bool fixed = (to_fixed(px, scale, tx) & to_fixed(py, scale, ty) &
+                        to_fixed(pz, scale, tz)) &&
+                       most - (1023u - kScaleSpan) < 2u * kScaleSpan && fs.most >= 0;
     __syncthreads();
     const u32 cnt = static_cast<u32>(min_u64(kST, j1 - base));
-    const u64 self = i - base;  // the target's place in this tile (past it: none)
+    // the target's place in this tile (past it: none)
+    const u32 self = i - base < kST ? static_cast<u32>(i - base) : kST;
     for (u32 k = 0; k < cnt; ++k) {
       if (k == self) continue;
-      const Body64 b = tile[k];
-      const double dx = px - b.x, dy = py - b.y, dz = pz - b.z;
-      double w, w3;  // 1/r, 1/r^3
-      if (!inverse_powers(dx, dy, dz, soft, w, w3)) {
-        w = rsqrt64(fma(dx, dx, fma(dy, dy, fma(dz, dz, eps2))));
-        w3 = w * w * w;
+      const Body64 &b = tile[k];
+      const Mass bm = b.mass;
+      Pair64 o;
+      bool done = false;
+      if (fixed && bm.e != 0u) {
+        u32 nx, ny, nz;
+        const Fixed x = difference(tx, b.p[0], nx), y = difference(ty, b.p[1], ny),
+                    z = difference(tz, b.p[2], nz);
+        done = pair_powers(x, y, z, fs, bm, scale, o.w, o.gm3);
+        done &= from_fixed(x, nx, scale, o.dx) & from_fixed(y, ny, scale, o.dy) &
+                from_fixed(z, nz, scale, o.dz);
       }
-      const double gm3 = b.m * w3;
-      ax = fma(-gm3, dx, ax);
-      ay = fma(-gm3, dy, ay);
-      az = fma(-gm3, dz, az);
-      phi = fma(-b.m, w, phi);
+      if (!done) {
+        Pair64 slow;
+        pair64(pos + 3 * (base + k), px, py, pz, b.m, soft, eps2, slow);
+        o = slow;
+      }
+      ax = fma(-o.gm3, o.dx, ax);
+      ay = fma(-o.gm3, o.dy, ay);
+      az = fma(-o.gm3, o.dz, az);
+      phi = fma(-b.m, o.w, phi);
     }
     __syncthreads();
   }

@@ -82,6 +82,132 @@ __device__ __forceinline__ bool inverse_powers(double dx, double dy, double dz,
   return true;
 }
 
+// ------------------------------------------------- differences in fixed point
+//
+// Coordinates as 96-bit integers in units of 2^(scale - 1115), `scale` the
+// largest biased exponent among those taken together: all 53 bits of a
+// coordinate down to 2^-40 of the largest fit, and differences are exact.
+
+struct Fixed {
+  u32 w[3];  // two's complement, w[2] highest; below 2^93 in magnitude
+};
+
+// False if v has bits below the unit (or is not finite or not normal).
+__device__ __forceinline__ bool to_fixed(double v, int scale, Fixed &f) {
+  const u32 hi = static_cast<u32>(__double2hiint(v)), lo = static_cast<u32>(__double2loint(v));
+  const int e = static_cast<int>(hi >> 20 & 0x7ffu), up = e - scale + 40;
+  const bool zero = (hi << 1 | lo) == 0u;
+  const u32 mh = zero ? 0u : (hi & 0xfffffu) | 0x100000u;
+  const u32 s = static_cast<u32>(up) & 31u;
+  const u32 a = lo << s, b = __funnelshift_l(lo, mh, s), c = mh >> 1 >> (31u - s);
+  const bool far = up >= 32;
+  const u32 x0 = far ? 0u : a, x1 = far ? a : b, x2 = far ? b : c;
+  const u32 n = static_cast<u32>(static_cast<int>(hi) >> 31);
+  const u64 y = (static_cast<u64>(x1 ^ n) << 32 | (x0 ^ n)) - static_cast<u64>(static_cast<long long>(static_cast<int>(n)));
+  f.w[0] = static_cast<u32>(y);
+  f.w[1] = static_cast<u32>(y >> 32);
+  f.w[2] = (x2 ^ n) + (n != 0u && y == 0ull ? 1u : 0u);
+  return zero || (e > 0 && up >= 0 && up <= 40);
+}
+
+// |a - b|; negative: 1 if a < b, else 0.
+__device__ __forceinline__ Fixed difference(const Fixed &a, const Fixed &b, u32 &negative) {
+  Fixed d;
+  asm("sub.cc.u32 %0, %3, %6;\n\t"
+      "subc.cc.u32 %1, %4, %7;\n\t"
+      "subc.u32 %2, %5, %8;"
+      : "=r"(d.w[0]), "=r"(d.w[1]), "=r"(d.w[2])
+      : "r"(a.w[0]), "r"(a.w[1]), "r"(a.w[2]), "r"(b.w[0]), "r"(b.w[1]), "r"(b.w[2]));
+  negative = d.w[2] >> 31;
+  const u32 n = 0u - negative;
+  Fixed m;
+  asm("add.cc.u32 %0, %3, %6;\n\t"
+      "addc.cc.u32 %1, %4, 0;\n\t"
+      "addc.u32 %2, %5, 0;"
+      : "=r"(m.w[0]), "=r"(m.w[1]), "=r"(m.w[2])
+      : "r"(d.w[0] ^ n), "r"(d.w[1] ^ n), "r"(d.w[2] ^ n), "r"(negative));
+  return m;
+}
+
+// A magnitude as FP64, rounded to nearest (ties away from zero). False if it is
+// below 2^-29 of the scale and not zero.
+__device__ __forceinline__ bool from_fixed(const Fixed &d, u32 negative, int scale, double &v) {
+  const u32 a = d.w[2];
+  const int lz = __clz(static_cast<int>(a));
+  const u32 hi = __funnelshift_l(d.w[1], a, lz), lo = __funnelshift_l(d.w[0], d.w[1], lz);
+  const u32 e = static_cast<u32>(scale + 2 - lz) << 20 | negative << 31;  // (leading bit added)
+  u32 r0, r1;
+  asm("{\n\t.reg .u32 t;\n\t"
+      "add.cc.u32 t, %2, 0x80000000;\n\t"
+      "addc.cc.u32 %0, %3, 0;\n\t"
+      "addc.u32 %1, %4, %5;\n\t}"
+      : "=r"(r0), "=r"(r1)
+      : "r"(lo << 21), "r"(__funnelshift_r(lo, hi, 11)), "r"(hi >> 11), "r"(e));
+  v = __hiloint2double(static_cast<int>(a != 0u ? r1 : 0u), static_cast<int>(r0));
+  return a != 0u || (d.w[1] | d.w[0]) == 0u;
+}
+
+// A mass's mantissa and exponent; e = 0 marks one that is not taken (see below).
+struct Mass {
+  u64 m;
+  u32 e, sign;
+};
+constexpr int kScaleSpan = 200, kMassSpan = 300;  // exponents about zero that are taken
+__device__ __forceinline__ Mass to_mass(double v) {
+  const u32 hi = static_cast<u32>(__double2hiint(v));
+  const u32 e = hi >> 20 & 0x7ffu;
+  int unused;
+  const u64 m = mantissa(fabs(v), unused);
+  return Mass{m, e - (1023u - kMassSpan) < 2u * kMassSpan ? e : 0u, hi & 0x80000000u};
+}
+
+// Softening in the units of squared differences, once per scale: the largest
+// shift of the differences that leaves it room (negative: none does).
+struct FixedSoftening {
+  u64 m;
+  int q, most;
+  __device__ __forceinline__ FixedSoftening(const Softening &s, int scale)
+      : m(s.m), q(2 * scale - 1016 - s.e), most(s.m ? (2 * scale - 1020 - s.e) >> 1 : 64) {}
+};
+
+// From the differences d of two bodies: w = (d^2 + eps2)^-1/2 and gm3 = mass w^3,
+// each within half a unit in the last place and 2^-55 of itself. False if the
+// bodies are too close for their unit.
+__device__ __forceinline__ bool pair_powers(const Fixed &x, const Fixed &y, const Fixed &z,
+                                            const FixedSoftening &soft, const Mass &mass,
+                                            int scale, double &w, double &gm3) {
+  // The differences to 62 bits, the largest (or the softening) leading: 64 bits
+  // of their squares' sum without l l, whose three are below a unit each. It is
+  // 2^58 to 2^62.
+  const int up = min(__clz(static_cast<int>(x.w[2] | y.w[2] | z.w[2])) - 2, soft.most);
+  if (up > 29) return false;
+  u64 hh = 0, hl = 0;
+  auto add = [&](const Fixed &d) {
+    const u32 h = __funnelshift_l(d.w[1], d.w[2], up), l = __funnelshift_l(d.w[0], d.w[1], up);
+    hh += static_cast<u64>(h) * h;
+    hl += static_cast<u64>(h) * l;
+  };
+  add(x);
+  add(y);
+  add(z);
+  const u64 sum = hh + (hl >> 31) + (soft.m >> min(soft.q - 2 * up, 63));
+  // r^2 = a 2^-62 4^h with a in [2^62, 2^64)
+  const int s = __clz(static_cast<int>(sum >> 32)) & ~1;
+  const int h = scale - 1020 - up - (s >> 1);
+  const u64 r = inverse_sqrt(sum << s);
+  w = __longlong_as_double((static_cast<long long>(1021 - h) << 52) +
+                           static_cast<long long>((r + (1ull << 8)) >> 9));
+  const u64 r1 = r << 2, g = mulhi(mulhi(mulhi(r1, r1), r1), mass.m);  // >= 2^59
+  const int lz = __clz(static_cast<int>(g >> 32));
+  const u64 c = g << lz;
+  const u64 v = (c >> 11) + ((c >> 10) & 1ull);
+  const int e = static_cast<int>(mass.e) - 1 - lz - 3 * h;
+  gm3 = __hiloint2double(
+      static_cast<int>((static_cast<u32>(v >> 32) + (static_cast<u32>(e) << 20)) | mass.sign),
+      static_cast<int>(static_cast<u32>(v)));
+  return true;
+}
+
 // ------------------------------------------- the same roundings as FP64's
 //
 // Products and 1/sqrt rounded as FP64 rounds them (to nearest, ties to even),

@@ -108,3 +108,48 @@ def test_fp64_sample_coincident_unsoftened(ctx, oracle):
     assert np.array_equal(np.isnan(acc), np.isnan(racc))
     assert np.array_equal(np.isinf(pot), np.isinf(rpot)) and np.array_equal(pot > 0, rpot > 0)
     assert np.allclose(acc[1], racc[1], rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("case", ["sheet", "line", "offset", "tiny", "masses", "soft", "hard"])
+def test_fp64_sample_fixed_point(ctx, oracle, case):
+    """What a tile's fixed point holds and what it does not: a sheet thinner
+    than its unit, zero differences, a far offset, coordinates near zero,
+    masses that are zero, negative and far apart, softening above and below
+    every distance. Each component within 1e-12 of its terms' absolute sum:
+    1500 additions and a few roundings a term in both sums, 2^-53 each."""
+    import torch
+    n = 1500
+    pos, mass = lopsided_sphere(n, 21)
+    eps = 0.05
+    if case == "sheet":
+        pos[:, 2] *= 1e-12
+    elif case == "line":
+        pos[:, 1] = 0.0
+        pos[:, 2] = -3.0
+    elif case == "offset":
+        pos += 1e9
+    elif case == "tiny":
+        pos[::5] *= 1e-16
+    elif case == "masses":
+        mass[::3] = 0.0
+        mass[1::3] *= -1e-120
+        mass[2::9] *= 1e60
+    else:
+        eps = {"soft": 1e4, "hard": 1e-9}[case]
+    idx = (np.arange(140) * 11 % n).astype(np.uint64)
+    G = 1.5
+    racc, rpot = oracle.direct_fp64(pos, mass, idx=idx, G=G, eps=eps)
+    d = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    dp, dm, di = d(pos), d(mass), d(idx.astype(np.int64))
+    acc = torch.zeros((140, 3), dtype=torch.float64, device="cuda")
+    pot = torch.zeros(140, dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    ctx.direct_fp64_device(dp.data_ptr(), dm.data_ptr(), n, di.data_ptr(), 140, acc.data_ptr(),
+                           pot.data_ptr(), G=G, eps=eps)
+    acc, pot = acc.cpu().numpy(), pot.cpu().numpy()
+    dx = pos[idx.astype(np.int64)][:, None, :] - pos[None]
+    r2 = (dx * dx).sum(2) + eps * eps
+    w = np.where(np.arange(n)[None] == idx[:, None].astype(np.int64), 0.0, 1 / np.sqrt(r2))
+    gm = G * np.abs(mass)
+    assert np.all(np.abs(acc - racc) <= 1e-12 * np.einsum("tn,tnk->tk", gm * w ** 3, np.abs(dx)))
+    assert np.all(np.abs(pot - rpot) <= 1e-12 * (gm * w).sum(1))
