@@ -32,7 +32,10 @@
 // into each other's shared memory, and each pair goes straight to its place in
 // the shared memory of the CTA that will hold it. Two cluster barriers a pass
 // replace the counting launches, the look-back and a launch per pass: five
-// passes of 5k pairs 64 -> 22 us, of 50k 68 -> 53 us.
+// passes of 5k pairs 64 -> 22 us, of 50k 68 -> 53 us. With eight pairs a thread
+// (to 131072) the one cluster is the slower: a solve of 65k bodies took the same
+// either way, one of 80k 0.537 ms against 0.504 in sweeps, of 131072 0.705 and
+// 0.661.
 
 #include <utility>
 
@@ -239,7 +242,7 @@ __global__ void __launch_bounds__(kThreads)
 constexpr int kCT = 1024;
 constexpr int kCWarps = kCT / 32;
 constexpr int kMaxCtas = 16;
-constexpr int kMostPerThread = 8;
+constexpr int kMostPerThread = 4;
 constexpr u32 kClusterItems = kCT * kMostPerThread;  // pairs per CTA at most
 
 __device__ __forceinline__ u32 cluster_rank() {
@@ -457,8 +460,7 @@ void radix_sort_pairs(u64 *keys, u32 *vals, u64 *alt_keys, u32 *alt_vals, u32 n,
     const bool wide = ctas == 16;
     if (n <= ctas * kCT) launch_cluster<1>(keys, vals, n, low_bit, passes, wide, s);
     else if (n <= ctas * kCT * 2) launch_cluster<2>(keys, vals, n, low_bit, passes, wide, s);
-    else if (n <= ctas * kCT * 4) launch_cluster<4>(keys, vals, n, low_bit, passes, wide, s);
-    else launch_cluster<8>(keys, vals, n, low_bit, passes, wide, s);
+    else launch_cluster<4>(keys, vals, n, low_bit, passes, wide, s);
     return;
   }
   // scratch, sized for the most passes whatever this call needs (so that a
