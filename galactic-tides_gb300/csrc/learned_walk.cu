@@ -611,15 +611,27 @@ __global__ void __launch_bounds__(kContWarps * 32) k_lcont(GArgs a, bool later) 
 // (accepted: the cell; opened: its subtree). Each step the lanes test the
 // first node of the 32 ranges on top; entries reach the lists in step order,
 // lane order within a step (fixed for given inputs), and the pairs deferred
-// now go to the group's pend slot for the next round.
+// now go to the group's pend slot for the next round. Leaf and small cells'
+// body runs are queued and listed 32 at a time, and a step's pushes are placed
+// by two ballots (a scan over the lanes for each, every step, before).
+//
+// Bound: the longest walks (200k: the SMs are busy 54% of the time to the last
+// one's end), then issue. Round 0 of 200k bodies 233 -> 197 us; 12 to 16 blocks an
+// SM, or stacks of 512 or 1024 ranges, measure the same.
 constexpr int kLWarps = 4;
-constexpr int kLStack = 1024;  // ranges per warp
+constexpr int kLStack = 256;  // ranges per warp
+
+struct LWarpWalk {
+  uint2 stk[kLStack];
+  u32 q_begin[64], q_count[64];  // body runs met, to be listed 32 at a time
+};
 
 __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
-  __shared__ uint2 stack_all[kLWarps][kLStack];
+  __shared__ LWarpWalk walks[kLWarps];
   const int lane = threadIdx.x & 31;
-  uint2 *stk = stack_all[threadIdx.x >> 5];
-  const unsigned below = (1u << lane) - 1u;
+  LWarpWalk &w = walks[threadIdx.x >> 5];
+  uint2 *stk = w.stk;
+  const unsigned below = (1u << lane) - 1u, above = ~below & ~(1u << lane);
   if (a.sc->list_overflow) return;  // a buffer was outgrown: the walk is redone
   const u32 root_end = lskip(a.lrec, 0);
   const bool root_leaf = a.nchild[0] == 0;
@@ -639,6 +651,20 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
     u32 *pl = a.pend + static_cast<u64>(g) * capp;  // part 0's pend slots come first
     u64 nc = round ? a.ncells[g] : 0, nb = round ? a.nbodies[g] : 0;
     u32 np = 0;
+    u32 queued = 0;
+    auto list_runs = [&](u32 runs) {  // the first of the queue, in queue order
+      const bool has = static_cast<u32>(lane) < runs;
+      const u32 begin = has ? w.q_begin[lane] : 0u, count = has ? w.q_count[lane] : 0u;
+      u32 incl = count;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const u32 t = __shfl_up_sync(kFullMask, incl, o);
+        if (lane >= o) incl += t;
+      }
+      const u64 at = nb + incl - count;
+      for (u32 j = 0; j < count && at + j < capb; ++j) bl[at + j] = begin + j;
+      nb += __shfl_sync(kFullMask, incl, 31);
+    };
     u32 kp = round ? a.roff[g] : 0u, k1 = round ? a.roff[g + 1] : 0u;
     int size = 0;
     if (round == 0) {
@@ -659,17 +685,20 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
       if (size > kLStack - 32) {
         // nearly full (a step adds at most one range per lane): lane 0
         // walks the range on top alone
+        list_runs(queued);
+        queued = 0;
+        __syncwarp();
         if (lane == 0) {
           const uint2 r = stk[size - 1];
           const bool pair = r.y >= kPairOpen;
-          LWalkState w{nc, nb, np, 0};
+          LWalkState one{nc, nb, np, 0};
           lwalk_range(a, gf, hf, acc_d2, open_d2, r.x, pair ? lskip(a.lrec, r.x) : r.y,
                       pair ? static_cast<int>(r.y - kPairOpen) : -1, cl, bl, pl, capc, capb, capp,
-                      ~0u, w);
-          nc = w.nc;
-          nb = w.nb;
-          np = w.np;
-          visits += w.visits;
+                      ~0u, one);
+          nc = one.nc;
+          nb = one.nb;
+          np = one.np;
+          visits += one.visits;
         }
         nc = __shfl_sync(kFullMask, nc, 0);
         nb = __shfl_sync(kFullMask, nb, 0);
@@ -715,19 +744,16 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
         const u64 at = np + __popc(bp & below);
         if (at < capp) pl[at] = r.x;
       }
-      u32 incl = nbo;  // bodies: inclusive scan over the lanes
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const u32 tt = __shfl_up_sync(kFullMask, incl, o);
-        if (lane >= o) incl += tt;
+      // body runs, queued in lane order and listed 32 at a time
+      const unsigned with_runs = __ballot_sync(kFullMask, nbo != 0u);
+      if (nbo) {
+        const u32 at = queued + __popc(with_runs & below);
+        w.q_begin[at] = first;
+        w.q_count[at] = nbo;
       }
-      for (u32 j = 0; j < nbo; ++j) {
-        const u64 at = nb + (incl - nbo) + j;
-        if (at < capb) bl[at] = first + j;
-      }
+      queued += __popc(with_runs);
       nc += __popc(bc);
       np += __popc(bp);
-      nb += __shfl_sync(kFullMask, incl, 31);
       // the next ranges: the opened node's children [r.x + 1, skip) above
       // the rest of its range [skip, r.y)
       bool has_rest = false, has_kids = false;
@@ -740,20 +766,28 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
           has_kids = verdict == 0 && !leaf && r.x + 1 < kids_end;
         }
       }
-      const u32 npush = (has_rest ? 1u : 0u) + (has_kids ? 1u : 0u);
-      u32 from = npush;  // pushes of this lane and the lanes above it
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const u32 tt = __shfl_down_sync(kFullMask, from, o);
-        if (lane + o < 32) from += tt;
-      }
-      const u32 base = static_cast<u32>(size) + from - npush;
-      if (has_rest) stk[base] = make_uint2(skip, rend);
-      if (has_kids) stk[base + (has_rest ? 1u : 0u)] = make_uint2(r.x + 1, kids_end);
-      size += static_cast<int>(__shfl_sync(kFullMask, from, 0));
+      const unsigned rests = __ballot_sync(kFullMask, has_rest),
+                     kids = __ballot_sync(kFullMask, has_kids);
+      u32 at = static_cast<u32>(size) + __popc(rests & above) + __popc(kids & above);
+      if (has_rest) stk[at++] = make_uint2(skip, rend);
+      if (has_kids) stk[at] = make_uint2(r.x + 1, kids_end);
+      size += __popc(rests) + __popc(kids);
       bad = __any_sync(kFullMask, bad);
       __syncwarp();
+      if (queued >= 32u) {
+        list_runs(32u);
+        queued -= 32u;
+        __syncwarp();
+        if (static_cast<u32>(lane) < queued) {
+          const u32 begin = w.q_begin[32 + lane], count = w.q_count[32 + lane];
+          w.q_begin[lane] = begin;
+          w.q_count[lane] = count;
+        }
+        __syncwarp();
+      }
     }
+    list_runs(queued);
+    __syncwarp();
     if (lane == 0) {
       a.ncells[g] = nc;
       a.nbodies[g] = nb;
