@@ -459,7 +459,7 @@ void group_force(gtc_context *ctx, const double *pos, const double *mass, u64 n,
                       ws.body_list.as<u32>(), ws.groups.as<uint4>(), ws.n_groups,
                       static_cast<float>(sp.G), static_cast<float>(sp.eps * sp.eps),
                       sp.quadrupole != 0, eo, &ws.scalars.as<gtc::Scalars>()->eval_next, s,
-                      ws.eval_shape);
+                      ws.eval_shape, &ws.scalars.as<gtc::Scalars>()->cell_interactions);
   GTC_CUDA(cudaEventRecord(ctx->ev[5], s));
   GTC_CUDA(cudaEventRecord(ctx->ev[3], s));
   read_scalars(ctx, s);

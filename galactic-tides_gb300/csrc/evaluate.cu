@@ -39,12 +39,18 @@
 // With many groups one warp works a group's passes one after another (groups
 // handed out by an atomic counter). Below kTeamGroups the four warps of a
 // block share a group's passes, so that long lists do not run alone at the
-// end. Kernel times against a kernel pairing two entries for one target, a
-// warp per group, the next round's entries loaded only when needed (seed 1
-// galaxies, quadrupoles): 5k bodies 139 -> 32 us (86 with a warp per group), 50k
-// 140 -> 101 us (133), 200k (8.9k groups) 359 -> 332 us (359 in teams), 2M 3.26 ->
-// 3.21 ms; monopoles only (a scalar kernel before) 200k 276 -> 219 us, 2M 2.39 ->
-// 1.97 ms.
+// end. From there to kWarpGroups a warp still has only a few groups to work,
+// and a group whose box spans much of the system (its list several times the
+// mean) ran on alone when the rest was done: such long groups are worked
+// first, by teams, and the others by a warp each. 200k bodies with one list of
+// 8765 entries (mean 1340): 0.415 -> 0.343 ms; with none above twice the mean 0.335
+// -> 0.342, 400k (17.7k groups) 0.637 -> 0.659, where it is not used.
+//
+// Kernel times against a kernel pairing two entries for one target, a warp per
+// group, the next round's entries loaded only when needed (seed 1 galaxies,
+// quadrupoles): 5k bodies 139 -> 32 us (86 with a warp per group), 50k 140 -> 101
+// us (133), 200k (8.9k groups) 359 -> 332 us (359 with all in teams), 2M 3.26 -> 3.21
+// ms; monopoles only (a scalar kernel before) 200k 276 -> 219 us, 2M 2.39 -> 1.97 ms.
 
 #include <algorithm>
 
@@ -57,6 +63,7 @@ constexpr int kWarpsPerBlock = 4;
 constexpr int kT = 32 * kWarpsPerBlock;
 constexpr int kBlocksPerSm = 5;   // 96 registers: 2M 3.21 ms; 4: 3.24, 6: 3.26, 7: 3.4 ms
 constexpr float kSoftEps2 = 1e-14f;  // eps^-5 stays below 1e35
+constexpr int kNoGroups = 0, kAllGroups = 1, kLongGroups = 2;  // worked by teams
 constexpr u32 kNone = 0xffffffffu;
 constexpr u32 kMaxSlices = 32;    // slices per group at most
 constexpr u32 kStage = 64;        // entries a warp stages per round, two per lane
@@ -199,209 +206,278 @@ __device__ __forceinline__ void add_cell(Targets &a, const float4 c, const float
 // end; nor do the zeros past a list's end need one. Otherwise the self term
 // is singular, or powers of 1/eps overflow: each entry is tested as in the
 // reference, and only real entries are worked (kU = 1).
-// kTeam: the block's warps share a group's passes (else a warp per group).
+// kTeam: the groups whose passes the block's warps share (else a warp per group).
 // kU: staged entries a lane works per inner-loop iteration (1 or 2, a
 // context option searched by gtc_autotune_eval): their arithmetic is
 // independent up to the accumulation, which stays in list order, so results
 // do not depend on it.
-template <bool kQuad, bool kSoft, bool kTeam, int kU>
+// Staged entries, per warp and round parity: slice area a of the pass holds W
+// entries from float4 a (kF4 W + 1) on (3 float4 per quadrupole cell, else 1); W
+// is even and the 16-byte gap puts the areas on different banks. Per warp
+// (kAllGroups: per slice) and target: the running sum (a, potential). (Arrays of
+// their own: one struct of them all ran 1.5% slower.)
+template <typename Stage, typename Sj, typename Sums>
+struct EvalShared {
+  Stage &stage;
+  Sj &sj;  // staged body indices (self test)
+  Sums &sums;
+};
+
+// Group g: by the warp (kNoGroups) or by the block's warps.
+template <bool kQuad, bool kSoft, int kTeam, int kU, typename Shared>
+__device__ __forceinline__ void eval_group(const Shared &sm, const float4 *__restrict__ bodies,
+                                           const float4 *__restrict__ cells,
+                                           const u32 *__restrict__ cell_list,
+                                           const u32 *__restrict__ body_list,
+                                           const uint4 *__restrict__ groups, u32 g, float G,
+                                           float eps2, const float2 e2, const EvalOut &eo,
+                                           u32 pass_cost) {
+  constexpr u32 kF4 = kQuad ? 3 : 1;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint4 q0 = groups[4ull * g], q1 = groups[4ull * g + 1], q2 = groups[4ull * g + 2],
+              q3 = groups[4ull * g + 3];
+  const SegView cs = cell_segs(q1, q2), bs = body_segs(q2, q3);  // list entry -> index
+  const u32 T = q0.y - q0.x, P = (T + 1) / 2;
+  const u32 ec = q0.z, eb = q0.w;
+  u32 S = 0;
+  float4 *sum = sm.sums[kTeam == kNoGroups ? warp : 0];
+  if (T > 0) {
+    S = choose_slices(T, ec, eb, lane, pass_cost);
+    const u32 slots = S * P;
+    const u32 passes = (slots + 31u) / 32u;
+    const float per_P = 1.f / static_cast<float>(P);
+    const Cut cut_c(ec, S), cut_b(eb, S);
+    if (kTeam != kAllGroups) {
+      if (kTeam == kNoGroups || warp == 0) sum[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+      __syncwarp();
+    }
+    // (kLongGroups: every warp of a team takes each turn's barriers)
+    const u32 ahead = kTeam == kLongGroups ? warp : 0u;
+    for (u32 p = kTeam != kNoGroups ? warp : 0u; p - ahead < passes;
+         p += kTeam != kNoGroups ? kWarpsPerBlock : 1u) {
+      const bool works = kTeam != kLongGroups || p < passes;
+      const u32 v = 32u * p + static_cast<u32>(lane);
+      const bool computes = works && v < slots;
+      const u32 slice = small_div(v, per_P), t0 = 2u * (v - slice * P),
+                t1 = min(t0 + 1u, T - 1u);
+      // the slices of the pass, and each one's share of the staging area
+      const u32 s_lo = __shfl_sync(kFullMask, slice, 0);
+      const u32 nsp = min(S - 1u, __shfl_sync(kFullMask, slice, 31)) - s_lo + 1u;
+      const u32 W = small_div(kStage, 1.f / static_cast<float>(nsp)) & ~1u;  // 2..64
+      const float per_W = 1.f / static_cast<float>(W);
+      const u32 area = slice - s_lo;
+      const float4 b0 = bodies[q0.x + (computes ? t0 : 0u)],
+                   b1 = bodies[q0.x + (computes ? t1 : 0u)];
+      Targets tg{f2(-b0.x, -b1.x), f2(-b0.y, -b1.y), f2(-b0.z, -b1.z),
+                 dup(0.f), dup(0.f), dup(0.f), dup(0.f)};
+      // The lane's two staging places (slice area and position in it) and
+      // the list entries that go there round by round: cells, then bodies.
+      u32 to_c[kPer], to_b[kPer], next[2][kPer], last[2][kPer];
+#pragma unroll
+      for (int h = 0; h < kPer; ++h) {
+        const u32 e = static_cast<u32>(lane) + 32u * h, a = small_div(e, per_W), pos = e - a * W;
+        to_c[h] = a < nsp ? a * (kF4 * W + 1u) + kF4 * pos : kNone;
+        to_b[h] = a * (W + 1u) + pos;
+#pragma unroll
+        for (int l = 0; l < 2; ++l) {
+          const Cut &cut = l ? cut_b : cut_c;
+          next[l][h] = cut.at(s_lo + a) + pos;
+          last[l][h] = a < nsp ? cut.at(s_lo + a + 1u) : 0u;
+        }
+      }
+      const u32 cell_rounds = works ? (cut_c.longest() + W - 1u) / W : 0u;
+      const u32 rounds = works ? cell_rounds + (cut_b.longest() + W - 1u) / W : 0u;
+      // the list indices of round r, kNone past the slice's end
+      u32 idx[kPer];
+      auto load_indices = [&](u32 r) {
+#pragma unroll
+        for (int h = 0; h < kPer; ++h) {
+          idx[h] = kNone;
+          if (r < cell_rounds) {
+            if (next[0][h] < last[0][h]) idx[h] = cell_list[cs.at(next[0][h])];
+            next[0][h] += W;
+          } else if (r < rounds) {
+            if (next[1][h] < last[1][h]) idx[h] = body_list[bs.at(next[1][h])];
+            next[1][h] += W;
+          }
+        }
+      };
+      // starts the copies of the entries idx names into round r's buffer
+      auto stage_round = [&](u32 r) {
+        if (r < rounds) {
+          float4 *buf = sm.stage[warp][r & 1u];
+#pragma unroll
+          for (int h = 0; h < kPer; ++h) {
+            if (to_c[h] == kNone) continue;
+            if (r < cell_rounds) {
+              copy_cell<kQuad>(buf + to_c[h], cells, idx[h]);
+            } else {
+              copy_async16(buf + to_b[h], bodies + (idx[h] == kNone ? 0u : idx[h]),
+                           idx[h] != kNone);
+              if (!kSoft) sm.sj[warp][r & 1u][to_b[h]] = idx[h];
+            }
+          }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+      };
+      load_indices(0);
+      stage_round(0);
+      load_indices(1);
+      u32 left_c = cut_c.base + (slice < cut_c.rest ? 1u : 0u),
+          left_b = cut_b.base + (slice < cut_b.rest ? 1u : 0u);
+      if (!computes) left_c = left_b = 0u;
+      for (u32 r = 0; r < rounds; ++r) {
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+        __syncwarp();  // every lane's copies of round r; round r - 1 read
+        stage_round(r + 1u);
+        load_indices(r + 2u);
+        const float4 *buf = sm.stage[warp][r & 1u];
+        if (r < cell_rounds) {
+          const u32 cnt = min(W, left_c);
+          left_c -= cnt;
+          const float4 *mine = buf + area * (kF4 * W + 1u);
+          for (u32 j = 0; j < cnt; j += kU) {
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+              const float4 c = mine[kF4 * u];
+              if (kQuad) {
+                const float4 q = mine[kF4 * u + 1];
+                const float2 w = *reinterpret_cast<const float2 *>(&mine[kF4 * u + 2]);
+                add_cell<kSoft>(tg, c, q, w, e2);
+              } else {
+                add_body<kSoft>(tg, c, e2);
+              }
+            }
+            mine += kF4 * kU;
+          }
+        } else {
+          const u32 cnt = min(W, left_b);
+          left_b -= cnt;
+          const float4 *mine = buf + area * (W + 1u);
+          for (u32 j = 0; j < cnt; j += kU) {
+#pragma unroll
+            for (int u = 0; u < kU; ++u) {
+              const float4 b = mine[u];
+              u32 self = kNone;  // the entry's target, if it is one
+              if (!kSoft) self = sm.sj[warp][r & 1u][kSoft ? 0u : area * (W + 1u) + j + u] - q0.x;
+              add_body<kSoft>(tg, b, e2, !kSoft && self == t0, !kSoft && self == t1);
+            }
+            mine += kU;
+          }
+        }
+      }
+      __syncwarp();  // the last round is read before the next pass stages
+      // this pass's partial sums onto the targets', slice by slice
+      const float4 r0 = make_float4(tg.ax.x, tg.ay.x, tg.az.x, tg.pot.x),
+                   r1 = make_float4(tg.ax.y, tg.ay.y, tg.az.y, tg.pot.y);
+      if (kTeam == kAllGroups) {
+        if (computes) {
+          sm.sums[slice][t0] = r0;
+          if (t1 != t0) sm.sums[slice][t1] = r1;
+        }
+      }
+      const int turns = kTeam == kAllGroups ? 0 : kTeam == kLongGroups ? kWarpsPerBlock : 1;
+      for (int turn = 0; turn < turns; ++turn) {
+        if (kTeam == kLongGroups) {  // the team's warps in pass order
+          __syncthreads();
+          if (turn != warp || !works) continue;
+        }
+        for (u32 a = 0; a < nsp; ++a) {
+          if (computes && area == a) {
+            float4 &u = sum[t0];
+            u = make_float4(u.x + r0.x, u.y + r0.y, u.z + r0.z, u.w + r0.w);
+            if (t1 != t0) {
+              float4 &w = sum[t1];
+              w = make_float4(w.x + r1.x, w.y + r1.y, w.z + r1.z, w.w + r1.w);
+            }
+          }
+          __syncwarp();
+        }
+      }
+    }
+  }
+  if (kTeam != kNoGroups) __syncthreads();
+  if (static_cast<u32>(lane) < T && (kTeam == kNoGroups || warp == 0)) {
+    const u32 i = q0.x + static_cast<u32>(lane);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (kTeam == kAllGroups) {
+      for (u32 s = 0; s < S; ++s) {
+        const float4 u = sm.sums[s][lane];
+        acc = make_float4(acc.x + u.x, acc.y + u.y, acc.z + u.z, acc.w + u.w);
+      }
+    } else {
+      acc = sum[lane];
+    }
+    // the self term (softened), taken back once
+    if (kSoft) acc.w -= __fmul_rn(bodies[i].w, rsqrtf(eps2));
+    write_target(eo, i, make_float4(G * acc.x, G * acc.y, G * acc.z, -G * acc.w));
+  }
+  if (kTeam != kNoGroups) __syncthreads();  // the sums are read before the next group's
+}
+
+template <bool kQuad, bool kSoft, int kTeam, int kU>
 __global__ void __launch_bounds__(kT, kBlocksPerSm)
     k_eval(const float4 *__restrict__ bodies, const float4 *__restrict__ cells,
            const u32 *__restrict__ cell_list, const u32 *__restrict__ body_list,
            const uint4 *__restrict__ groups, u32 ngroups, float G, float eps2, EvalOut eo,
-           u32 *next_group, const u32 *ng_dev, const u32 *abort, u32 pass_cost) {
-  // Staged entries, per warp and round parity: slice area a of the pass holds
-  // W entries from float4 a (kF4 W + 1) on (3 float4 per quadrupole cell, else
-  // 1); W is even and the 16-byte gap puts the areas on different banks.
-  constexpr u32 kF4 = kQuad ? 3 : 1;
-  __shared__ float4 stage[kWarpsPerBlock][2][kStage * kF4 + 32];
-  __shared__ u32 sj[kWarpsPerBlock][2][kSoft ? 1 : kStage + 32];  // staged body indices (self test)
-  // per target: the running sum (a, potential); per slice and target in a team
-  __shared__ float4 sums[kTeam ? kMaxSlices : kWarpsPerBlock][32];
+           u32 *next_group, const u32 *ng_dev, const u32 *abort, u32 pass_cost,
+           const unsigned long long *interactions) {
+  __shared__ float4 stage[kWarpsPerBlock][2][kStage * (kQuad ? 3 : 1) + 32];
+  __shared__ u32 sj[kWarpsPerBlock][2][kSoft ? 1 : kStage + 32];
+  __shared__ float4 sums[kTeam == kAllGroups ? kMaxSlices : kWarpsPerBlock][32];
   __shared__ u32 team_group;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const EvalShared<decltype(stage), decltype(sj), decltype(sums)> sm{stage, sj, sums};
+  const int lane = threadIdx.x & 31;
   if (abort && *abort) return;
   if (ng_dev) ngroups = min(ngroups, *ng_dev);
   const float2 e2 = dup(eps2);
-  for (;;) {
-    u32 g = 0;
-    if (kTeam) {
+  if (kTeam == kAllGroups) {
+    for (;;) {
       if (threadIdx.x == 0) team_group = atomicAdd(next_group, 1u);
       __syncthreads();
-      g = team_group;
-    } else {
-      if (lane == 0) g = atomicAdd(next_group, 1u);
-      g = __shfl_sync(kFullMask, g, 0);
+      const u32 g = team_group;
+      if (g >= ngroups) return;
+      eval_group<kQuad, kSoft, kAllGroups, kU>(
+          sm, bodies, cells, cell_list, body_list, groups, g, G, eps2, e2, eo, pass_cost);
     }
+  }
+  // A group's work: targets x (entries, a cell counted as so much of a body). Long:
+  // more than three quarters of a warp's share of it all.
+  constexpr u64 kCellCost = kQuad ? 5 : 2, kBodyCost = 2;
+  u64 long_work = ~0ull;
+  auto is_long = [&](const uint4 &q) {
+    return static_cast<u64>(q.y - q.x) * (kCellCost * q.z + kBodyCost * q.w) > long_work;
+  };
+  if (kTeam == kLongGroups) {
+    long_work = (kCellCost * interactions[0] + kBodyCost * interactions[1]) * 3ull /
+                (4ull * gridDim.x * kWarpsPerBlock);
+    // the long ones among the block's share, every gridDim.x-th group
+    for (u64 share = blockIdx.x; share < ngroups;) {
+      const u64 mine = share + static_cast<u64>(threadIdx.x) * gridDim.x;
+      if (threadIdx.x == 0) team_group = kNone;
+      __syncthreads();
+      if (mine < ngroups && is_long(groups[4ull * mine]))
+        atomicMin(&team_group, static_cast<u32>(mine));
+      __syncthreads();
+      const u32 g = team_group;
+      __syncthreads();
+      if (g == kNone) {
+        share += static_cast<u64>(kT) * gridDim.x;
+        continue;
+      }
+      eval_group<kQuad, kSoft, kLongGroups, kU>(
+          sm, bodies, cells, cell_list, body_list, groups, g, G, eps2, e2, eo, pass_cost);
+      share = static_cast<u64>(g) + gridDim.x;
+    }
+  }
+  for (;;) {
+    u32 g = 0;
+    if (lane == 0) g = atomicAdd(next_group, 1u);
+    g = __shfl_sync(kFullMask, g, 0);
     if (g >= ngroups) return;
-    const uint4 q0 = groups[4ull * g], q1 = groups[4ull * g + 1], q2 = groups[4ull * g + 2],
-                q3 = groups[4ull * g + 3];
-    const SegView cs = cell_segs(q1, q2), bs = body_segs(q2, q3);  // list entry -> index
-    const u32 T = q0.y - q0.x, P = (T + 1) / 2;
-    const u32 ec = q0.z, eb = q0.w;
-    u32 S = 0;
-    if (T > 0) {
-      S = choose_slices(T, ec, eb, lane, pass_cost);
-      const u32 slots = S * P;
-      const u32 passes = (slots + 31u) / 32u;
-      const float per_P = 1.f / static_cast<float>(P);
-      const Cut cut_c(ec, S), cut_b(eb, S);
-      if (!kTeam) {
-        sums[warp][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-        __syncwarp();
-      }
-      for (u32 p = kTeam ? warp : 0u; p < passes; p += kTeam ? kWarpsPerBlock : 1u) {
-        const u32 v = 32u * p + static_cast<u32>(lane);
-        const bool computes = v < slots;
-        const u32 slice = small_div(v, per_P), t0 = 2u * (v - slice * P),
-                  t1 = min(t0 + 1u, T - 1u);
-        // the slices of the pass, and each one's share of the staging area
-        const u32 s_lo = __shfl_sync(kFullMask, slice, 0);
-        const u32 nsp = min(S - 1u, __shfl_sync(kFullMask, slice, 31)) - s_lo + 1u;
-        const u32 W = small_div(kStage, 1.f / static_cast<float>(nsp)) & ~1u;  // 2..64
-        const float per_W = 1.f / static_cast<float>(W);
-        const u32 area = slice - s_lo;
-        const float4 b0 = bodies[q0.x + (computes ? t0 : 0u)],
-                     b1 = bodies[q0.x + (computes ? t1 : 0u)];
-        Targets tg{f2(-b0.x, -b1.x), f2(-b0.y, -b1.y), f2(-b0.z, -b1.z),
-                   dup(0.f), dup(0.f), dup(0.f), dup(0.f)};
-        // The lane's two staging places (slice area and position in it) and
-        // the list entries that go there round by round: cells, then bodies.
-        u32 to_c[kPer], to_b[kPer], next[2][kPer], last[2][kPer];
-#pragma unroll
-        for (int h = 0; h < kPer; ++h) {
-          const u32 e = static_cast<u32>(lane) + 32u * h, a = small_div(e, per_W), pos = e - a * W;
-          to_c[h] = a < nsp ? a * (kF4 * W + 1u) + kF4 * pos : kNone;
-          to_b[h] = a * (W + 1u) + pos;
-#pragma unroll
-          for (int l = 0; l < 2; ++l) {
-            const Cut &cut = l ? cut_b : cut_c;
-            next[l][h] = cut.at(s_lo + a) + pos;
-            last[l][h] = a < nsp ? cut.at(s_lo + a + 1u) : 0u;
-          }
-        }
-        const u32 cell_rounds = (cut_c.longest() + W - 1u) / W;
-        const u32 rounds = cell_rounds + (cut_b.longest() + W - 1u) / W;
-        // the list indices of round r, kNone past the slice's end
-        u32 idx[kPer];
-        auto load_indices = [&](u32 r) {
-#pragma unroll
-          for (int h = 0; h < kPer; ++h) {
-            idx[h] = kNone;
-            if (r < cell_rounds) {
-              if (next[0][h] < last[0][h]) idx[h] = cell_list[cs.at(next[0][h])];
-              next[0][h] += W;
-            } else if (r < rounds) {
-              if (next[1][h] < last[1][h]) idx[h] = body_list[bs.at(next[1][h])];
-              next[1][h] += W;
-            }
-          }
-        };
-        // starts the copies of the entries idx names into round r's buffer
-        auto stage_round = [&](u32 r) {
-          if (r < rounds) {
-            float4 *buf = stage[warp][r & 1u];
-#pragma unroll
-            for (int h = 0; h < kPer; ++h) {
-              if (to_c[h] == kNone) continue;
-              if (r < cell_rounds) {
-                copy_cell<kQuad>(buf + to_c[h], cells, idx[h]);
-              } else {
-                copy_async16(buf + to_b[h], bodies + (idx[h] == kNone ? 0u : idx[h]),
-                             idx[h] != kNone);
-                if (!kSoft) sj[warp][r & 1u][to_b[h]] = idx[h];
-              }
-            }
-          }
-          asm volatile("cp.async.commit_group;" ::: "memory");
-        };
-        load_indices(0);
-        stage_round(0);
-        load_indices(1);
-        u32 left_c = cut_c.base + (slice < cut_c.rest ? 1u : 0u),
-            left_b = cut_b.base + (slice < cut_b.rest ? 1u : 0u);
-        if (!computes) left_c = left_b = 0u;
-        for (u32 r = 0; r < rounds; ++r) {
-          asm volatile("cp.async.wait_group 0;" ::: "memory");
-          __syncwarp();  // every lane's copies of round r; round r - 1 read
-          stage_round(r + 1u);
-          load_indices(r + 2u);
-          const float4 *buf = stage[warp][r & 1u];
-          if (r < cell_rounds) {
-            const u32 cnt = min(W, left_c);
-            left_c -= cnt;
-            const float4 *mine = buf + area * (kF4 * W + 1u);
-            for (u32 j = 0; j < cnt; j += kU) {
-#pragma unroll
-              for (int u = 0; u < kU; ++u) {
-                const float4 c = mine[kF4 * u];
-                if (kQuad) {
-                  const float4 q = mine[kF4 * u + 1];
-                  const float2 w = *reinterpret_cast<const float2 *>(&mine[kF4 * u + 2]);
-                  add_cell<kSoft>(tg, c, q, w, e2);
-                } else {
-                  add_body<kSoft>(tg, c, e2);
-                }
-              }
-              mine += kF4 * kU;
-            }
-          } else {
-            const u32 cnt = min(W, left_b);
-            left_b -= cnt;
-            const float4 *mine = buf + area * (W + 1u);
-            for (u32 j = 0; j < cnt; j += kU) {
-#pragma unroll
-              for (int u = 0; u < kU; ++u) {
-                const float4 b = mine[u];
-                u32 self = kNone;  // the entry's target, if it is one
-                if (!kSoft) self = sj[warp][r & 1u][kSoft ? 0u : area * (W + 1u) + j + u] - q0.x;
-                add_body<kSoft>(tg, b, e2, !kSoft && self == t0, !kSoft && self == t1);
-              }
-              mine += kU;
-            }
-          }
-        }
-        __syncwarp();  // the last round is read before the next pass stages
-        // this pass's partial sums onto the targets', slice by slice
-        const float4 r0 = make_float4(tg.ax.x, tg.ay.x, tg.az.x, tg.pot.x),
-                     r1 = make_float4(tg.ax.y, tg.ay.y, tg.az.y, tg.pot.y);
-        if (kTeam) {
-          if (computes) {
-            sums[slice][t0] = r0;
-            if (t1 != t0) sums[slice][t1] = r1;
-          }
-        } else {
-          for (u32 a = 0; a < nsp; ++a) {
-            if (computes && area == a) {
-              float4 &u = sums[warp][t0];
-              u = make_float4(u.x + r0.x, u.y + r0.y, u.z + r0.z, u.w + r0.w);
-              if (t1 != t0) {
-                float4 &w = sums[warp][t1];
-                w = make_float4(w.x + r1.x, w.y + r1.y, w.z + r1.z, w.w + r1.w);
-              }
-            }
-            __syncwarp();
-          }
-        }
-      }
-    }
-    if (kTeam) __syncthreads();
-    if (static_cast<u32>(lane) < T && (!kTeam || warp == 0)) {
-      const u32 i = q0.x + static_cast<u32>(lane);
-      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (kTeam) {
-        for (u32 s = 0; s < S; ++s) {
-          const float4 u = sums[s][lane];
-          acc = make_float4(acc.x + u.x, acc.y + u.y, acc.z + u.z, acc.w + u.w);
-        }
-      } else {
-        acc = sums[warp][lane];
-      }
-      // the self term (softened), taken back once
-      if (kSoft) acc.w -= __fmul_rn(bodies[i].w, rsqrtf(eps2));
-      write_target(eo, i, make_float4(G * acc.x, G * acc.y, G * acc.z, -G * acc.w));
-    }
-    if (kTeam) __syncthreads();  // the sums are read before the next group's
+    if (kTeam == kLongGroups && is_long(groups[4ull * g])) continue;
+    eval_group<kQuad, kSoft, kNoGroups, kU>(sm, bodies, cells, cell_list, body_list, groups, g, G,
+                                            eps2, e2, eo, pass_cost);
   }
 }
 
@@ -416,25 +492,27 @@ struct EvalArgs {
   u32 *counter;
   EvalShape shape;
   const Scalars *sc;  // a graph replay: the group count and the abort word
+  const unsigned long long *interactions;  // the lists' totals: cells, bodies
 };
 
-template <bool kQuad, bool kSoft, bool kTeam, int kU>
+template <bool kQuad, bool kSoft, int kTeam, int kU>
 void launch_shape(const EvalArgs &a, int sms, cudaStream_t s) {
   int per_sm = 0;
   GTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
       &per_sm, k_eval<kQuad, kSoft, kTeam, kU>, kT, 0));
-  const u64 want = kTeam ? a.n_groups : (a.n_groups + kWarpsPerBlock - 1) / kWarpsPerBlock;
+  const u64 want = kTeam == kAllGroups ? a.n_groups : (a.n_groups + kWarpsPerBlock - 1) / kWarpsPerBlock;
   const u32 grid =
       static_cast<u32>(std::min<u64>(want, static_cast<u64>(sms) * std::max(1, per_sm)));
   k_eval<kQuad, kSoft, kTeam, kU><<<grid, kT, 0, s>>>(
       a.bodies, a.cells, a.cell_list, a.body_list, a.groups, static_cast<u32>(a.n_groups), a.G,
       a.eps2, a.eo, a.counter, a.sc ? &a.sc->n_groups : nullptr, a.sc ? &a.sc->abort : nullptr,
-      a.shape.pass_cost);
+      a.shape.pass_cost, a.interactions);
   GTC_LAUNCH_CHECK();
 }
 
-// Groups below which a block's warps share a group.
-constexpr u64 kTeamGroups = 6000;
+// Groups below which a block's warps share every group, and below which they
+// share the long ones (above).
+constexpr u64 kTeamGroups = 6000, kWarpGroups = 12000;
 
 template <bool kQuad, bool kSoft>
 void launch_eval(const EvalArgs &a, u64 groups_hint, cudaStream_t s) {
@@ -442,12 +520,16 @@ void launch_eval(const EvalArgs &a, u64 groups_hint, cudaStream_t s) {
   int dev = 0, sms = 0;
   GTC_CUDA(cudaGetDevice(&dev));
   GTC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const bool one = a.shape.pairs == 1;
   if (groups_hint < kTeamGroups) {
-    if (a.shape.pairs == 1) launch_shape<kQuad, kSoft, true, 1>(a, sms, s);
-    else launch_shape<kQuad, kSoft, true, kTwo>(a, sms, s);
+    if (one) launch_shape<kQuad, kSoft, kAllGroups, 1>(a, sms, s);
+    else launch_shape<kQuad, kSoft, kAllGroups, kTwo>(a, sms, s);
+  } else if (groups_hint < kWarpGroups && a.interactions) {
+    if (one) launch_shape<kQuad, kSoft, kLongGroups, 1>(a, sms, s);
+    else launch_shape<kQuad, kSoft, kLongGroups, kTwo>(a, sms, s);
   } else {
-    if (a.shape.pairs == 1) launch_shape<kQuad, kSoft, false, 1>(a, sms, s);
-    else launch_shape<kQuad, kSoft, false, kTwo>(a, sms, s);
+    if (one) launch_shape<kQuad, kSoft, kNoGroups, 1>(a, sms, s);
+    else launch_shape<kQuad, kSoft, kNoGroups, kTwo>(a, sms, s);
   }
 }
 
@@ -465,9 +547,9 @@ void launch_any(const EvalArgs &a, bool quadrupole, u64 groups_hint, cudaStream_
 void evaluate_lists(const float4 *bodies, const float4 *cells, const u32 *cell_list,
                     const u32 *body_list, const uint4 *groups, u64 n_groups, float G, float eps2,
                     bool quadrupole, const EvalOut &eo, u32 *counter, cudaStream_t s,
-                    const EvalShape &shape) {
+                    const EvalShape &shape, const unsigned long long *interactions) {
   launch_any(EvalArgs{bodies, cells, cell_list, body_list, groups, n_groups, G, eps2, eo, counter,
-                      shape, nullptr},
+                      shape, nullptr, interactions},
              quadrupole, n_groups, s);
 }
 
@@ -477,7 +559,7 @@ void evaluate_lists_graph(const float4 *bodies, const float4 *cells, const u32 *
                           bool quadrupole, const EvalOut &eo, u32 *counter, cudaStream_t s,
                           const EvalShape &shape) {
   launch_any(EvalArgs{bodies, cells, cell_list, body_list, groups, max_groups, G, eps2, eo,
-                      counter, shape, sc},
+                      counter, shape, sc, &sc->cell_interactions},
              quadrupole, groups_hint, s);
 }
 

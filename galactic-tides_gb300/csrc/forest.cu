@@ -262,7 +262,8 @@ void ForestRun::solve(int kick, double h, cudaStream_t s, bool write) {
                  ws.body_list.as<u32>(), ws.groups.as<uint4>(), ws.n_groups,
                  static_cast<float>(sp.G), static_cast<float>(sp.eps * sp.eps),
                  sp.quadrupole != 0, EvalOut{ws.out.as<float4>()},
-                 &ws.scalars.as<Scalars>()->eval_next, s, ws.eval_shape);
+                 &ws.scalars.as<Scalars>()->eval_next, s, ws.eval_shape,
+                 &ws.scalars.as<Scalars>()->cell_interactions);
   if (write) scatter(kick, h, nullptr, s);
   GTC_CUDA(cudaMemcpyAsync(host_sc, ws.scalars.ptr, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
   GTC_CUDA(cudaStreamSynchronize(s));

@@ -384,11 +384,13 @@ struct EvalOut {
 
 // Stage 3: warp-per-group evaluation of the lists into eo.
 // `counter` is one device word the kernel's work queue uses, zero at the start;
-// `shape` the tile shape.
+// `shape` the tile shape, `interactions` the lists' totals (cells, bodies; device; null:
+// not known, long groups then start in their turn).
 void evaluate_lists(const float4 *bodies, const float4 *cells, const u32 *cell_list,
                     const u32 *body_list, const uint4 *groups, u64 n_groups, float G, float eps2,
                     bool quadrupole, const EvalOut &eo, u32 *counter, cudaStream_t s,
-                    const EvalShape &shape = EvalShape{});
+                    const EvalShape &shape = EvalShape{},
+                    const unsigned long long *interactions = nullptr);
 
 // Capacities of a solve replayed from a CUDA graph: the sizes of the
 // buffers the graph was captured with. A replay whose tree, depth or lists

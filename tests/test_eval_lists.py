@@ -90,3 +90,40 @@ def test_small_softening_at_the_origin(ctx):
         got = ctx.tree(bodies, np.zeros((1, 12), np.float32), np.zeros(0, np.uint32),
                        np.arange(2, dtype=np.uint32), group, G=1.0, eps2=eps2)
         assert np.allclose(got, [[2, 0, 0, -2], [-1, 0, 0, -1]], rtol=1e-6, atol=0)
+
+
+@pytest.mark.parametrize("quad", [False, True])
+@pytest.mark.parametrize("eps", [0.0, 0.02])
+def test_long_groups_by_teams(gtc, quad, eps):
+    """Some 7500 groups, a few of them of bodies far apart with lists many
+    times as long: those are worked by teams of warps, the rest by a warp
+    each. The same bits as with twice the groups (a warp for every group)."""
+    import torch
+    rng = np.random.default_rng(3)
+    n = 170_000
+    pos = rng.normal(size=(n, 3))
+    pos *= (rng.random((n, 1)) ** 2 + 1e-3) / np.linalg.norm(pos, axis=1)[:, None]
+    pos[:300] = rng.uniform(-2, 2, (300, 3))
+    mass = rng.uniform(0.5, 1.5, n) / n
+    kw = dict(G=1.0, eps=eps, theta=0.75, quadrupole=quad, leaf_size=8, group_size=32, pack=1)
+    with gtc.Context(0) as ctx:
+        acc, pot = ctx.group_force(pos, mass, **kw)
+        g = ctx.export()["groups"].astype(np.int64)
+    assert 6000 <= len(g) < 12000
+    work = (g[:, 1] - g[:, 0]) * ((5 if quad else 2) * (g[:, 3] - g[:, 2])
+                                  + 2 * (g[:, 5] - g[:, 4]))
+    warps = torch.cuda.get_device_properties(0).multi_processor_count * 5 * 4
+    assert work.max() > 0.75 * work.sum() / warps
+    bufs = []
+    with gtc.Ensemble(2) as ens:
+        for i in range(2):
+            b = [torch.from_numpy(a.copy()).cuda()
+                 for a in (pos, np.zeros_like(pos), mass, np.zeros_like(pos), np.zeros(n))]
+            bufs.append(b)
+            ens.set_system(i, *[t.data_ptr() for t in b], n, **kw)
+        ens.set_option("forest", 1)
+        torch.cuda.synchronize()
+        ens.leapfrog(0.0, 1, prime=True, graph=False)
+        torch.cuda.synchronize()
+    for b in bufs:
+        assert np.array_equal(b[3].cpu().numpy(), acc) and np.array_equal(b[4].cpu().numpy(), pot)
