@@ -747,6 +747,7 @@ void set_contextless_error(const std::string &msg) { g_create_error = msg; }
 
 // Caller-order scatter for the direct path (identity order).
 __global__ void k_unpack_direct(const float4 *out, u32 n, double *acc, double *pot) {
+  grid_wait();
   const u32 i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   const float4 o = out[i];
@@ -1228,8 +1229,8 @@ gtc_status gtc_direct_force_device(gtc_context *ctx, const double *pos, const do
       throw gtc::InvalidArgument("pos, mass, acc and pot are required");
     direct_force(ctx, pos, mass, n, sp, acc, pot);
     if (n) {
-      gtc::k_unpack_direct<<<gtc::ceil_div(n, 256), 256, 0, ctx->stream>>>(
-          ctx->ws.out.as<float4>(), static_cast<u32>(n), acc, pot);
+      gtc::launch(gtc::k_unpack_direct, gtc::ceil_div(n, 256), 256, 0, ctx->stream,
+             ctx->ws.out.as<float4>(), static_cast<u32>(n), acc, pot);
       GTC_LAUNCH_CHECK();
       GTC_CUDA(cudaStreamSynchronize(ctx->stream));
     }
@@ -1256,8 +1257,8 @@ gtc_status gtc_direct_force(gtc_context *ctx, const double *pos, const double *m
     direct_force(ctx, ws.pos.as<double>(), ws.mass.as<double>(), n, sp, ws.acc.as<double>(),
                  ws.pot.as<double>());
     if (n) {
-      gtc::k_unpack_direct<<<gtc::ceil_div(n, 256), 256, 0, s>>>(
-          ws.out.as<float4>(), static_cast<u32>(n), ws.acc.as<double>(), ws.pot.as<double>());
+      gtc::launch(gtc::k_unpack_direct, gtc::ceil_div(n, 256), 256, 0, s, ws.out.as<float4>(),
+             static_cast<u32>(n), ws.acc.as<double>(), ws.pot.as<double>());
       GTC_LAUNCH_CHECK();
       GTC_CUDA(cudaMemcpyAsync(acc, ws.acc.ptr, n * 24, cudaMemcpyDeviceToHost, s));
       GTC_CUDA(cudaMemcpyAsync(pot, ws.pot.ptr, n * 8, cudaMemcpyDeviceToHost, s));
@@ -1400,8 +1401,8 @@ gtc_status gtc_leapfrog_device(gtc_context *ctx, double *pos, double *vel, const
         group_force(ctx, pos, mass, n, sp, acc, pot);
       } else {
         direct_force(ctx, pos, mass, n, sp, acc, pot);
-        gtc::k_unpack_direct<<<gtc::ceil_div(n, 256), 256, 0, s>>>(ctx->ws.out.as<float4>(),
-                                                                  static_cast<u32>(n), acc, pot);
+        gtc::launch(gtc::k_unpack_direct, gtc::ceil_div(n, 256), 256, 0, s, ctx->ws.out.as<float4>(),
+               static_cast<u32>(n), acc, pot);
         GTC_LAUNCH_CHECK();
       }
     };

@@ -62,6 +62,7 @@ template <int kDR>
 __global__ void __launch_bounds__(kDT)
     k_direct(const float4 *__restrict__ bodies, u32 n, u32 len, float G, float eps2,
              float4 *__restrict__ out) {
+  grid_wait();
   constexpr u32 kDTB = kDT * kDR;  // targets per block
   __shared__ float4 tile[kDT];  // kDT / 2 source pairs, two float4 each
   const u32 t0 = blockIdx.x * kDTB;
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(kDT)
 // out[i] = the sum of the slices' partial sums of target i, in slice order.
 __global__ void k_direct_sum(const float4 *__restrict__ part, u32 n, u32 slices,
                              float4 *__restrict__ out) {
+  grid_wait();
   const u32 i = blockIdx.x * 256 + threadIdx.x;
   if (i >= n) return;
   float4 a = part[i];
@@ -195,6 +197,7 @@ __global__ void __launch_bounds__(kST)
     k_direct64(const double *__restrict__ pos, const double *__restrict__ mass, u64 n,
                const u64 *__restrict__ idx, u64 m, u64 slice, double G, double eps2,
                double2 *part) {
+  grid_wait();
   __shared__ Body64 tile[kST];
   __shared__ u32 largest[kST / 32];
   const u64 s = static_cast<u64>(blockIdx.x) * kST + threadIdx.x;
@@ -279,6 +282,7 @@ __global__ void __launch_bounds__(kST)
 }
 
 __global__ void k_direct64_sum(const double2 *part, u64 m, u32 slices, double *acc, double *pot) {
+  grid_wait();
   const u64 s = static_cast<u64>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (s >= m) return;
   double ax = 0, ay = 0, az = 0, phi = 0;
@@ -317,12 +321,12 @@ void direct_fp32(const float4 *bodies, u32 n, float G, float eps2, float4 *out,
     dst = scratch.as<float4>();
   }
   if (targets == 4)
-    k_direct<4><<<dim3(tiles, slices), kDT, 0, s>>>(bodies, n, len, G, eps2, dst);
+    launch(k_direct<4>, dim3(tiles, slices), kDT, 0, s, bodies, n, len, G, eps2, dst);
   else
-    k_direct<2><<<dim3(tiles, slices), kDT, 0, s>>>(bodies, n, len, G, eps2, dst);
+    launch(k_direct<2>, dim3(tiles, slices), kDT, 0, s, bodies, n, len, G, eps2, dst);
   GTC_LAUNCH_CHECK();
   if (slices > 1) {
-    k_direct_sum<<<ceil_div(n, 256), 256, 0, s>>>(dst, n, slices, out);
+    launch(k_direct_sum, ceil_div(n, 256), 256, 0, s, dst, n, slices, out);
     GTC_LAUNCH_CHECK();
   }
 }
@@ -340,10 +344,10 @@ void launch_fp64_sample(const double *pos, const double *mass, u64 n, const u64 
                         double G, double eps, const Fp64SamplePlan &plan, double2 *part,
                         double *acc, double *pot, cudaStream_t s) {
   dim3 grid(ceil_div(m, kST), static_cast<u32>(plan.slices));
-  k_direct64<<<grid, kST, 0, s>>>(pos, mass, n, idx, m, plan.slice, G, eps * eps, part);
+  launch(k_direct64, grid, kST, 0, s, pos, mass, n, idx, m, plan.slice, G, eps * eps, part);
   GTC_LAUNCH_CHECK();
-  k_direct64_sum<<<ceil_div(m, 256), 256, 0, s>>>(part, m, static_cast<u32>(plan.slices), acc,
-                                                  pot);
+  launch(k_direct64_sum, ceil_div(m, 256), 256, 0, s, part, m, static_cast<u32>(plan.slices),
+         acc, pot);
   GTC_LAUNCH_CHECK();
 }
 
@@ -366,6 +370,7 @@ namespace {
 
 // Eight independent FMA chains per thread, long enough to hide latency.
 __global__ void __launch_bounds__(256) k_fma_peak(float *sink, int iters, float a, float b) {
+  grid_wait();
   float x[8];
 #pragma unroll
   for (int k = 0; k < 8; ++k) x[k] = threadIdx.x * 1e-3f + k;
@@ -395,7 +400,7 @@ double fp32_peak_tflops(cudaStream_t s) {
   float best = 1e30f;
   for (int rep = 0; rep < 4; ++rep) {
     GTC_CUDA(cudaEventRecord(a, s));
-    k_fma_peak<<<blocks, 256, 0, s>>>(sink.as<float>(), iters, 0.999f, 1e-3f);
+    launch(k_fma_peak, blocks, 256, 0, s, sink.as<float>(), iters, 0.999f, 1e-3f);
     GTC_LAUNCH_CHECK();
     GTC_CUDA(cudaEventRecord(b, s));
     GTC_CUDA(cudaEventSynchronize(b));

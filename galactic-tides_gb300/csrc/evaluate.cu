@@ -422,6 +422,7 @@ __global__ void __launch_bounds__(kT, kBlocksPerSm)
            const uint4 *__restrict__ groups, u32 ngroups, float G, float eps2, EvalOut eo,
            u32 *next_group, const u32 *ng_dev, const u32 *abort, u32 pass_cost,
            const unsigned long long *interactions) {
+  grid_wait();
   __shared__ float4 stage[kWarpsPerBlock][2][kStage * (kQuad ? 3 : 1) + 32];
   __shared__ u32 sj[kWarpsPerBlock][2][kSoft ? 1 : kStage + 32];
   __shared__ float4 sums[kTeam == kAllGroups ? kMaxSlices : kWarpsPerBlock][32];
@@ -503,10 +504,10 @@ void launch_shape(const EvalArgs &a, int sms, cudaStream_t s) {
   const u64 want = kTeam == kAllGroups ? a.n_groups : (a.n_groups + kWarpsPerBlock - 1) / kWarpsPerBlock;
   const u32 grid =
       static_cast<u32>(std::min<u64>(want, static_cast<u64>(sms) * std::max(1, per_sm)));
-  k_eval<kQuad, kSoft, kTeam, kU><<<grid, kT, 0, s>>>(
-      a.bodies, a.cells, a.cell_list, a.body_list, a.groups, static_cast<u32>(a.n_groups), a.G,
-      a.eps2, a.eo, a.counter, a.sc ? &a.sc->n_groups : nullptr, a.sc ? &a.sc->abort : nullptr,
-      a.shape.pass_cost, a.interactions);
+  launch(k_eval<kQuad, kSoft, kTeam, kU>, grid, kT, 0, s, a.bodies, a.cells, a.cell_list,
+         a.body_list, a.groups, static_cast<u32>(a.n_groups), a.G, a.eps2, a.eo, a.counter,
+         a.sc ? &a.sc->n_groups : nullptr, a.sc ? &a.sc->abort : nullptr, a.shape.pass_cost,
+         a.interactions);
   GTC_LAUNCH_CHECK();
 }
 

@@ -27,6 +27,7 @@ constexpr int kT = 256;
 // The arena's system of body i: start[k] <= i < start[k + 1].
 __global__ void __launch_bounds__(kT)
     k_forest_sys(const u32 *start, u32 systems, u32 n, u16 *sys) {
+  grid_wait();
   const u32 i = blockIdx.x * kT + threadIdx.x;
   if (i >= n) return;
   u32 lo = 0, hi = systems;  // start[lo] <= i < start[hi]
@@ -42,6 +43,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_forest_gather_bodies(const ForestSystemPtrs *sp, const u16 *sys, const u32 *start, u32 n,
                            double *apos, double *amass) {
+  grid_wait();
   const u32 i = blockIdx.x * kT + threadIdx.x;
   if (i >= n) return;
   const u16 k = sys[i];
@@ -58,6 +60,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_forest_kick_drift(const ForestSystemPtrs *sp, const u16 *sys, const u32 *start, u32 n,
                         double h, double dt, double *apos) {
+  grid_wait();
   const u32 i = blockIdx.x * kT + threadIdx.x;
   if (i >= n) return;
   const u16 k = sys[i];
@@ -79,6 +82,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_forest_scatter(const float4 *out, const u32 *order, u32 n, const ForestSystemPtrs *sp,
                      const u16 *sys, const u32 *start, int kick, double h, const u32 *abort) {
+  grid_wait();
   const u32 t = blockIdx.x * kT + threadIdx.x;
   if (t >= n || (abort && *abort)) return;
   const float4 o = out[t];
@@ -96,6 +100,7 @@ __global__ void __launch_bounds__(kT)
 // Per-system list statistics of the current lists (group records).
 __global__ void __launch_bounds__(kT)
     k_forest_stats(const uint4 *groups, u32 ng, const u16 *sys, ForestSystemStats *st) {
+  grid_wait();
   const u32 g = blockIdx.x * kT + threadIdx.x;
   if (g >= ng) return;
   const uint4 r = groups[4ull * g];  // begin, end, cells, bodies
@@ -218,35 +223,32 @@ void ForestRun::setup(const std::vector<ForestSystem> &systems, cudaStream_t s) 
   fv.slot_plan = slot_plan.as<uint4>();
   ptrs_dev = reinterpret_cast<const ForestSystemPtrs *>(t + off_ptrs);
   if (n == 0) return;
-  k_forest_sys<<<ceil_div(n, kT), kT, 0, s>>>(fv.start, k, static_cast<u32>(n), sysid.as<u16>());
+  launch(k_forest_sys, ceil_div(n, kT), kT, 0, s, fv.start, k, static_cast<u32>(n),
+         sysid.as<u16>());
   GTC_LAUNCH_CHECK();
-  k_forest_gather_bodies<<<ceil_div(n, kT), kT, 0, s>>>(ptrs_dev, fv.sys, fv.start,
-                                                        static_cast<u32>(n), apos.as<double>(),
-                                                        amass.as<double>());
+  launch(k_forest_gather_bodies, ceil_div(n, kT), kT, 0, s, ptrs_dev, fv.sys, fv.start,
+         static_cast<u32>(n), apos.as<double>(), amass.as<double>());
   GTC_LAUNCH_CHECK();
 }
 
 void ForestRun::gather(cudaStream_t s) {
   if (n == 0) return;
-  k_forest_gather_bodies<<<ceil_div(n, kT), kT, 0, s>>>(ptrs_dev, ws.forest.sys, ws.forest.start,
-                                                        static_cast<u32>(n), apos.as<double>(),
-                                                        amass.as<double>());
+  launch(k_forest_gather_bodies, ceil_div(n, kT), kT, 0, s, ptrs_dev, ws.forest.sys,
+         ws.forest.start, static_cast<u32>(n), apos.as<double>(), amass.as<double>());
   GTC_LAUNCH_CHECK();
 }
 
 void ForestRun::kick_drift(double h, double dt, cudaStream_t s) {
   if (n == 0) return;
-  k_forest_kick_drift<<<ceil_div(n, kT), kT, 0, s>>>(ptrs_dev, ws.forest.sys, ws.forest.start,
-                                                     static_cast<u32>(n), h, dt,
-                                                     apos.as<double>());
+  launch(k_forest_kick_drift, ceil_div(n, kT), kT, 0, s, ptrs_dev, ws.forest.sys,
+         ws.forest.start, static_cast<u32>(n), h, dt, apos.as<double>());
   GTC_LAUNCH_CHECK();
 }
 
 void ForestRun::scatter(int kick, double h, const u32 *abort, cudaStream_t s) {
   if (n == 0) return;
-  k_forest_scatter<<<ceil_div(n, kT), kT, 0, s>>>(ws.out.as<float4>(), ws.idx.as<u32>(),
-                                                  static_cast<u32>(n), ptrs_dev, ws.forest.sys,
-                                                  ws.forest.start, kick, h, abort);
+  launch(k_forest_scatter, ceil_div(n, kT), kT, 0, s, ws.out.as<float4>(), ws.idx.as<u32>(),
+         static_cast<u32>(n), ptrs_dev, ws.forest.sys, ws.forest.start, kick, h, abort);
   GTC_LAUNCH_CHECK();
 }
 
@@ -334,9 +336,8 @@ std::vector<ForestSystemStats> ForestRun::system_stats(cudaStream_t s) {
   if (k == 0) return out;
   GTC_CUDA(cudaMemsetAsync(stats.ptr, 0, k * sizeof(ForestSystemStats), s));
   if (ws.n_groups > 0) {
-    k_forest_stats<<<ceil_div(ws.n_groups, kT), kT, 0, s>>>(
-        ws.groups.as<uint4>(), static_cast<u32>(ws.n_groups), ws.forest.sys,
-        stats.as<ForestSystemStats>());
+    launch(k_forest_stats, ceil_div(ws.n_groups, kT), kT, 0, s, ws.groups.as<uint4>(),
+           static_cast<u32>(ws.n_groups), ws.forest.sys, stats.as<ForestSystemStats>());
     GTC_LAUNCH_CHECK();
   }
   GTC_CUDA(cudaMemcpyAsync(out.data(), stats.ptr, k * sizeof(ForestSystemStats),

@@ -52,6 +52,7 @@ struct NodeView {
 __global__ void __launch_bounds__(kT)
     k_group_marks(NodeView nv, u32 m, u32 gs, int pack, u32 *mark,
                   const u32 *m_dev = nullptr, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort) || p >= bounded(m, m_dev)) return;
   const u32 b0 = nv.nbegin[p], b1 = nv.nend[p];
@@ -103,6 +104,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_group_ranges(const u32 *mark, const u32 *scan, u32 n, u32 *gbegin, u32 *gend,
                    const u32 *abort = nullptr) {
+  grid_wait();
   const u32 b = blockIdx.x * kT + threadIdx.x;
   if (b >= n || aborted(abort)) return;
   const u32 g = scan[b];  // groups that start before b
@@ -118,10 +120,12 @@ __global__ void __launch_bounds__(kT)
 // together than the captured walk (before; walk_super 0: any), overflow pools
 // too small for the lists that outgrew their slots (after).
 __global__ void k_check_groups_graph(Scalars *sc, u32 groups, int walk_super) {
+  grid_wait();
   if (sc->n_groups > groups) sc->abort |= 8u;
   if (walk_super != 0 && walk_super_for(sc->n_groups) != walk_super) sc->abort |= 8u;
 }
 __global__ void k_check_slots_graph(Scalars *sc) {
+  grid_wait();
   if (sc->list_overflow) sc->abort |= 8u;
 }
 
@@ -148,6 +152,7 @@ __global__ void __launch_bounds__(kT)
     k_group_box(const u32 *gbegin, const u32 *gend, u32 ng, const double *tpos,
                 const TreeRoot *root, double *gbox, float *gboxf, const u32 *ng_dev,
                 const u32 *abort, ForestView fv) {
+  grid_wait();
   // gboxf per group: centre (3), half-extent (3), magnitude bound, pad
   const u32 g = (blockIdx.x * kT + threadIdx.x) / kBoxLanes;
   const u32 lane = threadIdx.x % kBoxLanes;
@@ -236,6 +241,7 @@ __global__ void __launch_bounds__(kT)
     k_walk(const WalkRec32 *walk32, const WalkRec64 *walk64, const double *gbox,
            const float *gboxf, u32 ng_cap, const Task *tasks, u32 ntasks, WalkOut out,
            Scalars *sc, const u32 *ng_dev, const u32 *abort, const u32 *group_root) {
+  grid_wait();
   const u64 tid = static_cast<u64>(blockIdx.x) * kT + threadIdx.x;
   if (aborted(abort)) return;
   const u32 ng = bounded(ng_cap, ng_dev);
@@ -356,6 +362,7 @@ __device__ __forceinline__ GroupSlots group_slots(const SplitOut &o, u32 g) {
 __global__ void __launch_bounds__(kT)
     k_sys_groups(const u32 *mscan, const u32 *start, u32 systems, const Scalars *sc,
                  u32 *groups) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= systems) return;
   const u32 next = k + 1 < systems ? mscan[start[k + 1]] : sc->n_groups;
@@ -368,6 +375,7 @@ __global__ void __launch_bounds__(kT)
     k_slot_plan(const u32 *gbegin, u32 ng_cap, const u32 *ng_dev, const u32 *abort,
                 const u16 *sys, const u32 *start, const u32 *mscan, const SysSlots *slots,
                 uint4 *plan) {
+  grid_wait();
   const u32 g = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort) || g >= bounded(ng_cap, ng_dev)) return;
   const u16 k = sys[gbegin[g]];
@@ -432,6 +440,7 @@ __global__ void __launch_bounds__(kWalkThreads)
                  const float *gboxf, const u32 *gbegin, const u32 *gend, const uint4 *kids,
                  const u8 *nchild, const u32 *nbegin, const u32 *nend, u32 ng_cap, SplitOut out,
                  Scalars *sc, const u32 *ng_dev, const u32 *abort, const u32 *group_root) {
+  grid_wait();
   const u64 tid = static_cast<u64>(blockIdx.x) * kWalkThreads + threadIdx.x;
   if (aborted(abort)) return;
   const u32 ng = bounded(ng_cap, ng_dev);
@@ -676,6 +685,7 @@ __global__ void __launch_bounds__(kWarpWalkThreads)
                 const float *gboxf, u32 ng_cap, WarpWalkOut out, u32 *next_chunk, Scalars *sc,
                 const u32 *ng_dev, const u32 *abort, const u32 *group_root, GroupSystems gs,
                 bool own_size) {
+  grid_wait();
   constexpr bool kWrite = kMode != kCount;
   __shared__ WarpWalk<kSuper> walks[kWarpWalkWarps];
   if (aborted(abort)) return;
@@ -965,6 +975,7 @@ __global__ void __launch_bounds__(kT)
     k_split_spill(const SplitOut out, u32 ng, u64 pool_cells_at, u64 pool_cells,
                   u64 pool_bodies_at, u64 pool_bodies, u32 *spill_cells, u32 *spill_bodies,
                   Scalars *sc, const u32 *ng_dev = nullptr, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 g = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort) || g >= bounded(ng, ng_dev)) return;
   const u64 rc = out.ncells[g], rb = out.nbodies[g];
@@ -994,6 +1005,7 @@ __global__ void __launch_bounds__(kT)
     k_split_records(const u32 *gbegin, const u32 *gend, u32 ng, const SplitOut out,
                     const u32 *spill_cells, const u32 *spill_bodies, uint4 *groups, Scalars *sc,
                     const u32 *ng_dev = nullptr, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 g = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort)) return;
   const bool valid = g < bounded(ng, ng_dev);
@@ -1049,6 +1061,7 @@ __global__ void __launch_bounds__(kT)
 // depth-2 task has an ancestor to test.
 __global__ void __launch_bounds__(kT)
     k_task_flags(const u8 *depth, const u8 *isleaf, u32 m, int split, u32 *flag) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (p >= m) return;
   flag[p] = (depth[p] == split || (isleaf[p] && depth[p] < split)) ? 1u : 0u;
@@ -1057,6 +1070,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_task_fill(const u32 *flag, const u32 *scan, const u8 *depth, const u32 *parent, u32 m,
                 Task *tasks) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (p >= m || !flag[p]) return;
   Task t{p, kNone, 0u, 0u};
@@ -1072,6 +1086,7 @@ __global__ void __launch_bounds__(kT)
     k_group_records(const u32 *gbegin, const u32 *gend, u32 ng, u32 ntasks, const u64 *cell_off,
                     const u64 *body_off, uint4 *groups, Scalars *sc, const u32 *ng_dev = nullptr,
                     const u16 *sys = nullptr, u32 *sys_max = nullptr) {
+  grid_wait();
   const u32 g = blockIdx.x * kT + threadIdx.x;
   if (sc->abort) return;
   const bool valid = g < bounded(ng, ng_dev);
@@ -1144,10 +1159,9 @@ void launch_warp_walk_of(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scal
   if (ws.forest)
     gs = GroupSystems{ws.gbegin.as<u32>(), ws.forest.sys, ws.forest.start,
                       ws.flags_scan.as<u32>(), ws.forest.systems};
-  k_walk_warp<kMode, kSuper><<<blocks, kWarpWalkThreads, 0, s>>>(
-      ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), ws.gbox.as<double>(),
-      ws.gboxf.as<float>(), ng_cap, out, next, sc, ng_dev, abort, ws.forest.group_root, gs,
-      ws.walk_super == 0);
+  launch(k_walk_warp<kMode, kSuper>, blocks, kWarpWalkThreads, 0, s, ws.walk32.as<WalkRec32>(),
+         ws.walk64.as<WalkRec64>(), ws.gbox.as<double>(), ws.gboxf.as<float>(), ng_cap, out,
+         next, sc, ng_dev, abort, ws.forest.group_root, gs, ws.walk_super == 0);
   GTC_LAUNCH_CHECK();
 }
 
@@ -1203,19 +1217,19 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   const bool split_tasks = !lw && !fv && ws.walk_split_depth > 0;
   if (split_tasks) {
     ws.tasks.ensure(m * sizeof(Task));
-    k_task_flags<<<mb, kT, 0, s>>>(ws.depth.as<u8>(), ws.isleaf.as<u8>(), m, ws.walk_split_depth,
-                                   mark);
+    launch(k_task_flags, mb, kT, 0, s, ws.depth.as<u8>(), ws.isleaf.as<u8>(), m,
+           ws.walk_split_depth, mark);
     GTC_LAUNCH_CHECK();
     exclusive_scan_u32(mark, mscan, m, &sc->aux, ws.scan_tmp, s, &sc->error);
-    k_task_fill<<<mb, kT, 0, s>>>(mark, mscan, ws.depth.as<u8>(), ws.parent.as<u32>(), m,
-                                  ws.tasks.as<Task>());
+    launch(k_task_fill, mb, kT, 0, s, mark, mscan, ws.depth.as<u8>(), ws.parent.as<u32>(), m,
+           ws.tasks.as<Task>());
     GTC_LAUNCH_CHECK();
   }
 
   // groups
-  GTC_CUDA(cudaMemsetAsync(mark, 0, n * 4, s));
+  clear({{mark, n * 4}}, s);
   const NodeView nv = node_view(ws);
-  k_group_marks<<<mb, kT, 0, s>>>(nv, m, gs, sp.pack, mark);
+  launch(k_group_marks, mb, kT, 0, s, nv, m, gs, sp.pack, mark);
   GTC_LAUNCH_CHECK();
   exclusive_scan_u32(mark, mscan, n, &sc->n_groups, ws.scan_tmp, s, &sc->error);
   ws.gbegin.ensure(n * 4);
@@ -1224,11 +1238,11 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   ws.gboxf.ensure(n * 32);
   ws.groups.ensure(n * kGroupRecWords * 4);
   u32 *gbegin = ws.gbegin.as<u32>(), *gend = ws.gend.as<u32>();
-  k_group_ranges<<<ceil_div(n, kT), kT, 0, s>>>(mark, mscan, n32, gbegin, gend);
+  launch(k_group_ranges, ceil_div(n, kT), kT, 0, s, mark, mscan, n32, gbegin, gend);
   GTC_LAUNCH_CHECK();
   if (fv) {  // each system's group count, read back with the total
-    k_sys_groups<<<ceil_div(fv.systems, kT), kT, 0, s>>>(mscan, fv.start, fv.systems, sc,
-                                                         fv.sys_groups);
+    launch(k_sys_groups, ceil_div(fv.systems, kT), kT, 0, s, mscan, fv.start, fv.systems, sc,
+           fv.sys_groups);
     GTC_LAUNCH_CHECK();
     GTC_CUDA(cudaMemcpyAsync(fv.host_groups, fv.sys_groups, fv.systems * sizeof(u32),
                              cudaMemcpyDeviceToHost, s));
@@ -1238,9 +1252,9 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   ws.n_groups = ng;
   ws.choose_walk(ng);
   const u32 gb = ceil_div(ng, kT);
-  k_group_box<<<ceil_div(static_cast<u64>(ng) * kBoxLanes, kT), kT, 0, s>>>(gbegin, gend, ng, ws.tpos.as<double>(),
-                                fv ? fv.roots : ws.root.as<TreeRoot>(), ws.gbox.as<double>(),
-                                ws.gboxf.as<float>(), nullptr, nullptr, fv);
+  launch(k_group_box, ceil_div(static_cast<u64>(ng) * kBoxLanes, kT), kT, 0, s, gbegin, gend, ng,
+         ws.tpos.as<double>(), fv ? fv.roots : ws.root.as<TreeRoot>(), ws.gbox.as<double>(),
+         ws.gboxf.as<float>(), nullptr, nullptr, fv);
   GTC_LAUNCH_CHECK();
   if (lw) {
     // the learned walk decides from FP32 moment estimates: the FP64 moments
@@ -1321,20 +1335,20 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
                   sl_c, sl_b, sn_c, sn_b, ng};
       so.sys = fv.sys;
       so.sys_max = fv.sys_max;
-      k_walk_split<<<ceil_div(2ull * ng, kWalkThreads), kWalkThreads, 0, s>>>(
-          w32, w64, gbox, gboxf, gbegin, gend, ws.kids.as<uint4>(), ws.nchild.as<u8>(),
-          ws.nbegin.as<u32>(), ws.nend.as<u32>(), ng, so, sc, nullptr, nullptr, fv.group_root);
+      launch(k_walk_split, ceil_div(2ull * ng, kWalkThreads), kWalkThreads, 0, s, w32, w64, gbox,
+             gboxf, gbegin, gend, ws.kids.as<uint4>(), ws.nchild.as<u8>(), ws.nbegin.as<u32>(),
+             ws.nend.as<u32>(), ng, so, sc, nullptr, nullptr, fv.group_root);
       GTC_LAUNCH_CHECK();
-      k_split_spill<<<gb, kT, 0, s>>>(so, ng, pool_at_c, pool_c, pool_at_b, pool_b, spill_c,
-                                      spill_b, sc);
+      launch(k_split_spill, gb, kT, 0, s, so, ng, pool_at_c, pool_c, pool_at_b, pool_b, spill_c,
+             spill_b, sc);
       GTC_LAUNCH_CHECK();
       WalkOut wo{ws.gcells.as<u64>(), ws.gbodies.as<u64>(), nullptr, nullptr,
                  ws.cell_list.as<u32>(), ws.body_list.as<u32>(), spill_c, spill_b};
-      k_walk<kSpill><<<tb, kT, 0, s>>>(w32, w64, gbox, gboxf, ng, tasks, 1, wo, sc, nullptr,
-                                       nullptr, fv.group_root);
+      launch(k_walk<kSpill>, tb, kT, 0, s, w32, w64, gbox, gboxf, ng, tasks, 1, wo, sc, nullptr,
+             nullptr, fv.group_root);
       GTC_LAUNCH_CHECK();
-      k_split_records<<<gb, kT, 0, s>>>(gbegin, gend, ng, so, spill_c, spill_b,
-                                        ws.groups.as<uint4>(), sc);
+      launch(k_split_records, gb, kT, 0, s, gbegin, gend, ng, so, spill_c, spill_b,
+             ws.groups.as<uint4>(), sc);
       GTC_LAUNCH_CHECK();
     }
     ws.stage(Workspace::kStWalk1, s);
@@ -1374,16 +1388,16 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   if (warps) {
     launch_warp_walk<kCount>(ws, wwo, ng, sc, s);
   } else {
-    k_walk<kCount><<<tb, kT, 0, s>>>(w32, w64, gbox, gboxf, ng, tasks, ntasks, wo, sc, nullptr,
-                                     nullptr, fv.group_root);
+    launch(k_walk<kCount>, tb, kT, 0, s, w32, w64, gbox, gboxf, ng, tasks, ntasks, wo, sc,
+           nullptr, nullptr, fv.group_root);
     GTC_LAUNCH_CHECK();
   }
   exclusive_scan_u64(ws.gcells.as<u64>(), cell_off, slots, cell_off + slots, ws.scan_tmp, s, &sc->error);
   exclusive_scan_u64(ws.gbodies.as<u64>(), body_off, slots, body_off + slots, ws.scan_tmp, s, &sc->error);
   GTC_CUDA(cudaMemcpyAsync(&sc->n_cell_list, cell_off + slots, 8, cudaMemcpyDeviceToDevice, s));
   GTC_CUDA(cudaMemcpyAsync(&sc->n_body_list, body_off + slots, 8, cudaMemcpyDeviceToDevice, s));
-  k_group_records<<<gb, kT, 0, s>>>(gbegin, gend, ng, ntasks, cell_off, body_off,
-                                    ws.groups.as<uint4>(), sc, nullptr, fv.sys, fv.sys_max);
+  launch(k_group_records, gb, kT, 0, s, gbegin, gend, ng, ntasks, cell_off, body_off,
+         ws.groups.as<uint4>(), sc, nullptr, fv.sys, fv.sys_max);
   GTC_LAUNCH_CHECK();
   read_sys_max();
   read_scalars(ws, host, s);
@@ -1401,8 +1415,8 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
     wwo.body_list = wo.body_list;
     launch_warp_walk<kFill>(ws, wwo, ng, sc, s);
   } else {
-    k_walk<kFill><<<tb, kT, 0, s>>>(w32, w64, gbox, gboxf, ng, tasks, ntasks, wo, sc, nullptr,
-                                    nullptr, fv.group_root);
+    launch(k_walk<kFill>, tb, kT, 0, s, w32, w64, gbox, gboxf, ng, tasks, ntasks, wo, sc,
+           nullptr, nullptr, fv.group_root);
     GTC_LAUNCH_CHECK();
   }
   ws.stage(Workspace::kStWalk1, s);
@@ -1421,24 +1435,25 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
   const u32 *abort = &sc->abort;
   const u32 nb = ceil_div(n, kT), mb = ceil_div(mcap, kT);
   // groups (the one walk task, the root, was written before capture)
-  GTC_CUDA(cudaMemsetAsync(mark, 0, n * 4, s));
+  clear({{mark, n * 4}}, s);
   const ForestView &fv = ws.forest;
   const NodeView nv = node_view(ws);
-  k_group_marks<<<mb, kT, 0, s>>>(nv, mcap, gs, sp.pack, mark, &sc->n_nodes, abort);
+  launch(k_group_marks, mb, kT, 0, s, nv, mcap, gs, sp.pack, mark, &sc->n_nodes, abort);
   GTC_LAUNCH_CHECK();
   exclusive_scan_u32(mark, mscan, n, &sc->n_groups, ws.scan_tmp, s, &sc->error);
   u32 *gbegin = ws.gbegin.as<u32>(), *gend = ws.gend.as<u32>();
-  k_group_ranges<<<nb, kT, 0, s>>>(mark, mscan, n32, gbegin, gend, abort);
+  launch(k_group_ranges, nb, kT, 0, s, mark, mscan, n32, gbegin, gend, abort);
   GTC_LAUNCH_CHECK();
   const u64 boxes = std::min<u64>(n, fv ? n : caps.groups);
-  k_group_box<<<ceil_div(boxes * kBoxLanes, kT), kT, 0, s>>>(gbegin, gend, static_cast<u32>(boxes), ws.tpos.as<double>(),
-                                fv ? fv.roots : ws.root.as<TreeRoot>(), ws.gbox.as<double>(),
-                                ws.gboxf.as<float>(), &sc->n_groups, abort, fv);
+  launch(k_group_box, ceil_div(boxes * kBoxLanes, kT), kT, 0, s, gbegin, gend,
+         static_cast<u32>(boxes), ws.tpos.as<double>(), fv ? fv.roots : ws.root.as<TreeRoot>(),
+         ws.gbox.as<double>(), ws.gboxf.as<float>(), &sc->n_groups, abort, fv);
   GTC_LAUNCH_CHECK();
   // one pass into the captured slots (near field and rest), outgrown groups
   // again into the pools
   if (!caps.sys_slots) {  // (per-system slots: a system past its capacity spills)
-    k_check_groups_graph<<<1, 1, 0, s>>>(sc, caps.groups, ws.walk_mode < 0 ? ws.walk_super : 0);
+    launch(k_check_groups_graph, 1, 1, 0, s, sc, caps.groups,
+           ws.walk_mode < 0 ? ws.walk_super : 0);
     GTC_LAUNCH_CHECK();
   }
   join_walk(ws, s);  // the walk reads the node records (the cells follow on the side stream)
@@ -1466,8 +1481,8 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
     so.sys_max = fv.sys_max;
     GTC_CUDA(cudaMemsetAsync(fv.sys_max, 0, 4ull * fv.systems * sizeof(u32), s));
     if (caps.sys_slots) {  // each system's own slots (and the pools after them)
-      k_slot_plan<<<nb, kT, 0, s>>>(gbegin, n32, &sc->n_groups, abort, fv.sys, fv.start, mscan,
-                                    caps.sys_slots, fv.slot_plan);
+      launch(k_slot_plan, nb, kT, 0, s, gbegin, n32, &sc->n_groups, abort, fv.sys, fv.start,
+             mscan, caps.sys_slots, fv.slot_plan);
       GTC_LAUNCH_CHECK();
       so.plan = fv.slot_plan;
       wwo.plan = fv.slot_plan;
@@ -1482,26 +1497,26 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
     wwo.pool_bodies = caps.pool_bodies;
     launch_warp_walk<kSlots>(ws, wwo, static_cast<u32>(boxes), sc, s, &sc->n_groups, abort);
   } else {
-    k_walk_split<<<ceil_div(2ull * n, kWalkThreads), kWalkThreads, 0, s>>>(
-        ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), ws.gbox.as<double>(),
-        ws.gboxf.as<float>(), gbegin, gend, ws.kids.as<uint4>(), ws.nchild.as<u8>(),
-        ws.nbegin.as<u32>(), ws.nend.as<u32>(), n32, so, sc, &sc->n_groups, abort,
-        fv.group_root);
+    launch(k_walk_split, ceil_div(2ull * n, kWalkThreads), kWalkThreads, 0, s,
+           ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), ws.gbox.as<double>(),
+           ws.gboxf.as<float>(), gbegin, gend, ws.kids.as<uint4>(), ws.nchild.as<u8>(),
+           ws.nbegin.as<u32>(), ws.nend.as<u32>(), n32, so, sc, &sc->n_groups, abort,
+           fv.group_root);
     GTC_LAUNCH_CHECK();
-    k_split_spill<<<nb, kT, 0, s>>>(so, n32, pool_at_c, caps.pool_cells, pool_at_b,
-                                    caps.pool_bodies, spill_c, spill_b, sc, &sc->n_groups, abort);
+    launch(k_split_spill, nb, kT, 0, s, so, n32, pool_at_c, caps.pool_cells, pool_at_b,
+           caps.pool_bodies, spill_c, spill_b, sc, &sc->n_groups, abort);
     GTC_LAUNCH_CHECK();
     WalkOut wo{ws.gcells.as<u64>(), ws.gbodies.as<u64>(), nullptr, nullptr,
                ws.cell_list.as<u32>(), ws.body_list.as<u32>(), spill_c, spill_b};
-    k_walk<kSpill><<<nb, kT, 0, s>>>(ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(),
-                                     ws.gbox.as<double>(), ws.gboxf.as<float>(), n32, nullptr, 1,
-                                     wo, sc, &sc->n_groups, abort, fv.group_root);
+    launch(k_walk<kSpill>, nb, kT, 0, s, ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(),
+           ws.gbox.as<double>(), ws.gboxf.as<float>(), n32, nullptr, 1, wo, sc, &sc->n_groups,
+           abort, fv.group_root);
     GTC_LAUNCH_CHECK();
-    k_split_records<<<nb, kT, 0, s>>>(gbegin, gend, n32, so, spill_c, spill_b,
-                                      ws.groups.as<uint4>(), sc, &sc->n_groups, abort);
+    launch(k_split_records, nb, kT, 0, s, gbegin, gend, n32, so, spill_c, spill_b,
+           ws.groups.as<uint4>(), sc, &sc->n_groups, abort);
     GTC_LAUNCH_CHECK();
   }
-  k_check_slots_graph<<<1, 1, 0, s>>>(sc);
+  launch(k_check_slots_graph, 1, 1, 0, s, sc);
   GTC_LAUNCH_CHECK();
 }
 

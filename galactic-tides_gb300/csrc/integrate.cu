@@ -17,6 +17,7 @@ constexpr int kDiagBlocks = 256;
 // v += h a; x += dt v (integrator.cpp:10-13)
 __global__ void __launch_bounds__(kT)
     k_kick_drift(double *pos, double *vel, const double *acc, u64 n3, double h, double dt) {
+  grid_wait();
   const u64 k = static_cast<u64>(blockIdx.x) * kT + threadIdx.x;
   if (k >= n3) return;
   const double v = vel[k] + h * acc[k];
@@ -27,6 +28,7 @@ __global__ void __launch_bounds__(kT)
 // v += h a (integrator.cpp:16); a graph replay skips it after an abort.
 __global__ void __launch_bounds__(kT)
     k_kick(double *vel, const double *acc, u64 n3, double h, const u32 *abort) {
+  grid_wait();
   const u64 k = static_cast<u64>(blockIdx.x) * kT + threadIdx.x;
   if (k >= n3 || (abort && *abort)) return;
   vel[k] = vel[k] + h * acc[k];
@@ -37,6 +39,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_diag_partials(const double *pos, const double *vel, const double *mass, const double *pot,
                     u64 n, double *part) {
+  grid_wait();
   __shared__ double s[kDiagTerms][kT / 32];
   double acc[kDiagTerms] = {};
   for (u64 i = static_cast<u64>(blockIdx.x) * kT + threadIdx.x; i < n;
@@ -76,19 +79,19 @@ __global__ void __launch_bounds__(kT)
 void kick_drift(double *pos, double *vel, const double *acc, u64 n, double h, double dt,
                 cudaStream_t s) {
   if (n == 0) return;
-  k_kick_drift<<<ceil_div(3 * n, kT), kT, 0, s>>>(pos, vel, acc, 3 * n, h, dt);
+  launch(k_kick_drift, ceil_div(3 * n, kT), kT, 0, s, pos, vel, acc, 3 * n, h, dt);
   GTC_LAUNCH_CHECK();
 }
 
 void kick(double *vel, const double *acc, u64 n, double h, cudaStream_t s, const u32 *abort) {
   if (n == 0) return;
-  k_kick<<<ceil_div(3 * n, kT), kT, 0, s>>>(vel, acc, 3 * n, h, abort);
+  launch(k_kick, ceil_div(3 * n, kT), kT, 0, s, vel, acc, 3 * n, h, abort);
   GTC_LAUNCH_CHECK();
 }
 
 void diagnostics_launch(const double *pos, const double *vel, const double *mass,
                         const double *pot, u64 n, double *part, cudaStream_t s) {
-  k_diag_partials<<<kDiagBlocks, kT, 0, s>>>(pos, vel, mass, pot, n, part);
+  launch(k_diag_partials, kDiagBlocks, kT, 0, s, pos, vel, mass, pot, n, part);
   GTC_LAUNCH_CHECK();
 }
 

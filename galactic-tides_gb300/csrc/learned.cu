@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(kT)
     k_sample_pairs(const WalkRec32 *walk32, const CellFeat *cfeat, u32 m, const float *gboxf,
                    u32 ng, u32 group_stride, u32 group_offset, float inv_theta_gen,
                    float inv_theta_guard, uint2 *pairs, u32 capacity, u32 *count) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   const u64 g64 = static_cast<u64>(k) * group_stride + group_offset;
   if (g64 >= ng) return;
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_pair_features(const uint2 *pairs, u32 np, const WalkRec32 *walk32, const CellFeat *cfeat,
                     const float *gboxf, const TreeRoot *root, const double2 *mom, float *feat) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= np) return;
   const FeatScale fs = scale_from(root, mom);
@@ -108,6 +110,7 @@ __global__ void __launch_bounds__(32 * kLabelWarps)
                   const u32 *nbegin, const u32 *nend, const double *tpos, const double *tmass,
                   const double2 *mom, const double2 *quad, const TreeRoot *root, double G,
                   double eps2, u32 max_bodies, float *label) {
+  grid_wait();
   const u32 k = blockIdx.x * kLabelWarps + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (k >= np) return;
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(32 * kLabelWarps)
 }
 
 __global__ void __launch_bounds__(kT) k_finite_flags(const float *label, u32 np, u32 *flag) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k < np) flag[k] = isfinite(label[k]) ? 1u : 0u;
 }
@@ -161,6 +165,7 @@ __global__ void __launch_bounds__(kT)
     k_append_samples(const u32 *flag, const u32 *scan, u32 np, const float *feat,
                      const float *label, const uint2 *pairs, u64 base, float *set_feat,
                      float *set_label, uint2 *set_pair) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= np || !flag[k]) return;
   const u64 o = base + scan[k];
@@ -184,6 +189,7 @@ constexpr int kStats = 2 * (kFeat + 1);
 
 __global__ void __launch_bounds__(kT)
     k_stat_partials(const float *feat, const float *label, u64 n, double *part) {
+  grid_wait();
   __shared__ double s[kStats][kT / 32];
   double acc[kStats] = {};
   for (u64 k = static_cast<u64>(blockIdx.x) * kT + threadIdx.x; k < n;
@@ -232,6 +238,7 @@ __global__ void __launch_bounds__(kTB)
     k_train_block(const float *__restrict__ model, const float *__restrict__ feat,
                   const float *__restrict__ label, u64 nsamples, u64 seed, u64 step, u32 batch,
                   const u32 *fixed, float *part, float *loss) {
+  grid_wait();
   extern __shared__ float smem[];
   float *sP = smem;                       // kModelFloats (+ padding)
   float *sZ1 = sP + kModelFloats + 4;     // kTB x kLd  (pre-activations, layer 1)
@@ -327,6 +334,7 @@ __global__ void __launch_bounds__(kTB)
 __global__ void __launch_bounds__(kT)
     k_reduce_adam(const float *part, u32 nblocks, float *grad, float *model, float *m, float *v,
                   float lr, float b1t, float b2t) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (p >= kParams) return;
   float g = 0.f;
@@ -350,6 +358,7 @@ constexpr int kBandBins = 1024;
 
 __global__ void __launch_bounds__(kT)
     k_band_hist(const float *model, const float *feat, u64 n, u64 stride, u32 *hist) {
+  grid_wait();
   __shared__ float sP[kModelFloats];
   __shared__ u32 sh[kBandBins];
   for (int i = threadIdx.x; i < kModelFloats; i += kT) sP[i] = model[i];
@@ -425,9 +434,8 @@ void learned_add_samples(gtc_context *ctx, const double *pos, const double *mass
   cnt.ensure(sizeof(u32));
   pairs.ensure(sizeof(uint2));
   GTC_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(u32), s));
-  k_sample_pairs<<<ceil_div(ng, kT), kT, 0, s>>>(ws.walk32.as<WalkRec32>(), cfeat, m,
-                                                 ws.gboxf.as<float>(), ng, 1, 0, igen, iguard,
-                                                 pairs.as<uint2>(), 0, cnt.as<u32>());
+  launch(k_sample_pairs, ceil_div(ng, kT), kT, 0, s, ws.walk32.as<WalkRec32>(), cfeat, m,
+         ws.gboxf.as<float>(), ng, 1, 0, igen, iguard, pairs.as<uint2>(), 0, cnt.as<u32>());
   GTC_LAUNCH_CHECK();
   u32 all = 0;
   read_back(&all, cnt.ptr, sizeof(u32), s);
@@ -437,9 +445,9 @@ void learned_add_samples(gtc_context *ctx, const double *pos, const double *mass
   const u32 cap = static_cast<u32>(std::min<u64>(all, 2 * max_new + 1024));
   pairs.ensure(static_cast<u64>(cap) * sizeof(uint2));
   GTC_CUDA(cudaMemsetAsync(cnt.ptr, 0, sizeof(u32), s));
-  k_sample_pairs<<<ceil_div(groups_used, kT), kT, 0, s>>>(
-      ws.walk32.as<WalkRec32>(), cfeat, m, ws.gboxf.as<float>(), ng, stride, stride / 2, igen,
-      iguard, pairs.as<uint2>(), cap, cnt.as<u32>());
+  launch(k_sample_pairs, ceil_div(groups_used, kT), kT, 0, s, ws.walk32.as<WalkRec32>(), cfeat,
+         m, ws.gboxf.as<float>(), ng, stride, stride / 2, igen, iguard, pairs.as<uint2>(), cap,
+         cnt.as<u32>());
   GTC_LAUNCH_CHECK();
   u32 np = 0;
   read_back(&np, cnt.ptr, sizeof(u32), s);
@@ -447,20 +455,19 @@ void learned_add_samples(gtc_context *ctx, const double *pos, const double *mass
   if (np == 0) return;
   feat.ensure(static_cast<u64>(np) * kFeat * sizeof(float));
   label.ensure(static_cast<u64>(np) * sizeof(float));
-  k_pair_features<<<ceil_div(np, kT), kT, 0, s>>>(pairs.as<uint2>(), np, ws.walk32.as<WalkRec32>(),
-                                                  cfeat, ws.gboxf.as<float>(),
-                                                  ws.root.as<TreeRoot>(), ws.mom.as<double2>(),
-                                                  feat.as<float>());
+  launch(k_pair_features, ceil_div(np, kT), kT, 0, s, pairs.as<uint2>(), np,
+         ws.walk32.as<WalkRec32>(), cfeat, ws.gboxf.as<float>(), ws.root.as<TreeRoot>(),
+         ws.mom.as<double2>(), feat.as<float>());
   GTC_LAUNCH_CHECK();
-  k_pair_labels<<<ceil_div(np, kLabelWarps), 32 * kLabelWarps, 0, s>>>(
-      pairs.as<uint2>(), np, ws.gbegin.as<u32>(), ws.gend.as<u32>(), ws.nbegin.as<u32>(),
-      ws.nend.as<u32>(), ws.tpos.as<double>(), ws.tmass.as<double>(), ws.mom.as<double2>(),
-      ws.quad.as<double2>(), ws.root.as<TreeRoot>(), sp.G, sp.eps * sp.eps, max_cell_bodies,
-      label.as<float>());
+  launch(k_pair_labels, ceil_div(np, kLabelWarps), 32 * kLabelWarps, 0, s, pairs.as<uint2>(), np,
+         ws.gbegin.as<u32>(), ws.gend.as<u32>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
+         ws.tpos.as<double>(), ws.tmass.as<double>(), ws.mom.as<double2>(),
+         ws.quad.as<double2>(), ws.root.as<TreeRoot>(), sp.G, sp.eps * sp.eps, max_cell_bodies,
+         label.as<float>());
   GTC_LAUNCH_CHECK();
   flag.ensure(static_cast<u64>(np) * 4);
   scan.ensure(static_cast<u64>(np) * 4 + 8);
-  k_finite_flags<<<ceil_div(np, kT), kT, 0, s>>>(label.as<float>(), np, flag.as<u32>());
+  launch(k_finite_flags, ceil_div(np, kT), kT, 0, s, label.as<float>(), np, flag.as<u32>());
   GTC_LAUNCH_CHECK();
   u32 *kept_dev = scan.as<u32>() + np;
   exclusive_scan_u32(flag.as<u32>(), scan.as<u32>(), np, kept_dev, ws.scan_tmp, s,
@@ -500,11 +507,9 @@ void learned_add_samples(gtc_context *ctx, const double *pos, const double *mass
     set.pair = npr;
     set.capacity = cap2;
   }
-  k_append_samples<<<ceil_div(np, kT), kT, 0, s>>>(flag.as<u32>(), scan.as<u32>(), np,
-                                                   feat.as<float>(), label.as<float>(),
-                                                   pairs.as<uint2>(), set.count,
-                                                   set.feat.as<float>(), set.label.as<float>(),
-                                                   set.pair.as<uint2>());
+  launch(k_append_samples, ceil_div(np, kT), kT, 0, s, flag.as<u32>(), scan.as<u32>(), np,
+         feat.as<float>(), label.as<float>(), pairs.as<uint2>(), set.count, set.feat.as<float>(),
+         set.label.as<float>(), set.pair.as<uint2>());
   GTC_LAUNCH_CHECK();
   GTC_CUDA(cudaStreamSynchronize(s));
   set.count += kept;
@@ -539,8 +544,8 @@ void learned_init_model(gtc_context *ctx, u64 seed) {
   cudaStream_t s = ctx->stream;
   DeviceBuffer part;
   part.ensure(kStatBlocks * kStats * sizeof(double));
-  k_stat_partials<<<kStatBlocks, kT, 0, s>>>(set.feat.as<float>(), set.label.as<float>(),
-                                             set.count, part.as<double>());
+  launch(k_stat_partials, kStatBlocks, kT, 0, s, set.feat.as<float>(), set.label.as<float>(),
+         set.count, part.as<double>());
   GTC_LAUNCH_CHECK();
   std::vector<double> hp(kStatBlocks * kStats);
   read_back(hp.data(), part.ptr, hp.size() * sizeof(double), s);
@@ -597,14 +602,13 @@ double learned_train_on(gtc_context *ctx, const float *feat, const float *label,
   float *model = ctx->model.as<float>();
   double b1t = 1.0, b2t = 1.0;
   for (u64 k = 0; k < steps; ++k) {
-    k_train_block<<<nblocks, kTB, smem, s>>>(model, feat, label, nsamples, seed, k, batch, fixed,
-                                             part, loss);
+    launch(k_train_block, nblocks, kTB, smem, s, model, feat, label, nsamples, seed, k, batch,
+           fixed, part, loss);
     GTC_LAUNCH_CHECK();
     b1t *= 0.9;
     b2t *= 0.999;
-    k_reduce_adam<<<ceil_div(kParams, kT), kT, 0, s>>>(part, nblocks, grad, model, mom1, mom2, lr,
-                                                       static_cast<float>(b1t),
-                                                       static_cast<float>(b2t));
+    launch(k_reduce_adam, ceil_div(kParams, kT), kT, 0, s, part, nblocks, grad, model, mom1,
+           mom2, lr, static_cast<float>(b1t), static_cast<float>(b2t));
     GTC_LAUNCH_CHECK();
   }
   std::vector<float> lb(nblocks);
@@ -633,8 +637,8 @@ void learned_update_band(gtc_context *ctx, double quantile) {
   DeviceBuffer hist;
   hist.ensure(kBandBins * sizeof(u32));
   GTC_CUDA(cudaMemsetAsync(hist.ptr, 0, kBandBins * sizeof(u32), s));
-  k_band_hist<<<ceil_div(used, kT), kT, 0, s>>>(ctx->model.as<float>(), set.feat.as<float>(),
-                                                set.count, stride, hist.as<u32>());
+  launch(k_band_hist, ceil_div(used, kT), kT, 0, s, ctx->model.as<float>(), set.feat.as<float>(),
+         set.count, stride, hist.as<u32>());
   GTC_LAUNCH_CHECK();
   std::vector<u32> h(kBandBins);
   read_back(h.data(), hist.ptr, kBandBins * sizeof(u32), s);

@@ -130,6 +130,7 @@ __device__ __forceinline__ FeatScale scale_of(const TreeRoot *root, const double
 
 __global__ void __launch_bounds__(kT)
     k_prepare_net(const float *model, LearnedNet *net) {
+  grid_wait();
   const int k = blockIdx.x * kT + threadIdx.x;
   const float *W1 = model + kOffW1, *B1 = model + kOffB1, *W2 = model + kOffW2;
   if (k < 8 * 32) {
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_cell_feat(const double2 *geom, const double2 *mom, const float4 *cells, const double *delta,
                 const TreeRoot *root, u32 m, CellFeat *out) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (p >= m) return;
   const FeatScale fs = scale_of(root, mom);
@@ -181,6 +183,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_cell_feat32(const double2 *geom, const double2 *rootmom, const float4 *cells32,
                   const float *delta32, const TreeRoot *root, u32 m, CellFeat *out) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (p >= m) return;
   const FeatScale fs = scale_of(root, rootmom);
@@ -195,6 +198,7 @@ __global__ void __launch_bounds__(kT)
                   const u32 *nbegin, const u32 *nend, const u32 *skip, const u8 *isleaf,
                   const TreeRoot *root, u32 m, float inv_theta_guard, float y_mean,
                   LWalkRec *out) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (p >= m) return;
   const double2 g0 = geom[2 * p], g1 = geom[2 * p + 1];
@@ -226,6 +230,7 @@ __global__ void __launch_bounds__(kT)
     k_group_tol(const u32 *gbegin, const u32 *gend, u32 ng, const u32 *order,
                 const float *prev_amag, const float *gboxf, const TreeRoot *root,
                 const double2 *mom, double alpha, double G, float2 *gtol) {
+  grid_wait();
   const u32 g = blockIdx.x * kT + threadIdx.x;
   if (g >= ng) return;
   const FeatScale fs = scale_of(root, mom);
@@ -394,6 +399,7 @@ __device__ __forceinline__ void lround_stats(Scalars *sc, int part, u64 nc, u64 
 // Round 0: thread (part, group) walks the part's range of the root's
 // children (the root itself, when it is a leaf, in part 0).
 __global__ void __launch_bounds__(kRoundThreads) k_lround0(GArgs a) {
+  grid_wait();
   const u64 tid = static_cast<u64>(blockIdx.x) * kRoundThreads + threadIdx.x;
   if (tid >= static_cast<u64>(kParts) * a.ng) return;
   const int part = static_cast<int>(tid / a.ng);
@@ -447,6 +453,7 @@ constexpr int kContStack = 1024;  // ranges per warp
 constexpr u32 kPairOpen = 0xfffffffeu, kPairAccept = 0xffffffffu;  // node counts stay below
 
 __global__ void __launch_bounds__(kContWarps * 32) k_lcont(GArgs a, bool later) {
+  grid_wait();
   __shared__ uint2 stack_all[kContWarps][kContStack];
   const int lane = threadIdx.x & 31;
   uint2 *stk = stack_all[threadIdx.x >> 5];
@@ -627,6 +634,7 @@ struct LWarpWalk {
 };
 
 __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
+  grid_wait();
   __shared__ LWarpWalk walks[kLWarps];
   const int lane = threadIdx.x & 31;
   LWarpWalk &w = walks[threadIdx.x >> 5];
@@ -823,6 +831,7 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
 // slot, so a part's lists are its round-0 walk followed by each later
 // round's.
 __global__ void __launch_bounds__(kRoundThreads) k_lround(GArgs a) {
+  grid_wait();
   const u64 pg = static_cast<u64>(blockIdx.x) * kRoundThreads + threadIdx.x;
   if (pg >= static_cast<u64>(kParts) * a.ng) return;
   if (a.sc->list_overflow) return;  // an earlier round outgrew a buffer: redone
@@ -866,6 +875,7 @@ __global__ void __launch_bounds__(kRoundThreads) k_lround(GArgs a) {
 // each, in the order they were deferred, if the row buffer holds `cap`
 // rows (else the overflow flag); also the round's rows in the statistics.
 __global__ void __launch_bounds__(kT) k_lrows(const GArgs a, uint2 *rows, u64 cap) {
+  grid_wait();
   const u64 pg = static_cast<u64>(blockIdx.x) * kT + threadIdx.x;
   const u64 nparts = static_cast<u64>(kParts) * a.ng;
   const u32 total = a.roff[nparts];
@@ -887,6 +897,7 @@ __global__ void __launch_bounds__(kT) k_lrows(const GArgs a, uint2 *rows, u64 ca
 // the list statistics.
 __global__ void __launch_bounds__(kT) k_lgroup_records(const GArgs a, const u32 *gbegin,
                                                        const u32 *gend, uint4 *groups) {
+  grid_wait();
   const u32 g = blockIdx.x * kT + threadIdx.x;
   const bool valid = g < a.ng;
   u64 t = 0, nc = 0, nb = 0;
@@ -913,6 +924,7 @@ __global__ void __launch_bounds__(kT)
               const float *gboxf, const float2 *gtol, const LearnedNet *net, const TreeRoot *root,
               const double2 *mom, u8 *dec, const u32 *nq_dev = nullptr,
               const u32 *overflow = nullptr) {
+  grid_wait();
   __shared__ NetShared sn;
   __shared__ uint4 rows[kT / 32][32];
   // rows counted on the device; none written when a buffer was outgrown
@@ -953,6 +965,7 @@ __global__ void __launch_bounds__(kT)
 // The walk's inference on given raw features (tests and diagnostics).
 __global__ void __launch_bounds__(kT)
     k_predict(const LearnedNet *net, const float *feat, u64 n, float *pred) {
+  grid_wait();
   __shared__ NetShared sn;
   __shared__ uint4 rows[kT / 32][32];
   load_net(net, sn);
@@ -974,14 +987,14 @@ __global__ void __launch_bounds__(kT)
 }  // namespace
 
 void learned_prepare_net(const float *model, LearnedNet *net, cudaStream_t s) {
-  k_prepare_net<<<4, kT, 0, s>>>(model, net);
+  launch(k_prepare_net, 4, kT, 0, s, model, net);
   GTC_LAUNCH_CHECK();
 }
 
 void learned_predict(const LearnedNet *net, const float *feat, u64 n, float *pred,
                      cudaStream_t s) {
   if (n == 0) return;
-  k_predict<<<ceil_div(n, kT), kT, 0, s>>>(net, feat, n, pred);
+  launch(k_predict, ceil_div(n, kT), kT, 0, s, net, feat, n, pred);
   GTC_LAUNCH_CHECK();
 }
 
@@ -989,9 +1002,9 @@ void learned_node_features(Workspace &ws, DeviceBuffer &cfeat, cudaStream_t s) {
   const u32 m = static_cast<u32>(ws.n_nodes);
   if (m == 0) return;
   cfeat.ensure(static_cast<u64>(m) * sizeof(CellFeat));
-  k_cell_feat<<<ceil_div(m, kT), kT, 0, s>>>(ws.geom.as<double2>(), ws.mom.as<double2>(),
-                                             ws.cells.as<float4>(), ws.delta.as<double>(),
-                                             ws.root.as<TreeRoot>(), m, cfeat.as<CellFeat>());
+  launch(k_cell_feat, ceil_div(m, kT), kT, 0, s, ws.geom.as<double2>(), ws.mom.as<double2>(),
+         ws.cells.as<float4>(), ws.delta.as<double>(), ws.root.as<TreeRoot>(), m,
+         cfeat.as<CellFeat>());
   GTC_LAUNCH_CHECK();
 }
 
@@ -1004,25 +1017,24 @@ void learned_walk_inputs(Workspace &ws, LearnedScratch &ls, DeviceBuffer &cfeat,
   ls.rootmom.ensure(2 * sizeof(double2));
   moments32(ws, ls.cells32.as<float4>(), ls.delta32.as<float>(), ls.rootmom.as<double2>(), s);
   cfeat.ensure(static_cast<u64>(m) * sizeof(CellFeat));
-  k_cell_feat32<<<ceil_div(m, kT), kT, 0, s>>>(ws.geom.as<double2>(), ls.rootmom.as<double2>(),
-                                               ls.cells32.as<float4>(), ls.delta32.as<float>(),
-                                               ws.root.as<TreeRoot>(), m, cfeat.as<CellFeat>());
+  launch(k_cell_feat32, ceil_div(m, kT), kT, 0, s, ws.geom.as<double2>(),
+         ls.rootmom.as<double2>(), ls.cells32.as<float4>(), ls.delta32.as<float>(),
+         ws.root.as<TreeRoot>(), m, cfeat.as<CellFeat>());
   GTC_LAUNCH_CHECK();
   ls.lrec.ensure(static_cast<u64>(m) * sizeof(LWalkRec));
-  k_lwalk_rec32<<<ceil_div(m, kT), kT, 0, s>>>(
-      ws.geom.as<double2>(), ls.cells32.as<float4>(), cfeat.as<CellFeat>(), ws.nbegin.as<u32>(),
-      ws.nend.as<u32>(), ws.skip.as<u32>(), ws.isleaf.as<u8>(), ws.root.as<TreeRoot>(), m,
-      inv_theta_guard, y_mean, ls.lrec.as<LWalkRec>());
+  launch(k_lwalk_rec32, ceil_div(m, kT), kT, 0, s, ws.geom.as<double2>(),
+         ls.cells32.as<float4>(), cfeat.as<CellFeat>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
+         ws.skip.as<u32>(), ws.isleaf.as<u8>(), ws.root.as<TreeRoot>(), m, inv_theta_guard,
+         y_mean, ls.lrec.as<LWalkRec>());
   GTC_LAUNCH_CHECK();
 }
 
 void learned_group_tolerances(Workspace &ws, const LearnedWalk &lw, u32 ng, cudaStream_t s) {
   if (ng == 0) return;
   lw.gtol->ensure(static_cast<u64>(ng) * sizeof(float2));
-  k_group_tol<<<ceil_div(ng, kT), kT, 0, s>>>(
-      ws.gbegin.as<u32>(), ws.gend.as<u32>(), ng, ws.idx.as<u32>(), lw.prev_amag,
-      ws.gboxf.as<float>(), ws.root.as<TreeRoot>(), lw.scratch->rootmom.as<double2>(), lw.alpha,
-      lw.G, lw.gtol->as<float2>());
+  launch(k_group_tol, ceil_div(ng, kT), kT, 0, s, ws.gbegin.as<u32>(), ws.gend.as<u32>(), ng,
+         ws.idx.as<u32>(), lw.prev_amag, ws.gboxf.as<float>(), ws.root.as<TreeRoot>(),
+         lw.scratch->rootmom.as<double2>(), lw.alpha, lw.G, lw.gtol->as<float2>());
   GTC_LAUNCH_CHECK();
 }
 
@@ -1109,16 +1121,15 @@ void learned_build_lists(Workspace &ws, const LearnedWalk &lw, u32 ng, Scalars *
     a.cells = ws.cell_list.as<u32>();
     a.bodies = ws.body_list.as<u32>();
     a.pend = ls.pend.as<u32>();
-    GTC_CUDA(cudaMemsetAsync(&sc->cell_interactions, 0, 3 * sizeof(unsigned long long), s));
-    GTC_CUDA(cudaMemsetAsync(&sc->max_group, 0, sizeof(u32), s));
-    GTC_CUDA(cudaMemsetAsync(&sc->list_overflow, 0, sizeof(u32), s));
-    GTC_CUDA(cudaMemsetAsync(sc->lmax_cells, 0,
-                             offsetof(Scalars, max_pend) + sizeof(u32) -
-                                 offsetof(Scalars, lmax_cells),
-                             s));  // lmax_cells, lmax_bodies, max_pend
-    GTC_CUDA(cudaMemsetAsync(&sc->walk_nodes, 0, sizeof(unsigned long long), s));
-    GTC_CUDA(cudaMemsetAsync(&sc->mlp_rows, 0, 2 * sizeof(unsigned long long), s));
-    GTC_CUDA(cudaMemsetAsync(&sc->max_rows, 0, sizeof(u32), s));
+    clear({{&sc->cell_interactions, 3 * sizeof(unsigned long long)},
+           {&sc->max_group, sizeof(u32)},
+           {&sc->list_overflow, sizeof(u32)},
+           {sc->lmax_cells,  // lmax_cells, lmax_bodies, max_pend
+            offsetof(Scalars, max_pend) + sizeof(u32) - offsetof(Scalars, lmax_cells)},
+           {&sc->walk_nodes, sizeof(unsigned long long)},
+           {&sc->mlp_rows, 2 * sizeof(unsigned long long)},
+           {&sc->max_rows, sizeof(u32)}},
+          s);
     u32 *roff = ls.roff.as<u32>();
     int qsel = 0;
     // one round: its walk, the warps' continuations, and the scan of the
@@ -1131,18 +1142,18 @@ void learned_build_lists(Workspace &ws, const LearnedWalk &lw, u32 ng, Scalars *
         a.dec = ls.dec[qsel].as<u8>();
       }
       if (warps) {
-        GTC_CUDA(cudaMemsetAsync(a.next, 0, sizeof(u32), s));
-        k_lwarp<<<warp_blocks, kLWarps * 32, 0, s>>>(a, r);
+        clear({{a.next, sizeof(u32)}}, s);
+        launch(k_lwarp, warp_blocks, kLWarps * 32, 0, s, a, r);
         GTC_LAUNCH_CHECK();
       } else {
         GTC_CUDA(cudaMemsetAsync(&sc->lcont, 0, 2 * sizeof(u32), s));
         a.budget = r == 0 ? lw.walk_budget : lw.pair_budget;
         if (r == 0)
-          k_lround0<<<rb, kRoundThreads, 0, s>>>(a);
+          launch(k_lround0, rb, kRoundThreads, 0, s, a);
         else
-          k_lround<<<rb, kRoundThreads, 0, s>>>(a);
+          launch(k_lround, rb, kRoundThreads, 0, s, a);
         GTC_LAUNCH_CHECK();
-        k_lcont<<<cont_blocks, kContWarps * 32, 0, s>>>(a, r > 0);
+        launch(k_lcont, cont_blocks, kContWarps * 32, 0, s, a, r > 0);
         GTC_LAUNCH_CHECK();
       }
       exclusive_scan_u32(a.pcount, roff, nparts, roff + nparts, ws.scan_tmp, s,
@@ -1153,13 +1164,12 @@ void learned_build_lists(Workspace &ws, const LearnedWalk &lw, u32 ng, Scalars *
     auto decide = [&](u64 launch_rows) {
       const int nq = qsel ^ 1;
       const u64 cap = std::min<u64>(ls.q[nq].bytes / sizeof(uint2), ls.dec[nq].bytes);  // rows held
-      k_lrows<<<pb, kT, 0, s>>>(a, ls.q[nq].as<uint2>(), cap);
+      launch(k_lrows, pb, kT, 0, s, a, ls.q[nq].as<uint2>(), cap);
       GTC_LAUNCH_CHECK();
       if (launch_rows > 0) {
-        k_ldecide<<<ceil_div(launch_rows, kT), kT, 0, s>>>(
-            ls.q[nq].as<uint2>(), launch_rows, a.lrec, lw.cfeat, a.gboxf, a.gtol, lw.net,
-            ws.root.as<TreeRoot>(), a.mom, ls.dec[nq].as<u8>(), roff + nparts,
-            &sc->list_overflow);
+        launch(k_ldecide, ceil_div(launch_rows, kT), kT, 0, s, ls.q[nq].as<uint2>(), launch_rows,
+               a.lrec, lw.cfeat, a.gboxf, a.gtol, lw.net, ws.root.as<TreeRoot>(), a.mom,
+               ls.dec[nq].as<u8>(), roff + nparts, &sc->list_overflow);
         GTC_LAUNCH_CHECK();
       }
       qsel = nq;
@@ -1230,9 +1240,9 @@ void learned_build_lists(Workspace &ws, const LearnedWalk &lw, u32 ng, Scalars *
     if (h.list_overflow & 2u) ls.row_cap = std::max<u32>(ls.row_cap, learned_slot(h.max_rows));
   }
   // group records and statistics
-  GTC_CUDA(cudaMemsetAsync(&sc->n_cell_list, 0, 2 * sizeof(u64), s));
-  k_lgroup_records<<<gb, kT, 0, s>>>(a, ws.gbegin.as<u32>(), ws.gend.as<u32>(),
-                                     ws.groups.as<uint4>());
+  clear({{&sc->n_cell_list, 2 * sizeof(u64)}}, s);
+  launch(k_lgroup_records, gb, kT, 0, s, a, ws.gbegin.as<u32>(), ws.gend.as<u32>(),
+         ws.groups.as<uint4>());
   GTC_LAUNCH_CHECK();
   GTC_CUDA(cudaMemcpyAsync(host, sc, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
   GTC_CUDA(cudaStreamSynchronize(s));

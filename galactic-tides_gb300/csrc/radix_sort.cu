@@ -87,6 +87,7 @@ __device__ __forceinline__ unsigned peers_of(u32 d, bool ok) {
 // Digit counts of every pass: hist[p][d] += pairs whose digit p is d.
 __global__ void __launch_bounds__(kThreads)
     k_digit_counts(const u64 *keys, u32 n, int low_bit, int passes, u32 *hist) {
+  grid_wait();
   __shared__ u32 h[kMaxPasses][kBins];
   for (int p = 0; p < passes; ++p) h[p][threadIdx.x] = 0;
   __syncthreads();
@@ -102,6 +103,7 @@ __global__ void __launch_bounds__(kThreads)
 
 // Each pass's digit starts: an exclusive scan of its 256 counts (block p).
 __global__ void __launch_bounds__(kThreads) k_digit_starts(const u32 *hist, u32 *start) {
+  grid_wait();
   __shared__ u32 wsum[kWarps];
   const int d = threadIdx.x, lane = d & 31, warp = d >> 5;
   const u32 c = hist[blockIdx.x * kBins + d];
@@ -121,6 +123,7 @@ __global__ void __launch_bounds__(kThreads) k_digit_starts(const u32 *hist, u32 
 __global__ void __launch_bounds__(kThreads)
     k_onesweep(const u64 *keys, const u32 *vals, u64 *keys_out, u32 *vals_out, u32 n, int shift,
                const u32 *digit_start, u64 *status, u32 *tile_counter, u32 *error) {
+  grid_wait();
   __shared__ u32 wh[kWarps][kBins];     // per-warp running counts
   __shared__ u32 woff[kWarps][kBins];   // per-warp start within the tile's digit run
   __shared__ u32 dstart[kBins];         // start of each digit's run inside the tile
@@ -285,6 +288,7 @@ struct ClusterSort {
 template <int kPer>
 __global__ void __launch_bounds__(kCT)
     k_sort_cluster(u64 *keys, u32 *vals, u32 n, u32 ctas, int low_bit, int passes) {
+  grid_wait();
   extern __shared__ __align__(16) unsigned char raw[];
   ClusterSort<kPer> &sm = *reinterpret_cast<ClusterSort<kPer> *>(raw);
   constexpr u32 kShare = kCT * kPer;
@@ -440,8 +444,9 @@ void launch_cluster(u64 *keys, u32 *vals, u32 n, int low_bit, int passes, bool s
   allow_cluster<kPer>(sixteen);
   u32 ctas = 1;
   while (ctas * kCT * kPer < n) ctas *= 2;
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = cluster_config<kPer>(ctas, &attr, s);
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = cluster_config<kPer>(ctas, attr, s);
+  add_early_start(cfg, attr);
   GTC_CUDA(cudaLaunchKernelEx(&cfg, k_sort_cluster<kPer>, keys, vals, n, ctas, low_bit, passes));
   GTC_LAUNCH_CHECK();
 }
@@ -476,15 +481,16 @@ void radix_sort_pairs(u64 *keys, u32 *vals, u64 *alt_keys, u32 *alt_vals, u32 n,
   u32 *start = hist + kMaxPasses * kBins;
   u32 *tiles = start + kMaxPasses * kBins;
   u32 *own_error = tiles + kMaxPasses;
-  GTC_CUDA(cudaMemsetAsync(status, 0, static_cast<u64>(passes) * ntiles * kBins * sizeof(u64), s));
-  GTC_CUDA(cudaMemsetAsync(hist, 0, small * sizeof(u32), s));
+  clear({{status, static_cast<u64>(passes) * ntiles * kBins * sizeof(u64)},
+         {hist, small * sizeof(u32)}},
+        s);
   int dev = 0, sms = 0;
   GTC_CUDA(cudaGetDevice(&dev));
   GTC_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const u32 hblocks = std::min<u32>(ceil_div(n, kThreads), 4u * static_cast<u32>(sms));
-  k_digit_counts<<<hblocks, kThreads, 0, s>>>(keys, n, low_bit, passes, hist);
+  launch(k_digit_counts, hblocks, kThreads, 0, s, keys, n, low_bit, passes, hist);
   GTC_LAUNCH_CHECK();
-  k_digit_starts<<<passes, kThreads, 0, s>>>(hist, start);
+  launch(k_digit_starts, passes, kThreads, 0, s, hist, start);
   GTC_LAUNCH_CHECK();
 
   // Ping-pong between the two buffers; an odd number of passes ends with
@@ -492,10 +498,9 @@ void radix_sort_pairs(u64 *keys, u32 *vals, u64 *alt_keys, u32 *alt_vals, u32 n,
   u64 *src_k = keys, *dst_k = alt_keys;
   u32 *src_v = vals, *dst_v = alt_vals;
   for (int p = 0; p < passes; ++p) {
-    k_onesweep<<<ntiles, kThreads, 0, s>>>(src_k, src_v, dst_k, dst_v, n, low_bit + 8 * p,
-                                           start + p * kBins,
-                                           status + static_cast<u64>(p) * ntiles * kBins,
-                                           tiles + p, error ? error : own_error);
+    launch(k_onesweep, ntiles, kThreads, 0, s, src_k, src_v, dst_k, dst_v, n, low_bit + 8 * p,
+           start + p * kBins, status + static_cast<u64>(p) * ntiles * kBins, tiles + p,
+           error ? error : own_error);
     GTC_LAUNCH_CHECK();
     std::swap(src_k, dst_k);
     std::swap(src_v, dst_v);

@@ -96,6 +96,7 @@ __device__ u64 look_back(const u64 *status, u32 tile, u32 *error) {
 template <class T>
 __global__ void __launch_bounds__(kThreads)
     k_scan(const T *in, T *out, u64 n, T *total_dev, u64 *status, u32 *counter, u32 *error) {
+  grid_wait();
   __shared__ T ws[kThreads / 32];
   __shared__ u32 tile_s;
   __shared__ u64 before_s;
@@ -139,6 +140,7 @@ constexpr u64 kSmall = kSmallThreads * kItems;
 template <class T>
 __global__ void __launch_bounds__(kSmallThreads)
     k_scan_small(const T *in, T *out, u32 n, T *total_dev) {
+  grid_wait();
   __shared__ T ws[kSmallThreads / 32];
   const u32 base = threadIdx.x * kItems;
   T v[kItems];
@@ -158,6 +160,25 @@ __global__ void __launch_bounds__(kSmallThreads)
   if (total_dev && threadIdx.x == kSmallThreads - 1) *total_dev = run;
 }
 
+struct ClearRanges {
+  u32 *ptr[kClearRanges];
+  u64 words[kClearRanges];
+};
+__global__ void __launch_bounds__(kThreads) k_clear(ClearRanges r) {
+  grid_wait();
+  const u64 first = blockIdx.x * static_cast<u64>(kThreads) + threadIdx.x,
+            stride = static_cast<u64>(gridDim.x) * kThreads;
+#pragma unroll
+  for (int k = 0; k < kClearRanges; ++k) {
+    u32 *p = r.ptr[k];
+    const u64 words = r.words[k];
+    const u64 vectors = (reinterpret_cast<uintptr_t>(p) & 15) == 0 ? words / 4 : 0;
+    for (u64 i = first; i < vectors; i += stride)
+      reinterpret_cast<uint4 *>(p)[i] = make_uint4(0u, 0u, 0u, 0u);
+    for (u64 i = 4 * vectors + first; i < words; i += stride) p[i] = 0u;
+  }
+}
+
 // Scratch: the tiles' words, their counter and an error word.
 u64 scratch_bytes(u64 n) { return (n + kTile - 1) / kTile * sizeof(u64) + 4 * sizeof(u32); }
 
@@ -169,7 +190,7 @@ void scan_impl(const T *in, T *out, u64 n, T *total_dev, DeviceBuffer &tmp, cuda
     return;
   }
   if (n <= kSmall) {
-    k_scan_small<T><<<1, kSmallThreads, 0, s>>>(in, out, static_cast<u32>(n), total_dev);
+    launch(k_scan_small<T>, 1, kSmallThreads, 0, s, in, out, static_cast<u32>(n), total_dev);
     GTC_LAUNCH_CHECK();
     return;
   }
@@ -177,13 +198,28 @@ void scan_impl(const T *in, T *out, u64 n, T *total_dev, DeviceBuffer &tmp, cuda
   tmp.ensure(scratch_bytes(n));
   u64 *status = tmp.as<u64>();
   u32 *counter = reinterpret_cast<u32 *>(status + tiles);
-  GTC_CUDA(cudaMemsetAsync(tmp.ptr, 0, scratch_bytes(n), s));
-  k_scan<T><<<tiles, kThreads, 0, s>>>(in, out, n, total_dev, status, counter,
-                                       error ? error : counter + 1);
+  clear({{tmp.ptr, scratch_bytes(n)}}, s);
+  launch(k_scan<T>, tiles, kThreads, 0, s, in, out, n, total_dev, status, counter,
+         error ? error : counter + 1);
   GTC_LAUNCH_CHECK();
 }
 
 }  // namespace
+
+void clear(std::initializer_list<ClearRange> ranges, cudaStream_t s) {
+  ClearRanges r{};
+  u64 most = 0;
+  int k = 0;
+  for (const ClearRange &c : ranges) {
+    if (k == kClearRanges || c.bytes % 4) throw RuntimeError("clear: ranges");
+    r.ptr[k] = static_cast<u32 *>(c.ptr);
+    r.words[k++] = c.bytes / 4;
+    most = std::max(most, c.bytes);
+  }
+  if (most == 0) return;
+  launch(k_clear, static_cast<u32>(std::min<u64>(1024, (most + 4095) / 4096)), kThreads, 0, s, r);
+  GTC_LAUNCH_CHECK();
+}
 
 void exclusive_scan_u32(const u32 *in, u32 *out, u64 n, u32 *total_dev, DeviceBuffer &tmp,
                         cudaStream_t s, u32 *error) {

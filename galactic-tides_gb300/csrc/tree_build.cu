@@ -219,6 +219,7 @@ __device__ void root_from_parts(const double *part, int nparts, TreeRoot *root, 
 // blocks and wraps to zero by itself.
 __global__ void __launch_bounds__(kT)
     k_bbox(const double *pos, u64 n, double *part, u32 *ticket, TreeRoot *root, double *split) {
+  grid_wait();
   const u64 inf_lo = order_key(INFINITY), inf_hi = order_key(-INFINITY);
   u64 lo[3] = {inf_lo, inf_lo, inf_lo}, hi[3] = {inf_hi, inf_hi, inf_hi};
   auto take = [&](int a, double v) {
@@ -284,6 +285,7 @@ __global__ void __launch_bounds__(kT)
 // root.
 __global__ void __launch_bounds__(kT)
     k_bbox_forest(const double *pos, const uint4 *blk, const u32 *start, double *part) {
+  grid_wait();
   const uint4 q = blk[blockIdx.x];
   const u64 b0 = start[q.x], b1 = start[q.x + 1];
   const u64 inf_lo = order_key(INFINITY), inf_hi = order_key(-INFINITY);
@@ -323,6 +325,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_root_forest(const double *part, const uint2 *sys_blk, TreeRoot *roots, int levels,
                   double *split) {
+  grid_wait();
   const uint2 q = sys_blk[blockIdx.x];
   root_from_parts(part + 6ull * q.x, static_cast<int>(q.y), roots + blockIdx.x, levels,
                   split + (static_cast<u64>(3u * blockIdx.x) << levels));
@@ -378,6 +381,7 @@ __device__ __forceinline__ bool grid_rank(double x, double centre, double grid, 
 __global__ void __launch_bounds__(kT)
     k_keys(const double *pos, u32 n, const u16 *sys, const TreeRoot *roots, u64 *key, u32 *idx,
            u8 *tiny, u32 *error) {
+  grid_wait();
   const u32 i = blockIdx.x * kT + threadIdx.x;
   if (i >= n) return;
   const TreeRoot *root = roots + (sys ? sys[i] : 0);  // (a forest: the body's system's)
@@ -426,6 +430,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_forest_sys_keys(const u64 *key, const u32 *idx, const u16 *sys, u32 n, u64 *skey, u32 *spos,
                       u64 *key_copy, u32 *idx_copy, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= n || aborted(abort)) return;
   const u32 i = idx[k];
@@ -438,6 +443,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_forest_gather(const u32 *spos, const u64 *key_copy, const u32 *idx_copy, u32 n, u64 *key,
                     u32 *idx, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= n || aborted(abort)) return;
   const u32 j = spos[k];
@@ -450,6 +456,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_levels(KeyView kv, const u32 *idx, const u8 *tiny, u32 n, int L, signed char *lcp_next,
              u8 *leafdepth, u32 *count, Scalars *sc) {
+  grid_wait();
   // win[i] = lcp(i, i + L) for the block's positions and the L before them,
   // each computed once; a body's w is the largest over its windows
   constexpr int kMaxWin = 64;
@@ -493,12 +500,14 @@ __global__ void __launch_bounds__(kT)
 
 __global__ void __launch_bounds__(kT)
     k_deep_flags(const u8 *leafdepth, u32 n, int limit, u32 *flag) {
+  grid_wait();
   const u32 b = blockIdx.x * kT + threadIdx.x;
   if (b < n) flag[b] = leafdepth[b] > limit ? 1u : 0u;
 }
 
 __global__ void __launch_bounds__(kT)
     k_compact(const u32 *flag, const u32 *scan, u32 n, u32 *out) {
+  grid_wait();
   const u32 b = blockIdx.x * kT + threadIdx.x;
   if (b < n && flag[b]) out[scan[b]] = b;
 }
@@ -508,6 +517,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_deep_keys(KeyView kv, const u32 *dpos, u32 nd, const u32 *idx, const double *pos,
                 const TreeRoot *root, u8 *tiny, u64 *word, u32 *rec, u32 *didx) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= nd) return;
   const u32 b = dpos[k];
@@ -540,6 +550,7 @@ __global__ void __launch_bounds__(kT)
 // words change (a different depth-21*words node).
 __global__ void __launch_bounds__(kT)
     k_deep_segments(KeyView kv, const u32 *dpos, u32 nd, u32 *flag) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= nd) return;
   bool start = k == 0;
@@ -553,6 +564,7 @@ __global__ void __launch_bounds__(kT)
 
 __global__ void __launch_bounds__(kT)
     k_seg_keys(const u32 *rec, const u32 *seg_scan, const u32 *seg_flag, u32 nd, u64 *key) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= nd) return;
   const u32 r = rec[k];
@@ -564,6 +576,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_deep_scatter(const u32 *dpos, const u32 *rec, const u32 *didx, const u64 *word, u32 nd,
                    u32 *idx, u64 *word_out) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= nd) return;
   const u32 r = rec[k];
@@ -579,6 +592,7 @@ __global__ void __launch_bounds__(kT)
             const u32 *count_scan, u32 n, const Scalars *sc, const TreeRoot *root,
             const double *split, double2 *geom, u32 *nbegin, u32 *nend, u32 *skip, u8 *depth,
             u8 *isleaf, int table_levels, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 table_size = 1u << table_levels;
   const u32 b = blockIdx.x * kT + threadIdx.x;
   if (b >= n || aborted(abort)) return;
@@ -668,6 +682,7 @@ __device__ __forceinline__ int children_of(u32 p, const u32 *skip, u32 ch[8]) {
 __global__ void __launch_bounds__(kT)
     k_children(const u32 *skip, const u8 *isleaf, u32 m, u32 *parent, u8 *nchild, uint4 *kids,
                const u32 *m_dev = nullptr, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort) || p >= bounded(m, m_dev)) return;
   if (p == 0) parent[0] = 0xffffffffu;
@@ -688,6 +703,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_forest_roots(const u32 *start, u32 systems, const u32 *count, const u32 *count_scan,
                    const Scalars *sc, u32 *root_node, u32 *parent, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= systems || aborted(abort)) return;
   const u32 last = start[k + 1] - 1;
@@ -700,6 +716,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_leaf_order(const u8 *isleaf, const u32 *nbegin, const u32 *nend, u32 m, u32 *idx,
                  const u32 *m_dev = nullptr, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort) || p >= bounded(m, m_dev) || !isleaf[p]) return;
   const u32 b0 = nbegin[p], b1 = nend[p];
@@ -717,6 +734,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_tree_order(const double *pos, const double *mass, const u32 *idx, u32 n, double *tpos,
                  double *tmass, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= n || aborted(abort)) return;
   const u64 i = idx[k];
@@ -1029,6 +1047,7 @@ __device__ __forceinline__ int bucket_of(const BucketView &v, u32 p) {
 __global__ void __launch_bounds__(kT)
     k_bucket_count(BucketView v, u32 m, u32 *count, const u32 *m_dev = nullptr,
                    const u32 *abort = nullptr) {
+  grid_wait();
   __shared__ u32 h[kBuckets];
   if (aborted(abort)) return;
   if (threadIdx.x < kBuckets) h[threadIdx.x] = 0;
@@ -1047,6 +1066,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_bucket_fill(BucketView v, u32 m, u32 *meta, u32 *bucket, const u32 *m_dev = nullptr,
                   const u32 *abort = nullptr) {
+  grid_wait();
   __shared__ u32 h[kBuckets], base[kBuckets];
   if (aborted(abort)) return;
   if (threadIdx.x < kBuckets) h[threadIdx.x] = 0;
@@ -1108,6 +1128,7 @@ template <bool kQuad>
 __global__ void __launch_bounds__(kUpThreads)
     k_moments_up(MomentArrays a, const u32 *bucket, const u32 *meta, const u8 *isleaf, u32 m,
                  u32 per_block, u32 *arrive, const u32 *m_dev, const u32 *abort) {
+  grid_wait();
   constexpr u32 kLanes = kQuad ? 8 : 4;
   __shared__ u32 queue[2][kMostLeaves];
   __shared__ u32 queued[2];
@@ -1163,6 +1184,7 @@ constexpr u32 kLeafThreads = 64;  // small blocks: small trees spread over the S
 __global__ void __launch_bounds__(kLeafThreads)
     k_leaf_quads(MomentArrays a, const u32 *bucket, const u32 *meta, const u8 *isleaf, u32 m,
                  const u32 *m_dev, const u32 *abort) {
+  grid_wait();
   if (aborted(abort)) return;
   const u32 p = nth_leaf(static_cast<u64>(blockIdx.x) * kLeafThreads + threadIdx.x, bucket, meta,
                          isleaf, bounded(m, m_dev));
@@ -1173,6 +1195,7 @@ __global__ void __launch_bounds__(kLeafThreads)
 // records, which hold them otherwise) its delta too.
 __global__ void __launch_bounds__(kLeafThreads)
     k_quad_terms(MomentArrays a, u32 m, bool deltas, const u32 *m_dev, const u32 *abort) {
+  grid_wait();
   const u32 p = blockIdx.x * kLeafThreads + threadIdx.x;
   if (aborted(abort) || p >= bounded(m, m_dev)) return;
   quad_term(a, p);
@@ -1189,6 +1212,7 @@ __global__ void __launch_bounds__(kLeafThreads)
 __global__ void __launch_bounds__(kT)
     k_moments32_up(Moment32Arrays a, const u32 *bucket, const u32 *meta, const u32 *parent,
                    u32 *arrive) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= leaf_count(meta)) return;
   u32 p = bucket[k];
@@ -1205,6 +1229,7 @@ __global__ void __launch_bounds__(kT)
 }
 
 __global__ void k_root_mass(const float4 *cells32, double2 *rootmom) {
+  grid_wait();
   rootmom[0] = make_double2(0.0, 0.0);
   rootmom[1] = make_double2(0.0, static_cast<double>(cells32[0].w));
 }
@@ -1213,6 +1238,7 @@ __global__ void k_root_mass(const float4 *cells32, double2 *rootmom) {
 // leaf below the sorted levels (bit 1), or more nodes than the node arrays
 // hold (bit 2).
 __global__ void k_check_tree_graph(Scalars *sc, u32 cap, int sorted_levels) {
+  grid_wait();
   if (sc->deep > 0 || static_cast<int>(sc->depth) > sorted_levels) sc->abort |= 1u;
   if (sc->n_nodes > cap) sc->abort |= 2u;
 }
@@ -1228,6 +1254,7 @@ __global__ void __launch_bounds__(kT)
                 double inv_theta, WalkRec32 *walk32, WalkRec64 *walk64,
                 const u32 *m_dev = nullptr, const u32 *abort = nullptr,
                 const u16 *sys = nullptr) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort) || p >= bounded(m, m_dev)) return;
   if (sys) root += sys[nbegin[p]];  // a forest: relative to the node's system's root
@@ -1270,6 +1297,7 @@ __global__ void __launch_bounds__(kT)
     k_pack_cells(const double2 *mom, const double2 *quad, const u32 *nbegin, u32 m,
                  const TreeRoot *root, float4 *cells, const u32 *m_dev = nullptr,
                  const u32 *abort = nullptr, const u16 *sys = nullptr) {
+  grid_wait();
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort) || p >= bounded(m, m_dev)) return;
   if (sys) root += sys[nbegin[p]];
@@ -1287,6 +1315,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_pack_bodies_forest(const double *tpos, const double *tmass, u32 n, const u16 *sys,
                          const TreeRoot *roots, float4 *bodies, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= n || aborted(abort)) return;
   const double *o = roots[sys[k]].center;
@@ -1300,6 +1329,7 @@ __global__ void __launch_bounds__(kT)
 __global__ void __launch_bounds__(kT)
     k_pack_bodies(const double *tpos, const double *tmass, u32 n, const double *origin,
                   float4 *bodies, const u32 *abort = nullptr) {
+  grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
   if (k >= n || aborted(abort)) return;
   bodies[k] = make_float4(static_cast<float>(tpos[3ull * k] - origin[0]),
@@ -1329,8 +1359,8 @@ void bbox_root(Workspace &ws, const double *pos, u64 n, cudaStream_t s, bool spl
     GTC_CUDA(cudaMemsetAsync(ws.bbox_ticket.ptr, 0, sizeof(u32), s));
   }
   if (split) ws.split.ensure(3ull * kSplitSize * sizeof(double));
-  k_bbox<<<nparts, kT, 0, s>>>(pos, n, ws.bbox_part.as<double>(), ws.bbox_ticket.as<u32>(),
-                               ws.root.as<TreeRoot>(), split ? ws.split.as<double>() : nullptr);
+  launch(k_bbox, nparts, kT, 0, s, pos, n, ws.bbox_part.as<double>(), ws.bbox_ticket.as<u32>(),
+         ws.root.as<TreeRoot>(), split ? ws.split.as<double>() : nullptr);
   GTC_LAUNCH_CHECK();
 }
 
@@ -1339,8 +1369,8 @@ void pack_bodies_bbox(Workspace &ws, const double *pos, const double *mass, u64 
   bbox_root(ws, pos, n, s, false);
   ws.bodies.ensure(n * sizeof(float4));
   const TreeRoot *root = ws.root.as<TreeRoot>();
-  k_pack_bodies<<<ceil_div(n, kT), kT, 0, s>>>(pos, mass, static_cast<u32>(n),
-                                               root_centre(root), ws.bodies.as<float4>());
+  launch(k_pack_bodies, ceil_div(n, kT), kT, 0, s, pos, mass, static_cast<u32>(n),
+         root_centre(root), ws.bodies.as<float4>());
   GTC_LAUNCH_CHECK();
 }
 
@@ -1387,9 +1417,8 @@ void join_walk(Workspace &ws, cudaStream_t s) {
 namespace {
 // The first key word of every body.
 void make_keys(Workspace &ws, const double *pos, u32 n, const TreeRoot *root, cudaStream_t s) {
-  k_keys<<<ceil_div(n, kT), kT, 0, s>>>(pos, n, ws.forest.sys, root, ws.key0.as<u64>(),
-                                        ws.idx.as<u32>(), ws.tiny.as<u8>(),
-                                        &ws.scalars.as<Scalars>()->error);
+  launch(k_keys, ceil_div(n, kT), kT, 0, s, pos, n, ws.forest.sys, root, ws.key0.as<u64>(),
+         ws.idx.as<u32>(), ws.tiny.as<u8>(), &ws.scalars.as<Scalars>()->error);
   GTC_LAUNCH_CHECK();
 }
 
@@ -1416,15 +1445,15 @@ int sort_top_levels(Workspace &ws, u32 n, int levels, cudaStream_t s,
     u64 *skey = ws.dkey.as<u64>();
     u32 *spos = ws.drec.as<u32>();
     const u32 nb = ceil_div(n, kT);
-    k_forest_sys_keys<<<nb, kT, 0, s>>>(ws.key0.as<u64>(), ws.idx.as<u32>(), fv.sys, n, skey,
-                                        spos, ws.key0_alt.as<u64>(), ws.idx_alt.as<u32>(), abort);
+    launch(k_forest_sys_keys, nb, kT, 0, s, ws.key0.as<u64>(), ws.idx.as<u32>(), fv.sys, n, skey,
+           spos, ws.key0_alt.as<u64>(), ws.idx_alt.as<u32>(), abort);
     GTC_LAUNCH_CHECK();
     int bits = 1;
     while (bits < 16 && (1u << bits) < fv.systems) ++bits;
     radix_sort_pairs(skey, spos, ws.dkey_alt.as<u64>(), ws.drec_alt.as<u32>(), n, bits, ws.radix,
                      s, 0, err);
-    k_forest_gather<<<nb, kT, 0, s>>>(spos, ws.key0_alt.as<u64>(), ws.idx_alt.as<u32>(), n,
-                                      ws.key0.as<u64>(), ws.idx.as<u32>(), abort);
+    launch(k_forest_gather, nb, kT, 0, s, spos, ws.key0_alt.as<u64>(), ws.idx_alt.as<u32>(), n,
+           ws.key0.as<u64>(), ws.idx.as<u32>(), abort);
     GTC_LAUNCH_CHECK();
   }
   return low == 0 ? kLevelsPerWord : (3 * kLevelsPerWord - low) / 3;
@@ -1435,31 +1464,31 @@ void forest_roots_and_tables(Workspace &ws, const double *pos, cudaStream_t s) {
   const ForestView &fv = ws.forest;
   ws.bbox_part.ensure(6 * sizeof(double) * fv.bbox_nblocks);
   ws.split.ensure((3ull * fv.systems << fv.split_levels) * sizeof(double));
-  k_bbox_forest<<<fv.bbox_nblocks, kT, 0, s>>>(pos, fv.bbox_blocks, fv.start,
-                                               ws.bbox_part.as<double>());
+  launch(k_bbox_forest, fv.bbox_nblocks, kT, 0, s, pos, fv.bbox_blocks, fv.start,
+         ws.bbox_part.as<double>());
   GTC_LAUNCH_CHECK();
-  k_root_forest<<<fv.systems, kT, 0, s>>>(ws.bbox_part.as<double>(), fv.sys_blocks, fv.roots,
-                                          fv.split_levels, ws.split.as<double>());
+  launch(k_root_forest, fv.systems, kT, 0, s, ws.bbox_part.as<double>(), fv.sys_blocks, fv.roots,
+         fv.split_levels, ws.split.as<double>());
   GTC_LAUNCH_CHECK();
 }
 
 void forest_roots(Workspace &ws, const u32 *abort, cudaStream_t s) {
   const ForestView &fv = ws.forest;
-  k_forest_roots<<<ceil_div(fv.systems, kT), kT, 0, s>>>(
-      fv.start, fv.systems, ws.count.as<u32>(), ws.count_scan.as<u32>(),
-      ws.scalars.as<Scalars>(), fv.root_node, ws.parent.as<u32>(), abort);
+  launch(k_forest_roots, ceil_div(fv.systems, kT), kT, 0, s, fv.start, fv.systems,
+         ws.count.as<u32>(), ws.count_scan.as<u32>(), ws.scalars.as<Scalars>(), fv.root_node,
+         ws.parent.as<u32>(), abort);
   GTC_LAUNCH_CHECK();
 }
 
 void pack_bodies_tree(Workspace &ws, u32 n, const TreeRoot *root, const u32 *abort,
                       cudaStream_t s) {
   if (ws.forest) {
-    k_pack_bodies_forest<<<ceil_div(n, kT), kT, 0, s>>>(ws.tpos.as<double>(), ws.tmass.as<double>(),
-                                                        n, ws.forest.sys, ws.forest.roots,
-                                                        ws.bodies.as<float4>(), abort);
+    launch(k_pack_bodies_forest, ceil_div(n, kT), kT, 0, s, ws.tpos.as<double>(),
+           ws.tmass.as<double>(), n, ws.forest.sys, ws.forest.roots, ws.bodies.as<float4>(),
+           abort);
   } else {
-    k_pack_bodies<<<ceil_div(n, kT), kT, 0, s>>>(ws.tpos.as<double>(), ws.tmass.as<double>(), n,
-                                                 root_centre(root), ws.bodies.as<float4>(), abort);
+    launch(k_pack_bodies, ceil_div(n, kT), kT, 0, s, ws.tpos.as<double>(), ws.tmass.as<double>(),
+           n, root_centre(root), ws.bodies.as<float4>(), abort);
   }
   GTC_LAUNCH_CHECK();
 }
@@ -1492,14 +1521,16 @@ MomentPlan plan_moments(Workspace &ws, u32 m, bool buckets, cudaStream_t s,
                       ws.mom.as<double2>(), ws.quad.as<double2>(), ws.delta.as<double>(),
                       ws.qterm.as<double>()};
   p.arrive = ws.climb.as<u32>();
-  GTC_CUDA(cudaMemsetAsync(p.arrive, 0, arrive_bytes(m), s));
-  if (buckets || m >= kBucketNodes) {
+  const bool use_buckets = buckets || m >= kBucketNodes;
+  clear({{p.arrive, arrive_bytes(m)},
+         {ws.arrive.ptr, use_buckets ? 2 * kBuckets * sizeof(u32) : 0}},
+        s);
+  if (use_buckets) {
     u32 *meta = ws.arrive.as<u32>(), *bucket = ws.bucket.as<u32>();
-    GTC_CUDA(cudaMemsetAsync(meta, 0, 2 * kBuckets * sizeof(u32), s));
     const BucketView bv{ws.isleaf.as<u8>(), ws.nbegin.as<u32>(), ws.nend.as<u32>()};
-    k_bucket_count<<<ceil_div(m, kT), kT, 0, s>>>(bv, m, meta, m_dev, abort);
+    launch(k_bucket_count, ceil_div(m, kT), kT, 0, s, bv, m, meta, m_dev, abort);
     GTC_LAUNCH_CHECK();
-    k_bucket_fill<<<ceil_div(m, kT), kT, 0, s>>>(bv, m, meta, bucket, m_dev, abort);
+    launch(k_bucket_fill, ceil_div(m, kT), kT, 0, s, bv, m, meta, bucket, m_dev, abort);
     GTC_LAUNCH_CHECK();
     p.bucket = bucket;
     p.meta = meta;
@@ -1513,8 +1544,8 @@ MomentPlan plan_moments(Workspace &ws, u32 m, bool buckets, cudaStream_t s,
 template <bool kQuad>
 void launch_up(const Workspace &ws, const MomentPlan &p, u32 *arrive, cudaStream_t s) {
   const u32 per_block = p.m >= kBucketNodes ? kMostLeaves : 32u;
-  k_moments_up<kQuad><<<ceil_div(p.m, per_block), kUpThreads, 0, s>>>(
-      p.ma, p.bucket, p.meta, ws.isleaf.as<u8>(), p.m, per_block, arrive, p.m_dev, p.abort);
+  launch(k_moments_up<kQuad>, ceil_div(p.m, per_block), kUpThreads, 0, s, p.ma, p.bucket, p.meta,
+         ws.isleaf.as<u8>(), p.m, per_block, arrive, p.m_dev, p.abort);
   GTC_LAUNCH_CHECK();
 }
 
@@ -1524,10 +1555,10 @@ void launch_coms(const Workspace &ws, const MomentPlan &p, cudaStream_t s) {
 
 void launch_pack_walk(Workspace &ws, const MomentPlan &p, const TreeRoot *root, double theta,
                       cudaStream_t s) {
-  k_pack_walk<<<ceil_div(p.m, kT), kT, 0, s>>>(
-      ws.geom.as<double2>(), ws.mom.as<double2>(), ws.delta.as<double>(), ws.nbegin.as<u32>(),
-      ws.nend.as<u32>(), ws.skip.as<u32>(), ws.isleaf.as<u8>(), p.m, root, 1.0 / theta,
-      ws.walk32.as<WalkRec32>(), ws.walk64.as<WalkRec64>(), p.m_dev, p.abort, ws.forest.sys);
+  launch(k_pack_walk, ceil_div(p.m, kT), kT, 0, s, ws.geom.as<double2>(), ws.mom.as<double2>(),
+         ws.delta.as<double>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(), ws.skip.as<u32>(),
+         ws.isleaf.as<u8>(), p.m, root, 1.0 / theta, ws.walk32.as<WalkRec32>(),
+         ws.walk64.as<WalkRec64>(), p.m_dev, p.abort, ws.forest.sys);
   GTC_LAUNCH_CHECK();
 }
 
@@ -1535,16 +1566,14 @@ void launch_pack_walk(Workspace &ws, const MomentPlan &p, const TreeRoot *root, 
 void launch_quads(Workspace &ws, const MomentPlan &p, const TreeRoot *root, bool deltas,
                   cudaStream_t s) {
   const u32 blocks = ceil_div(p.m, kLeafThreads);
-  k_leaf_quads<<<blocks, kLeafThreads, 0, s>>>(p.ma, p.bucket, p.meta, ws.isleaf.as<u8>(), p.m,
-                                               p.m_dev, p.abort);
+  launch(k_leaf_quads, blocks, kLeafThreads, 0, s, p.ma, p.bucket, p.meta, ws.isleaf.as<u8>(),
+         p.m, p.m_dev, p.abort);
   GTC_LAUNCH_CHECK();
-  k_quad_terms<<<blocks, kLeafThreads, 0, s>>>(p.ma, p.m, deltas, p.m_dev, p.abort);
+  launch(k_quad_terms, blocks, kLeafThreads, 0, s, p.ma, p.m, deltas, p.m_dev, p.abort);
   GTC_LAUNCH_CHECK();
   launch_up<true>(ws, p, p.arrive + p.m, s);
-  k_pack_cells<<<ceil_div(p.m, kT), kT, 0, s>>>(ws.mom.as<double2>(), ws.quad.as<double2>(),
-                                                ws.nbegin.as<u32>(), p.m, root,
-                                                ws.cells.as<float4>(), p.m_dev, p.abort,
-                                                ws.forest.sys);
+  launch(k_pack_cells, ceil_div(p.m, kT), kT, 0, s, ws.mom.as<double2>(), ws.quad.as<double2>(),
+         ws.nbegin.as<u32>(), p.m, root, ws.cells.as<float4>(), p.m_dev, p.abort, ws.forest.sys);
   GTC_LAUNCH_CHECK();
 }
 }  // namespace
@@ -1574,7 +1603,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   ws.scalars.ensure(sizeof(Scalars));
   join_side(ws, s);  // nothing of an earlier call may still write the buffers
   Scalars *sc = ws.scalars.as<Scalars>();
-  GTC_CUDA(cudaMemsetAsync(sc, 0, sizeof(Scalars), s));
+  clear({{sc, sizeof(Scalars)}}, s);
 
   ws.stage(Workspace::kStBuild, s);
   const ForestView &fv = ws.forest;
@@ -1600,7 +1629,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   auto count_nodes = [&] {
     exclusive_scan_u32(count, cscan, n, &sc->n_nodes, ws.scan_tmp, s, &sc->error);
   };
-  k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
+  launch(k_levels, nb, kT, 0, s, kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
   GTC_LAUNCH_CHECK();
   count_nodes();
   read_scalars(ws, host, s);
@@ -1609,7 +1638,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     sort_top_levels(ws, n32, kLevelsPerWord, s);
     GTC_CUDA(cudaMemsetAsync(&sc->deep, 0, sizeof(u32), s));
     GTC_CUDA(cudaMemsetAsync(&sc->depth, 0, sizeof(u32), s));
-    k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
+    launch(k_levels, nb, kT, 0, s, kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
     GTC_LAUNCH_CHECK();
     count_nodes();
     read_scalars(ws, host, s);
@@ -1625,7 +1654,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     ws.flags.ensure(n * 4);
     ws.flags_scan.ensure(n * 4);
     u32 *flag = ws.flags.as<u32>(), *fscan = ws.flags_scan.as<u32>();
-    k_deep_flags<<<nb, kT, 0, s>>>(leafdepth, n32, limit, flag);
+    launch(k_deep_flags, nb, kT, 0, s, leafdepth, n32, limit, flag);
     GTC_LAUNCH_CHECK();
     exclusive_scan_u32(flag, fscan, n, &sc->deep, ws.scan_tmp, s, &sc->error);
     read_scalars(ws, host, s);
@@ -1641,9 +1670,9 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     u32 *didx = ws.dtmp.as<u32>();
     u64 *dword = reinterpret_cast<u64 *>(ws.dtmp.as<char>() + idx_bytes);
     const u32 ndb = ceil_div(nd, kT);
-    k_compact<<<nb, kT, 0, s>>>(flag, fscan, n32, dpos);
+    launch(k_compact, nb, kT, 0, s, flag, fscan, n32, dpos);
     GTC_LAUNCH_CHECK();
-    k_deep_keys<<<ndb, kT, 0, s>>>(kv, dpos, nd, idx, pos, root, tiny, dword, drec, didx);
+    launch(k_deep_keys, ndb, kT, 0, s, kv, dpos, nd, idx, pos, root, tiny, dword, drec, didx);
     GTC_LAUNCH_CHECK();
     // order records by (segment, new word, input order): sort by the word,
     // then stably by segment number
@@ -1652,23 +1681,23 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     radix_sort_pairs(dkey, drec, ws.dkey_alt.as<u64>(), ws.drec_alt.as<u32>(), nd, 63, ws.radix, s,
                      0, &sc->error);
     u32 *sflag = ws.flags.as<u32>(), *sscan = ws.flags_scan.as<u32>();
-    k_deep_segments<<<ndb, kT, 0, s>>>(kv, dpos, nd, sflag);
+    launch(k_deep_segments, ndb, kT, 0, s, kv, dpos, nd, sflag);
     GTC_LAUNCH_CHECK();
     exclusive_scan_u32(sflag, sscan, nd, &sc->aux, ws.scan_tmp, s, &sc->error);
     read_scalars(ws, host, s);
     int seg_bits = 1;
     while (seg_bits < 32 && (1ull << seg_bits) <= host->aux) ++seg_bits;
-    k_seg_keys<<<ndb, kT, 0, s>>>(drec, sscan, sflag, nd, dkey);
+    launch(k_seg_keys, ndb, kT, 0, s, drec, sscan, sflag, nd, dkey);
     GTC_LAUNCH_CHECK();
     radix_sort_pairs(dkey, drec, ws.dkey_alt.as<u64>(), ws.drec_alt.as<u32>(), nd, seg_bits,
                      ws.radix, s, 0, &sc->error);
-    k_deep_scatter<<<ndb, kT, 0, s>>>(dpos, drec, didx, dword, nd, idx, wbuf.as<u64>());
+    launch(k_deep_scatter, ndb, kT, 0, s, dpos, drec, didx, dword, nd, idx, wbuf.as<u64>());
     GTC_LAUNCH_CHECK();
     if (kv.words == 1) kv.w1 = ws.key1.as<u64>();
     else kv.w2 = ws.key2.as<u64>();
     kv.words += 1;
     GTC_CUDA(cudaMemsetAsync(&sc->deep, 0, sizeof(u32), s));
-    k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
+    launch(k_levels, nb, kT, 0, s, kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
     GTC_LAUNCH_CHECK();
     read_scalars(ws, host, s);
   }
@@ -1702,19 +1731,21 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   ws.cells.ensure(m * 3 * sizeof(float4));
   const u32 mb = ceil_div(m, kT);
 
-  k_nodes<<<nb, kT, 0, s>>>(kv, lcp_next, leafdepth, count, cscan, n32, sc, root,
-                            ws.split.as<double>(), ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
-                            ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(),
-                            fv ? fv.split_levels : kSplitLevels, nullptr);
+  launch(k_nodes, nb, kT, 0, s, kv, lcp_next, leafdepth, count, cscan, n32, sc, root,
+         ws.split.as<double>(), ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
+         ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(),
+         fv ? fv.split_levels : kSplitLevels, nullptr);
   GTC_LAUNCH_CHECK();
   ws.kids.ensure(static_cast<u64>(m) * 8 * sizeof(u32));
-  k_children<<<mb, kT, 0, s>>>(ws.skip.as<u32>(), ws.isleaf.as<u8>(), m, ws.parent.as<u32>(),
-                               ws.nchild.as<u8>(), ws.kids.as<uint4>());
+  launch(k_children, mb, kT, 0, s, ws.skip.as<u32>(), ws.isleaf.as<u8>(), m, ws.parent.as<u32>(),
+         ws.nchild.as<u8>(), ws.kids.as<uint4>());
   GTC_LAUNCH_CHECK();
   if (fv) forest_roots(ws, nullptr, s);
-  k_leaf_order<<<mb, kT, 0, s>>>(ws.isleaf.as<u8>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(), m, idx);
+  launch(k_leaf_order, mb, kT, 0, s, ws.isleaf.as<u8>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
+         m, idx);
   GTC_LAUNCH_CHECK();
-  k_tree_order<<<nb, kT, 0, s>>>(pos, mass, idx, n32, ws.tpos.as<double>(), ws.tmass.as<double>());
+  launch(k_tree_order, nb, kT, 0, s, pos, mass, idx, n32, ws.tpos.as<double>(),
+         ws.tmass.as<double>());
   GTC_LAUNCH_CHECK();
   ws.stage(Workspace::kStTopo, s);
 
@@ -1742,11 +1773,11 @@ void moments32(Workspace &ws, float4 *cells32, float *delta32, double2 *rootmom,
                          ws.root.as<TreeRoot>(), cells32, delta32};
   const u32 *meta = ws.arrive.as<u32>(), *bucket = ws.bucket.as<u32>();
   ws.up_arrive.ensure(m * sizeof(u32));
-  GTC_CUDA(cudaMemsetAsync(ws.up_arrive.ptr, 0, m * sizeof(u32), s));
-  k_moments32_up<<<ceil_div(m, kT), kT, 0, s>>>(a, bucket, meta, ws.parent.as<u32>(),
-                                                ws.up_arrive.as<u32>());
+  clear({{ws.up_arrive.ptr, m * sizeof(u32)}}, s);
+  launch(k_moments32_up, ceil_div(m, kT), kT, 0, s, a, bucket, meta, ws.parent.as<u32>(),
+         ws.up_arrive.as<u32>());
   GTC_LAUNCH_CHECK();
-  k_root_mass<<<1, 1, 0, s>>>(cells32, rootmom);
+  launch(k_root_mass, 1, 1, 0, s, cells32, rootmom);
   GTC_LAUNCH_CHECK();
 }
 
@@ -1759,7 +1790,7 @@ void build_tree_graph(Workspace &ws, const double *pos, const double *mass, u64 
   const int L = std::max(1, sp.leaf_size);
   Scalars *sc = ws.scalars.as<Scalars>();
   u32 *abort = &sc->abort;
-  GTC_CUDA(cudaMemsetAsync(sc, 0, sizeof(Scalars), s));
+  clear({{sc, sizeof(Scalars)}}, s);
   const ForestView &fv = ws.forest;
   if (fv) forest_roots_and_tables(ws, pos, s);
   else bbox_root(ws, pos, n, s, true);
@@ -1774,26 +1805,26 @@ void build_tree_graph(Workspace &ws, const double *pos, const double *mass, u64 
   signed char *lcp_next = ws.lcp.as<signed char>();
   u8 *leafdepth = ws.leafdepth.as<u8>();
   u32 *count = ws.count.as<u32>(), *cscan = ws.count_scan.as<u32>();
-  k_levels<<<nb, kT, 0, s>>>(kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
+  launch(k_levels, nb, kT, 0, s, kv, idx, tiny, n32, L, lcp_next, leafdepth, count, sc);
   GTC_LAUNCH_CHECK();
   exclusive_scan_u32(count, cscan, n, &sc->n_nodes, ws.scan_tmp, s, &sc->error);
-  k_check_tree_graph<<<1, 1, 0, s>>>(sc, mcap, sorted);
+  launch(k_check_tree_graph, 1, 1, 0, s, sc, mcap, sorted);
   GTC_LAUNCH_CHECK();
   const u32 *m_dev = &sc->n_nodes;
-  k_nodes<<<nb, kT, 0, s>>>(kv, lcp_next, leafdepth, count, cscan, n32, sc, root,
-                            ws.split.as<double>(), ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
-                            ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(),
-                            fv ? fv.split_levels : kSplitLevels, abort);
+  launch(k_nodes, nb, kT, 0, s, kv, lcp_next, leafdepth, count, cscan, n32, sc, root,
+         ws.split.as<double>(), ws.geom.as<double2>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
+         ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(),
+         fv ? fv.split_levels : kSplitLevels, abort);
   GTC_LAUNCH_CHECK();
-  k_children<<<mb, kT, 0, s>>>(ws.skip.as<u32>(), ws.isleaf.as<u8>(), mcap, ws.parent.as<u32>(),
-                               ws.nchild.as<u8>(), ws.kids.as<uint4>(), m_dev, abort);
+  launch(k_children, mb, kT, 0, s, ws.skip.as<u32>(), ws.isleaf.as<u8>(), mcap,
+         ws.parent.as<u32>(), ws.nchild.as<u8>(), ws.kids.as<uint4>(), m_dev, abort);
   GTC_LAUNCH_CHECK();
   if (fv) forest_roots(ws, abort, s);
-  k_leaf_order<<<mb, kT, 0, s>>>(ws.isleaf.as<u8>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(), mcap,
-                                 idx, m_dev, abort);
+  launch(k_leaf_order, mb, kT, 0, s, ws.isleaf.as<u8>(), ws.nbegin.as<u32>(), ws.nend.as<u32>(),
+         mcap, idx, m_dev, abort);
   GTC_LAUNCH_CHECK();
-  k_tree_order<<<nb, kT, 0, s>>>(pos, mass, idx, n32, ws.tpos.as<double>(), ws.tmass.as<double>(),
-                                 abort);
+  launch(k_tree_order, nb, kT, 0, s, pos, mass, idx, n32, ws.tpos.as<double>(),
+         ws.tmass.as<double>(), abort);
   GTC_LAUNCH_CHECK();
   // the moments on the side stream, as in the eager build (the walk waits for
   // the walk records, the caller joins the rest before the evaluation)

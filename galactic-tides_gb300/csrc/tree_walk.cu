@@ -119,6 +119,7 @@ __device__ __noinline__ void terms64(const TreeWalkArgs &a, bool body, u32 j, do
 // kUnitG: G is 1, and a factor of it changes nothing.
 template <bool kQuad, bool kUnitG>
 __global__ void __launch_bounds__(kT, kBlocks) k_tree_walk(TreeWalkArgs a) {
+  grid_wait();
   __shared__ u32 lists[kT / 32][kList][32];
   const int lane = threadIdx.x & 31;
   u32 (*list)[32] = lists[threadIdx.x >> 5];
@@ -309,7 +310,7 @@ void tree_walk_forces(Workspace &ws, const SolverParams &sp, double *acc, double
   const bool unit = sp.G == 1.0;
   const auto kernel = sp.quadrupole ? (unit ? k_tree_walk<true, true> : k_tree_walk<true, false>)
                                     : (unit ? k_tree_walk<false, true> : k_tree_walk<false, false>);
-  kernel<<<ceil_div(ws.n, kT), kT, 0, s>>>(a);
+  launch(kernel, ceil_div(ws.n, kT), kT, 0, s, a);
   GTC_LAUNCH_CHECK();
 }
 
