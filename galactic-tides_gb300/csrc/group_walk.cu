@@ -22,6 +22,7 @@
 // two passes when a list outgrows its slot.
 
 #include <algorithm>
+#include <type_traits>
 
 #include "learned.cuh"
 #include "pipeline.cuh"
@@ -544,7 +545,10 @@ __global__ void __launch_bounds__(kWalkThreads)
 // scattered record loads). kSuper: walk_super_for.
 constexpr int kSlots = 2;
 constexpr int kWarpWalkWarps = 4;
-constexpr u32 kWarpStack = 640;   // ranges per warp
+// Ranges per warp. The less shared memory, the more L1 for the records: 640 ranges
+// 50k bodies 0.148 ms of lists, 2M 1.370, 352 to 192 0.132 and 1.327; at 160 the
+// single-lane walk of a full stack shows (400k 0.376 -> 0.452).
+constexpr u32 kWarpStack = 256;
 constexpr u32 kWarpWalkThreads = kWarpWalkWarps * 32;
 
 struct WarpWalkOut {
@@ -680,19 +684,14 @@ __device__ __forceinline__ void append_runs(const WarpWalk<kSuper> &w, u32 runs,
 }
 
 template <int kMode, int kSuper>
-__global__ void __launch_bounds__(kWarpWalkThreads)
-    k_walk_warp(const WalkRec32 *walk32, const WalkRec64 *walk64, const double *gbox,
-                const float *gboxf, u32 ng_cap, WarpWalkOut out, u32 *next_chunk, Scalars *sc,
-                const u32 *ng_dev, const u32 *abort, const u32 *group_root, GroupSystems gs,
-                bool own_size) {
-  grid_wait();
+__device__ __forceinline__ void walk_groups(WarpWalk<kSuper> &w, const WalkRec32 *walk32,
+                                            const WalkRec64 *walk64, const double *gbox,
+                                            const float *gboxf, u32 ng, const WarpWalkOut &out,
+                                            u32 *next_chunk, Scalars *sc, const u32 *group_root,
+                                            const GroupSystems &gs, bool own_size) {
   constexpr bool kWrite = kMode != kCount;
-  __shared__ WarpWalk<kSuper> walks[kWarpWalkWarps];
-  if (aborted(abort)) return;
-  const u32 ng = bounded(ng_cap, ng_dev);
   const u32 lane = threadIdx.x & 31u;
   const u32 below = (1u << lane) - 1u;
-  WarpWalk<kSuper> &w = walks[threadIdx.x >> 5];
   u32 exact = 0, visits = 0;
   if (kMode == kSlots && lane < kSuper) w.stats[lane] = WalkStats{};
   u32 g = 0, chunk_end = 0;  // groups of the taken chunk still to look at
@@ -968,6 +967,35 @@ __global__ void __launch_bounds__(kWarpWalkThreads)
   }
 }
 
+// kSuper 0: a forest, each system's groups as many at a time as suits its size, the
+// largest first and without a gap between them (16 systems of 10k to 200k bodies:
+// 630 us in three launches, each with its tail, 529 in one).
+template <int kMode, int kSuper>
+__global__ void __launch_bounds__(kWarpWalkThreads, 8)
+    k_walk_warp(const WalkRec32 *walk32, const WalkRec64 *walk64, const double *gbox,
+                const float *gboxf, u32 ng_cap, WarpWalkOut out, u32 *next_chunk, Scalars *sc,
+                const u32 *ng_dev, const u32 *abort, const u32 *group_root, GroupSystems gs) {
+  grid_wait();
+  __shared__ __align__(16) unsigned char
+      raw[kWarpWalkWarps][sizeof(WarpWalk<kSuper ? kSuper : 4>)];
+  if (aborted(abort)) return;
+  const u32 ng = bounded(ng_cap, ng_dev);
+  auto walk = [&](auto super) {
+    constexpr int kOf = decltype(super)::value;
+    walk_groups<kMode, kOf>(*reinterpret_cast<WarpWalk<kOf> *>(raw[threadIdx.x >> 5]), walk32,
+                            walk64, gbox, gboxf, ng, out, next_chunk + (kOf >> 1), sc, group_root,
+                            gs, kSuper == 0);
+    __syncwarp();
+  };
+  if constexpr (kSuper == 0) {
+    walk(std::integral_constant<int, 4>{});
+    walk(std::integral_constant<int, 2>{});
+    walk(std::integral_constant<int, 1>{});
+  } else {
+    walk(std::integral_constant<int, kSuper>{});
+  }
+}
+
 // Places in the overflow pools for the groups one of whose parts outgrew its
 // slot (their whole lists, walked again by one thread); pools too small flag
 // the lists as overflowing.
@@ -1146,14 +1174,14 @@ void launch_warp_walk_of(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scal
   GTC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_walk_warp<kMode, kSuper>,
                                                          kWarpWalkThreads, 0));
   // the one-pass walk's counters are zeroed with the scalars
-  u32 *next = kMode == kSlots ? &sc->walk_next[kSuper >> 1] : nullptr;
+  u32 *next = kMode == kSlots ? sc->walk_next : nullptr;
   if (!next) {
-    ws.walk_next.ensure(sizeof(u32));
+    ws.walk_next.ensure(sizeof(sc->walk_next));
     next = ws.walk_next.as<u32>();
-    GTC_CUDA(cudaMemsetAsync(next, 0, sizeof(u32), s));
+    clear({{next, sizeof(sc->walk_next)}}, s);
   }
   const u32 blocks = static_cast<u32>(std::max<u64>(
-      1, std::min<u64>(ceil_div(ng_cap, kWarpWalkWarps * kSuper),
+      1, std::min<u64>(ceil_div(ng_cap, kWarpWalkWarps * std::max(1, kSuper)),
                        static_cast<u64>(std::max(1, per_sm)) * static_cast<u64>(sms))));
   GroupSystems gs;
   if (ws.forest)
@@ -1161,7 +1189,7 @@ void launch_warp_walk_of(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scal
                       ws.flags_scan.as<u32>(), ws.forest.systems};
   launch(k_walk_warp<kMode, kSuper>, blocks, kWarpWalkThreads, 0, s, ws.walk32.as<WalkRec32>(),
          ws.walk64.as<WalkRec64>(), ws.gbox.as<double>(), ws.gboxf.as<float>(), ng_cap, out,
-         next, sc, ng_dev, abort, ws.forest.group_root, gs, ws.walk_super == 0);
+         next, sc, ng_dev, abort, ws.forest.group_root, gs);
   GTC_LAUNCH_CHECK();
 }
 
@@ -1172,10 +1200,7 @@ void launch_warp_walk(Workspace &ws, const WarpWalkOut &out, u32 ng_cap, Scalars
     case 1: return launch_warp_walk_of<kMode, 1>(ws, out, ng_cap, sc, s, ng_dev, abort);
     case 2: return launch_warp_walk_of<kMode, 2>(ws, out, ng_cap, sc, s, ng_dev, abort);
     case 4: return launch_warp_walk_of<kMode, 4>(ws, out, ng_cap, sc, s, ng_dev, abort);
-    default:  // a forest: each system in the launch of its size
-      launch_warp_walk_of<kMode, 4>(ws, out, ng_cap, sc, s, ng_dev, abort);
-      launch_warp_walk_of<kMode, 2>(ws, out, ng_cap, sc, s, ng_dev, abort);
-      launch_warp_walk_of<kMode, 1>(ws, out, ng_cap, sc, s, ng_dev, abort);
+    default: return launch_warp_walk_of<kMode, 0>(ws, out, ng_cap, sc, s, ng_dev, abort);
   }
 }
 

@@ -182,7 +182,7 @@ struct Workspace {
   // The current lists hold each group's entries in walk-step order rather
   // than the reference's visiting order (exports sort them back).
   bool lists_unordered = false;
-  DeviceBuffer walk_next;     // the warp walk's group counter (count and fill)
+  DeviceBuffer walk_next;     // the warp walk's group counters (count and fill)
   // One-pass walk: group g's lists start at g * slot_cells and g *
   // slot_bodies (capacities sized from the previous walk's longest lists);
   // 0 until a walk has measured them. `gapped`: the current lists use that
@@ -240,7 +240,7 @@ struct Scalars {
   unsigned long long spill_used[2];  // one-pass walk: overflow pool entries taken (cells, bodies)
   u32 spilled;            // one-pass walk: groups that outgrew their slots
   unsigned long long walk_nodes;  // node records the walk tested
-  u32 walk_next[3];       // the warp walk's group counters (one-pass walk: its launches)
+  u32 walk_next[3];       // the warp walk's group counters (a forest: by groups per warp)
   u32 eval_next;          // the evaluation's group counter
 };
 
