@@ -129,66 +129,89 @@ __device__ void build_split(const double *centre, const double *half_at, int lev
   }
 }
 
-// Root cube from the partial boxes (octree.cpp:184-198; min/max are exact in any
-// order), by one block, and its split table (null: none wanted).
-__device__ void root_from_parts(const double *part, int nparts, TreeRoot *root, int levels,
+// A block's partial box, from its warps', as order keys: lows, then highs. Not
+// a number counts as nothing, as in fmin and fmax.
+__device__ __forceinline__ u64 box_key(const u64 (*warps)[6], int a) {
+  u64 v = warps[0][a];
+  for (int w = 1; w < kT / 32; ++w) {
+    const u64 x = warps[w][a];
+    v = a < 3 ? (x < v ? x : v) : (x > v ? x : v);
+  }
+  const u64 least = order_key(-INFINITY), most = order_key(INFINITY);
+  if (v < least || v > most) v = a < 3 ? most : least;
+  return v;
+}
+__device__ __forceinline__ void box_of_warp(u64 (&lo)[3], u64 (&hi)[3]) {
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    for (int o = 16; o > 0; o >>= 1) {
+      const u64 l = __shfl_xor_sync(kFullMask, lo[a], o), h = __shfl_xor_sync(kFullMask, hi[a], o);
+      lo[a] = l < lo[a] ? l : lo[a];
+      hi[a] = h > hi[a] ? h : hi[a];
+    }
+}
+
+// Root cube from the partial boxes (octree.cpp:184-198; min and max are exact in
+// any order), by one block, and its split table (null: none wanted). A chain of
+// FP64 latencies (64 cycles an operation, some 600 a division): lanes 0 to 2 take
+// an axis each, lanes 0 and 1 a division.
+__device__ void root_from_parts(const u64 *part, int nparts, TreeRoot *root, int levels,
                                 double *split) {
-  __shared__ double s[kT / 32][6];
+  __shared__ u64 s[kT / 32][6];
   __shared__ double half_at[kMaxDepth + 1], centre[3], half_s;
   __shared__ long long tiny_bound;
   __shared__ int not_tiny[2];
-  double v[6];
+  u64 klo[3], khi[3];
   for (int a = 0; a < 3; ++a) {
-    v[a] = INFINITY;
-    v[3 + a] = -INFINITY;
+    klo[a] = order_key(INFINITY);
+    khi[a] = order_key(-INFINITY);
   }
   for (int p = threadIdx.x; p < nparts; p += kT)
     for (int a = 0; a < 3; ++a) {
-      v[a] = fmin(v[a], __ldcg(part + 6 * p + a));
-      v[3 + a] = fmax(v[3 + a], __ldcg(part + 6 * p + 3 + a));
+      const u64 l = __ldcg(part + 6 * p + a), h = __ldcg(part + 6 * p + 3 + a);
+      klo[a] = l < klo[a] ? l : klo[a];
+      khi[a] = h > khi[a] ? h : khi[a];
     }
-  for (int a = 0; a < 3; ++a)
-    for (int o = 16; o > 0; o >>= 1) {
-      v[a] = fmin(v[a], __shfl_xor_sync(kFullMask, v[a], o));
-      v[3 + a] = fmax(v[3 + a], __shfl_xor_sync(kFullMask, v[3 + a], o));
-    }
+  box_of_warp(klo, khi);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0)
-    for (int a = 0; a < 6; ++a) s[warp][a] = v[a];
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double lo[3], hi[3];
     for (int a = 0; a < 3; ++a) {
-      lo[a] = s[0][a];
-      hi[a] = s[0][3 + a];
-      for (int w = 1; w < kT / 32; ++w) {
-        lo[a] = fmin(lo[a], s[w][a]);
-        hi[a] = fmax(hi[a], s[w][3 + a]);
-      }
+      s[warp][a] = klo[a];
+      s[warp][3 + a] = khi[a];
     }
-    double half = 0.0, reach = 0.0;
+  __syncthreads();
+  if (warp == 0) {
+    const int axis = lane < 3 ? lane : 0;
+    const double lo = from_order_key(box_key(s, axis)), hi = from_order_key(box_key(s, 3 + axis));
+    const double c = (lo + hi) * 0.5, e = 0.5 * (hi - lo), far = fmax(fabs(lo), fabs(hi));
+    if (lane < 3) {
+      root->lo[lane] = lo;
+      root->hi[lane] = hi;
+      root->center[lane] = c;
+      centre[lane] = c;
+    }
+    double half = 0.0, reach = 0.0, m1 = 0.0;
     for (int a = 0; a < 3; ++a) {
-      root->lo[a] = lo[a];
-      root->hi[a] = hi[a];
-      centre[a] = (lo[a] + hi[a]) * 0.5;
-      root->center[a] = centre[a];
-      const double e = 0.5 * (hi[a] - lo[a]);
-      half = half < e ? e : half;
-      reach = fmax(reach, fabs(centre[a]));
+      const double ea = __shfl_sync(kFullMask, e, a);
+      half = half < ea ? ea : half;
+      reach = fmax(reach, fabs(__shfl_sync(kFullMask, c, a)));
+      m1 = m1 + __shfl_sync(kFullMask, far, a);
     }
     half = half * (1.0 + 1e-9) + 1e-300;
-    half_s = half;
     // the grid of the keys (grid_rank): its band covers the roundings of the
     // reference's centres, at most 20 of 2^-53 (|centre| + half) each, and of
     // the rank itself, in units of 2^-31 cells: 5 (|centre| + half) / half + 1
-    root->grid = static_cast<double>(1 << (kLevelsPerWord - 1)) / half;
-    const double band = 8.0 * ((reach + half) / half) + 8.0;
-    root->grid_band = band < 1e9 && half > 1e-280 ? static_cast<u32>(band) : ~0u;
-    // every body's |x| + |y| + |z| is at most this sum (rounding is monotone),
-    // so no body's tiny bound in k_keys exceeds this one
-    double m1 = 0.0;
-    for (int a = 0; a < 3; ++a) m1 = m1 + fmax(fabs(lo[a]), fabs(hi[a]));
-    tiny_bound = __double_as_longlong(2e-12 * (m1 + 1e-300));
+    const double q =
+        (lane == 0 ? static_cast<double>(1 << (kLevelsPerWord - 1)) : reach + half) / half;
+    const double band = 8.0 * __shfl_sync(kFullMask, q, 1) + 8.0;
+    if (lane == 0) {
+      half_s = half;
+      root->grid = q;
+      root->grid_band = band < 1e9 && half > 1e-280 ? static_cast<u32>(band) : ~0u;
+      // every body's |x| + |y| + |z| is at most m1 (rounding is monotone), so
+      // no body's tiny bound in k_keys exceeds this one
+      tiny_bound = __double_as_longlong(2e-12 * (m1 + 1e-300));
+    }
   }
   __syncthreads();
   if (threadIdx.x < 64) {  // (half falls with depth: the levels above the bound come first)
@@ -218,7 +241,7 @@ __device__ void root_from_parts(const double *part, int nparts, TreeRoot *root, 
 // thread loads two bodies as three 16-byte words. `ticket` counts finished
 // blocks and wraps to zero by itself.
 __global__ void __launch_bounds__(kT)
-    k_bbox(const double *pos, u64 n, double *part, u32 *ticket, TreeRoot *root, double *split) {
+    k_bbox(const double *pos, u64 n, u64 *part, u32 *ticket, TreeRoot *root, double *split) {
   grid_wait();
   const u64 inf_lo = order_key(INFINITY), inf_hi = order_key(-INFINITY);
   u64 lo[3] = {inf_lo, inf_lo, inf_lo}, hi[3] = {inf_hi, inf_hi, inf_hi};
@@ -246,13 +269,7 @@ __global__ void __launch_bounds__(kT)
     for (u64 i = first; i < n; i += stride)
       for (int a = 0; a < 3; ++a) take(a, pos[3 * i + a]);
   }
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-    for (int o = 16; o > 0; o >>= 1) {
-      const u64 l = __shfl_xor_sync(kFullMask, lo[a], o), h = __shfl_xor_sync(kFullMask, hi[a], o);
-      lo[a] = l < lo[a] ? l : lo[a];
-      hi[a] = h > hi[a] ? h : hi[a];
-    }
+  box_of_warp(lo, hi);
   __shared__ u64 s[kT / 32][6];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0)
@@ -262,12 +279,7 @@ __global__ void __launch_bounds__(kT)
     }
   __syncthreads();
   if (threadIdx.x < 6) {
-    u64 v = s[0][threadIdx.x];
-    for (int w = 1; w < kT / 32; ++w) {
-      const u64 x = s[w][threadIdx.x];
-      v = threadIdx.x < 3 ? (x < v ? x : v) : (x > v ? x : v);
-    }
-    part[6 * blockIdx.x + threadIdx.x] = from_order_key(v);
+    part[6 * blockIdx.x + threadIdx.x] = box_key(s, static_cast<int>(threadIdx.x));
     __threadfence();
   }
   __shared__ bool last;
@@ -284,7 +296,7 @@ __global__ void __launch_bounds__(kT)
 // reduces that system's partials (sys_blk: first block, blocks) into its
 // root.
 __global__ void __launch_bounds__(kT)
-    k_bbox_forest(const double *pos, const uint4 *blk, const u32 *start, double *part) {
+    k_bbox_forest(const double *pos, const uint4 *blk, const u32 *start, u64 *part) {
   grid_wait();
   const uint4 q = blk[blockIdx.x];
   const u64 b0 = start[q.x], b1 = start[q.x + 1];
@@ -297,13 +309,7 @@ __global__ void __launch_bounds__(kT)
       lo[a] = k < lo[a] ? k : lo[a];
       hi[a] = k > hi[a] ? k : hi[a];
     }
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-    for (int o = 16; o > 0; o >>= 1) {
-      const u64 l = __shfl_xor_sync(kFullMask, lo[a], o), h = __shfl_xor_sync(kFullMask, hi[a], o);
-      lo[a] = l < lo[a] ? l : lo[a];
-      hi[a] = h > hi[a] ? h : hi[a];
-    }
+  box_of_warp(lo, hi);
   __shared__ u64 s[kT / 32][6];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (lane == 0)
@@ -313,17 +319,12 @@ __global__ void __launch_bounds__(kT)
     }
   __syncthreads();
   if (threadIdx.x < 6) {
-    u64 v = s[0][threadIdx.x];
-    for (int w = 1; w < kT / 32; ++w) {
-      const u64 x = s[w][threadIdx.x];
-      v = threadIdx.x < 3 ? (x < v ? x : v) : (x > v ? x : v);
-    }
-    part[6 * blockIdx.x + threadIdx.x] = from_order_key(v);
+    part[6 * blockIdx.x + threadIdx.x] = box_key(s, static_cast<int>(threadIdx.x));
   }
 }
 
 __global__ void __launch_bounds__(kT)
-    k_root_forest(const double *part, const uint2 *sys_blk, TreeRoot *roots, int levels,
+    k_root_forest(const u64 *part, const uint2 *sys_blk, TreeRoot *roots, int levels,
                   double *split) {
   grid_wait();
   const uint2 q = sys_blk[blockIdx.x];
@@ -1352,14 +1353,14 @@ void read_scalars(Workspace &ws, Scalars *host, cudaStream_t s) {
 
 void bbox_root(Workspace &ws, const double *pos, u64 n, cudaStream_t s, bool split) {
   const u32 nparts = std::min<u32>(1024, std::max<u32>(1, ceil_div(n, kT)));
-  ws.bbox_part.ensure(6 * sizeof(double) * nparts);
+  ws.bbox_part.ensure(6 * sizeof(u64) * nparts);
   ws.root.ensure(sizeof(TreeRoot));
   if (!ws.bbox_ticket.ptr) {
     ws.bbox_ticket.ensure(sizeof(u32));
     GTC_CUDA(cudaMemsetAsync(ws.bbox_ticket.ptr, 0, sizeof(u32), s));
   }
   if (split) ws.split.ensure(3ull * kSplitSize * sizeof(double));
-  launch(k_bbox, nparts, kT, 0, s, pos, n, ws.bbox_part.as<double>(), ws.bbox_ticket.as<u32>(),
+  launch(k_bbox, nparts, kT, 0, s, pos, n, ws.bbox_part.as<u64>(), ws.bbox_ticket.as<u32>(),
          ws.root.as<TreeRoot>(), split ? ws.split.as<double>() : nullptr);
   GTC_LAUNCH_CHECK();
 }
@@ -1462,12 +1463,12 @@ int sort_top_levels(Workspace &ws, u32 n, int levels, cudaStream_t s,
 // A forest's root cubes and split tables (one per system).
 void forest_roots_and_tables(Workspace &ws, const double *pos, cudaStream_t s) {
   const ForestView &fv = ws.forest;
-  ws.bbox_part.ensure(6 * sizeof(double) * fv.bbox_nblocks);
+  ws.bbox_part.ensure(6 * sizeof(u64) * fv.bbox_nblocks);
   ws.split.ensure((3ull * fv.systems << fv.split_levels) * sizeof(double));
   launch(k_bbox_forest, fv.bbox_nblocks, kT, 0, s, pos, fv.bbox_blocks, fv.start,
-         ws.bbox_part.as<double>());
+         ws.bbox_part.as<u64>());
   GTC_LAUNCH_CHECK();
-  launch(k_root_forest, fv.systems, kT, 0, s, ws.bbox_part.as<double>(), fv.sys_blocks, fv.roots,
+  launch(k_root_forest, fv.systems, kT, 0, s, ws.bbox_part.as<u64>(), fv.sys_blocks, fv.roots,
          fv.split_levels, ws.split.as<double>());
   GTC_LAUNCH_CHECK();
 }
