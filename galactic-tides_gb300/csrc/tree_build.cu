@@ -944,15 +944,27 @@ __device__ __forceinline__ float3 centre32(const Moment32Arrays &a, u32 p) {
                      static_cast<float>(g.z - a.root->center[2]));
 }
 
+// Bodies k0.. of [k0, k1), at most eight, loaded together.
+__device__ __forceinline__ void bodies32(const Moment32Arrays &a, u32 k0, u32 k1, float4 (&b)[8]) {
+#pragma unroll
+  for (u32 j = 0; j < 8; ++j)
+    if (k0 + j < k1) b[j] = a.bodies[k0 + j];
+}
+
 __device__ void leaf_moments32(const Moment32Arrays &a, u32 p) {
   const u32 b0 = a.nbegin[p], b1 = a.nend[p];
   float m = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-  for (u32 k = b0; k < b1; ++k) {
-    const float4 b = a.bodies[k];
-    m += b.w;
-    cx += b.w * b.x;
-    cy += b.w * b.y;
-    cz += b.w * b.z;
+  float4 b[8];
+  for (u32 k = b0; k < b1; k += 8) {
+    bodies32(a, k, b1, b);
+#pragma unroll
+    for (u32 j = 0; j < 8; ++j) {
+      if (k + j >= b1) break;
+      m += b[j].w;
+      cx += b[j].w * b[j].x;
+      cy += b[j].w * b[j].y;
+      cz += b[j].w * b[j].z;
+    }
   }
   if (m > 0) {
     cx /= m;
@@ -965,40 +977,49 @@ __device__ void leaf_moments32(const Moment32Arrays &a, u32 p) {
     cz = c.z;
   }
   float q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (u32 k = b0; k < b1; ++k) {
-    const float4 b = a.bodies[k];
-    const float dx = b.x - cx, dy = b.y - cy, dz = b.z - cz;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    q[0] += b.w * (3.f * dx * dx - r2);
-    q[1] += b.w * (3.f * dy * dy - r2);
-    q[2] += b.w * (3.f * dz * dz - r2);
-    q[3] += b.w * 3.f * dx * dy;
-    q[4] += b.w * 3.f * dx * dz;
-    q[5] += b.w * 3.f * dy * dz;
+  for (u32 k = b0; k < b1; k += 8) {
+    if (b1 - b0 > 8) bodies32(a, k, b1, b);
+#pragma unroll
+    for (u32 j = 0; j < 8; ++j) {
+      if (k + j >= b1) break;
+      const float w = b[j].w, dx = b[j].x - cx, dy = b[j].y - cy, dz = b[j].z - cz;
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      q[0] += w * (3.f * dx * dx - r2);
+      q[1] += w * (3.f * dy * dy - r2);
+      q[2] += w * (3.f * dz * dz - r2);
+      q[3] += w * 3.f * dx * dy;
+      q[4] += w * 3.f * dx * dz;
+      q[5] += w * 3.f * dy * dz;
+    }
   }
   finish_moments32(a, p, m, cx, cy, cz, q);
 }
 
-// Children's cells written by other threads of the same launch are read
-// from L2 (kL2): an SM's L1 may hold an older copy of the line.
-template <bool kL2>
-__device__ __forceinline__ float4 cell32(const float4 *p) {
-  return kL2 ? __ldcg(p) : *p;
-}
-
-template <bool kL2 = false>
+// The children's cells, written by other threads of the same launch, are read
+// from L2 (an SM's L1 may hold an older copy of the line), all loads first.
 __device__ void node_moments32(const Moment32Arrays &a, u32 p) {
   const uint4 k0 = a.kids[2ull * p], k1 = a.kids[2ull * p + 1];
   const u32 ch[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w};
   const int nc = a.nchild[p];
+  float4 c[8], qa[8];
+  float2 qb[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j)
+    if (j < nc) {
+      const float4 *cell = &a.cells[3 * ch[j]];
+      c[j] = __ldcg(cell);
+      qa[j] = __ldcg(cell + 1);
+      qb[j] = __ldcg(reinterpret_cast<const float2 *>(cell + 2));
+    }
   float m = 0.f, cx = 0.f, cy = 0.f, cz = 0.f;
-  for (int j = nc - 1; j >= 0; --j) {
-    const float4 c = cell32<kL2>(&a.cells[3 * ch[j]]);
-    m += c.w;
-    cx += c.w * c.x;
-    cy += c.w * c.y;
-    cz += c.w * c.z;
-  }
+#pragma unroll
+  for (int j = 7; j >= 0; --j)
+    if (j < nc) {
+      m += c[j].w;
+      cx += c[j].w * c[j].x;
+      cy += c[j].w * c[j].y;
+      cz += c[j].w * c[j].z;
+    }
   if (m > 0) {
     cx /= m;
     cy /= m;
@@ -1010,18 +1031,18 @@ __device__ void node_moments32(const Moment32Arrays &a, u32 p) {
     cz = c.z;
   }
   float q[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-  for (int j = nc - 1; j >= 0; --j) {
-    const float4 c = cell32<kL2>(&a.cells[3 * ch[j]]), qa = cell32<kL2>(&a.cells[3 * ch[j] + 1]),
-                 qb = cell32<kL2>(&a.cells[3 * ch[j] + 2]);
-    const float dx = c.x - cx, dy = c.y - cy, dz = c.z - cz;
-    const float r2 = dx * dx + dy * dy + dz * dz;
-    q[0] += qa.x + c.w * (3.f * dx * dx - r2);
-    q[1] += qa.y + c.w * (3.f * dy * dy - r2);
-    q[2] += qa.z + c.w * (3.f * dz * dz - r2);
-    q[3] += qa.w + c.w * 3.f * dx * dy;
-    q[4] += qb.x + c.w * 3.f * dx * dz;
-    q[5] += qb.y + c.w * 3.f * dy * dz;
-  }
+#pragma unroll
+  for (int j = 7; j >= 0; --j)
+    if (j < nc) {
+      const float w = c[j].w, dx = c[j].x - cx, dy = c[j].y - cy, dz = c[j].z - cz;
+      const float r2 = dx * dx + dy * dy + dz * dz;
+      q[0] += qa[j].x + w * (3.f * dx * dx - r2);
+      q[1] += qa[j].y + w * (3.f * dy * dy - r2);
+      q[2] += qa[j].z + w * (3.f * dz * dz - r2);
+      q[3] += qa[j].w + w * 3.f * dx * dy;
+      q[4] += qb[j].x + w * 3.f * dx * dz;
+      q[5] += qb[j].y + w * 3.f * dy * dz;
+    }
   finish_moments32(a, p, m, cx, cy, cz, q);
 }
 
@@ -1221,10 +1242,8 @@ __global__ void __launch_bounds__(kT)
   for (int step = 0; step <= kMaxDepth; ++step) {
     const u32 q = parent[p];
     if (q == 0xffffffffu) return;
-    __threadfence();  // this node's values before its parent's count
-    if (atomicAdd(&arrive[q], 1u) + 1u != a.nchild[q]) return;
-    __threadfence();  // the siblings' values, counted before this, are visible
-    node_moments32<true>(a, q);
+    if (count_arrival(&arrive[q]) + 1u != a.nchild[q]) return;
+    node_moments32(a, q);
     p = q;
   }
 }
