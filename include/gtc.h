@@ -366,11 +366,11 @@ gtc_status gtc_autotune_direct(gtc_context *ctx, const double *pos, const double
                                double *best_ms);
 /* The list evaluation's tile shape (softened quadrupole evaluation): times
  * the evaluation kernel of gtc_group_force_device on these bodies (device
- * arrays, parameters gp) with 1 and 2 staged pairs per inner iteration and
+ * arrays, parameters gp) with 1 and 2 staged entries per inner iteration and
  * pass costs 8, 16, 24, 32 and 48 (how many slices a group's lists are cut
  * into), keeps the fastest in the context (options "eval_pairs" and
  * "eval_pass_cost") and returns it in *pairs and *pass_cost, its kernel time
- * in *best_ms. The staged pairs do not change the forces; the pass cost
+ * in *best_ms. The entry count does not change the forces; the pass cost
  * changes their summation order only. */
 gtc_status gtc_autotune_eval(gtc_context *ctx, const double *pos, const double *mass,
                              uint64_t n, const gtc_gravity_params *gp, int *pairs,
