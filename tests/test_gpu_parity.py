@@ -313,7 +313,7 @@ def test_keys_of_extreme_lengths(ctx, oracle, scale):
 @pytest.mark.parametrize("n", [2, 33, 1024, 1025, 4097, 16384, 16385, 32769, 65537, 131072,
                                131073, 150001])
 def test_tree_order_over_sort_sizes(ctx, oracle, n):
-    """The sort by one cluster (up to 131072 pairs, one to eight a thread) and by
+    """The sort by one cluster (up to 65536 pairs, one to four a thread) and by
     tiles (beyond): the oracle's order, equal keys in input order."""
     pos, mass = lopsided_sphere(n, 23)
     pos[n // 3:n // 3 + n // 50] = pos[n // 2]          # many equal keys
@@ -321,3 +321,21 @@ def test_tree_order_over_sort_sizes(ctx, oracle, n):
     order = ctx.export()["order"]
     nodes, want, _ = oracle.lists(pos, mass, theta=1.0)
     assert np.array_equal(order, want)
+
+
+@pytest.mark.parametrize("clump", [17, 31, 32, 33, 34, 64])
+@pytest.mark.parametrize("background", [0, 70_000])
+def test_first_bodies_of_long_chains(ctx, oracle, clump, background):
+    """Tight clumps end chains of some 36 nodes of about 16 to 64 bodies at one body
+    each: searches that stay near, that go to a block's warps, and (clumps of 33
+    and more: over 256 of them a block) past the room for those."""
+    rng = np.random.default_rng(5)
+    corner = np.array([[(o & 1) - 0.5, (o >> 1 & 1) - 0.5, (o >> 2) - 0.5] for o in range(8)])
+    pos = np.concatenate([1.3 * c + rng.uniform(-1, 1, (clump, 3)) * 2e-12 for c in corner]
+                         + [rng.uniform(-1, 1, (background + 2, 3))])
+    mass = rng.uniform(0.5, 1.5, len(pos))
+    ctx.group_force(pos, mass, theta=0.8, eps=0.05)
+    dev = ctx.export()
+    nodes, order, _ = oracle.lists(pos, mass, theta=0.8)
+    assert np.array_equal(dev["order"], order)
+    assert compare_trees(dev["nodes"], nodes) == []
