@@ -539,10 +539,14 @@ __global__ void __launch_bounds__(kWalkThreads)
 // others into their slots again; then the warp writes the groups' records and
 // keeps the statistics.
 //
-// Bound: instruction issue (75% of the issue slots busy at 1M bodies, four
-// groups to a warp; 190 instructions per 32 tests, the test itself 33). 2M
-// bodies 0.96 ms against 1.63 ms by threads (bound by their chains of
-// scattered record loads). kSuper: walk_super_for.
+// While the stack is short, an opened node's children get a range each: as one
+// range they come one a step, and a step had 11 of its 32 lanes at work (lists of
+// 50k bodies 0.130 -> 0.118 ms, 400k 0.374 -> 0.318, 2M 1.33 -> 1.24; from 48 or 64
+// ranges on instead of 32, slower).
+//
+// Bound: instruction issue at 2M (the test is 33 of 190 instructions per 32
+// tests), the longest walks at 200k. 2M bodies 0.70 ms against 1.63 ms by threads
+// (bound by their chains of scattered record loads). kSuper: walk_super_for.
 constexpr int kSlots = 2;
 constexpr int kWarpWalkWarps = 4;
 // Ranges per warp. The less shared memory, the more L1 for the records: 640 ranges
@@ -551,7 +555,10 @@ constexpr int kWarpWalkWarps = 4;
 constexpr u32 kWarpStack = 256;
 constexpr u32 kWarpWalkThreads = kWarpWalkWarps * 32;
 
+constexpr u32 kFewOpened = 16;    // opened nodes whose children get a range each, at most
+
 struct WarpWalkOut {
+  const uint4 *kids;              // the tree's children
   u32 *cell_list, *body_list;
   u64 *ncells, *nbodies;          // kCount
   const u64 *cell_off, *body_off; // kFill
@@ -683,6 +690,36 @@ __device__ __forceinline__ void append_runs(const WarpWalk<kSuper> &w, u32 runs,
   }
 }
 
+// A node's children (kids lists them in index order, zeros behind them).
+__device__ __forceinline__ u32 children_of(const uint4 *kids, u32 p, u32 (&ch)[8]) {
+  const uint4 k0 = __ldg(kids + 2ull * p), k1 = __ldg(kids + 2ull * p + 1);
+  ch[0] = k0.x;
+  ch[1] = k0.y;
+  ch[2] = k0.z;
+  ch[3] = k0.w;
+  ch[4] = k1.x;
+  ch[5] = k1.y;
+  ch[6] = k1.z;
+  ch[7] = k1.w;
+  u32 n = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) n += ch[j] ? 1u : 0u;
+  return n;
+}
+
+// A range for each child, from place `at` of the stack.
+template <int kSuper>
+__device__ __forceinline__ void push_children(WarpWalk<kSuper> &w, u32 at, const u32 (&ch)[8],
+                                              u32 end, u32 mask) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (!ch[j]) break;
+    const u32 next = j < 7 ? ch[j < 7 ? j + 1 : 7] : 0u;
+    w.stk[at + j] = make_uint2(ch[j], next ? next : end);
+    w.mask[at + j] = static_cast<u8>(mask);
+  }
+}
+
 template <int kMode, int kSuper>
 __device__ __forceinline__ void walk_groups(WarpWalk<kSuper> &w, const WalkRec32 *walk32,
                                             const WalkRec64 *walk64, const double *gbox,
@@ -744,11 +781,15 @@ __device__ __forceinline__ void walk_groups(WarpWalk<kSuper> &w, const WalkRec32
   again:
 #pragma unroll
     for (int k = 0; k < kSuper; ++k) nc[k] = nb[k] = 0u;
-    if (lane == 0) {
-      w.stk[0] = make_uint2((rr.nbody_leaf >> 31) != 0 ? root : root + 1, rr.skip);
+    u32 top = 1, queued = 0;
+    if ((rr.nbody_leaf >> 31) == 0) {
+      u32 ch[8];
+      top = children_of(out.kids, root, ch);
+      if (lane == 0) push_children(w, 0, ch, rr.skip, (1u << count) - 1u);
+    } else if (lane == 0) {
+      w.stk[0] = make_uint2(root, rr.skip);
       w.mask[0] = static_cast<u8>((1u << count) - 1u);
     }
-    u32 top = 1, queued = 0;
     __syncwarp();
     while (top > 0) {
       if (top > kWarpStack - 2 * 32) {
@@ -861,20 +902,41 @@ __device__ __forceinline__ void walk_groups(WarpWalk<kSuper> &w, const WalkRec32
         w.q_mask[at] = static_cast<u8>(runs);
       }
       queued += __popc(with_runs);
-      // pushes: each lane its rest, then its children's range (on top)
+      // pushes: each lane its rest, then its children's range (on top); where
+      // that leaves lanes idle, a range for each child
       const u32 rests = __ballot_sync(kFullMask, rest),
                 kids = __ballot_sync(kFullMask, opened != 0u);
-      u32 at = top + __popc(rests & below) + __popc(kids & below);
-      if (rest) {
-        w.stk[at] = make_uint2(r.skip, e.y);
-        w.mask[at] = static_cast<u8>(m);
-        ++at;
+      const u32 opens = __popc(kids);
+      u32 at = top + __popc(rests & below);
+      top += __popc(rests);
+      if (top + opens < 32u && opens <= kFewOpened) {
+        u32 ch[8] = {};
+        const u32 mine = opened ? children_of(out.kids, e.x, ch) : 0u;
+#pragma unroll
+        for (int bit = 0; bit < 4; ++bit) {  // the lanes' counts, at most 8
+          const u32 with = __ballot_sync(kFullMask, (mine >> bit) & 1u);
+          at += __popc(with & below) << bit;
+          top += __popc(with) << bit;
+        }
+        if (rest) {
+          w.stk[at] = make_uint2(r.skip, e.y);
+          w.mask[at] = static_cast<u8>(m);
+          ++at;
+        }
+        if (opened) push_children(w, at, ch, r.skip, opened);
+      } else {
+        at += __popc(kids & below);
+        top += opens;
+        if (rest) {
+          w.stk[at] = make_uint2(r.skip, e.y);
+          w.mask[at] = static_cast<u8>(m);
+          ++at;
+        }
+        if (opened) {
+          w.stk[at] = make_uint2(e.x + 1u, r.skip);
+          w.mask[at] = static_cast<u8>(opened);
+        }
       }
-      if (opened) {
-        w.stk[at] = make_uint2(e.x + 1u, r.skip);
-        w.mask[at] = static_cast<u8>(opened);
-      }
-      top += __popc(rests) + __popc(kids);
       __syncwarp();
       if (queued >= 32u) {
         append_runs<kWrite>(w, 32u, nb, out.body_list);
@@ -1336,6 +1398,7 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
     ws.body_list.ensure(ext_b * 4);
     if (ws.walk_warps) {
       WarpWalkOut wwo{};
+      wwo.kids = ws.kids.as<uint4>();
       wwo.cell_list = ws.cell_list.as<u32>();
       wwo.body_list = ws.body_list.as<u32>();
       wwo.slot_cells = sl_c;
@@ -1406,6 +1469,7 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
              nullptr, nullptr};
   const bool warps = ws.walk_warps && ntasks == 1;
   WarpWalkOut wwo{};
+  wwo.kids = ws.kids.as<uint4>();
   wwo.ncells = ws.gcells.as<u64>();
   wwo.nbodies = ws.gbodies.as<u64>();
   wwo.cell_off = cell_off;
@@ -1493,6 +1557,7 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
               caps.slot_cells, caps.slot_bodies, caps.slot_near_cells,
               caps.slot_near_bodies, n32};
   WarpWalkOut wwo{};
+  wwo.kids = ws.kids.as<uint4>();
   wwo.cell_list = ws.cell_list.as<u32>();
   wwo.body_list = ws.body_list.as<u32>();
   wwo.slot_cells = caps.slot_cells;

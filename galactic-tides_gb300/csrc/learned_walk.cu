@@ -619,14 +619,45 @@ __global__ void __launch_bounds__(kContWarps * 32) k_lcont(GArgs a, bool later) 
 // first node of the 32 ranges on top; entries reach the lists in step order,
 // lane order within a step (fixed for given inputs), and the pairs deferred
 // now go to the group's pend slot for the next round. Leaf and small cells'
-// body runs are queued and listed 32 at a time, and a step's pushes are placed
-// by two ballots (a scan over the lanes for each, every step, before).
+// body runs are queued and listed 32 at a time, a step's pushes are placed by
+// ballots (a scan over the lanes for each, every step, before), and while the
+// stack is short an opened node's children get a range each: as one range they
+// come one a step (learned solve of 200k bodies 0.74 -> 0.68 ms, 2M 3.67 -> 3.37; by
+// threads 1.13 and 3.57).
 //
 // Bound: the longest walks (200k: the SMs are busy 54% of the time to the last
 // one's end), then issue. Round 0 of 200k bodies 233 -> 197 us; 12 to 16 blocks an
 // SM, or stacks of 512 or 1024 ranges, measure the same.
 constexpr int kLWarps = 4;
 constexpr int kLStack = 256;  // ranges per warp
+
+constexpr int kLFewOpened = 16;  // opened nodes whose children get a range each, at most
+
+// A node's children (kids lists them in index order, zeros behind them), and a
+// range for each from place `at` of the stack.
+__device__ __forceinline__ u32 children_of(const uint4 *kids, u32 p, u32 (&ch)[8]) {
+  const uint4 k0 = __ldg(kids + 2ull * p), k1 = __ldg(kids + 2ull * p + 1);
+  ch[0] = k0.x;
+  ch[1] = k0.y;
+  ch[2] = k0.z;
+  ch[3] = k0.w;
+  ch[4] = k1.x;
+  ch[5] = k1.y;
+  ch[6] = k1.z;
+  ch[7] = k1.w;
+  u32 n = 0;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) n += ch[j] ? 1u : 0u;
+  return n;
+}
+__device__ __forceinline__ void push_children(uint2 *stk, u32 at, const u32 (&ch)[8], u32 end) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    if (!ch[j]) break;
+    const u32 next = j < 7 ? ch[j < 7 ? j + 1 : 7] : 0u;
+    stk[at + j] = make_uint2(ch[j], next ? next : end);
+  }
+}
 
 struct LWarpWalk {
   uint2 stk[kLStack];
@@ -676,8 +707,13 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
     u32 kp = round ? a.roff[g] : 0u, k1 = round ? a.roff[g + 1] : 0u;
     int size = 0;
     if (round == 0) {
-      if (lane == 0) stk[0] = root_leaf ? make_uint2(0u, root_end) : make_uint2(1u, root_end);
+      u32 ch[8] = {};
       size = 1;
+      if (!root_leaf) size = static_cast<int>(children_of(a.kids, 0, ch));
+      if (lane == 0) {
+        if (root_leaf) stk[0] = make_uint2(0u, root_end);
+        else push_children(stk, 0, ch, root_end);
+      }
     }
     __syncwarp();
     while ((size > 0 || kp < k1) && !bad) {
@@ -776,10 +812,27 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
       }
       const unsigned rests = __ballot_sync(kFullMask, has_rest),
                      kids = __ballot_sync(kFullMask, has_kids);
-      u32 at = static_cast<u32>(size) + __popc(rests & above) + __popc(kids & above);
-      if (has_rest) stk[at++] = make_uint2(skip, rend);
-      if (has_kids) stk[at] = make_uint2(r.x + 1, kids_end);
-      size += __popc(rests) + __popc(kids);
+      const int opens = __popc(kids);
+      u32 at = static_cast<u32>(size) + __popc(rests & above);
+      size += __popc(rests);
+      if (size + opens < 32 && opens <= kLFewOpened) {
+        // lanes would be idle: a range for each child
+        u32 ch[8] = {};
+        const u32 mine = has_kids ? children_of(a.kids, r.x, ch) : 0u;
+#pragma unroll
+        for (int bit = 0; bit < 4; ++bit) {  // the lanes' counts, at most 8
+          const u32 with = __ballot_sync(kFullMask, (mine >> bit) & 1u);
+          at += __popc(with & above) << bit;
+          size += __popc(with) << bit;
+        }
+        if (has_rest) stk[at++] = make_uint2(skip, rend);
+        if (has_kids) push_children(stk, at, ch, kids_end);
+      } else {
+        at += __popc(kids & above);
+        size += opens;
+        if (has_rest) stk[at++] = make_uint2(skip, rend);
+        if (has_kids) stk[at] = make_uint2(r.x + 1, kids_end);
+      }
       bad = __any_sync(kFullMask, bad);
       __syncwarp();
       if (queued >= 32u) {
@@ -1055,7 +1108,7 @@ void learned_build_lists(Workspace &ws, const LearnedWalk &lw, u32 ng, Scalars *
     throw RuntimeError("learned walk: too many tree nodes for 32 bit node ranges");
   Scalars *sc = ws.scalars.as<Scalars>();
   LearnedScratch &ls = *lw.scratch;
-  const bool warps = lw.warps_mode > 0 || (lw.warps_mode < 0 && ng < Workspace::kWarpWalkGroups);
+  const bool warps = lw.warps_mode != 0;
   if (ls.slot_cells[0] == 0) {  // the first learned walk: the theta walk's slots to start with
     for (int k = 0; k < kParts; ++k) {
       // the warp rounds write a group's whole lists into part 0

@@ -123,15 +123,13 @@ struct ForestView {
 // Neighbouring groups of a system of `groups` groups that a warp walks
 // together: more the more there are, since few groups leave most of the GPU
 // idle and want a warp each, and many are bound by instructions and share node
-// records and steps. The walk's time by groups per warp 1 / 2 / 4 (with the
-// spill and record kernels): 240 groups 71 / 82 / 110 us, 2.2k 98 / 100 / 143,
-// 4.4k 127 / 114 / 161, 8.8k 192 / 174 / 235, 17.6k 364 / 282 / 307 (the solve
-// 1.74 / 1.69 ms by 2 / 4: fewer warps beside the side stream), 87k 1720 / 1142 /
-// 962; by threads 1.63 ms at 87k, a warp each with two scans a step 276 us at
-// 8.8k. It depends on the system's own groups only, as does the order of
+// records and steps. The lists' time by groups per warp 1 / 2 / 4 in us: 240 groups
+// 78 / 87 / 109, 2.2k 124 / 151 / 230, 4.4k 163 / 177 / 253, 6.6k 207 / 178 / 257,
+// 8.9k 249 / 203 / 269, 13.2k 339 / 275 / 291, 17.6k 446 / 358 / 328.
+// It depends on the system's own groups only, as does the order of
 // their lists: a forest's systems keep the order each has alone.
 __host__ __device__ inline int walk_super_for(u64 groups) {
-  return groups < 3000 ? 1 : groups < 15000 ? 2 : 4;
+  return groups < 5000 ? 1 : groups < 15000 ? 2 : 4;
 }
 
 struct Workspace {
@@ -178,9 +176,6 @@ struct Workspace {
     walk_warps = walk_mode != 0;
     walk_super = walk_mode > 0 ? 2 : forest ? 0 : walk_super_for(groups);
   }
-  // Learned walk: rounds by warps below (43.8k groups 2.02 ms by warps, 2.20 by
-  // threads; 87k groups 3.67 and 3.60).
-  static constexpr u64 kWarpWalkGroups = 60000;
   // The current lists hold each group's entries in walk-step order rather
   // than the reference's visiting order (exports sort them back).
   bool lists_unordered = false;

@@ -411,7 +411,7 @@ gtc_status gtc_autotune_eval(gtc_context *ctx, const double *pos, const double *
  *   "learned_warps"      -1 (default), 0 or 1: the learned walk's rounds by
  *                        warps, one per group (1), or by three threads per
  *                        group with the long walks handed to warps (0, the
- *                        budgets above); -1 takes warps below 60000 groups.
+ *                        budgets above); -1 takes warps.
  *   "eval_pairs"         2 (default) or 1: staged entries each lane of the list
  *                        evaluation works per inner iteration (the forces do
  *                        not depend on it; gtc_autotune_eval picks it).
