@@ -161,7 +161,7 @@ struct LearnedWalk {
   u32 pair_budget = kLearnedPairBudget;  // later rounds: the same
   bool plan_rounds = true;  // walk the last call's rounds before reading anything back
   // each round by warps, one per group (1), by threads per part (0), or by
-  // warps below Workspace::kWarpWalkGroups groups (-1)
+  // warps (-1)
   int warps_mode = -1;
   // recorded after the walk's inputs (learned_walk_inputs) on another
   // stream: the walk's stream waits for it first (null: same stream)

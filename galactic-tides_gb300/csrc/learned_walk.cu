@@ -677,11 +677,39 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
   u32 visits = 0;
   u32 mc_max = 0, mb_max = 0, mp_max = 0;
   bool bad = false;
+  // Groups whose boxes span much of the root's may have walks several times as
+  // long as any other (one took 165 of round 0's 200 us at 200k): in round 0 they go
+  // first, each warp's share of them. 200 -> 179 us with such a group; with fewer
+  // groups than warps nothing waits, with many more the end is short.
+  const float wide = static_cast<float>(a.root->half_at[0]) * (1.f / 8.f);
+  auto spans = [&](u32 g) {
+    const float4 b0 = reinterpret_cast<const float4 *>(a.gboxf)[2ull * g],
+                 b1 = reinterpret_cast<const float4 *>(a.gboxf)[2ull * g + 1];
+    return fmaxf(b0.w, fmaxf(b1.x, b1.y)) > wide;
+  };
+  const u32 all_warps = gridDim.x * kLWarps;
+  const bool wide_first = round == 0 && a.ng >= 6000u && a.ng < 40000u;
+  u32 share = wide_first ? blockIdx.x * kLWarps + (threadIdx.x >> 5) : a.ng;
+  u32 first_of = 0;
+  unsigned wides = 0;
   for (;;) {
     u32 g = 0;
-    if (lane == 0) g = atomicAdd(a.next, 1u);
-    g = __shfl_sync(kFullMask, g, 0);
-    if (g >= a.ng) break;
+    if (wides) {
+      g = first_of + (static_cast<u32>(__ffs(static_cast<int>(wides))) - 1u) * all_warps;
+      wides &= wides - 1u;
+    } else if (share < a.ng) {
+      const u64 mine = share + static_cast<u64>(lane) * all_warps;
+      wides = __ballot_sync(kFullMask, mine < a.ng && spans(static_cast<u32>(mine)));
+      first_of = share;
+      const u64 after = share + 32ull * all_warps;
+      share = after < a.ng ? static_cast<u32>(after) : a.ng;
+      continue;
+    } else {
+      if (lane == 0) g = atomicAdd(a.next, 1u);
+      g = __shfl_sync(kFullMask, g, 0);
+      if (g >= a.ng) break;
+      if (wide_first && spans(g)) continue;
+    }
     float gf[3], hf[3], acc_d2, open_d2;
     group_scales(a, g, gf, hf, acc_d2, open_d2);
     const u32 capc = a.slot_cells[0], capb = a.slot_bodies[0], capp = a.slot_pend;
