@@ -253,9 +253,15 @@ __device__ __forceinline__ u32 cluster_rank() {
   asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;"
-               ::: "memory");
+  cluster_arrive();
+  cluster_wait();
 }
 // Address of this CTA's shared `p` in CTA `rank` of the cluster.
 __device__ __forceinline__ u32 remote(const void *p, u32 rank) {
@@ -289,6 +295,9 @@ template <int kPer>
 __global__ void __launch_bounds__(kCT)
     k_sort_cluster(u64 *keys, u32 *vals, u32 n, u32 ctas, int low_bit, int passes) {
   grid_wait();
+  // (a CTA's shared memory may be written once it runs: waited for before the first
+  // write into another's, behind the loads and the first ranking)
+  cluster_arrive();
   extern __shared__ __align__(16) unsigned char raw[];
   ClusterSort<kPer> &sm = *reinterpret_cast<ClusterSort<kPer> *>(raw);
   constexpr u32 kShare = kCT * kPer;
@@ -334,6 +343,7 @@ __global__ void __launch_bounds__(kCT)
       sm.quarter[q][d] = run;
     }
     __syncthreads();
+    if (p == 0) cluster_wait();
     if (threadIdx.x < kBins) {  // ... within the CTA, whose counts all CTAs get
       const u32 d = threadIdx.x;
       u32 run = 0;
