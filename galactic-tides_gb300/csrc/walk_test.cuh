@@ -39,10 +39,17 @@ __device__ __forceinline__ bool accept64(const WalkRec64 &r, const double *gc, c
 //   2^-24 of itself, which the factors (1 +- 2^-18) cover with the rounding of
 //   crit^2. (A lower and an upper bound per axis took half as many
 //   instructions again.)
-// A comparison outside its band has the FP64 outcome; otherwise the caller
+// All of which needs a square that FP32 holds: an infinite d^2 is no proof of a
+// large one, as its tolerance is finite (lengths near sqrt(FLT_MAX) = 1.84e19 in
+// a tree of 1e23 and more). So d^2 past kFarSquare is left to FP64, as are
+// scales where a rounding may be a subnormal's. (With d^2 + tol below kFarSquare an
+// overflown crit^2 is the larger in any case, and a tree whose centres, boxes or
+// bounds overflow has an infinite tolerance.)
+// A comparison outside its band then has the FP64 outcome; otherwise the caller
 // runs the FP64 test. Returns 1 accept, 0 open, 2 undecided (NaNs end up
 // undecided).
 constexpr float kBand = 1.0f / (1 << 20);
+constexpr float kFarSquare = 1e38f;
 
 __device__ __forceinline__ int accept32(const WalkRec32 &r, const float *gf, const float *hf,
                                         float gbound) {
@@ -58,8 +65,7 @@ __device__ __forceinline__ int accept32(const WalkRec32 &r, const float *gf, con
   const bool apart = d2 - tol > c2 * (1.f + 4.f * kBand);   // farther than crit for sure
   const bool close = d2 + tol < c2 * (1.f - 4.f * kBand);   // nearer for sure
   int verdict = over < -e || close ? 0 : (over > e && apart ? 1 : 2);
-  // scales where a rounding above may be a subnormal's: left to FP64
-  if (e < 1e-36f || fmaxf(d2 + tol, c2) < 1e-35f) verdict = 2;
+  if (e < 1e-36f || fmaxf(d2 + tol, c2) < 1e-35f || !(d2 + tol <= kFarSquare)) verdict = 2;
   return verdict;
 }
 

@@ -153,3 +153,39 @@ def test_fp64_sample_fixed_point(ctx, oracle, case):
     gm = G * np.abs(mass)
     assert np.all(np.abs(acc - racc) <= 1e-12 * np.einsum("tn,tnk->tk", gm * w ** 3, np.abs(dx)))
     assert np.all(np.abs(pot - rpot) <= 1e-12 * (gm * w).sum(1))
+
+
+def far_cluster(n=20_000):
+    """A cube of bodies 8e19 across, seen from a tree of 1e24: the FP32 squares
+    of its distances overflow at 1.84e19, their bound on the roundings is 1e18."""
+    pos = np.random.default_rng(1).uniform(-4e19, 4e19, (n, 3)) + np.array([2e24, 6e23, -4e23])
+    pos[0] *= -1.0
+    return pos, np.full(n, 1.0 / n)
+
+
+@pytest.mark.parametrize("theta", [0.44, 0.45, 0.47])
+def test_tree_walk_squares_beyond_fp32_bitwise(ctx, oracle, theta):
+    """Cells whose opening distance lies just below sqrt(FLT_MAX), and bodies
+    within the roundings of it whose FP32 square is infinite (6 to 28 such pairs
+    of a cell to open and a body, by these angles)."""
+    pos, mass = far_cluster()
+    kw = dict(G=1.0, theta=theta, eps=1e18, quadrupole=True)
+    acc, pot = ctx.tree_force(pos, mass, **kw)
+    st = ctx.stats()
+    want, wpot, (nc, npart) = oracle.tree_force(pos, mass, **kw)
+    assert (st["cell_interactions"], st["body_interactions"]) == (nc, npart)
+    assert np.array_equal(acc, want) and np.array_equal(pot, wpot)
+
+
+@pytest.mark.parametrize("warps", [-1, 0])
+def test_group_lists_squares_beyond_fp32(gtc, oracle, warps):
+    """The same for the grouped walk, by warps and by threads: groups of one body."""
+    from checks import compare_lists
+    pos, mass = far_cluster()
+    kw = dict(theta=0.44, group_size=1, leaf_size=8, pack=False)
+    nodes, _, lists = oracle.lists(pos, mass, **kw)
+    with gtc.Context(0) as c:
+        c.set_option("walk_warps", warps)
+        c.group_force(pos, mass, G=1.0, eps=1e18, quadrupole=True, **kw)
+        got = c.export()
+    assert compare_lists(got, got["nodes"], lists, nodes) == []
