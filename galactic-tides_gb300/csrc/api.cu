@@ -171,13 +171,13 @@ struct LearnedJoin {
   }
 };
 
-// The capacities of a captured solve of n bodies and the buffers they need:
-// the last eager solve's sizes (hs, ws) with headroom (list slots with
+// The capacities of a captured solve of n bodies: the last eager solve's sizes
+// (hs, ws) with headroom (list slots with
 // twice the headroom: the longest of many lists moves more than the totals
 // do); offsets stay below 2^32 (a replay that needs more aborts).
-void reserve_graph(gtc::Workspace &ws, const gtc::Scalars &hs, double headroom, u64 n,
-                   gtc::GraphCaps &caps, bool sized_lists = false) {
-  gtc::ensure_side(ws);  // the captured build forks the quadrupoles onto it
+gtc::GraphCaps graph_caps(const gtc::Workspace &ws, const gtc::Scalars &hs, double headroom,
+                          u64 n) {
+  gtc::GraphCaps caps{};
   const double f = 1.0 + headroom;
   const u64 pad = headroom > 0 ? 1024 : 0;
   caps.nodes = static_cast<u32>(std::min<u64>(static_cast<u64>(ws.n_nodes * f) + pad, 0xfffffff0ull));
@@ -208,33 +208,27 @@ void reserve_graph(gtc::Workspace &ws, const gtc::Scalars &hs, double headroom, 
   };
   caps.pool_cells = pool(caps.slot_cells, caps.slot_near_cells);
   caps.pool_bodies = pool(caps.slot_bodies, caps.slot_near_bodies);
+  return caps;
+}
+
+// The buffers of a solve of n bodies with those capacities.
+void reserve_graph(gtc::Workspace &ws, u64 n, const gtc::GraphCaps &caps,
+                   bool sized_lists = false) {
+  gtc::ensure_side(ws);  // the captured build forks the quadrupoles onto it
   const u64 m = caps.nodes;
-  ws.geom.ensure(m * 2 * sizeof(double2));
-  ws.mom.ensure(m * 2 * sizeof(double2));
-  ws.quad.ensure(m * 3 * sizeof(double2));
-  ws.delta.ensure(m * 8);
-  ws.nbegin.ensure(m * 4);
-  ws.nend.ensure(m * 4);
-  ws.skip.ensure(m * 4);
-  ws.parent.ensure(m * 4);
-  ws.depth.ensure(m);
-  ws.nchild.ensure(m);
-  ws.kids.ensure(m * 8 * sizeof(u32));
-  ws.isleaf.ensure(m);
-  ws.bucket.ensure(m * 4);
-  ws.climb.ensure(2 * m * sizeof(u32));
-  ws.qterm.ensure(m * 6 * sizeof(double));
-  ws.walk32.ensure(m * sizeof(gtc::WalkRec32));
-  ws.walk64.ensure(m * sizeof(gtc::WalkRec64));
-  ws.cells.ensure(m * 3 * sizeof(float4));
+  gtc::reserve_bodies(ws, n);
+  gtc::reserve_nodes(ws, m);
   ws.flags.ensure(std::max<u64>(n, m) * 4);
   ws.flags_scan.ensure(std::max<u64>(n, m) * 4);
+  ws.gbegin.ensure(n * 4);
+  ws.gend.ensure(n * 4);
+  ws.gbox.ensure(n * 48);
+  ws.gboxf.ensure(n * 32);
   ws.gcells.ensure(2 * n * 8);
   ws.gbodies.ensure(2 * n * 8);
   ws.gcell_off.ensure((n + 1) * 8);
   ws.gbody_off.ensure((n + 1) * 8);
   ws.groups.ensure(n * gtc::kGroupRecWords * 4);
-  caps.sys_slots = nullptr;
   if (!ws.forest || !sized_lists) {  // (a forest sizes them per system, when it can)
     ws.cell_list.ensure((static_cast<u64>(caps.groups) * (caps.slot_cells + caps.slot_near_cells) +
                          caps.pool_cells) * 4);
@@ -298,25 +292,22 @@ bool same_lists(const gtc::SolverParams &a, const gtc::SolverParams &b) {
          a.pack == b.pack;
 }
 
-// Remembers a theta solve's sizes for the next one.
-void plan_quick(gtc_context *ctx, u64 n, const gtc::SolverParams &sp) {
+// Remembers a theta solve's sizes for the next one (quick: the solve was
+// launched from the plan's).
+void plan_quick(gtc_context *ctx, u64 n, const gtc::SolverParams &sp, bool quick) {
   const gtc::Workspace &ws = ctx->ws;
   gtc_context::QuickPlan &q = ctx->quick;
   const gtc::Scalars &h = *ctx->host_sc;
   // the buffers reserved before serve on while the sizes stay well inside them
-  const bool fits = q.valid && q.reserved && q.n == n && same_lists(q.sp, sp) && h.spilled == 0 &&
-                    q.walk_super == ws.walk_super && ws.n_nodes < q.caps.nodes - q.caps.nodes / 16 &&
+  const bool fits = quick && h.spilled == 0 && ws.n_nodes < q.caps.nodes - q.caps.nodes / 16 &&
                     ws.n_groups < q.caps.groups - q.caps.groups / 16;
+  if (!fits) q.caps = graph_caps(ws, h, 0.25, n);
   q.valid = ws.key_words == 1 && ws.walk_warps && ws.walk_split_depth == 0;
-  q.reserved = fits;
   q.n = n;
-  q.n_nodes = ws.n_nodes;
   q.n_groups = ws.n_groups;
-  q.list_passes = ws.list_passes;
   q.walk_mode = ws.walk_mode;
   q.walk_super = ws.walk_super;
   q.sp = sp;
-  q.sizes = h;
 }
 
 // A theta solve launched whole from the last one's sizes, with nothing read
@@ -329,15 +320,11 @@ bool group_force_quick(gtc_context *ctx, const double *pos, const double *mass, 
                        const gtc::SolverParams &sp, double *acc, double *pot) {
   cudaStream_t s = ctx->stream;
   gtc::Workspace &ws = ctx->ws;
-  gtc_context::QuickPlan &q = ctx->quick;
-  if (!q.reserved) {
-    ws.n_nodes = q.n_nodes;
-    ws.n_groups = q.n_groups;
-    ws.list_passes = q.list_passes;
-    ws.walk_warps = true;
-    reserve_graph(ws, q.sizes, 0.25, n, q.caps);
-    q.reserved = true;
-  }
+  const gtc_context::QuickPlan &q = ctx->quick;
+  // (every time: other calls use the buffers too, and one that runs out of memory
+  // leaves the buffer it grew empty)
+  reserve_graph(ws, n, q.caps);
+  const gtc::EvalOut eo = solve_out(ctx, n, acc, pot);
   ws.walk_warps = true;
   ws.walk_super = q.walk_super;
   const gtc::Scalars *sc = ws.scalars.as<gtc::Scalars>();
@@ -355,8 +342,8 @@ bool group_force_quick(gtc_context *ctx, const double *pos, const double *mass, 
                               ws.cell_list.as<u32>(), ws.body_list.as<u32>(),
                               ws.groups.as<uint4>(), q.caps.groups, q.n_groups, sc,
                               static_cast<float>(sp.G), static_cast<float>(sp.eps * sp.eps),
-                              sp.quadrupole != 0, solve_out(ctx, n, acc, pot),
-                              &ws.scalars.as<gtc::Scalars>()->eval_next, s, ws.eval_shape);
+                              sp.quadrupole != 0, eo, &ws.scalars.as<gtc::Scalars>()->eval_next, s,
+                              ws.eval_shape);
     GTC_CUDA(cudaEventRecord(ctx->ev[5], s));
     GTC_CUDA(cudaEventRecord(ctx->ev[3], s));
   }
@@ -399,15 +386,15 @@ void group_force(gtc_context *ctx, const double *pos, const double *mass, u64 n,
   const bool learned = sp.criterion == GTC_CRITERION_LEARNED && ctx->have_model &&
                        ctx->prev_n == n;
   for (bool &h : ws.stage_hit) h = false;
-  if (!learned && ctx->quick.valid && ctx->quick.n == n && same_lists(ctx->quick.sp, sp) &&
-      ctx->quick.walk_mode == ws.walk_mode && !ws.stage_on && n >= kQuickBodies) {
-    if (group_force_quick(ctx, pos, mass, n, sp, acc, pot)) {
-      finish_solve(ctx, n, sp, false);
-      ctx->stats.kernel_launches = gtc::launches_so_far() - launches0;
-      plan_quick(ctx, n, sp);
-      return;
-    }
-    ctx->quick.valid = false;
+  gtc_context::QuickPlan &q = ctx->quick;
+  const bool quick = !learned && q.valid && q.n == n && same_lists(q.sp, sp) &&
+                     q.walk_mode == ws.walk_mode && !ws.stage_on && n >= kQuickBodies;
+  q.valid = false;  // until this solve has ended well
+  if (quick && group_force_quick(ctx, pos, mass, n, sp, acc, pot)) {
+    finish_solve(ctx, n, sp, false);
+    ctx->stats.kernel_launches = gtc::launches_so_far() - launches0;
+    plan_quick(ctx, n, sp, true);
+    return;
   }
   GTC_CUDA(cudaEventRecord(ctx->ev[0], s));
   const gtc::SideJoin side_join{ws, s};
@@ -466,8 +453,7 @@ void group_force(gtc_context *ctx, const double *pos, const double *mass, u64 n,
   gtc::check_device_error(ctx->host_sc->error);
   finish_solve(ctx, n, sp, learned);
   ctx->stats.kernel_launches = gtc::launches_so_far() - launches0;
-  if (learned) ctx->quick.valid = false;
-  else plan_quick(ctx, n, sp);
+  if (!learned) plan_quick(ctx, n, sp, false);
 }
 
 // One system's leapfrog step inside a captured CUDA graph: kick and drift,
@@ -488,7 +474,8 @@ struct GraphStep {
 
   void reserve() {
     gtc::Workspace &ws = ctx->ws;
-    reserve_graph(ws, *ctx->host_sc, ctx->graph_headroom, n, caps);
+    caps = graph_caps(ws, *ctx->host_sc, ctx->graph_headroom, n);
+    reserve_graph(ws, n, caps);
     if (ctx->have_model) ctx->prev_amag.ensure(n * sizeof(float));
   }
 
@@ -854,7 +841,8 @@ struct ForestGraph {
     // for every group
     gtc::GraphCaps probe{};
     const bool per_system = f->size_graph_slots(probe, headroom, s);
-    reserve_graph(f->ws, *f->host_sc, headroom, f->n, caps, per_system);
+    caps = graph_caps(f->ws, *f->host_sc, headroom, f->n);
+    reserve_graph(f->ws, f->n, caps, per_system);
     if (per_system) {
       caps.sys_slots = probe.sys_slots;
       caps.pool_at_cells = probe.pool_at_cells;

@@ -19,17 +19,14 @@ struct gtc_context {
   gtc::DeviceBuffer sample_scratch; // FP64 sample partial sums
   bool have_group = false;
   gtc::SolverParams last{};
-  // The sizes of the last theta solve, from which the next one of as many
-  // bodies with the same parameters is launched without reading any back
-  // (group_force); any option set forgets them.
+  // The sizes of the last theta solve with headroom, from which the next one
+  // of as many bodies with the same parameters is launched without reading any
+  // back (group_force); any option set and any solve that fails forgets them.
   struct QuickPlan {
-    bool valid = false;      // sizes below are a solve's
-    bool reserved = false;   // caps and the buffers follow them
-    gtc::u64 n = 0, n_nodes = 0, n_groups = 0;
-    gtc::u32 list_passes = 0;
+    bool valid = false;
+    gtc::u64 n = 0, n_groups = 0;
     int walk_mode = -1, walk_super = 1;
     gtc::SolverParams sp{};
-    gtc::Scalars sizes{};
     gtc::GraphCaps caps{};
   } quick;
   // learned opening criterion

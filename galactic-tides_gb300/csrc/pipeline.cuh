@@ -332,6 +332,10 @@ __device__ __forceinline__ void warp_add(unsigned long long *total, unsigned lon
   if ((threadIdx.x & 31) == 0 && v) atomicAdd(total, v);
 }
 
+// The build's buffers: per body, and (m nodes) per node.
+void reserve_bodies(Workspace &ws, u64 n);
+void reserve_nodes(Workspace &ws, u64 m);
+
 // Stage 1: octree on the device. pos (N x 3) and mass in caller order.
 // Fills geometry, moments, ranges, the tree-order permutation (idx), the
 // FP32 bodies and cells and the walk records. Returns the node count.

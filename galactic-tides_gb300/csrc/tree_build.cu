@@ -1706,16 +1706,7 @@ void launch_quads(Workspace &ws, const MomentPlan &p, const TreeRoot *root, bool
 }
 }  // namespace
 
-void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
-                const SolverParams &sp, cudaStream_t s, Scalars *host, bool walk_records) {
-  ws.n = n;
-  ws.n_nodes = 0;
-  ws.key_words = 1;
-  if (n == 0) return;
-  const u32 n32 = static_cast<u32>(n);
-  const u32 nb = ceil_div(n, kT);
-  const int L = std::max(1, sp.leaf_size);
-
+void reserve_bodies(Workspace &ws, u64 n) {
   ws.key0.ensure(n * 8);
   ws.key0_alt.ensure(n * 8);
   ws.idx.ensure(n * 4);
@@ -1729,6 +1720,41 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   ws.tmass.ensure(n * 8);
   ws.bodies.ensure(n * sizeof(float4));
   ws.scalars.ensure(sizeof(Scalars));
+}
+
+void reserve_nodes(Workspace &ws, u64 m) {
+  ws.geom.ensure(m * 2 * sizeof(double2));
+  ws.mom.ensure(m * 2 * sizeof(double2));
+  ws.quad.ensure(m * 3 * sizeof(double2));
+  ws.delta.ensure(m * 8);
+  ws.nbegin.ensure(m * 4);
+  ws.nend.ensure(m * 4);
+  ws.skip.ensure(m * 4);
+  ws.parent.ensure(m * 4);
+  ws.depth.ensure(m);
+  ws.nchild.ensure(m);
+  ws.kids.ensure(m * 8 * sizeof(u32));
+  ws.isleaf.ensure(m);
+  ws.arrive.ensure(2 * kBuckets * sizeof(u32));
+  ws.climb.ensure(arrive_bytes(m));
+  ws.qterm.ensure(m * 6 * sizeof(double));
+  ws.bucket.ensure(m * 4);
+  ws.walk32.ensure(m * sizeof(WalkRec32));
+  ws.walk64.ensure(m * sizeof(WalkRec64));
+  ws.cells.ensure(m * 3 * sizeof(float4));
+}
+
+void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
+                const SolverParams &sp, cudaStream_t s, Scalars *host, bool walk_records) {
+  ws.n = n;
+  ws.n_nodes = 0;
+  ws.key_words = 1;
+  if (n == 0) return;
+  const u32 n32 = static_cast<u32>(n);
+  const u32 nb = ceil_div(n, kT);
+  const int L = std::max(1, sp.leaf_size);
+
+  reserve_bodies(ws, n);
   join_side(ws, s);  // nothing of an earlier call may still write the buffers
   Scalars *sc = ws.scalars.as<Scalars>();
   clear({{sc, sizeof(Scalars)}}, s);
@@ -1839,24 +1865,7 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   const u32 m = host->n_nodes;
   ws.n_nodes = m;
   ws.tree_depth = static_cast<int>(host->depth);
-  ws.geom.ensure(m * 2 * sizeof(double2));
-  ws.mom.ensure(m * 2 * sizeof(double2));
-  ws.quad.ensure(m * 3 * sizeof(double2));
-  ws.delta.ensure(m * 8ull);
-  ws.nbegin.ensure(m * 4ull);
-  ws.nend.ensure(m * 4ull);
-  ws.skip.ensure(m * 4ull);
-  ws.parent.ensure(m * 4ull);
-  ws.depth.ensure(m);
-  ws.nchild.ensure(m);
-  ws.isleaf.ensure(m);
-  ws.arrive.ensure(2 * kBuckets * sizeof(u32));
-  ws.climb.ensure(arrive_bytes(m));
-  ws.qterm.ensure(m * 6 * sizeof(double));
-  ws.bucket.ensure(m * 4ull);
-  ws.walk32.ensure(m * sizeof(WalkRec32));
-  ws.walk64.ensure(m * sizeof(WalkRec64));
-  ws.cells.ensure(m * 3 * sizeof(float4));
+  reserve_nodes(ws, m);
   const u32 mb = ceil_div(m, kT);
 
   launch(k_nodes, nb, kT, 0, s, kv, lcp_next, leafdepth, count, cscan, n32, sc, root,
@@ -1864,7 +1873,6 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
          ws.skip.as<u32>(), ws.depth.as<u8>(), ws.isleaf.as<u8>(),
          fv ? fv.split_levels : kSplitLevels, nullptr);
   GTC_LAUNCH_CHECK();
-  ws.kids.ensure(static_cast<u64>(m) * 8 * sizeof(u32));
   launch(k_children, mb, kT, 0, s, ws.skip.as<u32>(), ws.isleaf.as<u8>(), m, ws.parent.as<u32>(),
          ws.nchild.as<u8>(), ws.kids.as<uint4>());
   GTC_LAUNCH_CHECK();
