@@ -211,6 +211,13 @@ gtc::GraphCaps graph_caps(const gtc::Workspace &ws, const gtc::Scalars &hs, doub
   return caps;
 }
 
+// Entries of both lists' slots and pools.
+u64 slot_entries(const gtc::GraphCaps &c) {
+  return static_cast<u64>(c.groups) * (static_cast<u64>(c.slot_cells) + c.slot_near_cells +
+                                       c.slot_bodies + c.slot_near_bodies) +
+         c.pool_cells + c.pool_bodies;
+}
+
 // The buffers of a solve of n bodies with those capacities.
 void reserve_graph(gtc::Workspace &ws, u64 n, const gtc::GraphCaps &caps,
                    bool sized_lists = false) {
@@ -302,7 +309,9 @@ void plan_quick(gtc_context *ctx, u64 n, const gtc::SolverParams &sp, bool quick
   const bool fits = quick && h.spilled == 0 && ws.n_nodes < q.caps.nodes - q.caps.nodes / 16 &&
                     ws.n_groups < q.caps.groups - q.caps.groups / 16;
   if (!fits) q.caps = graph_caps(ws, h, 0.25, n);
-  q.valid = ws.key_words == 1 && ws.walk_warps && ws.walk_split_depth == 0;
+  q.valid = ws.key_words == 1 && ws.walk_warps && ws.walk_split_depth == 0 &&
+            (fits || slot_entries(q.caps) <= gtc::Workspace::slot_limit(ws.n_cell_list +
+                                                                        ws.n_body_list));
   q.n = n;
   q.n_groups = ws.n_groups;
   q.walk_mode = ws.walk_mode;

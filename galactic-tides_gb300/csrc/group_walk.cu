@@ -1393,7 +1393,7 @@ void build_lists(Workspace &ws, const SolverParams &sp, cudaStream_t s, Scalars 
   const u64 pool_c = Workspace::pool_for(ng, sl_c + sn_c), pool_b = Workspace::pool_for(ng, sl_b + sn_b);
   const u64 ext_c = pool_at_c + pool_c, ext_b = pool_at_b + pool_b;
   if (sl_c > 0 && ntasks == 1 && ext_c <= 0xffffffffull && ext_b <= 0xffffffffull &&
-      ext_c + ext_b <= std::max<u64>(16 * prev_entries, 1ull << 28)) {
+      ext_c + ext_b <= Workspace::slot_limit(prev_entries)) {
     ws.cell_list.ensure(ext_c * 4);
     ws.body_list.ensure(ext_b * 4);
     if (ws.walk_warps) {

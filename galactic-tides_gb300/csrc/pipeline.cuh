@@ -208,6 +208,12 @@ struct Workspace {
   // Overflow pool behind n_groups slots of `slot` entries: a sixteenth of
   // the slots plus four slots.
   static u64 pool_for(u64 n_groups, u32 slot) { return n_groups * slot / 16 + 4ull * slot; }
+  // What per-group slots and their pools may take in all (entries), given the
+  // lists' own: past it (a few lists many times as long as the others) lists are
+  // counted first and written back to back.
+  static u64 slot_limit(u64 entries) {
+    return 16 * entries > (1ull << 28) ? 16 * entries : 1ull << 28;
+  }
   void release_all();
 };
 

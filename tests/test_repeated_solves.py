@@ -52,3 +52,23 @@ def test_after_a_call_that_ran_out_of_memory(gtc):
             s.solve(n=2**32 - 1)
         assert same(s.solve(), want)
         assert same(s.solve(), want)
+
+
+def test_one_long_list_among_many_keeps_its_memory(gtc):
+    """100000 bodies in a small cube and seven at the corners of the root's, whose
+    group's box holds them all: its list is 100000 long, the others' 800. Slots of
+    that length for every group would take 3 GB; the lists, 14 MB in all, stay
+    counted first and back to back, as the first solve has them."""
+    import torch
+    n = 100_000
+    rng = np.random.default_rng(0)
+    corners = np.array([[x, y, z] for x in (-1, 1) for y in (-1, 1) for z in (-1, 1)][1:], float)
+    with Solver(gtc, n) as s:
+        s.set(np.concatenate([rng.uniform(-0.7, -0.3, (n - 7, 3)), corners]), np.full(n, 1.0 / n))
+        want = s.solve()
+        assert s.ctx.stats()["max_list"] > 90_000
+        free = torch.cuda.mem_get_info()[0]
+        for _ in range(3):
+            assert same(s.solve(), want)
+            assert s.ctx.stats()["list_passes"] == 2
+        assert free - torch.cuda.mem_get_info()[0] < 2**28
