@@ -309,7 +309,8 @@ void plan_quick(gtc_context *ctx, u64 n, const gtc::SolverParams &sp, bool quick
   const bool fits = quick && h.spilled == 0 && ws.n_nodes < q.caps.nodes - q.caps.nodes / 16 &&
                     ws.n_groups < q.caps.groups - q.caps.groups / 16;
   if (!fits) q.caps = graph_caps(ws, h, 0.25, n);
-  q.valid = ws.key_words == 1 && ws.walk_warps && ws.walk_split_depth == 0 &&
+  q.refused = q.refused && q.n == n && same_lists(q.sp, sp);
+  q.valid = !q.refused && ws.key_words == 1 && ws.walk_warps && ws.walk_split_depth == 0 &&
             (fits || slot_entries(q.caps) <= gtc::Workspace::slot_limit(ws.n_cell_list +
                                                                         ws.n_body_list));
   q.n = n;
@@ -399,7 +400,15 @@ void group_force(gtc_context *ctx, const double *pos, const double *mass, u64 n,
   const bool quick = !learned && q.valid && q.n == n && same_lists(q.sp, sp) &&
                      q.walk_mode == ws.walk_mode && !ws.stage_on && n >= kQuickBodies;
   q.valid = false;  // until this solve has ended well
-  if (quick && group_force_quick(ctx, pos, mass, n, sp, acc, pot)) {
+  bool done = false;
+  if (quick) {
+    try {
+      done = group_force_quick(ctx, pos, mass, n, sp, acc, pot);
+    } catch (const gtc::OutOfMemory &) {
+      q.refused = true;  // the sizes themselves may fit
+    }
+  }
+  if (done) {
     finish_solve(ctx, n, sp, false);
     ctx->stats.kernel_launches = gtc::launches_so_far() - launches0;
     plan_quick(ctx, n, sp, true);

@@ -24,6 +24,7 @@ struct gtc_context {
   // back (group_force); any option set and any solve that fails forgets them.
   struct QuickPlan {
     bool valid = false;
+    bool refused = false;  // no memory for this n's and these lists' headroom
     gtc::u64 n = 0, n_groups = 0;
     int walk_mode = -1, walk_super = 1;
     gtc::SolverParams sp{};

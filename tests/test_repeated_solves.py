@@ -72,3 +72,25 @@ def test_one_long_list_among_many_keeps_its_memory(gtc):
             assert same(s.solve(), want)
             assert s.ctx.stats()["list_passes"] == 2
         assert free - torch.cuda.mem_get_info()[0] < 2**28
+
+
+def test_without_memory_for_the_headroom(gtc):
+    """With the GPU's memory full but for 32 MB, the buffers of a solve launched
+    from the last one's sizes (a quarter more groups, half as long again lists)
+    cannot be had: it reads its sizes, whose buffers fit, this time and the next."""
+    import torch
+    with Solver(gtc, 200_003) as s:
+        for _ in range(3):  # (an option set: sizes are read each time)
+            s.ctx.set_option("eval_pairs", 2)
+            want = s.solve()
+        before = s.ctx.stats()["kernel_launches"]
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - 2**25, dtype=torch.uint8, device="cuda")
+        try:
+            for _ in range(3):
+                assert same(s.solve(), want)
+                assert s.ctx.stats()["kernel_launches"] == before
+        finally:
+            del hog
+            torch.cuda.empty_cache()
+        assert same(s.solve(), want)
