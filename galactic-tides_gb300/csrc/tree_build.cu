@@ -1361,12 +1361,13 @@ __global__ void k_root_mass(const float4 *cells32, double2 *rootmom) {
   rootmom[1] = make_double2(0.0, static_cast<double>(cells32[0].w));
 }
 
-// A graph replay's checks after the node count: deeper keys needed, or a
-// leaf below the sorted levels (bit 1), or more nodes than the node arrays
-// hold (bit 2).
+// A graph replay's checks after the node count: an error so far (positions that
+// are not finite), deeper keys needed, or a leaf below the sorted levels (bit
+// 1), or more nodes than the node arrays hold (bit 2). The host looks at the error
+// first; the abort keeps the later kernels from writing results.
 __global__ void k_check_tree_graph(Scalars *sc, u32 cap, int sorted_levels) {
   grid_wait();
-  if (sc->deep > 0 || static_cast<int>(sc->depth) > sorted_levels) sc->abort |= 1u;
+  if (sc->error || sc->deep > 0 || static_cast<int>(sc->depth) > sorted_levels) sc->abort |= 1u;
   if (sc->n_nodes > cap) sc->abort |= 2u;
 }
 

@@ -94,3 +94,20 @@ def test_without_memory_for_the_headroom(gtc):
             del hog
             torch.cuda.empty_cache()
         assert same(s.solve(), want)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_positions_not_finite_leave_the_results(gtc, bad):
+    """A body without a place is refused before anything is written: results, and
+    the sizes of accelerations kept for a learned solve, stay the last solve's."""
+    with Solver(gtc, 70_001) as s:
+        want = s.solve()
+        assert same(s.solve(), want)
+        x = float(s.pos[123, 1])
+        s.pos[123, 1] = bad
+        with pytest.raises(gtc.GtcInvalidArgument, match="finite"):
+            s.solve()
+        assert same((s.acc.cpu().numpy(), s.pot.cpu().numpy()), want)
+        s.pos[123, 1] = x
+        assert same(s.solve(), want)
+        assert same(s.solve(), want)
