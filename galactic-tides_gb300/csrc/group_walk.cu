@@ -116,13 +116,13 @@ __global__ void __launch_bounds__(kT)
   if (b == n - 1 && g + mark[b] > 0) gend[g + mark[b] - 1] = n;
 }
 
-// A graph replay's checks around the one-pass walk (bit 8): more groups
-// than the captured slots cover, or so many that a warp walks more or fewer
+// A graph replay's checks around the one-pass walk (bit 8): an error so far, more
+// groups than the captured slots cover, or so many that a warp walks more or fewer
 // together than the captured walk (before; walk_super 0: any), overflow pools
 // too small for the lists that outgrew their slots (after).
 __global__ void k_check_groups_graph(Scalars *sc, u32 groups, int walk_super) {
   grid_wait();
-  if (sc->n_groups > groups) sc->abort |= 8u;
+  if (sc->error || sc->n_groups > groups) sc->abort |= 8u;
   if (walk_super != 0 && walk_super_for(sc->n_groups) != walk_super) sc->abort |= 8u;
 }
 __global__ void k_check_slots_graph(Scalars *sc) {
@@ -1201,9 +1201,12 @@ __global__ void __launch_bounds__(kT)
 }
 
 
+// (The counts read back size buffers and the scans behind them give places: neither
+// is used after an error.)
 void read_scalars(Workspace &ws, Scalars *host, cudaStream_t s) {
   GTC_CUDA(cudaMemcpyAsync(host, ws.scalars.ptr, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
   GTC_CUDA(cudaStreamSynchronize(s));
+  check_device_error(host->error);
 }
 
 // Slots for the next one-pass walk: this walk's longest lists plus a half
@@ -1540,11 +1543,10 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
   GTC_LAUNCH_CHECK();
   // one pass into the captured slots (near field and rest), outgrown groups
   // again into the pools
-  if (!caps.sys_slots) {  // (per-system slots: a system past its capacity spills)
-    launch(k_check_groups_graph, 1, 1, 0, s, sc, caps.groups,
-           ws.walk_mode < 0 ? ws.walk_super : 0);
-    GTC_LAUNCH_CHECK();
-  }
+  // (per-system slots: a system past its capacity spills)
+  launch(k_check_groups_graph, 1, 1, 0, s, sc, caps.sys_slots ? ~0u : caps.groups,
+         ws.walk_mode < 0 && !caps.sys_slots ? ws.walk_super : 0);
+  GTC_LAUNCH_CHECK();
   join_walk(ws, s);  // the walk reads the node records (the cells follow on the side stream)
   u32 *spill_c = ws.spill.as<u32>(), *spill_b = spill_c + n;
   // (the replays' walk: the choice of the eager solve before the capture)

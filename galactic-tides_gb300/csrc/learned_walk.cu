@@ -960,6 +960,10 @@ __global__ void __launch_bounds__(kT) k_lrows(const GArgs a, uint2 *rows, u64 ca
   const u64 pg = static_cast<u64>(blockIdx.x) * kT + threadIdx.x;
   const u64 nparts = static_cast<u64>(kParts) * a.ng;
   const u32 total = a.roff[nparts];
+  if (a.sc->error) {  // no places for the rows: nothing more is walked or decided
+    if (pg == 0) atomicOr(&a.sc->list_overflow, 4u);
+    return;
+  }
   if (a.sc->list_overflow & 1u) return;  // a slot was outgrown: the walk is redone
   if (pg == 0) {
     atomicMax(&a.sc->max_rows, total);
@@ -1263,9 +1267,7 @@ void learned_build_lists(Workspace &ws, const LearnedWalk &lw, u32 ng, Scalars *
       GTC_CUDA(cudaMemcpyAsync(flags, &sc->list_overflow, sizeof(u32), cudaMemcpyDeviceToHost, s));
       GTC_CUDA(cudaMemcpyAsync(flags + 1, &sc->error, sizeof(u32), cudaMemcpyDeviceToHost, s));
       GTC_CUDA(cudaStreamSynchronize(s));
-      if (flags[1])
-        throw RuntimeError("cuda: inconsistent tree detected on the device (code " +
-                           std::to_string(flags[1]) + ")");
+      check_device_error(flags[1]);
       return flags[0] != 0;
     };
     bool overflow = false;

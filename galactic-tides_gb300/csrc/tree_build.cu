@@ -1471,9 +1471,12 @@ const double *root_centre(const TreeRoot *root) {
                                           offsetof(TreeRoot, center));
 }
 
+// (The counts read back size buffers and the scans behind them give places: neither
+// is used after an error.)
 void read_scalars(Workspace &ws, Scalars *host, cudaStream_t s) {
   GTC_CUDA(cudaMemcpyAsync(host, ws.scalars.ptr, sizeof(Scalars), cudaMemcpyDeviceToHost, s));
   GTC_CUDA(cudaStreamSynchronize(s));
+  check_device_error(host->error);
 }
 
 }  // namespace
@@ -1788,7 +1791,6 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
   GTC_LAUNCH_CHECK();
   count_nodes();
   read_scalars(ws, host, s);
-  if (host->error & 4u) throw InvalidArgument("cuda: positions must be finite");
   if (sorted < kLevelsPerWord && static_cast<int>(host->depth) > sorted) {
     sort_top_levels(ws, n32, kLevelsPerWord, s);
     GTC_CUDA(cudaMemsetAsync(&sc->deep, 0, sizeof(u32), s));
