@@ -111,3 +111,34 @@ def test_positions_not_finite_leave_the_results(gtc, bad):
         s.pos[123, 1] = x
         assert same(s.solve(), want)
         assert same(s.solve(), want)
+
+
+def test_which_way_each_solve_takes(gtc):
+    """Two galaxies of as many bodies, on either side of the 5000 groups from which a
+    warp walks two groups instead of one. The launches tell the ways apart: a solve
+    from the last sizes has as many on the same bodies each time; one that finds
+    another number of groups stops and is solved by reading them, both ways' launches.
+    The forces are a fresh context's either way."""
+    n = 112_000
+    bodies = {k: gtc.make_galaxy(n, seed=k)[0::2] for k in (1, 2)}
+    want = {}
+    for k, (pos, mass) in bodies.items():
+        with Solver(gtc, n, seed=k) as fresh:
+            want[k] = fresh.solve()
+            groups = fresh.ctx.stats()["n_groups"]
+            assert (groups >= 5000) == (k == 1) and abs(groups - 5000) < 250
+    with Solver(gtc, n, seed=1) as s:
+        def solve(k):
+            s.set(*bodies[k])
+            assert same(s.solve(), want[k])
+            return s.ctx.stats()["kernel_launches"]
+        solve(1)
+        quick = solve(1)
+        s.ctx.set_option("eval_pairs", 2)  # forgets the sizes
+        read = solve(1)
+        assert read != quick
+        assert [solve(1), solve(1)] == [quick, quick]
+        for k in (2, 1):
+            redone = solve(k)
+            assert quick + read - 4 <= redone <= quick + read + 4
+            assert solve(k) == quick
