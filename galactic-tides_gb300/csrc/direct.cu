@@ -147,22 +147,6 @@ struct alignas(16) Body64 {
   double m;
 };
 
-// 1/sqrt(x) in FP64: the SFU's estimate (rsqrt.approx.ftz.f64) and one step
-// of the third-order (Halley) iteration: with e = 1 - x y^2 exactly the
-// relative deficit of y^2, 1/sqrt(x) = y (1 - e)^(-1/2) = y (1 + e/2 + 3/8 e^2
-// + O(e^3)). An estimate good to 2^-18 leaves 5/16 e^3 < 2^-52 / 8, so the
-// result is within about one unit in the last place (sqrt and a division
-// round twice). Zero, subnormal, negative, infinite and NaN inputs take the
-// plain division. For the distances inverse_powers does not take.
-__device__ __forceinline__ double rsqrt64(double x) {
-  const u32 hi = static_cast<u32>(__double2hiint(x));
-  if (hi - 0x00100000u >= 0x7fe00000u) return 1.0 / sqrt(x);
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
 // What a source adds to its target, in FP64 coordinates: for tiles and bodies
 // that their tile's fixed point does not hold.
 struct Pair64 {

@@ -82,6 +82,27 @@ __device__ __forceinline__ bool inverse_powers(double dx, double dy, double dz,
   return true;
 }
 
+// 1/sqrt(x) in FP64, for the distances inverse_powers does not take: the SFU's
+// estimate y (rsqrt.approx.ftz.f64) and one step of the third-order (Halley)
+// iteration: with e = 1 - x y^2 exactly, 1/sqrt(x) = y (1 - e)^(-1/2) = y (1 + e/2
+// + 3/8 e^2 + 5/16 e^3 + ...). |e| is at most 1.9e-6 < 2^-18 (on every high word;
+// tests/test_rsqrt64.py), so what is left out is below 2^-55; the rounding of x y
+// leaves 2^-54 in e / 2, the last one 2^-53: within 2^-52 of the value in all
+// (1.24e-16 measured; sqrt and a division round twice). Zero, subnormal,
+// negative, infinite and NaN inputs take the plain division.
+__device__ __forceinline__ double rsqrt64_estimate(double x) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  return y;
+}
+__device__ __forceinline__ double rsqrt64(double x) {
+  const u32 hi = static_cast<u32>(__double2hiint(x));
+  if (hi - 0x00100000u >= 0x7fe00000u) return 1.0 / sqrt(x);
+  const double y = rsqrt64_estimate(x);
+  const double e = fma(-(x * y), y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
 // ------------------------------------------------- differences in fixed point
 //
 // Coordinates as 96-bit integers in units of 2^(scale - 1115), `scale` the
