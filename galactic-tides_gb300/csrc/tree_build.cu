@@ -427,13 +427,14 @@ __global__ void __launch_bounds__(kT)
 
 // A forest's last sort pass, by system: the system of each sorted body as
 // the key, the position as the value; the key words and bodies are copied
-// aside for the gather that follows the pass.
+// aside for the gather that follows the pass. (Here and below: what a sort that
+// failed leaves behind is not used as places; the solve ends with its error.)
 __global__ void __launch_bounds__(kT)
     k_forest_sys_keys(const u64 *key, const u32 *idx, const u16 *sys, u32 n, u64 *skey, u32 *spos,
-                      u64 *key_copy, u32 *idx_copy, const u32 *abort = nullptr) {
+                      u64 *key_copy, u32 *idx_copy, const u32 *error) {
   grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
-  if (k >= n || aborted(abort)) return;
+  if (k >= n || *error) return;
   const u32 i = idx[k];
   skey[k] = sys[i];
   spos[k] = k;
@@ -443,10 +444,10 @@ __global__ void __launch_bounds__(kT)
 
 __global__ void __launch_bounds__(kT)
     k_forest_gather(const u32 *spos, const u64 *key_copy, const u32 *idx_copy, u32 n, u64 *key,
-                    u32 *idx, const u32 *abort = nullptr) {
+                    u32 *idx, const u32 *error) {
   grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
-  if (k >= n || aborted(abort)) return;
+  if (k >= n || *error) return;
   const u32 j = spos[k];
   key[k] = key_copy[j];
   idx[k] = idx_copy[j];
@@ -462,6 +463,7 @@ __global__ void __launch_bounds__(kT)
   // each computed once; a body's w is the largest over its windows
   constexpr int kMaxWin = 64;
   __shared__ signed char win[kT + kMaxWin];
+  if (sc->error) return;
   const u32 base = blockIdx.x * kT, b = base + threadIdx.x;
   const bool shared_win = L <= kMaxWin;
   if (shared_win) {
@@ -564,10 +566,11 @@ __global__ void __launch_bounds__(kT)
 }
 
 __global__ void __launch_bounds__(kT)
-    k_seg_keys(const u32 *rec, const u32 *seg_scan, const u32 *seg_flag, u32 nd, u64 *key) {
+    k_seg_keys(const u32 *rec, const u32 *seg_scan, const u32 *seg_flag, u32 nd, u64 *key,
+               const u32 *error) {
   grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
-  if (k >= nd) return;
+  if (k >= nd || *error) return;
   const u32 r = rec[k];
   key[k] = seg_scan[r] + seg_flag[r];  // 1-based segment number
 }
@@ -576,10 +579,10 @@ __global__ void __launch_bounds__(kT)
 // new word, input order).
 __global__ void __launch_bounds__(kT)
     k_deep_scatter(const u32 *dpos, const u32 *rec, const u32 *didx, const u64 *word, u32 nd,
-                   u32 *idx, u64 *word_out) {
+                   u32 *idx, u64 *word_out, const u32 *error) {
   grid_wait();
   const u32 k = blockIdx.x * kT + threadIdx.x;
-  if (k >= nd) return;
+  if (k >= nd || *error) return;
   const u32 r = rec[k];
   idx[dpos[k]] = didx[r];
   word_out[dpos[k]] = word[r];
@@ -1559,8 +1562,7 @@ void make_keys(Workspace &ws, const double *pos, u32 n, const TreeRoot *root, cu
 // keep their input order, which is all the tree needs while no leaf lies
 // deeper. A forest's pairs are then sorted by system, stably: (system,
 // key), each system at its own bodies' positions.
-int sort_top_levels(Workspace &ws, u32 n, int levels, cudaStream_t s,
-                    const u32 *abort = nullptr) {
+int sort_top_levels(Workspace &ws, u32 n, int levels, cudaStream_t s) {
   const int passes = levels >= kLevelsPerWord ? 8 : (3 * std::max(levels, 1) + 7) / 8;
   const int low = std::max(0, 3 * kLevelsPerWord - 8 * passes);
   ws.sort_passes = passes;
@@ -1577,14 +1579,14 @@ int sort_top_levels(Workspace &ws, u32 n, int levels, cudaStream_t s,
     u32 *spos = ws.drec.as<u32>();
     const u32 nb = ceil_div(n, kT);
     launch(k_forest_sys_keys, nb, kT, 0, s, ws.key0.as<u64>(), ws.idx.as<u32>(), fv.sys, n, skey,
-           spos, ws.key0_alt.as<u64>(), ws.idx_alt.as<u32>(), abort);
+           spos, ws.key0_alt.as<u64>(), ws.idx_alt.as<u32>(), err);
     GTC_LAUNCH_CHECK();
     int bits = 1;
     while (bits < 16 && (1u << bits) < fv.systems) ++bits;
     radix_sort_pairs(skey, spos, ws.dkey_alt.as<u64>(), ws.drec_alt.as<u32>(), n, bits, ws.radix,
                      s, 0, err);
     launch(k_forest_gather, nb, kT, 0, s, spos, ws.key0_alt.as<u64>(), ws.idx_alt.as<u32>(), n,
-           ws.key0.as<u64>(), ws.idx.as<u32>(), abort);
+           ws.key0.as<u64>(), ws.idx.as<u32>(), err);
     GTC_LAUNCH_CHECK();
   }
   return low == 0 ? kLevelsPerWord : (3 * kLevelsPerWord - low) / 3;
@@ -1844,11 +1846,12 @@ void build_tree(Workspace &ws, const double *pos, const double *mass, u64 n,
     read_scalars(ws, host, s);
     int seg_bits = 1;
     while (seg_bits < 32 && (1ull << seg_bits) <= host->aux) ++seg_bits;
-    launch(k_seg_keys, ndb, kT, 0, s, drec, sscan, sflag, nd, dkey);
+    launch(k_seg_keys, ndb, kT, 0, s, drec, sscan, sflag, nd, dkey, &sc->error);
     GTC_LAUNCH_CHECK();
     radix_sort_pairs(dkey, drec, ws.dkey_alt.as<u64>(), ws.drec_alt.as<u32>(), nd, seg_bits,
                      ws.radix, s, 0, &sc->error);
-    launch(k_deep_scatter, ndb, kT, 0, s, dpos, drec, didx, dword, nd, idx, wbuf.as<u64>());
+    launch(k_deep_scatter, ndb, kT, 0, s, dpos, drec, didx, dword, nd, idx, wbuf.as<u64>(),
+           &sc->error);
     GTC_LAUNCH_CHECK();
     if (kv.words == 1) kv.w1 = ws.key1.as<u64>();
     else kv.w2 = ws.key2.as<u64>();

@@ -1,7 +1,8 @@
-"""A scan whose look-back outwaits its bound leaves sums that are too small, and
-sums are places in memory. (Read from the source: no input makes a wait run out.)
-Host code checks the error word with every read back of sizes, and of the kernels
-that work from counts on the device the first after each scan looks at it."""
+"""A scan whose look-back outwaits its bound leaves sums that are too small, a sort
+places that were not written, and both are places in memory. (Read from the source:
+no input makes a wait run out.) Host code checks the error word with every read
+back of sizes, and of the kernels that work on the device's own the first after each
+scan or sort looks at it."""
 
 import pathlib
 import re
@@ -28,6 +29,11 @@ def body(path, name):
     ("tree_build.cu", "k_check_tree_graph", "sc->error"),     # the node count's scan
     ("group_walk.cu", "k_check_groups_graph", "sc->error"),   # the groups'
     ("learned_walk.cu", "k_lrows", "sc->error"),              # the deferred pairs'
+    ("tree_build.cu", "k_levels", "sc->error"),               # the keys' sort
+    ("tree_build.cu", "k_forest_sys_keys", "*error"),         # a forest's, by key
+    ("tree_build.cu", "k_forest_gather", "*error"),           # and by system
+    ("tree_build.cu", "k_seg_keys", "*error"),                # the deeper keys', by word
+    ("tree_build.cu", "k_deep_scatter", "*error"),            # and by segment
 ])
 def test_errors_are_seen_before_places_are_used(path, name, check):
     assert check in body(path, name)
