@@ -12,14 +12,16 @@
 // the marks into the group array, which comes out in tree order as in the
 // reference.
 //
-// Walk. By warps (below) or by threads: one thread per group traverses the
-// nodes in their stored order (the order the reference's stack pops them): accept -> record and jump to
-// the node's skip link, leaf -> record its bodies and jump, otherwise step
-// to the next node (its last child). A counting pass sizes the lists; after
-// the offsets are scanned a second pass writes them. Once a walk has
-// measured the longest lists, later walks run once, writing each group's
-// lists into fixed per-group slots (half as long again), and fall back to the
-// two passes when a list outgrows its slot.
+// Walk. By warps, each walking one, two or four neighbouring groups with a stack of
+// node ranges (k_walk_warp, the default), or by threads (option walk_warps 0), which
+// traverse the nodes in their stored order (the order the reference's stack pops
+// them): accept -> record and jump to the node's skip link, leaf -> record its
+// bodies and jump, otherwise step to the next node (its last child). A counting pass
+// sizes the lists; after the offsets are scanned a second pass writes them. Once a
+// walk has measured the longest lists, later walks run once, writing each group's
+// lists into per-group slots (half as long again). A group that outgrows its slot
+// is walked again into an overflow pool; pools too small, or slots past
+// Workspace::slot_limit, fall back to the two passes.
 
 #include <algorithm>
 #include <type_traits>
@@ -1526,7 +1528,7 @@ void build_lists_graph(Workspace &ws, const SolverParams &sp, const GraphCaps &c
   u32 *mark = ws.flags.as<u32>(), *mscan = ws.flags_scan.as<u32>();
   const u32 *abort = &sc->abort;
   const u32 nb = ceil_div(n, kT), mb = ceil_div(mcap, kT);
-  // groups (the one walk task, the root, was written before capture)
+  // groups
   clear({{mark, n * 4}}, s);
   const ForestView &fv = ws.forest;
   const NodeView nv = node_view(ws);

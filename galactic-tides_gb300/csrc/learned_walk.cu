@@ -625,8 +625,8 @@ __global__ void __launch_bounds__(kContWarps * 32) k_lcont(GArgs a, bool later) 
 // come one a step (learned solve of 200k bodies 0.74 -> 0.68 ms, 2M 3.67 -> 3.37; by
 // threads 1.13 and 3.57).
 //
-// Bound: the longest walks (200k: the SMs are busy 54% of the time to the last
-// one's end), then issue. Round 0 of 200k bodies 233 -> 197 us; 12 to 16 blocks an
+// Bound: the longest walks (round 0 of 200k: 178 us, the SMs busy 46% of the time to
+// the last one's end, issuing in 61% of those cycles), then issue. 12 to 16 blocks an
 // SM, or stacks of 512 or 1024 ranges, measure the same.
 constexpr int kLWarps = 4;
 constexpr int kLStack = 256;  // ranges per warp
@@ -679,8 +679,11 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
   bool bad = false;
   // Groups whose boxes span much of the root's may have walks several times as
   // long as any other (one took 165 of round 0's 200 us at 200k): in round 0 they go
-  // first, each warp's share of them. 200 -> 179 us with such a group; with fewer
-  // groups than warps nothing waits, with many more the end is short.
+  // first, each warp's share of them. Walks of five galaxies a size: at 200k the one
+  // with such a group 0.429 -> 0.412 ms, the others and those of 130k, 400k and 1M
+  // the same within 1% with and without, as with boxes from 1/4 or 1/16 of the root's
+  // half on. The rule is kept to where it can matter: with fewer groups than warps
+  // (4864) nothing waits, with many more the end is short.
   const float wide = static_cast<float>(a.root->half_at[0]) * (1.f / 8.f);
   auto spans = [&](u32 g) {
     const float4 b0 = reinterpret_cast<const float4 *>(a.gboxf)[2ull * g],

@@ -405,7 +405,7 @@ void evaluate_lists(const float4 *bodies, const float4 *cells, const u32 *cell_l
 // returns at once (memory stays in bounds; the step is then redone eagerly).
 struct GraphCaps {
   u32 nodes;        // node arrays
-  int depth;        // deepest node the per-depth moment launches cover
+  int depth;        // deepest leaf: the sort covers it and one level more
   u32 groups;       // groups the list slots cover
   u32 slot_cells, slot_bodies;  // each group's list slots (one-pass walk, its rest)
   u32 slot_near_cells, slot_near_bodies;  // ... and its near-field walk

@@ -6,7 +6,7 @@
 // once for all passes) and one small launch scans them into each digit's
 // start in each pass. Then each pass is a single launch: a block takes the
 // next tile (2048 pairs) from a counter, ranks its keys stably (each warp
-// with __match_any_sync and a warp-private histogram, equal digits in input
+// by ballots and a warp-private histogram, equal digits in input
 // order), publishes its digit counts, and finds how many pairs of each digit
 // the earlier tiles hold by looking back over their published counts --
 // each tile publishes first its own counts, then, once it knows them, the
@@ -14,7 +14,7 @@
 // running total it meets. The tile is put in digit order in shared memory
 // and written out in that order (consecutive threads, consecutive places of
 // a digit's run). Per pass a pair is read once and written once (12 B each
-// way); the former per-pass histogram read (8 B) and scan launches are gone.
+// way), with no histogram read or scan launch of its own.
 //
 // (Time at 2M, six passes: 248 us with __match_any_sync and each load beside its
 // ranking, 238 with the loads first, 215 with ballots; 35 us a pass, bound by
@@ -24,7 +24,8 @@
 // A look-back waits only on tiles taken earlier from the counter, whose
 // blocks are running or done and publish their counts before waiting
 // themselves, so the waits end. Each wait is bounded all the same: past the
-// limit the kernel records error bit 16 (and the pass's output is garbage).
+// limit the kernel records error bit 16 (and the pass's output is garbage, which
+// the solve does not use).
 //
 // Up to kClusterItems pairs a CTA of one thread-block cluster (16 CTAs where the
 // GPU takes such clusters, else 8) the whole sort is one launch: the pairs stay
@@ -32,7 +33,9 @@
 // into each other's shared memory, and each pair goes straight to its place in
 // the shared memory of the CTA that will hold it. Two cluster barriers a pass
 // replace the counting launches, the look-back and a launch per pass: five
-// passes of 5k pairs 64 -> 22 us, of 50k 68 -> 53 us. With eight pairs a thread
+// passes of 5k pairs 64 -> 22 us, of 50k 68 -> 53 us. (One more at the start, after
+// which every CTA's shared memory may be written, measures nothing: it is waited
+// for behind the first ranking.) With eight pairs a thread
 // (to 131072) the one cluster is the slower: a solve of 65k bodies took the same
 // either way, one of 80k 0.537 ms against 0.504 in sweeps, of 131072 0.705 and
 // 0.661.

@@ -1338,9 +1338,8 @@ __global__ void __launch_bounds__(kLeafThreads)
 // the leaf buckets' order) computes its leaf, then climbs while it is the
 // last child of its parent to finish, computing that parent from its
 // children in child order as node_moments32 does. So every node is computed
-// once, after all its children, with the same operations as the per-depth
-// launches; the climb ends at the root or at a parent a sibling will
-// finish (at most kMaxDepth steps).
+// once, after all its children; the climb ends at the root or at a parent a sibling
+// will finish (at most kMaxDepth steps).
 __global__ void __launch_bounds__(kT)
     k_moments32_up(Moment32Arrays a, const u32 *bucket, const u32 *meta, const u32 *parent,
                    u32 *arrive) {
