@@ -681,8 +681,8 @@ __global__ void __launch_bounds__(kLWarps * 32) k_lwarp(GArgs a, u32 round) {
   // long as any other (one took 165 of round 0's 200 us at 200k): in round 0 they go
   // first, each warp's share of them. Walks of five galaxies a size: at 200k the one
   // with such a group 0.429 -> 0.412 ms, the others and those of 130k, 400k and 1M
-  // the same within 1% with and without, as with boxes from 1/4 or 1/16 of the root's
-  // half on. The rule is kept to where it can matter: with fewer groups than warps
+  // the same within the runs' spread with and without, as with boxes from 1/4 or 1/16 of
+  // the root's half on. The rule is kept to where it can matter: with fewer groups than warps
   // (4864) nothing waits, with many more the end is short.
   const float wide = static_cast<float>(a.root->half_at[0]) * (1.f / 8.f);
   auto spans = [&](u32 g) {

@@ -189,3 +189,16 @@ def test_group_lists_squares_beyond_fp32(gtc, oracle, warps):
         c.group_force(pos, mass, G=1.0, eps=1e18, quadrupole=True, **kw)
         got = c.export()
     assert compare_lists(got, got["nodes"], lists, nodes) == []
+
+
+@pytest.mark.parametrize("scale", [1e-19, 1e-17, 1e-15, 1e-13, 1e-12, 1e17, 1e18, 1e19, 1e20])
+def test_tree_walk_at_the_ends_of_fp32_squares_bitwise(ctx, oracle, scale):
+    """Trees of which some tests are within what the FP32 test takes (d^2 from 1e-35
+    to 1e38) and some beyond."""
+    pos, mass = lopsided_sphere(2000, 15)
+    kw = dict(G=1.0, theta=0.6, eps=0.02 * scale, quadrupole=True)
+    acc, pot = ctx.tree_force(pos * scale, mass, **kw)
+    st = ctx.stats()
+    want, wpot, (nc, npart) = oracle.tree_force(pos * scale, mass, **kw)
+    assert np.array_equal(acc, want, equal_nan=True) and np.array_equal(pot, wpot, equal_nan=True)
+    assert (st["cell_interactions"], st["body_interactions"]) == (nc, npart)
